@@ -7,10 +7,8 @@
 // (CompareHuffmanNode, huffman.cc:9-18); the first popped becomes the 0
 // branch.  Leaves are symbol indices 0..S-1 (S = bins, +1 for the zero-run
 // key), merged nodes are numbered from S upward.  Here the leaves are sorted
-// by (count asc, index desc) and merged nodes wait in a queue of equal-count
-// groups; merged counts never decrease, so the group at the front holds the
-// smallest merged count and its newest node is the one the reference pops
-// next.  On equal counts a merged node beats a leaf (it has the larger index).
+// by (count asc, index desc), the order they are popped in, and merged in
+// rounds of independent pairs (huffman_build_kernel).
 // Codes are root-first, bit d of the code word = branch taken at depth d
 // (computeEncodedBits :147-174), the decode table lists nodes breadth first
 // as (left id, right id) or (0, symbol) (computeDecodeTable :177-228).
@@ -29,66 +27,109 @@ namespace {
 constexpr int kMaxCodeBits = 58;  // + 3 dup bits fits 61 bits -> at most 3 words
 
 // ---- tree -------------------------------------------------------------------
+// Shared memory of one tree build for up to S symbols (P = S rounded up to a
+// power of two).  The sort keys are dead once the leaf list is taken from
+// them and the lists are dead after the last round, so their space is reused.
 struct BuildSmem {
-  unsigned long long *keys;  // sorted leaves, later codes of all nodes
-  short *lch, *rch;          // children of merged node (id - S)
-  unsigned long long *icnt;  // counts of merged nodes
-  short *gs, *ge;            // equal-count groups of the merged-node queue
-  short *istack;             // merged-node storage of the groups
-  unsigned char *depth;      // per node
-  short *bfs, *bfsId;        // breadth-first order / position
+  unsigned long long *keys;        // P sort keys
+  unsigned *cntA, *cntB;           // S each: counts of the active list (two buffers)
+  uint16_t *idA, *idB;             // S each: its node ids
+  unsigned *sum;                   // S / 2 + 1: counts of the round's new nodes
+  uint16_t *lch, *rch;             // S each: children of merged node (id - S)
+  uint16_t *par;                   // 2 S: parent's (id - S) * 2 + branch
+  uint16_t *bfs;                   // 2 S: nodes in breadth-first order
 };
 
-__host__ __device__ inline size_t build_smem_bytes(int S) {
-  int P = 1;
+__host__ __device__ inline int build_pow2(int S) {
+  int P = 32;
   while (P < S) P <<= 1;
-  const size_t nodes = 2 * (size_t)S;
-  size_t b = 0;
-  b += (size_t)(P > (int)nodes ? P : nodes) * 8;  // keys / codes
-  b += 2 * (size_t)S * 2;                         // lch, rch
-  b += (size_t)S * 8;                             // icnt
-  b += 2 * (size_t)S * 2;                         // gs, ge
-  b += (size_t)S * 2;                             // istack
-  b += nodes;                                     // depth
-  b += 2 * nodes * 2;                             // bfs, bfsId
-  return (b + 15) & ~(size_t)15;
+  return P;
+}
+// keys (aliased by cntB, idB) | cntA (aliased by bfs) | sum | idA |
+// lch | rch | par
+__host__ __device__ inline size_t build_smem_bytes(int S) {
+  const size_t s = (size_t)((S + 3) & ~3);
+  return (size_t)build_pow2(S) * 8 + s * 4 + (s / 2 + 4) * 4 + s * 2 * 3 + s * 2 * 2;
 }
 
-// 256 threads: the merge, depths and decode table are one thread's work, so a
-// small CTA lets every cubelet of a large batch build at once (eight CTAs per
-// SM) instead of waiting for a second wave.
-constexpr int kBuildThreads = 256;
-__global__ void __launch_bounds__(kBuildThreads) huffman_build_kernel(DevBatch b) {
-  extern __shared__ unsigned long long hsm[];
+// number of entries of the ascending list v[0..n) below x (below or equal
+// with LE)
+template <bool LE> __device__ __forceinline__ int list_rank(const unsigned *v, int n, unsigned x) {
+  int pos = 0;
+  for (int step = n ? 1 << (31 - __clz(n)) : 0; step > 0; step >>= 1)
+    if (step <= n - pos && (LE ? v[pos + step - 1] <= x : v[pos + step - 1] < x)) pos += step;
+  return pos;
+}
+// the same for one x by a whole warp: 32 probes at a time
+__device__ __forceinline__ int list_rank_warp(const unsigned *v, int n, unsigned x, int lane) {
+  int lo = 0, len = n;
+  while (len > 0) {
+    const int step = (len + 31) >> 5;
+    const int p = lo + (lane + 1) * step - 1;
+    const int c = __popc(__ballot_sync(0xffffffffu, p < lo + len && v[p] < x));
+    lo += c * step;
+    len = min(step - 1, len - c * step);
+  }
+  return lo;
+}
+
+// One CTA builds one cubelet's tree, codes and decode table; nothing in it is
+// a serial chain over the symbols.  It is bound by shared-memory latency: a
+// one-thread merge, depth pass and breadth-first walk took 120 and 578 us for
+// 257 and 1025 symbols; with this form a whole call on a 2048^2 image (257
+// symbols) went from 624 to 523 us, on a 256^3 volume (1025) from 1079 to 623.
+//
+// Merging in rounds.  The active list holds the parentless nodes in the order
+// the reference pops them (count ascending, on equal counts the larger index
+// first).  With s the sum of its two smallest counts, every node created from
+// now on counts at least s, so the entries below s are popped in list order:
+// they pair off two by two at once (an odd last one stays for the next
+// round), and the new nodes -- counts ascending, equal counts in reverse
+// order, before old nodes of equal count since their indices are larger --
+// are merged into the rest of the list by rank.  Two rounds at least double
+// the smallest count, so there are at most about 62 of them (25 in practice),
+// each a handful of shared-memory searches.
+//
+// Codes: a thread per symbol walks up the parents (at most 58 steps).  The
+// decode table's breadth-first numbering is a scan of the inner nodes, level
+// by level.
+template <int T>
+__global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
+  constexpr int kWarps = T / 32;
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char hsm[];
   __shared__ int nLeaves;
+  __shared__ int wSum[2][kWarps];
   const int ci = blockIdx.x;
   const CubeletDev cd = b.cub[ci];
   CubeletState *st = b.state + ci;
   const int dupV = st->dupValue;
   const int S = cd.binCount + (dupV >= 0 ? 1 : 0);
-  int P = 1;
-  while (P < S) P <<= 1;
-  const int nodesMax = 2 * S;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   BuildSmem m;
-  char *p = reinterpret_cast<char *>(hsm);
-  m.keys = reinterpret_cast<unsigned long long *>(p); p += (size_t)(P > nodesMax ? P : nodesMax) * 8;
-  m.icnt = reinterpret_cast<unsigned long long *>(p); p += (size_t)S * 8;
-  m.lch = reinterpret_cast<short *>(p); p += (size_t)S * 2;
-  m.rch = reinterpret_cast<short *>(p); p += (size_t)S * 2;
-  m.gs = reinterpret_cast<short *>(p); p += (size_t)S * 2;
-  m.ge = reinterpret_cast<short *>(p); p += (size_t)S * 2;
-  m.istack = reinterpret_cast<short *>(p); p += (size_t)S * 2;
-  m.bfs = reinterpret_cast<short *>(p); p += (size_t)nodesMax * 2;
-  m.bfsId = reinterpret_cast<short *>(p); p += (size_t)nodesMax * 2;
-  m.depth = reinterpret_cast<unsigned char *>(p);
+  {
+    const int s4 = (S + 3) & ~3;
+    unsigned char *p = hsm;
+    m.keys = reinterpret_cast<unsigned long long *>(p);
+    m.cntB = reinterpret_cast<unsigned *>(p);
+    m.idB = reinterpret_cast<uint16_t *>(p + 4 * s4);
+    p += (size_t)build_pow2(S) * 8;
+    m.cntA = reinterpret_cast<unsigned *>(p);
+    m.bfs = reinterpret_cast<uint16_t *>(p); p += 4 * s4;
+    m.sum = reinterpret_cast<unsigned *>(p); p += (s4 / 2 + 4) * 4;
+    m.idA = reinterpret_cast<uint16_t *>(p); p += 2 * s4;
+    m.lch = reinterpret_cast<uint16_t *>(p); p += 2 * s4;
+    m.rch = reinterpret_cast<uint16_t *>(p); p += 2 * s4;
+    m.par = reinterpret_cast<uint16_t *>(p);
+  }
 
+  // ---- leaves with a nonzero count, key = count:51 | (8191 - symbol):13
   const unsigned long long *cnt = b.hist + (size_t)ci * kMaxSymbols;
-  if (threadIdx.x == 0) nLeaves = 0;
+  if (tid == 0) nLeaves = 0;
   __syncthreads();
-  // leaves with a nonzero count, key = count:51 | (8191 - symbol):13
-  for (int i = threadIdx.x; i < S; i += blockDim.x) {
-    const unsigned long long c = (i == cd.binCount) ? cnt[cd.binCount] : cnt[i];
+  for (int i = tid; i < S; i += T) {
+    const unsigned long long c = cnt[i];
     if (c > 0) {
       const int slot = atomicAdd(&nLeaves, 1);
       m.keys[slot] = (c << 13) | (unsigned long long)(8191 - i);
@@ -96,129 +137,160 @@ __global__ void __launch_bounds__(kBuildThreads) huffman_build_kernel(DevBatch b
   }
   __syncthreads();
   const int nL = nLeaves;
-  for (int i = nL + threadIdx.x; i < P; i += blockDim.x) m.keys[i] = ~0ull;
+  const int P = build_pow2(nL);
+  for (int i = nL + tid; i < P; i += T) m.keys[i] = ~0ull;
   __syncthreads();
-  // bitonic sort, ascending
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        const int l = i ^ j;
-        if (l > i) {
-          const unsigned long long a = m.keys[i], c = m.keys[l];
-          const bool up = (i & k) == 0;
-          if ((a > c) == up) { m.keys[i] = c; m.keys[l] = a; }
-        }
+  // ---- bitonic sort, ascending: distances below 32 inside a warp
+  auto warp_stages = [&](unsigned long long v, int i, int k, int j0) {
+    for (int j = j0; j > 0; j >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(kAll, v, j);
+      const bool keepMin = ((i & k) == 0) == ((i & j) == 0);
+      v = keepMin == (v < o) ? v : o;
+    }
+    return v;
+  };
+  for (int i = tid; i < P; i += T) {  // P is a multiple of 32: whole warps
+    unsigned long long v = m.keys[i];
+    for (int k = 2; k <= 32; k <<= 1) v = warp_stages(v, i, k, k >> 1);
+    m.keys[i] = v;
+  }
+  __syncthreads();
+  for (int k = 64; k <= P; k <<= 1) {
+    for (int j = k >> 1; j >= 32; j >>= 1) {
+      for (int p = tid; p < P / 2; p += T) {
+        const int i = 2 * p - (p & (j - 1)), l = i + j;
+        const unsigned long long a = m.keys[i], c = m.keys[l];
+        if ((a > c) == ((i & k) == 0)) { m.keys[i] = c; m.keys[l] = a; }
       }
       __syncthreads();
     }
+    for (int i = tid; i < P; i += T) m.keys[i] = warp_stages(m.keys[i], i, k, 16);
+    __syncthreads();
   }
-
-  if (threadIdx.x == 0) {
-    int err = 0;
-    // ---- merge (single thread, O(S)) ----
-    int lf = 0;                 // next leaf
-    int gF = 0, gL = -1;        // active groups gF..gL
-    int top = 0;                // next free istack slot
-    int next = S;               // next merged node id
-    int root = -1;
-    int remaining = nL;
-    auto popNode = [&](unsigned long long &count) -> int {
-      const bool haveLeaf = lf < nL;
-      const bool haveInt = gF <= gL;
-      bool takeInt = false;
-      unsigned long long ic = 0;
-      if (haveInt) ic = m.icnt[m.istack[m.gs[gF]] - S];
-      if (haveInt && haveLeaf) takeInt = ic <= (m.keys[lf] >> 13);
-      else takeInt = haveInt;
-      if (takeInt) {
-        const int id = m.istack[m.ge[gF] - 1];
-        m.ge[gF]--;
-        if (m.ge[gF] == m.gs[gF]) gF++;
-        count = ic;
-        return id;
-      }
-      const unsigned long long key = m.keys[lf++];
-      count = key >> 13;
-      return 8191 - (int)(key & 8191ull);
-    };
-    while (remaining > 1) {
-      unsigned long long ca, cb2;
-      const int a = popNode(ca);
-      const int c = popNode(cb2);
-      const int id = next++;
-      const unsigned long long sum = ca + cb2;
-      m.lch[id - S] = (short)a;
-      m.rch[id - S] = (short)c;
-      m.icnt[id - S] = sum;
-      if (gF <= gL && m.icnt[m.istack[m.gs[gL]] - S] == sum) {
-        m.istack[m.ge[gL]++] = (short)id;
-        top = m.ge[gL];
-      } else {
-        gL++;
-        if (gL < gF) gF = gL;
-        m.gs[gL] = (short)top;
-        m.ge[gL] = (short)(top + 1);
-        m.istack[top++] = (short)id;
-      }
-      remaining--;
-    }
-    if (nL == 1) root = 8191 - (int)(m.keys[0] & 8191ull);
-    else if (nL > 1) root = next - 1;
-    const int nInternal = next - S;
-
-    // ---- depths and codes (parents are created after their children) ----
-    unsigned long long *code = m.keys;  // reuse: codes per node id
-    const int nodes = S + nInternal;
-    for (int i = 0; i < nodes; i++) { m.depth[i] = 0; code[i] = 0; }
-    int longest = 0;
-    for (int j = nInternal - 1; j >= 0; j--) {
-      const int id = S + j;
-      const int d = m.depth[id];
-      const int l = m.lch[j], r = m.rch[j];
-      m.depth[l] = (unsigned char)(d + 1);
-      m.depth[r] = (unsigned char)(d + 1);
-      code[l] = code[id];
-      code[r] = code[id] | (d < 64 ? (1ull << d) : 0ull);
-      if (d + 1 > longest) longest = d + 1;
-    }
-    if (longest > kMaxCodeBits) err = 2;
-
-    // ---- decode table, breadth first ----
-    int *dec = b.decode + (size_t)ci * 4 * kMaxSymbols;
-    int nb = 0;
-    if (root >= 0) {
-      m.bfs[nb++] = (short)root;
-      for (int h = 0; h < nb; h++) {
-        const int nd = m.bfs[h];
-        m.bfsId[nd] = (short)h;
-        if (nd >= S) {
-          m.bfs[nb++] = m.lch[nd - S];
-          m.bfs[nb++] = m.rch[nd - S];
-        }
-      }
-      for (int h = 0; h < nb; h++) {
-        const int nd = m.bfs[h];
-        if (nd >= S) {
-          dec[2 * h] = m.bfsId[m.lch[nd - S]];
-          dec[2 * h + 1] = m.bfsId[m.rch[nd - S]];
-        } else {
-          dec[2 * h] = 0;
-          dec[2 * h + 1] = nd;
-        }
-      }
-    }
-    st->nDecode = 2 * nb;
-    st->longest = longest;
-    st->nLeaves = nL;
-    if (err) st->error = err;
+  // the counts of a cubelet's tokens sum to at most its element count (below
+  // 2^31), so 32 bits hold every node's count
+  for (int i = tid; i < nL; i += T) {
+    const unsigned long long key = m.keys[i];
+    m.cntA[i] = (unsigned)(key >> 13);
+    m.idA[i] = (uint16_t)(8191 - (int)(key & 8191ull));
   }
   __syncthreads();
-  // code table for the encoder
+
+  // ---- merge rounds
+  unsigned *cc = m.cntA, *cn = m.cntB;
+  uint16_t *ic = m.idA, *in = m.idB;
+  int len = nL, next = S;
+  bool bad = false;
+  while (len > 1) {
+    const unsigned s = cc[0] + cc[1];
+    const int kp = list_rank_warp(cc, len, s, lane) & ~1;  // entries paired off
+    bad = kp < 2;  // the counts overflow 32 bits: not from a token count
+    if (bad) break;
+    const int q = kp >> 1, r = len - kp;
+    for (int j = tid; j < q; j += T) {
+      const int a = ic[2 * j], c = ic[2 * j + 1], node = next - S + j;
+      m.sum[j] = cc[2 * j] + cc[2 * j + 1];
+      m.lch[node] = (uint16_t)a;
+      m.rch[node] = (uint16_t)c;
+      m.par[a] = (uint16_t)(2 * node);
+      m.par[c] = (uint16_t)(2 * node + 1);
+    }
+    __syncthreads();
+    const unsigned *rest = cc + kp;
+    for (int j = tid; j < q; j += T) {
+      const unsigned c = m.sum[j];
+      int at = j;  // among the new nodes: a run of equal counts is reversed
+      const bool le = j > 0 && m.sum[j - 1] == c, re = j + 1 < q && m.sum[j + 1] == c;
+      if (le || re) {
+        const int gs = le ? list_rank<false>(m.sum, j, c) : j;
+        const int ge = re ? list_rank<true>(m.sum, q, c) - 1 : j;
+        at = gs + ge - j;
+      }
+      at += list_rank<false>(rest, r, c);
+      cn[at] = c;
+      in[at] = (uint16_t)(next + j);
+    }
+    for (int i = tid; i < r; i += T) {
+      const unsigned c = rest[i];
+      const int at = i + list_rank<true>(m.sum, q, c);
+      cn[at] = c;
+      in[at] = ic[kp + i];
+    }
+    next += q;
+    len = q + r;
+    unsigned *tc = cc;
+    cc = cn;
+    cn = tc;
+    uint16_t *ti = ic;
+    ic = in;
+    in = ti;
+    __syncthreads();
+  }
+
+  // ---- codes: up from each leaf (root-first bits, bit d = branch at depth d)
+  const int root = next - 1;  // with two or more leaves
   unsigned long long *gcode = b.codes + (size_t)ci * kMaxSymbols;
   uint8_t *glen = b.codeLen + (size_t)ci * kMaxSymbols;
-  for (int i = threadIdx.x; i < S; i += blockDim.x) {
-    gcode[i] = m.keys[i];
-    glen[i] = m.depth[i];
+  for (int i = tid; i < S; i += T) {
+    unsigned long long code = 0;
+    int d = 0;
+    if (nL > 1 && cnt[i] > 0 && !bad) {
+      int nd = i;
+      while (nd != root && d < 64) {
+        const int pb = m.par[nd];
+        code = (code << 1) | (unsigned)(pb & 1);
+        d++;
+        nd = S + (pb >> 1);
+      }
+    }
+    gcode[i] = code;
+    glen[i] = (uint8_t)d;
+  }
+
+  // ---- decode table, breadth first: (left id, right id) or (0, symbol)
+  int2 *dec = reinterpret_cast<int2 *>(b.decode + (size_t)ci * 4 * kMaxSymbols);
+  int base = 0, width = nL > 0 && !bad ? 1 : 0, levels = 0, par = 0;
+  if (nL > 0 && tid == 0) m.bfs[0] = (uint16_t)(nL > 1 ? root : 8191 - (int)(m.keys[0] & 8191ull));
+  __syncthreads();
+  while (width > 0) {
+    const int nb = base + width;  // the next level's first node
+    int inner = 0;                // inner nodes of this level so far
+    for (int t0 = 0; t0 < width; t0 += T) {
+      const int t = t0 + tid;
+      const int nd = t < width ? m.bfs[base + t] : 0;
+      const bool isIn = t < width && nd >= S;
+      const unsigned bal = __ballot_sync(kAll, isIn);
+      if (lane == 0) wSum[par][warp] = __popc(bal);
+      __syncthreads();
+      int before = 0, all = 0;
+#pragma unroll
+      for (int v = 0; v < kWarps; v++) {
+        const int x = wSum[par][v];
+        before += v < warp ? x : 0;
+        all += x;
+      }
+      par ^= 1;  // two sets: a warp overwrites one only after the next barrier
+      if (isIn) {
+        const int c = nb + 2 * (inner + before + __popc(bal & ((1u << lane) - 1u)));
+        m.bfs[c] = m.lch[nd - S];
+        m.bfs[c + 1] = m.rch[nd - S];
+        dec[base + t] = make_int2(c, c + 1);
+      } else if (t < width) {
+        dec[base + t] = make_int2(0, nd);
+      }
+      inner += all;
+    }
+    __syncthreads();
+    base = nb;
+    width = 2 * inner;
+    levels++;
+  }
+  if (tid == 0) {
+    const int longest = levels > 0 ? levels - 1 : 0;
+    st->nDecode = 2 * base;
+    st->longest = longest;
+    st->nLeaves = nL;
+    if (longest > kMaxCodeBits || bad) st->error = 2;
   }
 }
 
@@ -529,9 +601,17 @@ __global__ void __launch_bounds__(kEncThreads, 8) encode_write_kernel(DevBatch b
 }  // namespace
 
 void launch_huffman_build(DevBatch &b, int maxSymbols, cudaStream_t s) {
-  const size_t smem = build_smem_bytes(maxSymbols);
-  raise_smem_limit(huffman_build_kernel, (int)smem);
-  huffman_build_kernel<<<b.n, kBuildThreads, smem, s>>>(b);
+  const int smem = (int)build_smem_bytes(maxSymbols);
+  // wide CTAs for a large alphabet (the sort and the list moves are as long as
+  // it is); a batch of more than two cubelets per SM keeps 256 threads, eight
+  // CTAs to an SM, so that all of them build in one wave
+  if (maxSymbols > 600 && b.n <= 2 * 152) {
+    raise_smem_limit(huffman_build_kernel<1024>, smem);
+    huffman_build_kernel<1024><<<b.n, 1024, smem, s>>>(b);
+  } else {
+    raise_smem_limit(huffman_build_kernel<256>, smem);
+    huffman_build_kernel<256><<<b.n, 256, smem, s>>>(b);
+  }
 }
 
 void launch_pack_meta(DevBatch &b, cudaStream_t s) { pack_meta_kernel<<<b.n, 256, 0, s>>>(b); }
