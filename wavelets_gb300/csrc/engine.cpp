@@ -299,7 +299,7 @@ struct wl_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   DevBuf input, coef, coef2, bins, tokCount, state, selHist, lloydHist, qtable, dqtable, qlut,
-      hist, chunkRun, chunkRunCtx, chunkBits, chunkCub, groupCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
+      hist, chunkRun, chunkBits, chunkCub, groupCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
       words, passes, logHdr, outbuf, decWords, decTable, decWs, meta, optIn, optOut, optErr,
       errIn, errRest, errPart;
   HostBuf hState, hDecode, hPasses, hTab, hLogHdr, hPrefix, hIn, hVals, hFlags;
@@ -976,7 +976,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   TRY(ensure(ctx, ctx->hist, (size_t)n * kMaxSymbols * 8));
   TRY(ensure(ctx, ctx->chunkRun, chunkTotal * sizeof(int4)));
   TRY(ensure(ctx, ctx->chunkSpan, chunkTotal * sizeof(int2)));
-  TRY(ensure(ctx, ctx->chunkRunCtx, chunkTotal * 2 * sizeof(long long)));
   TRY(ensure(ctx, ctx->chunkBits, chunkTotal * 8));
   TRY(ensure(ctx, ctx->codes, (size_t)n * kMaxSymbols * 8));
   TRY(ensure(ctx, ctx->codeLen, (size_t)n * kMaxSymbols));
@@ -1143,7 +1142,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.hist = P<unsigned long long>(ctx->hist);
   b.chunkRun = P<int4>(ctx->chunkRun);
   b.chunkSpan = P<int2>(ctx->chunkSpan);
-  b.chunkRunCtx = P<long long>(ctx->chunkRunCtx);
   b.chunkBits = P<unsigned long long>(ctx->chunkBits);
   b.codes = P<unsigned long long>(ctx->codes);
   b.codeLen = P<uint8_t>(ctx->codeLen);
@@ -1160,6 +1158,12 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.logHdr = P<int4>(ctx->logHdr);
   b.meta = P<int>(ctx->meta);
   b.totalChunks = chunkTotal;
+  int maxChunks[2] = {0, 0};
+  for (int i = 0; i < n; i++) {
+    int &m = maxChunks[half_of(i)];
+    m = std::max(m, plans[i].nChunks);
+  }
+  b.maxChunks = maxChunks[0];
   constexpr long long kMetaPer = 4LL * kMaxSymbols + 2LL * kMaxBins;  // ints per cubelet
   DevBatch bh[2] = {b, b};
   if (nh == 2) {
@@ -1183,7 +1187,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       v.chunkTok += ch;
       v.chunkSpan += ch;
       v.chunkRun += ch;
-      v.chunkRunCtx += 2 * ch;
       v.chunkBits += ch;
       v.chunkCub += ch;
       v.groupCub += g;
@@ -1194,6 +1197,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       v.words += words0[h];
       v.meta += c0 * kMetaPer;
       v.totalChunks = (h ? chunkTotal : chunk0[1]) - ch;
+      v.maxChunks = maxChunks[h];
       v.totalGroups = (h ? groupTotal : group0[1]) - g;
     }
   }
@@ -2302,7 +2306,7 @@ void wl_destroy(wl_ctx *ctx) {
   DevBuf *dbs[] = {&ctx->input, &ctx->coef, &ctx->coef2, &ctx->bins, &ctx->tokCount,
                    &ctx->state,
                    &ctx->selHist, &ctx->lloydHist, &ctx->qtable, &ctx->dqtable, &ctx->qlut, &ctx->hist,
-                   &ctx->chunkRun, &ctx->chunkRunCtx, &ctx->chunkBits, &ctx->chunkCub, &ctx->groupCub,
+                   &ctx->chunkRun, &ctx->chunkBits, &ctx->chunkCub, &ctx->groupCub,
                    &ctx->encCub, &ctx->sliceOff,
                    &ctx->chunkSpan, &ctx->optIn, &ctx->optOut, &ctx->optErr,
                    &ctx->codes, &ctx->codeLen, &ctx->decode, &ctx->words, &ctx->passes,

@@ -31,19 +31,6 @@ namespace {
 constexpr int kThreads = kChunkThreads;
 constexpr int INF = 0x7fffffff;
 
-// greedy split of a zero-bin run (HuffmanDup::dupCount, huffman.h:46-57)
-__device__ __forceinline__ void run_split(long long L, long long &singles, long long &dups) {
-  dups = L / 1024;  // dupFindLongest returns 7 (1024) while L >= 1024
-  int r = (int)(L % 1024);
-  while (r > 8) {
-    int p = 8;
-    while ((p << 1) <= r) p <<= 1;
-    r -= p;
-    dups++;
-  }
-  singles = r;
-}
-
 // ---- quantizer parameters ---------------------------------------------------
 __global__ void quant_params_kernel(DevBatch b) {
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
@@ -429,8 +416,10 @@ __device__ __forceinline__ QParams load_qparams(const CubeletDev &cd, const Cube
 // count) give every warp the run before its first value and its place in the
 // chunk, and each warp writes that run's tokens and its staged ones to the
 // chunk's slot with coalesced stores.
-// greedy split of a zero-bin run into dup tokens and single zero-bin tokens
-// (closed form of run_split; the same counts as run_token_count)
+// Greedy split of a zero-bin run into dup tokens and single zero-bin tokens
+// (HuffmanDup::dupCount, huffman.h:46-57) in closed form: runs of 1024, then
+// one dup token per set bit of the remainder at or above 8 -- except that a
+// last 8 left over is coded as 8 single tokens.
 __device__ __forceinline__ void run_split_closed(int L, int &singles, int &dups) {
   const int q = L >> 10, r = L & 1023, hi = r & ~7, lo = r & 7;
   const int big = __popc(hi >> 4);
@@ -709,160 +698,125 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff) {
     if (hist[i]) atomicAdd(&gh[i], (unsigned long long)hist[i]);
 }
 
-// Join zero runs across chunk edges; one CTA per cubelet.
-__device__ __forceinline__ int block_scan_max_excl(int v, int *sh, int &total) {
-  // exclusive max-scan over 1024 threads (identity -1)
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int inc = v;
-  for (int off = 1; off < 32; off <<= 1) {
-    int t = __shfl_up_sync(0xffffffffu, inc, off);
-    if (lane >= off) inc = max(inc, t);
-  }
-  if (lane == 31) sh[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    int x = sh[lane];
-    for (int off = 1; off < 32; off <<= 1) {
-      int t = __shfl_up_sync(0xffffffffu, x, off);
-      if (lane >= off) x = max(x, t);
-    }
-    sh[32 + lane] = x;
-  }
-  __syncthreads();
-  int before = w > 0 ? sh[32 + w - 1] : -1;
-  int ex = __shfl_up_sync(0xffffffffu, inc, 1);
-  if (lane == 0) ex = -1;
-  total = sh[32 + 31];
-  __syncthreads();
-  return max(before, ex);
-}
+// Join zero runs across chunk edges: the tokens of the runs entering and
+// leaving every chunk, and their counts.  A CTA takes kRunChunks consecutive
+// chunks of one cubelet (blockIdx.y), one thread each; the nearest chunks
+// with a value before and after the CTA's range are searched kRunChunks at a
+// time, usually found in the first step, whose loads are issued with the
+// CTA's own.  Bound by the latency of a few dependent loads and the tokens a
+// thread writes: one CTA of 1024 threads per cubelet left most SMs idle (59
+// us for a 2048^2 image of 1024 chunks, 93 us for a 256^3 volume); spread
+// over the SMs a whole call went from 523 to 468 us and from 623 to 529 us.
+constexpr int kRunChunks = 256;
 
-__device__ __forceinline__ int block_scan_min_excl_rev(int v, int *sh, int &total) {
-  // exclusive min-scan from the right (identity INF)
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int inc = v;
-  for (int off = 1; off < 32; off <<= 1) {
-    int t = __shfl_down_sync(0xffffffffu, inc, off);
-    if (lane + off < 32) inc = min(inc, t);
-  }
-  if (lane == 0) sh[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    int x = sh[lane];
-    for (int off = 1; off < 32; off <<= 1) {
-      int t = __shfl_down_sync(0xffffffffu, x, off);
-      if (lane + off < 32) x = min(x, t);
-    }
-    sh[32 + lane] = x;
-  }
-  __syncthreads();
-  int after = w < 31 ? sh[32 + w + 1] : INF;
-  int ex = __shfl_down_sync(0xffffffffu, inc, 1);
-  if (lane == 31) ex = INF;
-  total = sh[32];
-  __syncthreads();
-  return min(after, ex);
-}
-
-__global__ void __launch_bounds__(1024) runs_kernel(DevBatch b) {
-  __shared__ int sh[64];
-  __shared__ unsigned long long sSingles, sDups;
-  const int ci = blockIdx.x;
+__global__ void __launch_bounds__(kRunChunks) runs_kernel(DevBatch b) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kWarps = kRunChunks / 32;
+  __shared__ unsigned sMask[kWarps];
+  __shared__ int sPrev, sNext;
+  const int ci = blockIdx.y;
   const CubeletDev cd = b.cub[ci];
-  const CubeletState *st = b.state + ci;
-  const int dupV = st->dupValue;
+  const int nc = cd.nChunks, c0 = (int)blockIdx.x * kRunChunks;
+  if (c0 >= nc) return;
+  const int dupV = b.state[ci].dupValue;
   if (dupV < 0) return;
-  const int nc = cd.nChunks;
-  const long long base = cd.chunkBase;
-  int4 *cr = b.chunkRun + base;
-  long long *ctx = b.chunkRunCtx + 2 * base;
-  if (threadIdx.x == 0) { sSingles = 0; sDups = 0; }
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int4 *cr = b.chunkRun + cd.chunkBase;
+  const int c = c0 + tid;
+  // chunks past the end count as all zero and are not written
+  const int4 me = c < nc ? cr[c] : make_int4(0, 0, 1, 0);
+  const bool val = !me.z;  // the chunk holds a value
+  const int back = c0 - 1 - tid, ahead = c0 + kRunChunks + tid;
+  bool hitB = back >= 0 && !cr[back].z, hitA = ahead < nc && !cr[ahead].z;
+  if (tid == 0) {
+    sPrev = -1;
+    sNext = INF;
+  }
+  const unsigned m = __ballot_sync(kAll, val);
+  if (lane == 0) sMask[w] = m;
   __syncthreads();
+  // nearest chunks with a value before and after the CTA's range
+  for (int k = 0;; k++) {
+    const unsigned mb = __ballot_sync(kAll, hitB), ma = __ballot_sync(kAll, hitA);
+    if (lane == 0) {
+      const int o = k * kRunChunks + 32 * w;
+      if (mb) atomicMax(&sPrev, c0 - 1 - (o + __ffs(mb) - 1));
+      if (ma) atomicMin(&sNext, c0 + kRunChunks + o + __ffs(ma) - 1);
+    }
+    __syncthreads();
+    const bool fb = sPrev >= 0 || c0 - (k + 1) * kRunChunks <= 0;
+    const bool fa = sNext != INF || c0 + (k + 2) * kRunChunks >= nc;
+    if (fb && fa) break;
+    __syncthreads();  // everyone has read this step's result
+    const int pb = back - (k + 1) * kRunChunks, pa = ahead + (k + 1) * kRunChunks;
+    hitB = !fb && pb >= 0 && !cr[pb].z;
+    hitA = !fa && pa < nc && !cr[pa].z;
+  }
+  // and of this chunk
+  int prev = -1, next = INF;
+  const unsigned lo = m & ((1u << lane) - 1u), hi = m & ~((2u << lane) - 1u);
+  if (lo) {
+    prev = c0 + 32 * w + 31 - __clz(lo);
+  } else {
+    for (int v = w - 1; v >= 0 && prev < 0; v--)
+      if (sMask[v]) prev = c0 + 32 * v + 31 - __clz(sMask[v]);
+    if (prev < 0) prev = sPrev;
+  }
+  if (hi) {
+    next = c0 + 32 * w + __ffs(hi) - 1;
+  } else {
+    for (int v = w + 1; v < kWarps && next == INF; v++)
+      if (sMask[v]) next = c0 + 32 * v + __ffs(sMask[v]) - 1;
+    if (next == INF) next = sNext;
+  }
 
-  // forward: previous non-all-zero chunk (exclusive)
-  int carry = -1;
-  for (int seg = 0; seg < nc; seg += 1024) {
-    const int c = seg + threadIdx.x;
-    const int v = (c < nc && !cr[c].z) ? c : -1;
-    int total;
-    int ex = block_scan_max_excl(v, sh, total);
-    ex = max(ex, carry);
-    if (c < nc) {
-      long long s0 = 0;
-      if (ex >= 0) {
-        const int4 o = cr[ex];
-        s0 = (long long)ex * kChunk + o.w - o.y;
-      }
-      ctx[2 * c] = s0;  // start of the run entering chunk c
+  int singles = 0, dups = 0;
+  if (c < nc) {
+    const int n = (int)cd.n, dupKey = cd.binCount;  // positions stay below 2^31
+    // the run entering the chunk starts at runIn, the one leaving it ends at e
+    int runIn = 0, e = n;
+    if (prev >= 0) {
+      const int4 o = cr[prev];
+      runIn = prev * kChunk + o.w - o.y;
     }
-    carry = max(carry, total);
+    if (next != INF) e = next * kChunk + cr[next].x;
+    const int cstart = c * kChunk;
+    if (val) run_split_closed(e - (cstart + me.w - me.y), singles, dups);
+    if (c == 0) {  // the run starting at element 0 belongs to no chunk's tail
+      int sg, dp;
+      run_split_closed(val ? me.x : e, sg, dp);
+      singles += sg;
+      dups += dp;
+    }
+    // Tokens of the zero runs at the chunk's edges that start inside it, in
+    // stream order around the stored tokens [lead, lead + nInt): the entering
+    // run's right before them, the leaving run's right after.
+    uint16_t *slot = b.tok + cd.coefOff + cstart;
+    const int nInt = b.chunkTok[cd.chunkBase + c];
+    int nPre = 0, nPost = 0;
+    if (me.x > 0) {
+      const int re = me.z ? e : cstart + me.x, w1 = cstart + (me.z ? me.w : me.x);
+      run_tokens(runIn, re, cstart, w1, dupKey, dupV, [&](uint16_t) { nPre++; });
+      int i = me.x - nPre;
+      run_tokens(runIn, re, cstart, w1, dupKey, dupV, [&](uint16_t t) { slot[i++] = t; });
+    }
+    if (val && me.y > 0) {
+      const int s0 = cstart + me.w - me.y;
+      int i = me.x + nInt;
+      run_tokens(s0, e, s0, cstart + me.w, dupKey, dupV, [&](uint16_t t) { slot[i++] = t; });
+      nPost = i - (me.x + nInt);
+    }
+    b.chunkSpan[cd.chunkBase + c] = make_int2(me.x - nPre, nPre + nInt + nPost);
   }
-  // backward: next non-all-zero chunk (exclusive); run ends and lengths
-  int carryN = INF;
-  long long singles = 0, dups = 0;
-  for (int seg = ((nc - 1) / 1024) * 1024; seg >= 0; seg -= 1024) {
-    const int c = seg + threadIdx.x;
-    const int v = (c < nc && !cr[c].z) ? c : INF;
-    int total;
-    int ex = block_scan_min_excl_rev(v, sh, total);
-    ex = min(ex, carryN);
-    if (c < nc) {
-      const long long e = ex == INF ? cd.n : (long long)ex * kChunk + cr[ex].x;
-      ctx[2 * c + 1] = e;  // end of the run leaving chunk c
-      const int4 me = cr[c];
-      if (!me.z) {
-        const long long s0 = (long long)c * kChunk + me.w - me.y;
-        if (e > s0) {
-          long long sg, dp;
-          run_split(e - s0, sg, dp);
-          singles += sg;
-          dups += dp;
-        }
-      }
-      // Tokens of the zero runs at the chunk's edges that start inside it,
-      // in stream order around the stored tokens [lead, lead + nInt): the
-      // entering run's right before them, the leaving run's right after.
-      const long long cstart = (long long)c * kChunk;
-      uint16_t *slot = b.tok + cd.coefOff + cstart;
-      const int nInt = b.chunkTok[base + c];
-      const int dupKey = cd.binCount;
-      int nPre = 0, nPost = 0;
-      if (me.x > 0) {
-        const long long runIn = ctx[2 * c];
-        const long long re = me.z ? e : cstart + me.x;
-        const long long w1 = cstart + (me.z ? me.w : me.x);
-        run_tokens(runIn, re, cstart, w1, dupKey, dupV, [&](uint16_t) { nPre++; });
-        int i = me.x - nPre;
-        run_tokens(runIn, re, cstart, w1, dupKey, dupV, [&](uint16_t t) { slot[i++] = t; });
-      }
-      if (!me.z && me.y > 0) {
-        const long long s0 = cstart + me.w - me.y;
-        int i = me.x + nInt;
-        run_tokens(s0, e, s0, cstart + me.w, dupKey, dupV, [&](uint16_t t) { slot[i++] = t; });
-        nPost = i - (me.x + nInt);
-      }
-      b.chunkSpan[base + c] = make_int2(me.x - nPre, nPre + nInt + nPost);
-    }
-    // the run starting at element 0 belongs to no chunk's tail
-    if (seg == 0 && threadIdx.x == 0) {
-      const int first = (v != INF) ? 0 : ex;
-      const long long e = first == INF ? cd.n : (long long)first * kChunk + cr[first].x;
-      if (e > 0) {
-        long long sg, dp;
-        run_split(e, sg, dp);
-        singles += sg;
-        dups += dp;
-      }
-    }
-    carryN = min(carryN, total);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    singles += __shfl_xor_sync(kAll, singles, d);
+    dups += __shfl_xor_sync(kAll, dups, d);
   }
-  if (singles) atomicAdd(&sSingles, (unsigned long long)singles);
-  if (dups) atomicAdd(&sDups, (unsigned long long)dups);
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (lane == 0) {
     unsigned long long *gh = b.hist + (size_t)ci * kMaxSymbols;
-    gh[dupV] += sSingles;
-    gh[cd.binCount] += sDups;
+    if (singles) atomicAdd(&gh[dupV], (unsigned long long)singles);
+    if (dups) atomicAdd(&gh[cd.binCount], (unsigned long long)dups);
   }
 }
 
@@ -890,6 +844,8 @@ void launch_quantize(DevBatch &b, const float *coef, int maxTable, int maxSymbol
   quantize_kernel<<<(unsigned)b.totalGroups, kThreads, smem, s>>>(b, coef, histOff);
 }
 
-void launch_runs(DevBatch &b, cudaStream_t s) { runs_kernel<<<b.n, 1024, 0, s>>>(b); }
+void launch_runs(DevBatch &b, cudaStream_t s) {
+  runs_kernel<<<dim3((b.maxChunks + kRunChunks - 1) / kRunChunks, b.n), kRunChunks, 0, s>>>(b);
+}
 
 }  // namespace wl

@@ -60,42 +60,26 @@ __host__ __device__ inline uint16_t make_token(int sym, int v) {
 // more than 8 remain, then single zero-bin tokens).  Calls f(token).  At
 // most 19 tokens start in a window of kChunk elements.
 template <class F>
-__host__ __device__ inline void run_tokens(long long s, long long e, long long w0,
-                                           long long w1, int dupKey, int dupV, F f) {
-  const long long L = e - s;
-  const long long q = L >> 10;
-  long long j0 = 0;
-  if (w0 > s) j0 = (w0 - s + 1023) >> 10;
-  for (long long j = j0; j < q; j++) {
-    const long long pos = s + (j << 10);
-    if (pos >= w1) break;
+__host__ __device__ inline void run_tokens(int s, int e, int w0, int w1, int dupKey, int dupV,
+                                           F f) {
+  const int L = e - s;
+  const int q = L >> 10;
+  int j0 = 0;
+  if (w0 > s) j0 = (int)(((unsigned)(w0 - s) + 1023u) >> 10);
+  for (int j = j0; j < q; j++) {
+    if (s + (j << 10) >= w1) break;
     f(make_token(dupKey, 7));
   }
-  long long pos = s + (q << 10);
-  int r = (int)(L - (q << 10));
+  int pos = s + (q << 10);
+  int r = L - (q << 10);
   while (r > 8) {
     int lg = 31 - clz32(r);
     if (pos >= w0 && pos < w1) f(make_token(dupKey, lg - 3));
     pos += 1 << lg;
     r -= 1 << lg;
   }
-  long long a = pos > w0 ? pos : w0, z = pos + r < w1 ? pos + r : w1;
-  for (long long x = a; x < z; x++) f(make_token(dupV, 0));
-}
-
-// Number of tokens of a zero-bin run of length L (the same split as
-// run_tokens): runs of 1024, then one token per set bit of the remainder at
-// or above 8 -- except that a last 8 left over is coded as 8 single tokens.
-__host__ __device__ inline int run_token_count(long long L) {
-  const int q = (int)(L >> 10), r = (int)(L & 1023);
-  const int hi = r & ~7, lo = r & 7;
-#ifdef __CUDA_ARCH__
-  int big = __popc(hi >> 4);
-#else
-  int big = __builtin_popcount(hi >> 4);
-#endif
-  if (hi & 8) return q + big + (lo > 0 ? 1 + lo : 8);
-  return q + big + lo;
+  const int a = pos > w0 ? pos : w0, z = pos + r < w1 ? pos + r : w1;
+  for (int x = a; x < z; x++) f(make_token(dupV, 0));
 }
 
 struct CubeletState;
@@ -200,7 +184,6 @@ struct DevBatch {
   float *dqtable;                 // dequant values [n][binCount]
   unsigned long long *hist;       // [n][kMaxSymbols] Huffman counts
   int4 *chunkRun;                 // per chunk: lead, trail, allZero, len
-  long long *chunkRunCtx;         // per chunk: start of incoming run, end of outgoing run (2 each)
   unsigned long long *chunkBits;  // per chunk bit count / offset
   unsigned long long *codes;      // [n][kMaxSymbols] code bits
   uint8_t *codeLen;               // [n][kMaxSymbols]
@@ -217,6 +200,7 @@ struct DevBatch {
   int4 *logHdr;                   // [n] log table layout from the host
   int *meta;                      // packed decode tables and Lloyd codebooks
   long long totalChunks;
+  int maxChunks;                  // most chunks of one cubelet
 };
 
 // launchers (dwt.cu)
