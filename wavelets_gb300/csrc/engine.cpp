@@ -1087,12 +1087,16 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   long long groupTotal = 0, encTotal = 0;
   long long chunk0[2] = {0, 0}, group0[2] = {0, 0}, words0[2] = {0, 0}, enc0[2] = {0, 0};
   long long wordsAcc = 0;
-  // bit-packer slices per chunk, from each half's chunk count
-  int encF[2] = {1, 1};
+  // bit-packer slices per chunk and chunks per quantize group, from each
+  // half's chunk count
+  int encF[2] = {1, 1}, group[2] = {1, 1};
   {
     long long halfChunks[2] = {0, 0};
     for (int i = 0; i < n; i++) halfChunks[half_of(i)] += plans[i].nChunks;
-    for (int h = 0; h < nh; h++) encF[h] = ctx->encSlices ? ctx->encSlices : enc_slices(halfChunks[h]);
+    for (int h = 0; h < nh; h++) {
+      encF[h] = ctx->encSlices ? ctx->encSlices : enc_slices(halfChunks[h]);
+      group[h] = quant_group(halfChunks[h]);
+    }
   }
   for (int i = 0; i < n; i++) {
     const Plan &pl = plans[i];
@@ -1118,7 +1122,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     c.lloydIters = pl.p.lloyd_iters > 0 ? pl.p.lloyd_iters : 20;
     c.tableOff = pl.tableOff;
     c.groupBase = (int)(groupTotal - group0[h]);
-    groupTotal += (pl.nChunks + kQuantGroup - 1) / kQuantGroup;
+    groupTotal += (pl.nChunks + group[h] - 1) / group[h];
     c.encBase = (int)(encTotal - enc0[h]);
     encTotal += ((long long)pl.nChunks * encF[h] + kEncThreads - 1) / kEncThreads;
     wordsAcc += pl.wordsCap;
@@ -1151,6 +1155,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.chunkCub = P<int>(ctx->chunkCub);
   b.groupCub = P<int>(ctx->groupCub);
   b.totalGroups = groupTotal;
+  b.group = group[0];
   b.encCub = P<int>(ctx->encCub);
   b.totalEnc = encTotal;
   b.encF = encF[0];
@@ -1198,6 +1203,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       v.meta += c0 * kMetaPer;
       v.totalChunks = (h ? chunkTotal : chunk0[1]) - ch;
       v.maxChunks = maxChunks[h];
+      v.group = group[h];
       v.totalGroups = (h ? groupTotal : group0[1]) - g;
     }
   }

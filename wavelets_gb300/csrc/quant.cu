@@ -395,7 +395,7 @@ __device__ __forceinline__ QParams load_qparams(const CubeletDev &cd, const Cube
 // in order: a token for every value that is not the zero bin, preceded by the
 // tokens of the zero-bin run before it when that run starts inside the chunk.
 // Runs touching a chunk edge are left to runs_kernel (counts) and the encoder
-// (tokens).  A CTA codes kQuantGroup consecutive chunks of one cubelet; warp
+// (tokens).  A CTA codes b.group consecutive chunks of one cubelet; warp
 // w owns elements [512 w, 512 w + 512) of each chunk, and everything but one
 // CTA barrier per chunk is warp-local.
 //
@@ -491,8 +491,8 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff) {
   const int dupV = st->dupValue;
   const int B = cd.binCount;
   const int nTab = q.alg == WL_LLOYD ? q.nb : (q.alg == WL_LOG ? q.nPos + q.nNeg : 0);
-  const int c0 = ((int)blockIdx.x - cd.groupBase) * kQuantGroup;  // first chunk of the cubelet
-  const int nc = min(kQuantGroup, cd.nChunks - c0);
+  const int c0 = ((int)blockIdx.x - cd.groupBase) * b.group;  // first chunk of the cubelet
+  const int nc = min(b.group, cd.nChunks - c0);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int base = w * kSpan;
   const unsigned ltMask = (1u << lane) - 1u;

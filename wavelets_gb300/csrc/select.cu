@@ -58,7 +58,7 @@ __device__ __forceinline__ void load_chunk(const float *src, int len, float (&v)
 }
 
 // First digit (bits 31..20 of |c|) plus min, max and the two largest |c|.
-// A CTA takes kQuantGroup consecutive chunks of one cubelet (one histogram
+// A CTA takes b.group consecutive chunks of one cubelet (one histogram
 // flush per group); a thread's 16 loads of a chunk are issued together, and
 // six CTAs per SM keep enough of them in flight.
 __global__ void __launch_bounds__(kThreads, 6)
@@ -67,8 +67,8 @@ select_pass0(DevBatch b, const float *__restrict__ coef) {
   const int ci = b.groupCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
   if (cd.selFused) return;  // the last transform pass gathered these already
-  const int c0 = ((int)blockIdx.x - cd.groupBase) * kQuantGroup;
-  const int nc = min(kQuantGroup, cd.nChunks - c0);
+  const int c0 = ((int)blockIdx.x - cd.groupBase) * b.group;
+  const int nc = min(b.group, cd.nChunks - c0);
   auto chunk_len = [&](int k) {
     return (int)min((long long)kChunk, cd.n - (long long)(c0 + k) * kChunk);
   };
@@ -102,8 +102,8 @@ select_compact(DevBatch b, const float *__restrict__ coef, unsigned *__restrict_
   __shared__ unsigned lh[kLloydBins];
   const int ci = b.groupCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
-  const int c0 = ((int)blockIdx.x - cd.groupBase) * kQuantGroup;
-  const int nc = min(kQuantGroup, cd.nChunks - c0);
+  const int c0 = ((int)blockIdx.x - cd.groupBase) * b.group;
+  const int nc = min(b.group, cd.nChunks - c0);
   CubeletState *st = b.state + ci;
   const unsigned prefix = st->prefix;
   const bool lloyd = cd.quantAlg == WL_LLOYD && !st->lloydDeferred;
@@ -292,7 +292,7 @@ __global__ void chunk_map_kernel(DevBatch b) {
   const CubeletDev cd = b.cub[blockIdx.x];
   for (int j = threadIdx.x; j < cd.nChunks; j += blockDim.x)
     b.chunkCub[cd.chunkBase + j] = (int)blockIdx.x;
-  const int groups = (cd.nChunks + kQuantGroup - 1) / kQuantGroup;
+  const int groups = (cd.nChunks + b.group - 1) / b.group;
   for (int j = threadIdx.x; j < groups; j += blockDim.x)
     b.groupCub[cd.groupBase + j] = (int)blockIdx.x;
   const int enc = (int)(((long long)cd.nChunks * b.encF + kEncThreads - 1) / kEncThreads);

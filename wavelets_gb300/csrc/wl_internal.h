@@ -28,7 +28,18 @@ constexpr int kLloydBins = 4096;        // |coefficient| histogram for Lloyd
 constexpr int kCandSlices = 64;        // CTAs per cubelet over its threshold candidates
 constexpr int kLutCells = 4096;         // Lloyd bin lookup: cells of the float order key
 constexpr int kLutStride = kLutCells + 8;  // per-cubelet table stride (16-byte rows)
-constexpr int kQuantGroup = 8;          // chunks per select / quantize / encode CTA
+// Chunks per select / quantize CTA: up to eight for large batches (few table
+// loads and histogram flushes), fewer where eight would leave CTA slots empty
+// (four CTAs of 256 threads on each of a GB300's 152 SMs: the quantizer's
+// occupancy).  With eight always, the quantizer of a 2048^2 image (1024
+// chunks) ran 128 CTAs of eight chunks in a row: the call took 468 us against
+// 435 us with two, a 147 x 181 x 93 stack 483 against 448 us; 256^3 (4096
+// chunks, seven) 529 and 531 us.
+constexpr int kMaxQuantGroup = 8;
+inline int quant_group(long long chunks) {
+  const long long slots = 152 * 4, g = (chunks + slots - 1) / slots;
+  return (int)(g < 1 ? 1 : g > kMaxQuantGroup ? kMaxQuantGroup : g);
+}
 // Bit packer: a chunk's tokens are split into F slices (F a power of two,
 // 1..32), one lane each; a CTA of kEncThreads lanes packs kEncThreads / F
 // consecutive chunks of one cubelet (four warps: few CTAs, so kernels of
@@ -160,7 +171,7 @@ struct CubeletDev {
   int lloydIters;
   int tableOff;           // offset into per-cubelet quantizer tables (floats)
   int nTable;             // entries in the table (log: boundaries; lloyd: boundaries)
-  int groupBase;          // first quantize group (kQuantGroup chunks per group)
+  int groupBase;          // first quantize group (DevBatch::group chunks per group)
   int encBase;            // first bit-packer CTA (kEncThreads / F chunks per CTA)
   int selFused;           // 1: the last transform pass gathered the first select
                           // digit and the extremes (no stand-alone first pass)
@@ -193,6 +204,7 @@ struct DevBatch {
   int *chunkCub;                  // [totalChunks] cubelet of every chunk
   int *groupCub;                  // [totalGroups] cubelet of every quantize group
   long long totalGroups;
+  int group;                      // chunks per quantize group
   int *encCub;                    // [totalEnc] cubelet of every bit-packer CTA
   long long totalEnc;
   int encF;                       // bit-packer slices per chunk
