@@ -1,536 +1,430 @@
 // Huffman decoding on the device for streams without any index (files the
-// reference wrote decode too).
+// reference wrote decode too), a batch of streams at a time, straight to the
+// dequantized values.
 //
 // Reference: HuffmanDecoder::decodeFromStream (huffman.h:96-131) walks the
 // breadth-first decode table bit by bit; a zero-run key is followed by 3
 // length bits and expands to 2^(v+3) copies of the zero bin.
 //
-// The stream is cut into subsequences of kSubBits bits.  Phase 1: every
-// subsequence is decoded speculatively from its first bit until the decoder
-// crosses into the next subsequence; it records where that happens (its exit,
-// a token boundary) and how many elements it produced.  Huffman codes
-// resynchronise after a few tokens, so the exit rarely depends on where the
-// decoding started.  Rounds: a subsequence whose start differs from its
-// predecessor's exit is decoded again from that exit; rounds repeat until no
-// start changes (each round fixes at least the first wrong subsequence).
-// The first kSync token boundaries of every speculative decode are kept, so a
-// later round stops as soon as it lands on one of them: from there on its
-// tokens are the speculative ones, and the exit and element count follow
-// from the record (without it every subsequence would be decoded again,
-// since a speculative start is almost never a token boundary).
-// Then an exclusive scan of the element counts gives every subsequence its
-// output offset, and a last pass decodes again and writes the elements (the
-// bins, or for batched decompression their dequantized values, where zero-bin
-// runs were set beforehand and are only skipped).  A 12-bit lookup table
-// resolves most codes in one step; each thread reads its stream through a
-// window of three words in registers.
+// The stream is cut into subsequences of 256 bits, one thread each, and a CTA
+// decodes a tile of kTileSubs consecutive ones:
+//  - tile_kernel: every thread decodes speculatively from its first bit to
+//    the end of its subsequence and keeps its first kRec token boundaries.
+//    Huffman codes resynchronise after a few tokens, so a thread's exit (the
+//    first boundary past its end) rarely depends on where it started.  Then,
+//    in rounds inside the CTA, a thread whose start differs from its
+//    predecessor's exit decodes again from there until it meets one of its
+//    recorded boundaries.  Thread 0 decodes the subsequence before the tile
+//    only to find the tile's entry.
+//  - check_kernel: a tile whose entry is not the exit of the tile before it
+//    (rare: no resynchronisation within a subsequence) is decoded again from
+//    that exit.  It is launched twice; the second launch changes nothing
+//    unless a chain of tiles was wrong, which the host sees at the end and
+//    repairs with more launches (codes that never resynchronise, e.g. all of
+//    one length).
+//  - scan_kernel: output offset of every tile.
+//  - write_kernel: decodes each subsequence from its true start and writes
+//    the values.
+// A token costs two shared-memory reads of the stream and one of a 12-bit
+// table that also expands zero-run lengths where they fit; longer codes go on
+// four bits at a time.
+//
+// Bound by the latency of the token chain on small streams, which is why a
+// thread has only 256 bits and nothing waits on the host between the passes:
+// with 1024 bits a thread, tables in global memory and a host wait after
+// every round, decoding a 2048^2 image (4.7 Mbit) took 830 us of a 1213 us
+// call; the call now takes 394 us.  256^3 volume 900 -> 339 us, mixed batch
+// of 512 (464 Mbit) 7.02 -> 5.86 ms.
 #include <cstring>
-#include <vector>
 
 #include "wl_internal.h"
 
 namespace wl {
 namespace {
 
-constexpr int kSubBits = 1024;
-constexpr int kSync = 8;  // token boundaries kept per speculative decode
-constexpr int kLutBits = 12;
 constexpr int kThreads = 256;
+constexpr int kSubBits = 256, kSubWords = kSubBits / 32;
+constexpr int kTileSubs = kThreads - 1;      // thread 0 warms up on the one before
+constexpr int kTileBits = kTileSubs * kSubBits;
+constexpr int kTileWords = kTileSubs * kSubWords;
+constexpr int kRec = 8;                      // token boundaries kept per speculative decode
+constexpr int kLutBits = 12, kLutSize = 1 << kLutBits;
+constexpr int kStepBits = 4, kStep = 1 << kStepBits;  // longer codes, per step
+constexpr int kMaxCode = 60;                 // longest code accepted
+// words of a tile in shared memory: kThreads subsequences of 8 words and the
+// longest token past the end; after every eighth word the next one again, so
+// that words k and k + 1 are always neighbours, which also spreads the
+// threads' words over the banks (stride 9)
+constexpr int kStageWords = kThreads * kSubWords + 4;
+constexpr int kStageSize = kStageWords + kStageWords / 8 + 1;
+constexpr int kBuildNodes = 2 * kMaxSymbols;  // decode tables staged in shared memory
 
-struct DecCub {
-  const uint32_t *words;
-  long long nWords;
-  const int *table;
-  int nTable;
-  int dupKey, dupValue;
-  int binCount;
-  long long n;        // elements
-  int *out;           // bins
-  float *fout = nullptr;  // or the dequantized values dq[bin]
-  const float *dq = nullptr;
-  long long subBase;  // first subsequence
-  long long nSub;
-  int lutOff;
+// Table entry.  Token: bits 0-5 bits consumed, 6-9 log2 of its elements,
+// 10-22 symbol.  kSlow: kRun: the zero-run key with a code of bits 0-5 bits
+// whose length bits come after it (kBad: malformed table), else bits 0-15
+// the step table to go on with.
+constexpr unsigned kSlow = 1u << 31, kRun = 1u << 30, kBad = 1u << 29;
+
+struct TileAt {
+  int tile;    // tile of the cubelet
+  int tot;     // bits of the stream from the staged words' start (bounded)
 };
 
-__device__ __forceinline__ int find_cub(const DecCub *c, int n, long long sub) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (c[mid].subBase <= sub) lo = mid; else hi = mid - 1;
+// stage the words of a tile: local subsequence s (thread s) is subsequence
+// kTileSubs * tile + s - 1 of the stream
+__device__ __forceinline__ TileAt stage_words(const DecodeCub &c, int tile, uint32_t *sw) {
+  TileAt t;
+  t.tile = tile;
+  const long long w0 = (long long)tile * kTileWords - kSubWords;
+  for (int k = threadIdx.x; k < kStageWords; k += kThreads) {
+    const long long g = w0 + k;
+    const uint32_t v = g >= 0 && g < c.nWords ? c.words[g] : 0u;
+    sw[k + (k >> 3)] = v;
+    if ((k & 7) == 0 && k > 0) sw[k + (k >> 3) - 1] = v;
   }
-  return lo;
+  const long long bits = (c.nWords - w0) * 32;
+  t.tot = (int)min(bits, (long long)2 * kTileBits);
+  return t;
 }
-
-// LUT entry: bit 31 leaf; leaf: bits 16-23 code length, bits 0-15 symbol;
-// not a leaf: bits 0-30 node offset in the decode table after kLutBits bits
-__global__ void build_lut_kernel(const DecCub *cubs, unsigned *lut) {
-  const DecCub c = cubs[blockIdx.x];
-  unsigned *L = lut + (size_t)c.lutOff;
-  for (int p = threadIdx.x; p < (1 << kLutBits); p += blockDim.x) {
-    if (c.nTable == 2) {  // one node: a zero-length code
-      L[p] = 0x80000000u | (unsigned)c.table[1];
-      continue;
-    }
-    int node = 0;
-    unsigned e = 0;
-    bool leaf = false;
-    for (int d = 0; d < kLutBits; d++) {
-      const int bit = (p >> d) & 1;
-      const int nx = c.table[node + bit] * 2;
-      if (nx < 0 || nx + 1 >= c.nTable) { e = 0x80000000u | (0xffu << 16) | 0xffffu; leaf = true; break; }
-      node = nx;
-      if (c.table[node] == 0) {
-        e = 0x80000000u | ((unsigned)(d + 1) << 16) | (unsigned)c.table[node + 1];
-        leaf = true;
-        break;
-      }
-    }
-    L[p] = leaf ? e : (unsigned)node;
-  }
-}
-
-// Decode one token at bit p.  Returns bits consumed (0 = malformed), sets the
-// element count and the value.
-// Three stream words from word i on (zero past the end), moved on a word at a
-// time as the bit position advances (it never goes back): a token loads a
-// word only when it crosses into the next one.
-struct Window {
-  const uint32_t *w;
-  long long nw, i;
-  unsigned a, b, c;
-  __device__ unsigned ld(long long k) const { return k < nw ? w[k] : 0u; }
-  __device__ void init(const uint32_t *words, long long n, long long p) {
-    w = words;
-    nw = n;
-    i = p >> 5;
-    a = ld(i);
-    b = ld(i + 1);
-    c = ld(i + 2);
-  }
-  // 64 bits of the stream from bit p (p >= 32 i), as peek64
-  __device__ unsigned long long peek(long long p) {
-    const long long k = p >> 5;
-    while (i < k) {
-      a = b;
-      b = c;
-      c = ld(i + 3);
-      i++;
-    }
-    // bits o .. o + 63 of c:b:a, as two 32-bit funnel shifts (o = 0 included)
-    const unsigned o = (unsigned)(p & 31);
-    const unsigned lo = __funnelshift_r(a, b, o), hi = __funnelshift_r(b, c, o);
-    return lo | ((unsigned long long)hi << 32);
-  }
-};
-
-__device__ __forceinline__ int decode_token(const DecCub &c, const unsigned *L, Window &win,
-                                            long long p, int &count, int &value) {
-  const unsigned long long b0 = win.peek(p);  // bits p .. p + 63
-  unsigned long long bits = b0;
-  const unsigned e = L[bits & ((1u << kLutBits) - 1)];
-  int len, sym;
-  if (e & 0x80000000u) {
-    len = (e >> 16) & 0xff;
-    sym = e & 0xffff;
-    if (len == 0xff) return 0;
-  } else {
-    int node = (int)e;
-    len = kLutBits;
-    bits >>= kLutBits;
-    while (true) {
-      const int nx = c.table[node + (int)(bits & 1)] * 2;
-      bits >>= 1;
-      len++;
-      if (nx < 0 || nx + 1 >= c.nTable || len > 60) return 0;
-      node = nx;
-      if (c.table[node] == 0) break;
-    }
-    sym = c.table[node + 1];
-  }
-  if (sym == c.dupKey && c.dupKey >= 0) {
-    // the 3 length bits follow the code; len <= 60, so they are in b0
-    const unsigned v = (unsigned)((b0 >> len) & 7u);
-    count = 1 << (v + 3);
-    value = c.dupValue;
-    return len + 3;
-  }
-  count = 1;
-  value = sym;
-  return len > 0 ? len : -1;  // -1: zero-length code (one-symbol stream)
-}
-
-// Decode tokens from `start` until the position reaches `limit`; returns the
-// exit position and the number of elements.
-__device__ long long decode_span(const DecCub &c, const unsigned *L, long long start, long long limit,
-                                 long long &elems, bool &bad) {
-  long long p = start, e = 0;
-  const long long total = c.nWords * 32;
-  Window win;
-  win.init(c.words, c.nWords, p);
-  while (p < limit && p < total) {
-    int cnt, val;
-    const int used = decode_token(c, L, win, p, cnt, val);
-    if (used <= 0) { bad = true; break; }
-    p += used;
-    e += cnt;
-  }
-  elems = e;
-  return p;
-}
-
-// Speculative decode of subsequence i from its first bit, keeping the first
-// kSync token boundaries: rec[k * totalSub + i] = (boundary - start) | (elements
-// before it << 16), all ones where the subsequence ends first (a boundary is at
-// most kSync * 61 bits and 8192 elements past the start).
-__device__ long long decode_span_rec(const DecCub &c, const unsigned *L, long long start,
-                                     long long limit, long long &elems, bool &bad,
-                                     unsigned *rec, long long stride) {
-  long long p = start, e = 0;
-  const long long total = c.nWords * 32;
-  Window win;
-  win.init(c.words, c.nWords, p);
+__device__ __forceinline__ void stage_lut(const DecodeCub &c, const unsigned *lut, unsigned *sl) {
+  const uint4 *g = reinterpret_cast<const uint4 *>(lut + c.lutOff);
+  uint4 *s = reinterpret_cast<uint4 *>(sl);
 #pragma unroll
-  for (int k = 0; k < kSync; k++) {
+  for (int i = 0; i < kLutSize / 4 / kThreads; i++)
+    s[threadIdx.x + i * kThreads] = g[threadIdx.x + i * kThreads];
+}
+__device__ __forceinline__ unsigned bits_at(const uint32_t *sw, int p) {
+  const int k = p >> 5, a = k + (k >> 3);
+  return __funnelshift_r(sw[a], sw[a + 1], p & 31);
+}
+
+// a code longer than the table, or a zero-run key whose length bits are
+// outside it; returns the bits consumed, 0 when malformed
+__device__ __noinline__ int slow_token(const uint32_t *sw, const unsigned *steps, int p,
+                                       unsigned e, int dupValue, int &lg, int &sym) {
+  int used = 0, width = kLutBits;
+  while (e & kSlow) {
+    if (e & kRun) {
+      if (e & kBad) return 0;
+      used += (int)(e & 63u);
+      lg = (int)(bits_at(sw, p + used) & 7u) + 3;
+      sym = dupValue;
+      return used + 3;
+    }
+    used += width;
+    width = kStepBits;
+    e = steps[(e & 0xffffu) * kStep + (bits_at(sw, p + used) & (kStep - 1))];
+  }
+  lg = (int)((e >> 6) & 15u);
+  sym = (int)((e >> 10) & 0x1fffu);
+  return used + (int)(e & 63u);
+}
+
+// one token at bit p of the staged words: bits consumed (0: malformed)
+__device__ __forceinline__ int token_at(const uint32_t *sw, const unsigned *sl,
+                                        const unsigned *steps, int p, int dupValue, int &lg,
+                                        int &sym) {
+  const unsigned e = sl[bits_at(sw, p) & (kLutSize - 1)];
+  if (e & kSlow) return slow_token(sw, steps, p, e, dupValue, lg, sym);
+  lg = (int)((e >> 6) & 15u);
+  sym = (int)((e >> 10) & 0x1fffu);
+  return (int)(e & 63u);
+}
+
+struct TileSmem {
+  uint32_t sw[kStageSize];
+  __align__(16) unsigned lut[kLutSize];
+  unsigned rec[kRec][kThreads];
+  int exits[kThreads];
+  unsigned sums[kThreads / 32];
+};
+
+// Decode a tile; entry: the tile's true first token boundary (bits past the
+// tile's first bit), or -1 to find it speculatively.  Writes the start and
+// element count of every subsequence and the tile's entry, exit and total.
+__device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, TileSmem &sm,
+                            int entry) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int tile = t - c.tileBase, tid = threadIdx.x;
+  const TileAt at = stage_words(c, tile, sm.sw);
+  stage_lut(c, d.lut, sm.lut);
+  __syncthreads();
+  const unsigned *steps = d.steps + (size_t)c.stepOff * kStep;
+  const long long sub = (long long)tile * kTileSubs + tid - 1;  // subsequence of the stream
+  const bool active = sub >= 0 && sub < c.nSub;
+  const int s0 = tid * kSubBits, lim = min(s0 + kSubBits, at.tot);
+  int p = s0;
+  unsigned n = 0;
+  bool bad = false;
+  // speculative decode, the first boundaries recorded (unused: all ones)
+#pragma unroll
+  for (int k = 0; k < kRec; k++) {
     unsigned r = ~0u;
-    if (!bad && p < limit && p < total) {
-      int cnt, val;
-      const int used = decode_token(c, L, win, p, cnt, val);
-      if (used <= 0) {
-        bad = true;
-      } else {
+    if (active && !bad && p < lim) {
+      int lg, sym;
+      const int used = token_at(sm.sw, sm.lut, steps, p, c.dupValue, lg, sym);
+      bad = used == 0;
+      if (!bad) {
         p += used;
-        e += cnt;
-        r = (unsigned)(p - start) | ((unsigned)e << 16);
+        n += 1u << lg;
+        r = (unsigned)(p - s0) | (n << 16);
       }
     }
-    rec[k * stride] = r;
+    sm.rec[k][tid] = r;
   }
-  while (!bad && p < limit && p < total) {
-    int cnt, val;
-    const int used = decode_token(c, L, win, p, cnt, val);
-    if (used <= 0) { bad = true; break; }
+  while (active && !bad && p < lim) {
+    int lg, sym;
+    const int used = token_at(sm.sw, sm.lut, steps, p, c.dupValue, lg, sym);
+    if (used == 0) { bad = true; break; }
     p += used;
-    e += cnt;
+    n += 1u << lg;
   }
-  elems = e;
-  return p;
-}
+  const int x0 = p;           // the speculative exit and element count
+  const unsigned n0 = n;
+  int start = s0;
+  // the first tile starts with the stream
+  if (tid == 0 && tile == 0) p = kSubBits;
+  if (tid == 0 && entry >= 0) p = kSubBits + entry;
 
-// Decode from a true token boundary s (s >= s0, the speculative start) until
-// the position meets a boundary of the speculative decode (then its exit x0
-// and element count e0 hold, less the elements it produced before that
-// boundary) or the subsequence ends.
-__device__ long long decode_span_sync(const DecCub &c, const unsigned *L, long long s,
-                                      long long limit, long long s0, long long x0, long long e0,
-                                      const unsigned *rec, long long stride, long long &elems,
-                                      bool &bad) {
-  long long p = s, e = 0;
-  const long long total = c.nWords * 32;
-  int k = -1;                 // speculative boundary below or at p: k = -1 is s0
-  long long bk = s0, ck = 0;  // its position and the elements before it
-  Window win;
-  win.init(c.words, c.nWords, p);
+  // rounds: each fixes at least the first wrong subsequence
   for (;;) {
-    while (bk < p && k + 1 < kSync) {
-      const unsigned r = rec[(k + 1) * stride];
-      if (r == ~0u) break;
-      k++;
-      bk = s0 + (r & 0xffffu);
-      ck = r >> 16;
+    sm.exits[tid] = p;
+    __syncthreads();
+    const int ns = tid > 0 ? sm.exits[tid - 1] : start;
+    bool changed = false;
+    if (active && tid > 0 && ns != start) {
+      start = ns;
+      int q = ns, k = -1, bk = s0;  // boundary k of the speculative decode (-1: s0)
+      unsigned m = 0, ck = 0;
+      for (;;) {
+        while (bk < q && k + 1 < kRec) {
+          const unsigned r = sm.rec[k + 1][tid];
+          if (r == ~0u) break;
+          k++;
+          bk = s0 + (int)(r & 0xffffu);
+          ck = r >> 16;
+        }
+        if (bk == q) {  // on the speculative path from here
+          m += n0 - ck;
+          q = x0;
+          break;
+        }
+        if (bad || q >= lim) break;
+        int lg, sym;
+        const int used = token_at(sm.sw, sm.lut, steps, q, c.dupValue, lg, sym);
+        if (used == 0) { bad = true; break; }
+        q += used;
+        m += 1u << lg;
+      }
+      changed = q != p;
+      p = q;
+      n = m;
     }
-    if (bk == p) {  // on the speculative path from here
-      elems = e + (e0 - ck);
-      return x0;
-    }
-    if (!(p < limit && p < total)) break;
-    int cnt, val;
-    const int used = decode_token(c, L, win, p, cnt, val);
-    if (used <= 0) { bad = true; break; }
-    p += used;
-    e += cnt;
+    if (!__syncthreads_or(changed)) break;
   }
-  elems = e;
-  return p;
+  const bool out = active && tid > 0;
+  if (out) {
+    d.subStart[c.subBase + sub] = (uint8_t)(start - s0);
+    d.subCount[c.subBase + sub] = n;
+  }
+  unsigned sum = out ? n : 0u;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
+  if ((tid & 31) == 0) sm.sums[tid >> 5] = sum;
+  if (tid == 1) d.tileEntry[t] = start - s0;
+  if (tid == kThreads - 1) d.tileExit[t] = p - (s0 + kSubBits);
+  if (bad) atomicAdd(&d.flags[kDecodeBad], 1);
+  __syncthreads();
+  if (tid == 0) {
+    unsigned all = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; w++) all += sm.sums[w];
+    d.tileCount[t] = all;
+  }
 }
 
-__global__ void spec_kernel(const DecCub *cubs, int nCub, const unsigned *lut, long long totalSub,
-                            long long *start, long long *exitPos, long long *elems, int *flags,
-                            int round, unsigned *rec, long long *spec0) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= totalSub) return;
-  const int ci = find_cub(cubs, nCub, i);
-  const DecCub c = cubs[ci];
-  const long long local = i - c.subBase;
-  const long long s0 = local * kSubBits, limit = (local + 1) * kSubBits;
-  bool bad = false;
-  long long e, x;
-  if (round == 0) {
-    start[i] = s0;
-    x = decode_span_rec(c, lut + c.lutOff, s0, limit, e, bad, rec + i, totalSub);
-    spec0[2 * i] = x;
-    spec0[2 * i + 1] = e;
-  } else {
-    if (local == 0) {  // always starts right; carry its exit to this round's buffer
-      exitPos[2 * i + (round & 1)] = exitPos[2 * i + ((round - 1) & 1)];
-      return;
-    }
-    const long long s = exitPos[2 * (i - 1) + ((round - 1) & 1)];
-    if (s == start[i]) {
-      exitPos[2 * i + (round & 1)] = exitPos[2 * i + ((round - 1) & 1)];
-      return;
-    }
-    atomicAdd(&flags[0], 1);
-    start[i] = s;
-    x = decode_span_sync(c, lut + c.lutOff, s, limit, s0, spec0[2 * i], spec0[2 * i + 1],
-                         rec + i, totalSub, e, bad);
-  }
-  exitPos[2 * i + (round & 1)] = x;
-  elems[i] = e;
-  if (bad) atomicAdd(&flags[1], 1);
+__global__ void __launch_bounds__(kThreads) tile_kernel(const DecodeCub *__restrict__ cubs,
+                                                        DecodeArrays d) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const DecodeCub c = cubs[d.tileCub[blockIdx.x]];
+  decode_tile(c, d, blockIdx.x, *reinterpret_cast<TileSmem *>(dsm), -1);
 }
 
-// per cubelet exclusive scan of element counts (one CTA per cubelet)
-__global__ void __launch_bounds__(1024) elem_scan_kernel(const DecCub *cubs, long long *elems,
-                                                         long long *totalOut) {
-  __shared__ long long sh[32];
-  const DecCub c = cubs[blockIdx.x];
+// flag: counter of tiles decoded again
+__global__ void __launch_bounds__(kThreads) check_kernel(const DecodeCub *__restrict__ cubs,
+                                                         DecodeArrays d, int flag) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  __shared__ int entry;
+  const int t = blockIdx.x;
+  const DecodeCub c = cubs[d.tileCub[t]];
+  if (t == c.tileBase) return;
+  // read once for the CTA: the tile before may be decoded again meanwhile
+  // (the next launch then sees its new exit)
+  if (threadIdx.x == 0) {
+    const int e = d.tileExit[t - 1];
+    entry = e == d.tileEntry[t] ? -1 : e;
+  }
+  __syncthreads();
+  const int e = entry;
+  if (e < 0) return;
+  if (threadIdx.x == 0) atomicAdd(&d.flags[flag], 1);
+  decode_tile(c, d, t, *reinterpret_cast<TileSmem *>(dsm), e);
+}
+
+// per cubelet: exclusive scan of its tiles' element counts
+__global__ void __launch_bounds__(kThreads) scan_kernel(const DecodeCub *__restrict__ cubs,
+                                                        DecodeArrays d) {
+  __shared__ long long sh[kThreads / 32];
+  const DecodeCub c = cubs[blockIdx.x];
   long long carry = 0;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (long long seg = 0; seg < c.nSub; seg += 1024) {
-    const long long j = seg + threadIdx.x;
-    const long long v = j < c.nSub ? elems[c.subBase + j] : 0;
+  for (int seg = 0; seg < c.nTiles; seg += kThreads) {
+    const int j = seg + threadIdx.x;
+    const long long v = j < c.nTiles ? d.tileCount[c.tileBase + j] : 0;
     long long inc = v;
-    for (int off = 1; off < 32; off <<= 1) {
-      const long long t = __shfl_up_sync(0xffffffffu, inc, off);
-      if (lane >= off) inc += t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
     }
     if (lane == 31) sh[w] = inc;
     __syncthreads();
-    long long before = 0, tot = 0;
-    for (int k = 0; k < 32; k++) { if (k < w) before += sh[k]; tot += sh[k]; }
-    if (j < c.nSub) elems[c.subBase + j] = carry + before + inc - v;
-    carry += tot;
+    long long before = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < kThreads / 32; k++) {
+      if (k < w) before += sh[k];
+      all += sh[k];
+    }
+    if (j < c.nTiles) d.tileOff[c.tileBase + j] = carry + before + inc - v;
+    carry += all;
     __syncthreads();
   }
-  if (threadIdx.x == 0) totalOut[blockIdx.x] = carry;
+  // fewer values than the cubelet holds
+  if (threadIdx.x == 0 && carry < c.n) atomicAdd(&d.flags[kDecodeShort], 1);
 }
 
-__global__ void write_kernel(const DecCub *cubs, int nCub, const unsigned *lut, long long totalSub,
-                             const long long *start, const long long *exitPos, const long long *offs,
-                             int lastRound) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= totalSub) return;
-  const int ci = find_cub(cubs, nCub, i);
-  const DecCub c = cubs[ci];
-  const unsigned *L = lut + c.lutOff;
-  const long long limit = exitPos[2 * i + (lastRound & 1)];
-  long long p = start[i], o = offs[i];
-  const long long total = c.nWords * 32;
-  Window win;
-  win.init(c.words, c.nWords, p);
-  if (c.fout) {
-    // dequantized on the way.  With zero runs the output already holds the
-    // zero bin's value everywhere (launch_fill_batch), so only the other
-    // values are written; runs and single zero-bin tokens just move on.
-    float *F = c.fout;
-    if (c.dupValue >= 0) {
-      // prefilled: a zero-run token or a single zero-bin token only moves on,
-      // every other token is one value (only the zero-run key counts more
-      // than one element)
-      while (p < limit && p < total && o < c.n) {
-        int cnt, val;
-        const int used = decode_token(c, L, win, p, cnt, val);
-        if (used <= 0) break;
-        p += used;
-        if (val != c.dupValue) F[o] = c.dq[min(max(val, 0), c.binCount - 1)];
-        o = min(o + cnt, c.n);
-      }
-      return;
-    }
-    while (p < limit && p < total && o < c.n) {
-      int cnt, val;
-      const int used = decode_token(c, L, win, p, cnt, val);
-      if (used <= 0) break;
-      p += used;
-      const float fv = c.dq[min(max(val, 0), c.binCount - 1)];
-      const long long e = min(o + cnt, c.n);
-      for (; o < e; o++) F[o] = fv;
-    }
-    return;
+struct WriteSmem {
+  uint32_t sw[kStageSize];
+  __align__(16) unsigned lut[kLutSize];
+  unsigned sums[kThreads / 32];
+  float dq[1];  // binCount entries
+};
+
+// The values, from each subsequence's true start.  With zero runs
+// (dupValue >= 0) the output already holds the zero bin's value everywhere
+// (launch_fill_batch), so only the other values are written.
+__global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__restrict__ cubs,
+                                                         DecodeArrays d) {
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char dsm[];
+  WriteSmem &sm = *reinterpret_cast<WriteSmem *>(dsm);
+  const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const DecodeCub c = cubs[d.tileCub[t]];
+  const long long tileOff = d.tileOff[t];
+  if (tileOff >= c.n) return;  // padding bits after the last value
+  const int tile = t - c.tileBase;
+  const TileAt at = stage_words(c, tile, sm.sw);
+  stage_lut(c, d.lut, sm.lut);
+  for (int i = tid; i < c.binCount; i += kThreads) sm.dq[i] = c.dq[i];
+  const long long sub = (long long)tile * kTileSubs + tid - 1;
+  const bool active = tid > 0 && sub < c.nSub;
+  const unsigned n = active ? d.subCount[c.subBase + sub] : 0u;
+  int p = tid * kSubBits + (active ? (int)d.subStart[c.subBase + sub] : 0);
+  unsigned inc = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned x = __shfl_up_sync(kAll, inc, o);
+    if (lane >= o) inc += x;
   }
-  while (p < limit && p < total && o < c.n) {
-    int cnt, val;
-    const int used = decode_token(c, L, win, p, cnt, val);
-    if (used <= 0) break;
+  if (lane == 31) sm.sums[w] = inc;
+  __syncthreads();
+  unsigned before = inc - n;
+#pragma unroll
+  for (int k = 0; k < kThreads / 32; k++) before += k < w ? sm.sums[k] : 0u;
+  if (!active) return;
+  const long long room = c.n - tileOff;  // elements from the tile's first on
+  const unsigned end = (unsigned)min(room, (long long)0xffffffffu);
+  const int lim = min(tid * kSubBits + kSubBits, at.tot);
+  const unsigned *steps = d.steps + (size_t)c.stepOff * kStep;
+  float *F = c.out + tileOff;
+  unsigned o = before;
+  while (p < lim && o < end) {
+    int lg, sym;
+    const int used = token_at(sm.sw, sm.lut, steps, p, c.dupValue, lg, sym);
+    if (used == 0) break;
     p += used;
-    for (int k = 0; k < cnt && o < c.n; k++) c.out[o++] = val;
+    if (sym != c.dupValue) F[o] = sm.dq[min(sym, c.binCount - 1)];
+    o += 1u << lg;
   }
 }
 
-// Fallback when rounds do not converge (codes that never resynchronise, e.g.
-// all of one length): one thread per cubelet fixes its subsequences in order.
-__global__ void seq_fix_kernel(const DecCub *cubs, const unsigned *lut, long long *start,
-                               long long *exitPos, long long *elems, int buf, int *flags) {
-  const DecCub c = cubs[blockIdx.x];
-  for (long long j = 1; j < c.nSub; j++) {
-    const long long i = c.subBase + j;
-    const long long s = exitPos[2 * (i - 1) + buf];
-    if (s == start[i]) continue;
-    start[i] = s;
-    bool bad = false;
-    long long e;
-    exitPos[2 * i + buf] = decode_span(c, lut + c.lutOff, s, (j + 1) * kSubBits, e, bad);
-    elems[i] = e;
-    if (bad) atomicAdd(&flags[1], 1);
+// 12-bit table and step tables of every stream's decode table
+__global__ void __launch_bounds__(1024) build_lut_kernel(const DecodeCub *__restrict__ cubs,
+                                                         DecodeArrays d) {
+  extern __shared__ ushort2 nodes[];  // the decode table, when it fits
+  __shared__ int nSlots;
+  const DecodeCub c = cubs[blockIdx.x];
+  const int nNodes = c.nTable / 2;
+  const bool staged = nNodes <= kBuildNodes && c.dupKey < 0x10000;  // 16 bits an entry
+  const int2 *tab = reinterpret_cast<const int2 *>(c.table);
+  if (staged)
+    for (int i = threadIdx.x; i < nNodes; i += blockDim.x) {
+      const int2 v = tab[i];
+      nodes[i] = make_ushort2((unsigned short)v.x, (unsigned short)v.y);
+    }
+  if (threadIdx.x == 0) nSlots = 0;
+  __syncthreads();
+  auto node = [&](int k) {
+    if (!staged) return tab[k];
+    const ushort2 v = nodes[k];
+    return make_int2(v.x, v.y);
+  };
+  unsigned *L = d.lut + c.lutOff, *T = d.steps + (size_t)c.stepOff * kStep;
+  // the entry reached from node `k` with `width` bits `p`, `above` bits
+  // already consumed
+  auto entry = [&](int k, unsigned p, int width, int above) {
+    int dep = 0;
+    int2 v = node(k);
+    while (v.x != 0 && dep < width) {  // x == 0: a leaf, y its symbol
+      k = (p >> dep) & 1u ? v.y : v.x;
+      dep++;
+      if (k < 0 || k >= nNodes) return kSlow | kRun | kBad;
+      v = node(k);
+    }
+    if (v.x != 0) {  // goes on: a step table of its own
+      if (above + dep + kStepBits > kMaxCode) return kSlow | kRun | kBad;
+      const int slot = atomicAdd(&nSlots, 1);
+      if (slot >= c.nSteps) return kSlow | kRun | kBad;
+      T[slot * kStep] = (unsigned)k;  // until it is filled
+      return kSlow | (unsigned)slot;
+    }
+    if (v.y == c.dupKey && c.dupKey >= 0) {
+      if (above > 0 || dep + 3 > width) return kSlow | kRun | (unsigned)dep;
+      const unsigned run = ((p >> dep) & 7u) + 3;
+      return (unsigned)(dep + 3) | (run << 6) | ((unsigned)c.dupValue << 10);
+    }
+    if (above + dep == 0) return kSlow | kRun | kBad;  // a zero-length code
+    return (unsigned)dep | ((unsigned)v.y << 10);
+  };
+  for (int p = threadIdx.x; p < kLutSize; p += blockDim.x) L[p] = entry(0, (unsigned)p, kLutBits, 0);
+  __syncthreads();
+  int head = 0, above = kLutBits;
+  for (;;) {
+    const int tail = min(nSlots, c.nSteps);
+    __syncthreads();  // everyone has read the count
+    if (head >= tail) break;
+    // whole warps, kStep lanes per table
+    const int lo = head * kStep, hi = tail * kStep;
+    for (int i = (lo & ~31) + threadIdx.x; i < ((hi + 31) & ~31); i += blockDim.x) {
+      const bool ok = i >= lo && i < hi;
+      const int k = ok ? (int)T[i & ~(kStep - 1)] : 0;
+      __syncwarp();
+      if (ok) T[i] = entry(k, (unsigned)(i & (kStep - 1)), kStepBits, above);
+    }
+    __syncthreads();
+    head = tail;
+    above += kStepBits;
   }
-}
-
-__global__ void fill_kernel(int *out, long long n, int v) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    out[i] = v;
-}
-
-}  // namespace
-
-// Decode n streams at once (the DecCub records and scratch in ws: see
-// decode_batch_workspace_bytes).  Streams are the items with a real tree
-// (items whose table is one node are filled by the caller).  Returns 0 on
-// success, 1 when a stream is malformed or holds fewer elements than its
-// cubelet, -1 on a CUDA error; bad[i] (host, may be NULL) marks the items.
-// per subsequence: start, two exits, element count (32 bytes), the
-// speculative exit and count (16) and its kSync boundaries (4 each)
-constexpr size_t kSubBytes = 48 + 4 * kSync;
-
-size_t decode_batch_workspace_bytes(int n, long long totalSub) {
-  return (size_t)n * sizeof(DecCub) + 256 + (size_t)n * 4096 * 4 + (size_t)totalSub * kSubBytes +
-         (size_t)n * 8 + 64 + 256;
-}
-
-int decode_streams(const DecodeItem *items, int n, void *ws, int *hostFlags,
-                   long long *hostTotals, cudaStream_t s) {
-  if (n <= 0) return 0;
-  std::vector<DecCub> cs(n);
-  long long totalSub = 0;
-  for (int i = 0; i < n; i++) {
-    const DecodeItem &it = items[i];
-    DecCub &c = cs[i];
-    const long long nSub = (it.nWords * 32 + kSubBits - 1) / kSubBits > 0
-                               ? (it.nWords * 32 + kSubBits - 1) / kSubBits : 1;
-    c.words = it.words; c.nWords = it.nWords; c.table = it.table; c.nTable = it.nTable;
-    c.dupKey = it.dupKey; c.dupValue = it.dupValue; c.binCount = it.binCount; c.n = it.n;
-    c.out = it.out; c.fout = it.fout; c.dq = it.dq;
-    c.subBase = totalSub; c.nSub = nSub; c.lutOff = i * 4096;
-    totalSub += nSub;
-  }
-  char *p = static_cast<char *>(ws);
-  DecCub *dc = reinterpret_cast<DecCub *>(p);
-  p += ((size_t)n * sizeof(DecCub) + 255) & ~(size_t)255;
-  unsigned *lut = reinterpret_cast<unsigned *>(p); p += (size_t)n * 4096 * 4;
-  long long *start = reinterpret_cast<long long *>(p); p += totalSub * 8;
-  long long *exitPos = reinterpret_cast<long long *>(p); p += totalSub * 16;
-  long long *elems = reinterpret_cast<long long *>(p); p += totalSub * 8;
-  long long *spec0 = reinterpret_cast<long long *>(p); p += totalSub * 16;
-  unsigned *rec = reinterpret_cast<unsigned *>(p); p += totalSub * 4 * kSync;
-  long long *total = reinterpret_cast<long long *>(p); p += (size_t)n * 8;
-  int *flags = reinterpret_cast<int *>(p);
-  if (cudaMemcpyAsync(dc, cs.data(), (size_t)n * sizeof(DecCub), cudaMemcpyHostToDevice, s) !=
-      cudaSuccess)
-    return -1;
-  build_lut_kernel<<<n, 1024, 0, s>>>(dc, lut);
-  const unsigned grid = (unsigned)((totalSub + kThreads - 1) / kThreads);
-  constexpr int kRounds = 6;
-  int round = 0;
-  cudaMemsetAsync(flags, 0, 8, s);
-  spec_kernel<<<grid, kThreads, 0, s>>>(dc, n, lut, totalSub, start, exitPos, elems, flags, 0,
-                                        rec, spec0);
-  bool converged = false;
-  for (round = 1; round <= kRounds; round++) {
-    cudaMemsetAsync(flags, 0, 4, s);
-    spec_kernel<<<grid, kThreads, 0, s>>>(dc, n, lut, totalSub, start, exitPos, elems, flags,
-                                          round, rec, spec0);
-    cudaMemcpyAsync(hostFlags, flags, 8, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-    if (hostFlags[0] == 0) { converged = true; break; }
-  }
-  if (!converged) {
-    round = kRounds;
-    seq_fix_kernel<<<n, 1, 0, s>>>(dc, lut, start, exitPos, elems, round & 1, flags);
-    cudaMemcpyAsync(hostFlags, flags, 8, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-  }
-  if (hostFlags[1]) return 1;
-  elem_scan_kernel<<<n, 1024, 0, s>>>(dc, elems, total);
-  cudaMemcpyAsync(hostTotals, total, (size_t)n * 8, cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-  for (int i = 0; i < n; i++)
-    if (hostTotals[i] < items[i].n) return 1;  // fewer values than the cubelet holds
-  write_kernel<<<grid, kThreads, 0, s>>>(dc, n, lut, totalSub, start, exitPos, elems, round);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-// Decode one stream (device words/table) into n ints at out.  Synchronizes
-// the stream between rounds.  Returns 0 on success, 1 malformed stream,
-// -1 CUDA error.  Scratch comes from `ws` (decode_workspace_bytes).  A
-// one-node table whose symbol is not the zero-run key codes every element
-// with zero bits: fill_value() handles that case.
-size_t decode_workspace_bytes(long long nWords) {
-  const long long nSub = (nWords * 32 + kSubBits - 1) / kSubBits + 1;
-  return (size_t)nSub * kSubBytes + 4096 * 4 + 256 + 64;
-}
-
-int decode_stream(const uint32_t *words, long long nWords, const int *table, int nTable,
-                  int dupKey, int dupValue, int binCount, long long n, int *out, void *ws,
-                  int *hostFlags, cudaStream_t s) {
-  const long long nSub = (nWords * 32 + kSubBits - 1) / kSubBits > 0
-                             ? (nWords * 32 + kSubBits - 1) / kSubBits : 1;
-  char *p = static_cast<char *>(ws);
-  DecCub *dc = reinterpret_cast<DecCub *>(p); p += 256;
-  unsigned *lut = reinterpret_cast<unsigned *>(p); p += 4096 * 4;
-  long long *start = reinterpret_cast<long long *>(p); p += nSub * 8;
-  long long *exitPos = reinterpret_cast<long long *>(p); p += nSub * 16;
-  long long *elems = reinterpret_cast<long long *>(p); p += nSub * 8;
-  long long *spec0 = reinterpret_cast<long long *>(p); p += nSub * 16;
-  unsigned *rec = reinterpret_cast<unsigned *>(p); p += nSub * 4 * kSync;
-  long long *total = reinterpret_cast<long long *>(p); p += 8;
-  int *flags = reinterpret_cast<int *>(p);
-  DecCub c{};  // bins out (fout stays null)
-  c.words = words; c.nWords = nWords; c.table = table; c.nTable = nTable;
-  c.dupKey = dupKey; c.dupValue = dupValue; c.binCount = binCount; c.n = n; c.out = out;
-  c.subBase = 0; c.nSub = nSub; c.lutOff = 0;
-  if (cudaMemcpyAsync(dc, &c, sizeof c, cudaMemcpyHostToDevice, s) != cudaSuccess) return -1;
-  build_lut_kernel<<<1, 1024, 0, s>>>(dc, lut);
-  const unsigned grid = (unsigned)((nSub + kThreads - 1) / kThreads);
-  constexpr int kRounds = 6;
-  int round = 0;
-  cudaMemsetAsync(flags, 0, 8, s);
-  spec_kernel<<<grid, kThreads, 0, s>>>(dc, 1, lut, nSub, start, exitPos, elems, flags, 0, rec,
-                                        spec0);
-  bool converged = false;
-  for (round = 1; round <= kRounds; round++) {
-    cudaMemsetAsync(flags, 0, 4, s);
-    spec_kernel<<<grid, kThreads, 0, s>>>(dc, 1, lut, nSub, start, exitPos, elems, flags, round,
-                                          rec, spec0);
-    cudaMemcpyAsync(hostFlags, flags, 8, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-    if (hostFlags[0] == 0) { converged = true; break; }
-  }
-  if (!converged) {
-    round = kRounds;
-    seq_fix_kernel<<<1, 1, 0, s>>>(dc, lut, start, exitPos, elems, round & 1, flags);
-    cudaMemcpyAsync(hostFlags, flags, 8, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-  }
-  if (hostFlags[1]) return 1;
-  elem_scan_kernel<<<1, 1024, 0, s>>>(dc, elems, total);
-  cudaMemcpyAsync(hostFlags + 2, total, 8, cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-  long long got;
-  memcpy(&got, hostFlags + 2, 8);
-  if (got < n) return 1;  // the reference stops with fewer values than the cubelet holds
-  write_kernel<<<grid, kThreads, 0, s>>>(dc, 1, lut, nSub, start, exitPos, elems, round);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 __global__ void __launch_bounds__(256) fill_batch_kernel(const FillItem *__restrict__ items,
@@ -551,15 +445,49 @@ __global__ void __launch_bounds__(256) fill_batch_kernel(const FillItem *__restr
   if (threadIdx.x < e - tail) it.out[tail + threadIdx.x] = it.v;
 }
 
+}  // namespace
+
 void launch_fill_batch(const FillItem *items, int nItems, long long totalBlocks, cudaStream_t s) {
   if (nItems > 0 && totalBlocks > 0)
     fill_batch_kernel<<<(unsigned)totalBlocks, 256, 0, s>>>(items, nItems);
 }
 
-void fill_value(int *out, long long n, int v, cudaStream_t s) {
-  long long blocks = (n + 255) / 256;
-  if (blocks > 152 * 32) blocks = 152 * 32;
-  fill_kernel<<<(unsigned)(blocks > 0 ? blocks : 1), 256, 0, s>>>(out, n, v);
+long long decode_subs(long long nWords) {
+  const long long k = (nWords * 32 + kSubBits - 1) / kSubBits;
+  return k > 0 ? k : 1;
+}
+int decode_tiles(long long nWords) {
+  return (int)((decode_subs(nWords) + kTileSubs - 1) / kTileSubs);
+}
+int decode_lut_size() { return kLutSize; }
+// step tables a decode table of nTable ints can need: one per inner node
+int decode_steps(int nTable) {
+  const int k = nTable / 4 + 1;
+  return k < 0xffff ? k : 0xffff;
+}
+size_t decode_step_bytes(long long steps) { return (size_t)steps * kStep * sizeof(unsigned); }
+
+int launch_decode(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
+                  cudaStream_t s) {
+  const int build = (b.maxTable / 2 <= kBuildNodes ? b.maxTable / 2 : kBuildNodes) * 4 + 16;
+  if (build > 48 * 1024) raise_smem_limit(build_lut_kernel, build);
+  build_lut_kernel<<<b.n, 1024, build, s>>>(cubs, d);
+  tile_kernel<<<b.tiles, kThreads, sizeof(TileSmem), s>>>(cubs, d);
+  check_kernel<<<b.tiles, kThreads, sizeof(TileSmem), s>>>(cubs, d, kDecodeFirst);
+  check_kernel<<<b.tiles, kThreads, sizeof(TileSmem), s>>>(cubs, d, kDecodeAgain);
+  return 4 + launch_decode_write(cubs, b, d, s);
+}
+void launch_decode_check(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
+                         cudaStream_t s) {
+  check_kernel<<<b.tiles, kThreads, sizeof(TileSmem), s>>>(cubs, d, kDecodeAgain);
+}
+int launch_decode_write(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
+                        cudaStream_t s) {
+  scan_kernel<<<b.n, kThreads, 0, s>>>(cubs, d);
+  const int smem = (int)sizeof(WriteSmem) + b.maxBins * 4;
+  if (smem > 48 * 1024) raise_smem_limit(write_kernel, smem);
+  write_kernel<<<b.tiles, kThreads, smem, s>>>(cubs, d);
+  return 2;
 }
 
 }  // namespace wl

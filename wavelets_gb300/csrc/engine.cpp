@@ -302,7 +302,7 @@ struct wl_ctx {
       hist, chunkRun, chunkBits, chunkCub, groupCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
       words, passes, logHdr, outbuf, decWords, decTable, decWs, meta, optIn, optOut, optErr,
       errIn, errRest, errPart;
-  HostBuf hState, hDecode, hPasses, hTab, hLogHdr, hPrefix, hIn, hVals, hFlags;
+  HostBuf hState, hDecode, hPasses, hTab, hLogHdr, hIn, hFlags;
   HostBuf hStage[2];  // staging buffers of the container pipeline
   // CUDA graphs: 0 = off, 1 = capture a batch geometry seen twice in a row
   // and replay it from then on
@@ -1505,15 +1505,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
 }
 
 // ---- decompression -----------------------------------------------------------
-}  // namespace
-
-// dequantize kernel launcher lives in dwt.cu
-namespace wl {
-void launch_dequant(const int *bins, const float *table, float *out, long long n, int nTable,
-                    cudaStream_t s);
-}
-
-namespace {
 
 // Column-tile inverse passes (the forward layouts in reverse): z in place on
 // z-x-y (only with z levels), y z-x-y -> z-y-x into c2, x z-y-x -> x-y-z with
@@ -1638,17 +1629,21 @@ void inverse_passes(const int size[3], const int steps[3], int wavelet, const in
   }
 }
 
-// Stage the three inverse phases (one upload) and launch them in order; the
-// groups of a phase run concurrently.  pb receives the phase boundaries.
-wl_status run_inverse_phases(wl_ctx *ctx, PassGroups ph[3]) {
+// Staged launches of the three inverse phases.
+struct InversePhases {
+  std::vector<GroupLaunch> gl;
+  size_t bound[4] = {0, 0, 0, 0};
+};
+
+// Stage the three inverse phases (one upload, queued on the context's stream).
+wl_status stage_inverse_phases(wl_ctx *ctx, PassGroups ph[3], InversePhases &ip) {
   size_t hoff = 0, count = 0;
   for (int k = 0; k < 3; k++)
     for (const auto &kv : ph[k]) count += kv.second.size();
   const size_t need = count * (sizeof(PassDesc) + sizeof(int) + 260) + 4096;
   TRY(ensure(ctx, ctx->passes, need));
   TRY(ensure_host(ctx, ctx->hPasses, need));
-  std::vector<GroupLaunch> gl;
-  size_t bound[4] = {0, 0, 0, 0};
+  std::vector<GroupLaunch> &gl = ip.gl;
   const int kinds[3] = {kTuneInvZ, kTuneInvY, kTuneInvX};
   for (int k = 0; k < 3; k++) {
     for (const auto &kv : ph[k]) {
@@ -1666,10 +1661,15 @@ wl_status run_inverse_phases(wl_ctx *ctx, PassGroups ph[3]) {
       const int outT = (kv.first >> 8) & 15;
       TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, outT, true, cols, false, gl));
     }
-    bound[k + 1] = gl.size();
+    ip.bound[k + 1] = gl.size();
   }
   CU(cudaMemcpyAsync(ctx->passes.p, ctx->hPasses.p, hoff, cudaMemcpyHostToDevice, ctx->stream));
-  for (int k = 0; k < 3; k++) TRY(launch_phase(ctx, gl, bound[k], bound[k + 1]));
+  return WL_OK;
+}
+
+// Launch them in order; the groups of a phase run concurrently.
+wl_status launch_inverse_phases(wl_ctx *ctx, const InversePhases &ip) {
+  for (int k = 0; k < 3; k++) TRY(launch_phase(ctx, ip.gl, ip.bound[k], ip.bound[k + 1]));
   return WL_OK;
 }
 
@@ -1684,7 +1684,9 @@ wl_status inverse_impl(wl_ctx *ctx, const int size[3], const int steps[3], int w
   PassGroups ph[3];
   inverse_passes(size, steps, wavelet, original_size, outType, two_d, P<float>(ctx->coef),
                  P<float>(ctx->coef2), dst, ph);
-  TRY(run_inverse_phases(ctx, ph));
+  InversePhases ip;
+  TRY(stage_inverse_phases(ctx, ph, ip));
+  TRY(launch_inverse_phases(ctx, ip));
   if (!outOnDevice) CU(cudaMemcpyAsync(out, dst, outBytes, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
   return WL_OK;
@@ -1735,43 +1737,13 @@ bool single_symbol(const wl_result *r) {
   return r->n_decode == 2 && r->decode[0] == 0 && r->decode[1] != r->dup_key;
 }
 
+wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const int *outTypes,
+                                void *const *outs, int outOnDevice);
+
+// one cubelet: a batch of one
 wl_status decompress_impl(wl_ctx *ctx, const wl_result *r, int outType, void *out, int outOnDevice) {
-  CU(cudaSetDevice(ctx->device));
   if (!r || !out) return fail(ctx, WL_EINVAL, "null argument");
-  long long n;
-  TRY(check_result(ctx, r, outType, n));
-  std::vector<float> dq(r->bin_count);
-  if (r->quant_alg == WL_LLOYD && (!r->values || r->n_values != r->bin_count))
-    return fail(ctx, WL_EFORMAT, "codebook values missing");
-  dequant_values(r->quant_alg, r->bin_count, r->threshold_value, r->max_value, r->values, dq.data());
-  const long long padded = (n + 63) & ~63LL;
-  TRY(ensure(ctx, ctx->coef, padded * 4));
-  TRY(ensure(ctx, ctx->coef2, padded * 4));
-  TRY(ensure(ctx, ctx->bins, padded * 4));  // int bins for the dequant kernel
-  TRY(ensure(ctx, ctx->dqtable, (size_t)kMaxBins * 4));
-  TRY(ensure(ctx, ctx->decWords, (size_t)r->n_words * 4 + 16));
-  TRY(ensure(ctx, ctx->decTable, (size_t)r->n_decode * 4 + 16));
-  TRY(ensure(ctx, ctx->decWs, decode_workspace_bytes(r->n_words)));
-  TRY(ensure_host(ctx, ctx->hFlags, 64));
-  cudaStream_t s = ctx->stream;
-  CU(cudaMemcpyAsync(ctx->decWords.p, r->words, (size_t)r->n_words * 4, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(ctx->decTable.p, r->decode, (size_t)r->n_decode * 4, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(ctx->dqtable.p, dq.data(), dq.size() * 4, cudaMemcpyHostToDevice, s));
-  if (r->n_decode == 2 && r->decode[0] == 0 && r->decode[1] != r->dup_key) {
-    fill_value(P<int>(ctx->bins), n, r->decode[1], s);  // one symbol, zero-length code
-  } else {
-    const int rc = decode_stream(P<uint32_t>(ctx->decWords), r->n_words, P<int>(ctx->decTable),
-                                 r->n_decode, r->dup_key, r->dup_value, r->bin_count, n,
-                                 P<int>(ctx->bins), ctx->decWs.p, H<int>(ctx->hFlags), s);
-    if (rc < 0) return fail(ctx, WL_ECUDA, "decode failed: %s", cudaGetErrorString(cudaGetLastError()));
-    if (rc > 0) return fail(ctx, WL_EFORMAT, "corrupt Huffman stream");
-  }
-  ctx->launches = 1;
-  launch_dequant(P<int>(ctx->bins), P<float>(ctx->dqtable), P<float>(ctx->coef), n,
-                 r->bin_count, s);
-  CU(cudaGetLastError());
-  return inverse_impl(ctx, r->size, r->steps, r->wavelet, r->original_size, outType, out,
-                      outOnDevice, r->transform_2d != 0);
+  return decompress_batch_impl(ctx, r, 1, &outType, &out, outOnDevice);
 }
 
 // ---- error metrics (-err) ----------------------------------------------------------
@@ -2025,18 +1997,22 @@ wl_status optimize_impl(wl_ctx *ctx, const void *data, const int size[3], int on
   return WL_OK;
 }
 
-// Decompress n cubelets at once: one copy of all streams, decode tables and
-// dequantization tables; every stream decoded by one set of decoder launches;
-// one dequantization launch; the inverse transform as three phases of
-// concurrent launch groups; the outputs copied back per cubelet.
+// Decompress n cubelets at once: one copy of all streams and one of their
+// records, decode tables and dequantization tables; every stream decoded by
+// one set of launches straight to the dequantized values; the inverse
+// transform as three phases of concurrent launch groups; the outputs copied
+// back per cubelet.  The host waits once, at the end, and looks at the
+// decoder's flags then: a malformed stream is refused, and a batch whose
+// tiles the two checks did not settle is repaired and written again.
 wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const int *outTypes,
                                 void *const *outs, int outOnDevice) {
   CU(cudaSetDevice(ctx->device));
   if (n <= 0) return fail(ctx, WL_EINVAL, "empty batch");
   if (!rs || !outs) return fail(ctx, WL_EINVAL, "null argument");
-  std::vector<long long> N(n), coefOff(n), wordsOff(n), tableOff(n), outOff(n);
+  std::vector<long long> N(n), coefOff(n), wordsOff(n), outOff(n);
   std::vector<int> ot(n);
-  long long coefTotal = 0, wordsTotal = 0, tableTotal = 0, outTotal = 0, totalSub = 0;
+  long long coefTotal = 0, wordsTotal = 0, tableTotal = 0, outTotal = 0, binTotal = 0;
+  long long subTotal = 0, tileTotal = 0, stepTotal = 0;
   int nStreams = 0;
   // results whose words follow each other in memory (the results of one
   // compression call) keep that layout on the device: one copy per run
@@ -2053,62 +2029,45 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
     coefTotal += (N[i] + 63) & ~63LL;
     wordsOff[i] = follows(i) ? wordsOff[i - 1] + rs[i - 1].n_words : (wordsTotal + 3) & ~3LL;
     wordsTotal = wordsOff[i] + r->n_words;
-    tableOff[i] = tableTotal;
     tableTotal += ((long long)r->n_decode + 3) & ~3LL;
+    binTotal += (r->bin_count + 3) & ~3;
     outOff[i] = outTotal;
     outTotal += ((long long)r->original_size[0] * r->original_size[1] * r->original_size[2] *
                      dtype_size(ot[i]) + 255) & ~255LL;
     if (!single_symbol(r)) {
       nStreams++;
-      totalSub += decode_subsequences(r->n_words);
+      subTotal += decode_subs(r->n_words);
+      tileTotal += decode_tiles(r->n_words);
+      stepTotal += decode_steps(r->n_decode);
     }
   }
-  const size_t decWsBytes = decode_batch_workspace_bytes(nStreams, totalSub);
-  const size_t fillOff = (decWsBytes + 255) & ~(size_t)255;
+  if (tileTotal > 0x7fffffffLL) return fail(ctx, WL_EINVAL, "batch too large");
+  // upload block: stream records | fill records | tile map | decode tables |
+  // dequantization tables
+  auto up16 = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t cubAt = 0, fillAt = cubAt + up16((size_t)nStreams * sizeof(DecodeCub)),
+               mapAt = fillAt + up16((size_t)n * sizeof(FillItem)),
+               tabAt = mapAt + up16((size_t)tileTotal * 4),
+               dqAt = tabAt + up16((size_t)tableTotal * 4),
+               upBytes = dqAt + up16((size_t)binTotal * 4);
+  // device scratch of the decoder
+  const size_t lutAt = 0, stepAt = lutAt + up16((size_t)nStreams * decode_lut_size() * 4),
+               offAt = stepAt + up16(decode_step_bytes(stepTotal)),
+               cntAt = offAt + up16((size_t)tileTotal * 8),
+               entAt = cntAt + up16((size_t)subTotal * 4),
+               extAt = entAt + up16((size_t)tileTotal * 4),
+               totAt = extAt + up16((size_t)tileTotal * 4),
+               flagAt = totAt + up16((size_t)tileTotal * 4),
+               subAt = flagAt + 256, wsBytes = subAt + (size_t)subTotal;
   TRY(ensure(ctx, ctx->coef, (size_t)coefTotal * 4 + 256));
   TRY(ensure(ctx, ctx->coef2, (size_t)coefTotal * 4 + 256));
-  TRY(ensure(ctx, ctx->bins, (size_t)coefTotal * 4 + 256));
   TRY(ensure(ctx, ctx->decWords, (size_t)wordsTotal * 4 + 16));
-  TRY(ensure(ctx, ctx->decTable, (size_t)tableTotal * 4 + 16));
-  TRY(ensure(ctx, ctx->dqtable, (size_t)n * kMaxBins * 4));
-  TRY(ensure(ctx, ctx->decWs, fillOff + (size_t)n * sizeof(FillItem)));
+  TRY(ensure(ctx, ctx->decTable, upBytes));
+  TRY(ensure(ctx, ctx->decWs, wsBytes));
   if (!outOnDevice) TRY(ensure(ctx, ctx->outbuf, (size_t)outTotal + 16));
-  TRY(ensure_host(ctx, ctx->hDecode, (size_t)tableTotal * 4 + 16));
-  TRY(ensure_host(ctx, ctx->hVals, (size_t)n * kMaxBins * 4 + (size_t)n * sizeof(FillItem)));
-  TRY(ensure_host(ctx, ctx->hFlags, 64 + (size_t)n * 8));
+  TRY(ensure_host(ctx, ctx->hDecode, upBytes));
+  TRY(ensure_host(ctx, ctx->hFlags, 64));
   cudaStream_t s = ctx->stream;
-  // decode tables and dequantization tables gathered into page-locked staging
-  int *ht = H<int>(ctx->hDecode);
-  float *hq = H<float>(ctx->hVals);
-  // ranges set to one value before decoding: a single-symbol cubelet whole,
-  // and the cubelets with zero runs to the zero bin's value (the decoder
-  // then writes only the other values)
-  FillItem *hfill = reinterpret_cast<FillItem *>(hq + (size_t)n * kMaxBins);
-  int nFill = 0;
-  long long fillBlocks = 0;
-  std::vector<DecodeItem> items;
-  items.reserve(nStreams);
-  for (int i = 0; i < n; i++) {
-    const wl_result *r = rs + i;
-    memcpy(ht + tableOff[i], r->decode, (size_t)r->n_decode * 4);
-    dequant_values(r->quant_alg, r->bin_count, r->threshold_value, r->max_value, r->values,
-                   hq + (size_t)i * kMaxBins);
-    const bool single = single_symbol(r);
-    if (single || r->dup_value >= 0) {
-      const int v = std::min(std::max(single ? r->decode[1] : r->dup_value, 0), r->bin_count - 1);
-      hfill[nFill++] = FillItem{P<float>(ctx->coef) + coefOff[i], N[i],
-                                hq[(size_t)i * kMaxBins + v], fillBlocks};
-      fillBlocks += (N[i] + kFillBlock - 1) / kFillBlock;
-    }
-    if (!single) {
-      DecodeItem it{P<uint32_t>(ctx->decWords) + wordsOff[i], r->n_words,
-                    P<int>(ctx->decTable) + tableOff[i], r->n_decode, r->dup_key,
-                    r->dup_value, r->bin_count, N[i], P<int>(ctx->bins) + coefOff[i]};
-      it.fout = P<float>(ctx->coef) + coefOff[i];
-      it.dq = P<float>(ctx->dqtable) + (size_t)i * kMaxBins;
-      items.push_back(it);
-    }
-  }
   for (int i = 0; i < n;) {  // the words, run by run
     int j = i + 1;
     long long nw = rs[i].n_words;
@@ -2118,24 +2077,60 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
                          cudaMemcpyHostToDevice, s));
     i = j;
   }
-  CU(cudaMemcpyAsync(ctx->decTable.p, ht, (size_t)tableTotal * 4, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(ctx->dqtable.p, hq, (size_t)n * kMaxBins * 4, cudaMemcpyHostToDevice, s));
-  ctx->launches = 0;
-  if (nFill) {
-    FillItem *dfill = reinterpret_cast<FillItem *>(P<char>(ctx->decWs) + fillOff);
-    CU(cudaMemcpyAsync(dfill, hfill, (size_t)nFill * sizeof(FillItem), cudaMemcpyHostToDevice, s));
-    launch_fill_batch(dfill, nFill, fillBlocks, s);
-    ctx->launches++;
+  char *hu = H<char>(ctx->hDecode), *du = P<char>(ctx->decTable), *ws = P<char>(ctx->decWs);
+  DecodeCub *hc = reinterpret_cast<DecodeCub *>(hu + cubAt);
+  // ranges set to one value before decoding: a single-symbol cubelet whole,
+  // and the cubelets with zero runs to the zero bin's value (the decoder
+  // then writes only the other values)
+  FillItem *hfill = reinterpret_cast<FillItem *>(hu + fillAt);
+  int *hmap = reinterpret_cast<int *>(hu + mapAt);
+  int *ht = reinterpret_cast<int *>(hu + tabAt);
+  float *hq = reinterpret_cast<float *>(hu + dqAt);
+  DecodeBatch db{nStreams, (int)tileTotal, 2, 2};
+  int nFill = 0, k = 0;
+  long long fillBlocks = 0, tableOff = 0, binOff = 0, subOff = 0, tileOff = 0, stepOff = 0;
+  for (int i = 0; i < n; i++) {
+    const wl_result *r = rs + i;
+    dequant_values(r->quant_alg, r->bin_count, r->threshold_value, r->max_value, r->values,
+                   hq + binOff);
+    const bool single = single_symbol(r);
+    if (single || r->dup_value >= 0) {
+      const int v = std::min(std::max(single ? r->decode[1] : r->dup_value, 0), r->bin_count - 1);
+      hfill[nFill++] = FillItem{P<float>(ctx->coef) + coefOff[i], N[i], hq[binOff + v], fillBlocks};
+      fillBlocks += (N[i] + kFillBlock - 1) / kFillBlock;
+    }
+    if (!single) {
+      memcpy(ht + tableOff, r->decode, (size_t)r->n_decode * 4);
+      DecodeCub &c = hc[k];
+      c.words = P<uint32_t>(ctx->decWords) + wordsOff[i];
+      c.nWords = r->n_words;
+      c.table = reinterpret_cast<int *>(du + tabAt) + tableOff;
+      c.nTable = r->n_decode;
+      c.dupKey = r->dup_key;
+      c.dupValue = r->dup_value;
+      c.binCount = r->bin_count;
+      c.n = N[i];
+      c.out = P<float>(ctx->coef) + coefOff[i];
+      c.dq = reinterpret_cast<float *>(du + dqAt) + binOff;
+      c.subBase = subOff;
+      c.nSub = decode_subs(r->n_words);
+      c.tileBase = (int)tileOff;
+      c.nTiles = decode_tiles(r->n_words);
+      c.lutOff = (long long)k * decode_lut_size();
+      c.stepOff = stepOff;
+      c.nSteps = decode_steps(r->n_decode);
+      std::fill(hmap + tileOff, hmap + tileOff + c.nTiles, k);
+      subOff += c.nSub;
+      tileOff += c.nTiles;
+      stepOff += c.nSteps;
+      db.maxTable = std::max(db.maxTable, r->n_decode);
+      db.maxBins = std::max(db.maxBins, r->bin_count);
+      k++;
+    }
+    tableOff += ((long long)r->n_decode + 3) & ~3LL;
+    binOff += (r->bin_count + 3) & ~3;
   }
-  if (!items.empty()) {
-    int *hf = H<int>(ctx->hFlags);
-    long long *totals = reinterpret_cast<long long *>(hf + 16);
-    const int rc = decode_streams(items.data(), (int)items.size(), ctx->decWs.p, hf, totals, s);
-    if (rc < 0) return fail(ctx, WL_ECUDA, "decode failed: %s", cudaGetErrorString(cudaGetLastError()));
-    if (rc > 0) return fail(ctx, WL_EFORMAT, "corrupt Huffman stream in the batch");
-    ctx->launches += 5;
-  }
-  CU(cudaGetLastError());
+  CU(cudaMemcpyAsync(du, hu, upBytes, cudaMemcpyHostToDevice, s));
   PassGroups ph[3];
   for (int i = 0; i < n; i++) {
     void *dst = outOnDevice ? outs[i] : (void *)(P<char>(ctx->outbuf) + outOff[i]);
@@ -2143,16 +2138,70 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
                    rs[i].transform_2d != 0, P<float>(ctx->coef) + coefOff[i],
                    P<float>(ctx->coef2) + coefOff[i], dst, ph);
   }
-  TRY(run_inverse_phases(ctx, ph));
-  if (!outOnDevice)
-    for (int i = 0; i < n; i++) {
-      const wl_result *r = rs + i;
-      const size_t bytes = (size_t)r->original_size[0] * r->original_size[1] *
-                           r->original_size[2] * dtype_size(ot[i]);
-      CU(cudaMemcpyAsync(outs[i], P<char>(ctx->outbuf) + outOff[i], bytes,
-                         cudaMemcpyDeviceToHost, s));
+  InversePhases ip;
+  TRY(stage_inverse_phases(ctx, ph, ip));
+
+  const DecodeCub *dc = reinterpret_cast<const DecodeCub *>(du + cubAt);
+  DecodeArrays da;
+  da.lut = reinterpret_cast<unsigned *>(ws + lutAt);
+  da.steps = reinterpret_cast<unsigned *>(ws + stepAt);
+  da.subStart = reinterpret_cast<uint8_t *>(ws + subAt);
+  da.subCount = reinterpret_cast<unsigned *>(ws + cntAt);
+  da.tileCub = reinterpret_cast<const int *>(du + mapAt);
+  da.tileEntry = reinterpret_cast<int *>(ws + entAt);
+  da.tileExit = reinterpret_cast<int *>(ws + extAt);
+  da.tileCount = reinterpret_cast<unsigned *>(ws + totAt);
+  da.tileOff = reinterpret_cast<long long *>(ws + offAt);
+  da.flags = reinterpret_cast<int *>(ws + flagAt);
+  int *hf = H<int>(ctx->hFlags);
+  ctx->launches = 0;
+  auto fill = [&] {
+    if (!nFill) return;
+    launch_fill_batch(reinterpret_cast<const FillItem *>(du + fillAt), nFill, fillBlocks, s);
+    ctx->launches++;
+  };
+  // the values on, and the flags and outputs back
+  auto finish = [&]() -> wl_status {
+    CU(cudaGetLastError());
+    TRY(launch_inverse_phases(ctx, ip));
+    CU(cudaMemcpyAsync(hf, da.flags, kDecodeFlags * 4, cudaMemcpyDeviceToHost, s));
+    if (!outOnDevice)
+      for (int i = 0; i < n; i++) {
+        const wl_result *r = rs + i;
+        const size_t bytes = (size_t)r->original_size[0] * r->original_size[1] *
+                             r->original_size[2] * dtype_size(ot[i]);
+        CU(cudaMemcpyAsync(outs[i], P<char>(ctx->outbuf) + outOff[i], bytes,
+                           cudaMemcpyDeviceToHost, s));
+      }
+    CU(cudaStreamSynchronize(s));
+    return WL_OK;
+  };
+  CU(cudaMemsetAsync(da.flags, 0, kDecodeFlags * 4, s));
+  fill();
+  if (nStreams) ctx->launches += launch_decode(dc, db, da, s);
+  TRY(finish());
+  if (hf[kDecodeAgain] && !hf[kDecodeBad]) {
+    // a chain of tiles took another entry: each check settles at least the
+    // first wrong one, so they end within the longest stream's tile count
+    for (long long round = 0; hf[kDecodeAgain] && round <= tileTotal; round++) {
+      CU(cudaMemsetAsync(da.flags, 0, kDecodeFlags * 4, s));
+      launch_decode_check(dc, db, da, s);
+      ctx->launches++;
+      CU(cudaGetLastError());
+      CU(cudaMemcpyAsync(hf, da.flags, kDecodeFlags * 4, cudaMemcpyDeviceToHost, s));
+      CU(cudaStreamSynchronize(s));
+      if (hf[kDecodeBad]) break;
     }
-  CU(cudaStreamSynchronize(s));
+    if (!hf[kDecodeBad]) {
+      CU(cudaMemsetAsync(da.flags, 0, kDecodeFlags * 4, s));
+      fill();
+      ctx->launches += launch_decode_write(dc, db, da, s);
+      TRY(finish());
+    }
+  }
+  if (hf[kDecodeBad] || hf[kDecodeShort])
+    return fail(ctx, WL_EFORMAT, n == 1 ? "corrupt Huffman stream"
+                                        : "corrupt Huffman stream in the batch");
   return WL_OK;
 }
 
@@ -2321,7 +2370,7 @@ void wl_destroy(wl_ctx *ctx) {
   for (DevBuf *d : dbs) if (d->p) cudaFree(d->p);
   for (GraphEntry &g : ctx->graphs) drop_graph(g);
   HostBuf *hbs[] = {&ctx->hStage[0], &ctx->hStage[1], &ctx->hState, &ctx->hDecode, &ctx->hPasses,
-                    &ctx->hTab, &ctx->hLogHdr, &ctx->hPrefix, &ctx->hIn, &ctx->hVals,
+                    &ctx->hTab, &ctx->hLogHdr, &ctx->hIn,
                     &ctx->hFlags};
   for (HostBuf *h : hbs) if (h->p) cudaFreeHost(h->p);
   for (auto &e : ctx->ev) if (e) cudaEventDestroy(e);

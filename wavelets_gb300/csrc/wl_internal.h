@@ -308,26 +308,57 @@ void launch_huffman_build(DevBatch &b, int maxSymbols, cudaStream_t s);
 void launch_encode(DevBatch &b, int maxSymbols, cudaStream_t s);
 void launch_pack_meta(DevBatch &b, cudaStream_t s);
 
-// GPU Huffman decoding (decode.cu)
-size_t decode_workspace_bytes(long long nWords);
-// batched decoding (decode.cu)
-struct DecodeItem {
+// batched Huffman decoding (decode.cu): the streams of n cubelets to their
+// dequantized values
+struct DecodeCub {
   const uint32_t *words;  // device
   long long nWords;
   const int *table;       // device
   int nTable;
   int dupKey, dupValue, binCount;
   long long n;            // elements
-  int *out;               // device bins
-  // instead of bins: the dequantized values dq[bin] (binCount entries)
-  float *fout = nullptr;
-  const float *dq = nullptr;
+  float *out;             // values; holds dq[dupValue] everywhere when dupValue >= 0
+  const float *dq;        // dequantized value of every bin
+  long long subBase, nSub;   // subsequences (decode_subs)
+  int tileBase, nTiles;      // tiles (decode_tiles)
+  long long lutOff;          // decode_lut_size() entries
+  long long stepOff;         // step tables (decode_steps)
+  int nSteps;
 };
-inline long long decode_subsequences(long long nWords) {
-  const long long k = (nWords * 32 + 1023) / 1024;
-  return k > 0 ? k : 1;
-}
-size_t decode_batch_workspace_bytes(int n, long long totalSub);
+struct DecodeArrays {
+  unsigned *lut, *steps;
+  uint8_t *subStart;      // first token boundary of every subsequence
+  unsigned *subCount;     // elements of every subsequence
+  const int *tileCub;     // cubelet of every tile
+  int *tileEntry, *tileExit;
+  unsigned *tileCount;
+  long long *tileOff;
+  int *flags;             // kDecodeFlags counters, zero before the first launch
+};
+enum {
+  kDecodeFirst, kDecodeAgain,  // tiles decoded again by the first / second check
+  kDecodeBad,                  // malformed streams
+  kDecodeShort,                // streams with fewer values than their cubelet
+  kDecodeFlags
+};
+struct DecodeBatch {
+  int n, tiles;           // streams, tiles in all
+  int maxTable, maxBins;
+};
+long long decode_subs(long long nWords);
+int decode_tiles(long long nWords);
+int decode_lut_size();
+int decode_steps(int nTable);
+size_t decode_step_bytes(long long steps);
+// the whole decode (returns the kernels launched); if flags[kDecodeAgain] is
+// not zero afterwards: zero it and launch_decode_check until it stays zero,
+// then fill the outputs and launch_decode_write again
+int launch_decode(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
+                  cudaStream_t s);
+void launch_decode_check(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
+                         cudaStream_t s);
+int launch_decode_write(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
+                        cudaStream_t s);
 // n floats at out set to v, for many ranges in one launch (blocks of
 // kFillBlock elements; blockBase = the range's first block)
 constexpr int kFillBlock = 4096;
@@ -338,12 +369,6 @@ struct FillItem {
   long long blockBase;
 };
 void launch_fill_batch(const FillItem *items, int nItems, long long totalBlocks, cudaStream_t s);
-int decode_streams(const DecodeItem *items, int n, void *ws, int *hostFlags, long long *hostTotals,
-                   cudaStream_t s);
-int decode_stream(const uint32_t *words, long long nWords, const int *table, int nTable,
-                  int dupKey, int dupValue, int binCount, long long n, int *out, void *ws,
-                  int *hostFlags, cudaStream_t s);
-void fill_value(int *out, long long n, int v, cudaStream_t s);
 
 // host-side exact log-quantizer tables (quant_host.cpp)
 struct LogTable {
