@@ -38,6 +38,11 @@ def _tree(shape):
         for i in range(k - 1, -1, -1):
             t = (i, t)
         return t, k + 1
+    if kind == "keys":      # the zero-run key (last leaf) has the one-bit code
+        t = 0
+        for i in range(1, k + 1):
+            t = (i, t)
+        return t, k + 1
     # mixed: a random tree of k leaves
     rng = np.random.default_rng(k)
     nodes = list(range(k))
@@ -75,6 +80,8 @@ def _stream(shape, bits, runs, seed):
     rng = np.random.default_rng(seed)
     mean = np.mean([len(c) for c in codes.values()])
     syms = rng.integers(0, leaves, max(1, int(bits / mean)))
+    if shape[0] == "keys":  # mostly runs: a tile covers millions of elements
+        syms[rng.random(syms.size) < 0.9] = leaves - 1
     parts = []
     n = 0
     for s in syms:
@@ -90,7 +97,7 @@ def _stream(shape, bits, runs, seed):
     values = np.linspace(-3.0, 5.0, bins).astype(np.float32)
     # the largest box the stream has values for
     x = min(n, 64)
-    y = min(n // x, 128)
+    y = min(n // x, 1024)
     z = n // (x * y)
     c = lib.Compressed((x, y, z), (x, y, z), lib.WL_F32, (0, 0, 0), P.CDF97,
                        P.LLOYD, bins, 0.5, 0.1, 5.0, -3.0, 5.0, max(zero, 0), key, zero,
@@ -100,7 +107,8 @@ def _stream(shape, bits, runs, seed):
     return c, values[want][:x * y * z].reshape(z, y, x)
 
 
-SHAPES = [("flat", 9), ("flat", 8), ("comb", 20), ("comb", 57), ("mixed", 300), ("mixed", 4096)]
+SHAPES = [("flat", 9), ("flat", 8), ("comb", 20), ("comb", 57), ("keys", 8), ("mixed", 300),
+          ("mixed", 4096)]
 LENGTHS = [1, 256, 300, TILE - 40, TILE + 90, 2 * TILE + 5000]
 
 

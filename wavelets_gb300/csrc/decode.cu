@@ -51,6 +51,10 @@ constexpr int kRec = 8;                      // token boundaries kept per specul
 constexpr int kLutBits = 12, kLutSize = 1 << kLutBits;
 constexpr int kStepBits = 4, kStep = 1 << kStepBits;  // longer codes, per step
 constexpr int kMaxCode = 60;                 // longest code accepted
+// step tables kept in shared memory: the first ones built belong to the
+// shortest of the long codes (a global read of a step costs the whole warp
+// several hundred cycles, and with 1024 bins most warps have one per token)
+constexpr int kStageSteps = 128;
 // words of a tile in shared memory: kThreads subsequences of 8 words and the
 // longest token past the end; after every eighth word the next one again, so
 // that words k and k + 1 are always neighbours, which also spreads the
@@ -86,12 +90,23 @@ __device__ __forceinline__ TileAt stage_words(const DecodeCub &c, int tile, uint
   t.tot = (int)min(bits, (long long)2 * kTileBits);
   return t;
 }
-__device__ __forceinline__ void stage_lut(const DecodeCub &c, const unsigned *lut, unsigned *sl) {
-  const uint4 *g = reinterpret_cast<const uint4 *>(lut + c.lutOff);
-  uint4 *s = reinterpret_cast<uint4 *>(sl);
+// A stream's tables for one CTA: the 12-bit table and the first step tables
+// in shared memory, the other step tables in global memory.
+struct Tables {
+  __align__(16) unsigned lut[kLutSize];
+  __align__(16) unsigned steps[kStageSteps * kStep];
+};
+__device__ __forceinline__ void stage_tables(const DecodeCub &c, const DecodeArrays &d, int ci,
+                                             Tables &t) {
+  const uint4 *g = reinterpret_cast<const uint4 *>(d.lut + c.lutOff);
+  uint4 *s = reinterpret_cast<uint4 *>(t.lut);
+  const int n = min(d.stepCount[ci], kStageSteps) * (kStep / 4);
 #pragma unroll
   for (int i = 0; i < kLutSize / 4 / kThreads; i++)
     s[threadIdx.x + i * kThreads] = g[threadIdx.x + i * kThreads];
+  g = reinterpret_cast<const uint4 *>(d.steps + (size_t)c.stepOff * kStep);
+  s = reinterpret_cast<uint4 *>(t.steps);
+  for (int i = threadIdx.x; i < n; i += kThreads) s[i] = g[i];
 }
 __device__ __forceinline__ unsigned bits_at(const uint32_t *sw, int p) {
   const int k = p >> 5, a = k + (k >> 3);
@@ -100,8 +115,9 @@ __device__ __forceinline__ unsigned bits_at(const uint32_t *sw, int p) {
 
 // a code longer than the table, or a zero-run key whose length bits are
 // outside it; returns the bits consumed, 0 when malformed
-__device__ __noinline__ int slow_token(const uint32_t *sw, const unsigned *steps, int p,
-                                       unsigned e, int dupValue, int &lg, int &sym) {
+__device__ __noinline__ int slow_token(const uint32_t *sw, const unsigned *near,
+                                       const unsigned *steps, int p, unsigned e, int dupValue,
+                                       int &lg, int &sym) {
   int used = 0, width = kLutBits;
   while (e & kSlow) {
     if (e & kRun) {
@@ -113,7 +129,9 @@ __device__ __noinline__ int slow_token(const uint32_t *sw, const unsigned *steps
     }
     used += width;
     width = kStepBits;
-    e = steps[(e & 0xffffu) * kStep + (bits_at(sw, p + used) & (kStep - 1))];
+    const unsigned slot = e & 0xffffu;
+    const unsigned at = slot * kStep + (bits_at(sw, p + used) & (kStep - 1));
+    e = slot < kStageSteps ? near[at] : steps[at];
   }
   lg = (int)((e >> 6) & 15u);
   sym = (int)((e >> 10) & 0x1fffu);
@@ -121,19 +139,19 @@ __device__ __noinline__ int slow_token(const uint32_t *sw, const unsigned *steps
 }
 
 // one token at bit p of the staged words: bits consumed (0: malformed)
-__device__ __forceinline__ int token_at(const uint32_t *sw, const unsigned *sl,
+__device__ __forceinline__ int token_at(const uint32_t *sw, const Tables &t,
                                         const unsigned *steps, int p, int dupValue, int &lg,
                                         int &sym) {
-  const unsigned e = sl[bits_at(sw, p) & (kLutSize - 1)];
-  if (e & kSlow) return slow_token(sw, steps, p, e, dupValue, lg, sym);
+  const unsigned e = t.lut[bits_at(sw, p) & (kLutSize - 1)];
+  if (e & kSlow) return slow_token(sw, t.steps, steps, p, e, dupValue, lg, sym);
   lg = (int)((e >> 6) & 15u);
   sym = (int)((e >> 10) & 0x1fffu);
   return (int)(e & 63u);
 }
 
 struct TileSmem {
+  Tables tab;
   uint32_t sw[kStageSize];
-  __align__(16) unsigned lut[kLutSize];
   unsigned rec[kRec][kThreads];
   int exits[kThreads];
   unsigned sums[kThreads / 32];
@@ -147,7 +165,7 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
   constexpr unsigned kAll = 0xffffffffu;
   const int tile = t - c.tileBase, tid = threadIdx.x;
   const TileAt at = stage_words(c, tile, sm.sw);
-  stage_lut(c, d.lut, sm.lut);
+  stage_tables(c, d, d.tileCub[t], sm.tab);
   __syncthreads();
   const unsigned *steps = d.steps + (size_t)c.stepOff * kStep;
   const long long sub = (long long)tile * kTileSubs + tid - 1;  // subsequence of the stream
@@ -162,7 +180,7 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
     unsigned r = ~0u;
     if (active && !bad && p < lim) {
       int lg, sym;
-      const int used = token_at(sm.sw, sm.lut, steps, p, c.dupValue, lg, sym);
+      const int used = token_at(sm.sw, sm.tab, steps, p, c.dupValue, lg, sym);
       bad = used == 0;
       if (!bad) {
         p += used;
@@ -174,7 +192,7 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
   }
   while (active && !bad && p < lim) {
     int lg, sym;
-    const int used = token_at(sm.sw, sm.lut, steps, p, c.dupValue, lg, sym);
+    const int used = token_at(sm.sw, sm.tab, steps, p, c.dupValue, lg, sym);
     if (used == 0) { bad = true; break; }
     p += used;
     n += 1u << lg;
@@ -211,7 +229,7 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
         }
         if (bad || q >= lim) break;
         int lg, sym;
-        const int used = token_at(sm.sw, sm.lut, steps, q, c.dupValue, lg, sym);
+        const int used = token_at(sm.sw, sm.tab, steps, q, c.dupValue, lg, sym);
         if (used == 0) { bad = true; break; }
         q += used;
         m += 1u << lg;
@@ -304,15 +322,19 @@ __global__ void __launch_bounds__(kThreads) scan_kernel(const DecodeCub *__restr
 }
 
 struct WriteSmem {
+  Tables tab;
   uint32_t sw[kStageSize];
-  __align__(16) unsigned lut[kLutSize];
   unsigned sums[kThreads / 32];
   float dq[1];  // binCount entries
 };
 
 // The values, from each subsequence's true start.  With zero runs
-// (dupValue >= 0) the output already holds the zero bin's value everywhere
-// (launch_fill_batch), so only the other values are written.
+// (dupValue >= 0) only the other values are written one by one; the zero
+// bin's value is set before: by this CTA over its tile's output range
+// (DecodeCub::fill), so that the scattered values land in lines still in L2,
+// or, where a tile covers so much output that one CTA would be long at it, by
+// launch_fill_batch.  Filling everything first cost the mixed batch (1.5 GB
+// of output) 252 us and 48 us more in this kernel.
 __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__restrict__ cubs,
                                                          DecodeArrays d) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -324,7 +346,7 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__rest
   if (tileOff >= c.n) return;  // padding bits after the last value
   const int tile = t - c.tileBase;
   const TileAt at = stage_words(c, tile, sm.sw);
-  stage_lut(c, d.lut, sm.lut);
+  stage_tables(c, d, d.tileCub[t], sm.tab);
   for (int i = tid; i < c.binCount; i += kThreads) sm.dq[i] = c.dq[i];
   const long long sub = (long long)tile * kTileSubs + tid - 1;
   const bool active = tid > 0 && sub < c.nSub;
@@ -341,16 +363,28 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__rest
   unsigned before = inc - n;
 #pragma unroll
   for (int k = 0; k < kThreads / 32; k++) before += k < w ? sm.sums[k] : 0u;
-  if (!active) return;
   const long long room = c.n - tileOff;  // elements from the tile's first on
   const unsigned end = (unsigned)min(room, (long long)0xffffffffu);
+  if (c.fill) {
+    const float v = sm.dq[min(c.dupValue, c.binCount - 1)];
+    float *g = c.out + tileOff;
+    const int total = (int)min(end, d.tileCount[t]);
+    const int head = min((int)((16 - (reinterpret_cast<size_t>(g) & 15)) & 15) / 4, total);
+    const int quads = (total - head) / 4, tail = head + 4 * quads;
+    if (tid < head) g[tid] = v;
+    float4 *g4 = reinterpret_cast<float4 *>(g + head);
+    for (int i = tid; i < quads; i += kThreads) g4[i] = make_float4(v, v, v, v);
+    if (tid < total - tail) g[tail + tid] = v;
+    __syncthreads();  // the values below come after
+  }
+  if (!active) return;
   const int lim = min(tid * kSubBits + kSubBits, at.tot);
   const unsigned *steps = d.steps + (size_t)c.stepOff * kStep;
   float *F = c.out + tileOff;
   unsigned o = before;
   while (p < lim && o < end) {
     int lg, sym;
-    const int used = token_at(sm.sw, sm.lut, steps, p, c.dupValue, lg, sym);
+    const int used = token_at(sm.sw, sm.tab, steps, p, c.dupValue, lg, sym);
     if (used == 0) break;
     p += used;
     if (sym != c.dupValue) F[o] = sm.dq[min(sym, c.binCount - 1)];
@@ -425,6 +459,7 @@ __global__ void __launch_bounds__(1024) build_lut_kernel(const DecodeCub *__rest
     head = tail;
     above += kStepBits;
   }
+  if (threadIdx.x == 0) d.stepCount[blockIdx.x] = min(nSlots, c.nSteps);
 }
 
 __global__ void __launch_bounds__(256) fill_batch_kernel(const FillItem *__restrict__ items,

@@ -2057,7 +2057,8 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
                entAt = cntAt + up16((size_t)subTotal * 4),
                extAt = entAt + up16((size_t)tileTotal * 4),
                totAt = extAt + up16((size_t)tileTotal * 4),
-               flagAt = totAt + up16((size_t)tileTotal * 4),
+               scntAt = totAt + up16((size_t)tileTotal * 4),
+               flagAt = scntAt + up16((size_t)nStreams * 4),
                subAt = flagAt + 256, wsBytes = subAt + (size_t)subTotal;
   TRY(ensure(ctx, ctx->coef, (size_t)coefTotal * 4 + 256));
   TRY(ensure(ctx, ctx->coef2, (size_t)coefTotal * 4 + 256));
@@ -2080,8 +2081,8 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
   char *hu = H<char>(ctx->hDecode), *du = P<char>(ctx->decTable), *ws = P<char>(ctx->decWs);
   DecodeCub *hc = reinterpret_cast<DecodeCub *>(hu + cubAt);
   // ranges set to one value before decoding: a single-symbol cubelet whole,
-  // and the cubelets with zero runs to the zero bin's value (the decoder
-  // then writes only the other values)
+  // and sparse cubelets with zero runs to the zero bin's value (the decoder
+  // then writes only the other values; it fills the denser ones itself)
   FillItem *hfill = reinterpret_cast<FillItem *>(hu + fillAt);
   int *hmap = reinterpret_cast<int *>(hu + mapAt);
   int *ht = reinterpret_cast<int *>(hu + tabAt);
@@ -2094,7 +2095,10 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
     dequant_values(r->quant_alg, r->bin_count, r->threshold_value, r->max_value, r->values,
                    hq + binOff);
     const bool single = single_symbol(r);
-    if (single || r->dup_value >= 0) {
+    // the zero bin's value: by the decoder, or beforehand
+    const bool fillHere = !single && r->dup_value >= 0 &&
+                          N[i] <= kDecodeFillTile * decode_tiles(r->n_words);
+    if (single || (r->dup_value >= 0 && !fillHere)) {
       const int v = std::min(std::max(single ? r->decode[1] : r->dup_value, 0), r->bin_count - 1);
       hfill[nFill++] = FillItem{P<float>(ctx->coef) + coefOff[i], N[i], hq[binOff + v], fillBlocks};
       fillBlocks += (N[i] + kFillBlock - 1) / kFillBlock;
@@ -2111,6 +2115,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
       c.binCount = r->bin_count;
       c.n = N[i];
       c.out = P<float>(ctx->coef) + coefOff[i];
+      c.fill = fillHere ? 1 : 0;
       c.dq = reinterpret_cast<float *>(du + dqAt) + binOff;
       c.subBase = subOff;
       c.nSub = decode_subs(r->n_words);
@@ -2152,6 +2157,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
   da.tileExit = reinterpret_cast<int *>(ws + extAt);
   da.tileCount = reinterpret_cast<unsigned *>(ws + totAt);
   da.tileOff = reinterpret_cast<long long *>(ws + offAt);
+  da.stepCount = reinterpret_cast<int *>(ws + scntAt);
   da.flags = reinterpret_cast<int *>(ws + flagAt);
   int *hf = H<int>(ctx->hFlags);
   ctx->launches = 0;

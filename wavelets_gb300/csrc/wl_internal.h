@@ -317,7 +317,9 @@ struct DecodeCub {
   int nTable;
   int dupKey, dupValue, binCount;
   long long n;            // elements
-  float *out;             // values; holds dq[dupValue] everywhere when dupValue >= 0
+  float *out;             // values
+  int fill;               // dupValue >= 0: 1: the decoder sets dq[dupValue] everywhere
+                          // first, 0: the output holds it already
   const float *dq;        // dequantized value of every bin
   long long subBase, nSub;   // subsequences (decode_subs)
   int tileBase, nTiles;      // tiles (decode_tiles)
@@ -325,8 +327,11 @@ struct DecodeCub {
   long long stepOff;         // step tables (decode_steps)
   int nSteps;
 };
+// elements of a tile's output up to which the decoder fills it itself
+constexpr long long kDecodeFillTile = 1 << 20;
 struct DecodeArrays {
   unsigned *lut, *steps;
+  int *stepCount;         // step tables of every stream
   uint8_t *subStart;      // first token boundary of every subsequence
   unsigned *subCount;     // elements of every subsequence
   const int *tileCub;     // cubelet of every tile
