@@ -292,6 +292,8 @@ struct GraphEntry {
   unsigned long long lastUse = 0;
 };
 constexpr size_t kGraphCache = 4;
+// largest slab a call's results are delivered to by a kernel
+constexpr size_t kDeliverMax = (size_t)8 << 20;
 }  // namespace
 
 struct wl_ctx {
@@ -300,9 +302,9 @@ struct wl_ctx {
   std::string err;
   DevBuf input, coef, coef2, bins, tokCount, state, selHist, lloydHist, qtable, dqtable, qlut,
       hist, chunkRun, chunkBits, chunkCub, groupCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
-      words, passes, logHdr, outbuf, decWords, decTable, decWs, meta, optIn, optOut, optErr,
+      words, passes, outbuf, head, decWords, decTable, decWs, meta, optIn, optOut, optErr,
       errIn, errRest, errPart;
-  HostBuf hState, hDecode, hPasses, hTab, hLogHdr, hIn, hFlags;
+  HostBuf hState, hDecode, hPasses, hTab, hIn, hFlags, hHead, hSel;
   HostBuf hStage[2];  // staging buffers of the container pipeline
   // CUDA graphs: 0 = off, 1 = capture a batch geometry seen twice in a row
   // and replay it from then on
@@ -334,6 +336,7 @@ struct wl_ctx {
   cudaEvent_t pev[10] = {};
   float ktimes[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   int launches = 0;
+  size_t outBytes = 0;     // result bytes of the last call delivered by a kernel
   size_t devBytes = 0;     // device workspace held (grow-only buffers)
   size_t memLimit = 0;     // wl_set_memory_limit (0: none)
 };
@@ -970,7 +973,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   TRY(ensure(ctx, ctx->sliceOff, chunkTotal * 32 * sizeof(unsigned)));
   TRY(ensure(ctx, ctx->selHist, (size_t)n * kSelectBins * 4));
   if (anyLloyd) TRY(ensure(ctx, ctx->lloydHist, (size_t)n * kLloydBins * 4));
-  TRY(ensure(ctx, ctx->qtable, (size_t)tableTotal * 4));
+  // log table headers, then the quantizer tables
+  const size_t hdrBytes = ((size_t)n * sizeof(int4) + 255) & ~(size_t)255;
+  TRY(ensure(ctx, ctx->qtable, hdrBytes + (size_t)tableTotal * 4));
   if (anyLloyd) TRY(ensure(ctx, ctx->qlut, (size_t)n * kLutStride * 2));
   TRY(ensure(ctx, ctx->dqtable, (size_t)n * kMaxBins * 4));
   TRY(ensure(ctx, ctx->hist, (size_t)n * kMaxSymbols * 8));
@@ -981,18 +986,21 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   TRY(ensure(ctx, ctx->codeLen, (size_t)n * kMaxSymbols));
   TRY(ensure(ctx, ctx->decode, (size_t)n * 4 * kMaxSymbols * 4));
   TRY(ensure(ctx, ctx->words, wordsTotal * 4));
-  TRY(ensure(ctx, ctx->logHdr, n * sizeof(int4)));
+  TRY(ensure(ctx, ctx->head, kHeadCount * sizeof(long long)));
   TRY(ensure(ctx, ctx->meta, (size_t)n * (4 * kMaxSymbols + 2 * kMaxBins) * 4));
-  // upload block: cubelet records | chunk prefix | transform pass groups
+  // upload block: result slab | cubelet records | chunk prefix | transform
+  // pass groups
+  const size_t slabBytes = 256;
   const size_t cubBytes = ((size_t)n * sizeof(CubeletDev) + 255) & ~(size_t)255;
   const size_t prefBytes = ((size_t)n * sizeof(long long) + 255) & ~(size_t)255;
   const size_t passBytes =
-      cubBytes + prefBytes + (size_t)3 * n * (sizeof(PassDesc) + sizeof(int) + 260) + 4096;
+      slabBytes + cubBytes + prefBytes + (size_t)3 * n * (sizeof(PassDesc) + sizeof(int) + 260) + 4096;
   TRY(ensure(ctx, ctx->passes, passBytes));
   TRY(ensure_host(ctx, ctx->hPasses, passBytes));
   TRY(ensure_host(ctx, ctx->hState, n * sizeof(CubeletState)));
-  TRY(ensure_host(ctx, ctx->hLogHdr, n * sizeof(int4)));
-  if (anyLog) TRY(ensure_host(ctx, ctx->hTab, (size_t)tableTotal * 4));
+  TRY(ensure_host(ctx, ctx->hHead, kHeadCount * sizeof(long long)));
+  if (anyLog) TRY(ensure_host(ctx, ctx->hSel, (size_t)n * sizeof(float2)));
+  if (anyLog) TRY(ensure_host(ctx, ctx->hTab, hdrBytes + (size_t)tableTotal * 4));
 
   cudaStream_t s = ctx->stream;
   CU(cudaEventRecord(ctx->ev[0], s));
@@ -1000,6 +1008,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   // ---- inputs ----
   std::vector<const void *> dIn(n);
   std::vector<char> hostIn(n, 0);  // input read in place from page-locked host memory
+  bool stagedInput = false;
   if (onDevice) {
     for (int i = 0; i < n; i++) dIn[i] = plans[i].data;
   } else {
@@ -1023,6 +1032,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
         staged = true;
       }
     }
+    stagedInput = staged;
     if (staged) TRY(ensure(ctx, ctx->input, inBytes));
     for (int i = 0; i < n; i++) {
       if (dIn[i]) continue;
@@ -1059,6 +1069,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     }
   }
 
+  if (stagedInput) CU(cudaEventRecord(ctx->ev[1], s));
+
   // ---- halves ----
   // A large batch runs as two halves (cubelets [0, cut) and [cut, n), cut at
   // half of the padded elements) on two streams: the second half's transform
@@ -1082,8 +1094,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   auto half_of = [&](int i) { return i < cut ? 0 : 1; };
 
   // ---- descriptors (host side of the upload block) ----
-  CubeletDev *hc = H<CubeletDev>(ctx->hPasses);
-  long long *hp = reinterpret_cast<long long *>(H<char>(ctx->hPasses) + cubBytes);
+  CubeletDev *hc = reinterpret_cast<CubeletDev *>(H<char>(ctx->hPasses) + slabBytes);
+  long long *hp = reinterpret_cast<long long *>(H<char>(ctx->hPasses) + slabBytes + cubBytes);
   long long groupTotal = 0, encTotal = 0;
   long long chunk0[2] = {0, 0}, group0[2] = {0, 0}, words0[2] = {0, 0}, enc0[2] = {0, 0};
   long long wordsAcc = 0;
@@ -1132,7 +1144,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   DevBatch b;
   memset(&b, 0, sizeof b);
   b.n = n;
-  b.cub = reinterpret_cast<CubeletDev *>(P<char>(ctx->passes));
+  b.cub = reinterpret_cast<CubeletDev *>(P<char>(ctx->passes) + slabBytes);
   b.state = P<CubeletState>(ctx->state);
   b.coef = P<float>(ctx->coef);
   b.coef2 = P<float>(ctx->coef2);
@@ -1140,7 +1152,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.chunkTok = P<int>(ctx->tokCount);
   b.selHist = P<unsigned>(ctx->selHist);
   b.lloydHist = P<float>(ctx->lloydHist);
-  b.qtable = P<float>(ctx->qtable);
+  b.qtable = reinterpret_cast<float *>(P<char>(ctx->qtable) + hdrBytes);
   b.qlut = P<uint16_t>(ctx->qlut);
   b.dqtable = P<float>(ctx->dqtable);
   b.hist = P<unsigned long long>(ctx->hist);
@@ -1151,7 +1163,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.codeLen = P<uint8_t>(ctx->codeLen);
   b.decode = P<int>(ctx->decode);
   b.words = P<uint32_t>(ctx->words);
-  b.chunkPrefix = reinterpret_cast<long long *>(P<char>(ctx->passes) + cubBytes);
+  b.chunkPrefix = reinterpret_cast<long long *>(P<char>(ctx->passes) + slabBytes + cubBytes);
   b.chunkCub = P<int>(ctx->chunkCub);
   b.groupCub = P<int>(ctx->groupCub);
   b.totalGroups = groupTotal;
@@ -1160,7 +1172,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.totalEnc = encTotal;
   b.encF = encF[0];
   b.sliceOff = P<unsigned>(ctx->sliceOff);
-  b.logHdr = P<int4>(ctx->logHdr);
+  b.logHdr = P<int4>(ctx->qtable);
   b.meta = P<int>(ctx->meta);
   b.totalChunks = chunkTotal;
   int maxChunks[2] = {0, 0};
@@ -1169,6 +1181,20 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     m = std::max(m, plans[i].nChunks);
   }
   b.maxChunks = maxChunks[0];
+  b.head = P<long long>(ctx->head);
+  b.hostSel = anyLog ? H<float2>(ctx->hSel) : nullptr;
+  // Small results go to the host by a kernel at the end of the call, into a
+  // slab acquired beforehand: room for a quarter more than the last such
+  // call's and at most what the streams can take.  Larger ones are copied by
+  // the copy engine once the host knows their size.
+  size_t outCap = std::max<size_t>((size_t)1 << 20, ctx->outBytes + ctx->outBytes / 4);
+  outCap = std::min(outCap, (size_t)wordsTotal * 4 + (size_t)n * (4 * kMaxSymbols + 2 * kMaxBins) * 4);
+  const bool deliver = nh == 1 && !coefOut && outCap <= kDeliverMax;
+  b.outSlab = reinterpret_cast<const OutSlab *>(P<char>(ctx->passes));
+  if (deliver) {
+    b.hostState = H<CubeletState>(ctx->hState);
+    b.hostHead = H<long long>(ctx->hHead);
+  }
   constexpr long long kMetaPer = 4LL * kMaxSymbols + 2LL * kMaxBins;  // ints per cubelet
   DevBatch bh[2] = {b, b};
   if (nh == 2) {
@@ -1188,6 +1214,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       v.codeLen += (size_t)c0 * kMaxSymbols;
       v.decode += (size_t)c0 * 4 * kMaxSymbols;
       v.logHdr += c0;
+      if (v.hostSel) v.hostSel += c0;
+      if (h) v.head = nullptr;
       v.chunkPrefix += c0;
       v.chunkTok += ch;
       v.chunkSpan += ch;
@@ -1219,7 +1247,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     pass0[h] |= !fused;
   }
   std::vector<GroupLaunch> gl;
-  size_t hoff = cubBytes + prefBytes;
+  size_t hoff = slabBytes + cubBytes + prefBytes;
   size_t gb[2][4];  // per half: group index bounds of the x, y, z phases
   for (int h = 0; h < nh; h++) {
     gb[h][0] = gl.size();
@@ -1240,7 +1268,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   auto post = [&](int h, cudaStream_t st) -> wl_status {
     DevBatch &v = bh[h];
     const bool first = h == 0;
-    if (first) CU(record(ctx, ctx->ev[2]));
     launch_quant_params(v, st);
     ctx->launches += 1;
     if (anyLloyd) { launch_lloyd(v, v.coef, maxLloyd, st); ctx->launches += 3; }
@@ -1251,18 +1278,16 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     ctx->launches += 2;
     if (first) mark(ctx, 7);
     CU(cudaGetLastError());
-    if (first) CU(record(ctx, ctx->ev[3]));
     launch_huffman_build(v, maxS, st);
     ctx->launches += 1;
     if (first) mark(ctx, 8);
     CU(cudaGetLastError());
-    if (first) CU(record(ctx, ctx->ev[4]));
     launch_encode(v, maxS, st);
-    launch_pack_meta(v, st);
+    if (deliver) launch_deliver(v, st);
+    else launch_pack_meta(v, st);
     ctx->launches += 6;
     if (first) mark(ctx, 9);
     CU(cudaGetLastError());
-    if (first) CU(record(ctx, ctx->ev[5]));
     return WL_OK;
   };
   // the second half's stream joins the context's stream
@@ -1273,11 +1298,19 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     }
     return WL_OK;
   };
+  // the states and the marks, where no kernel delivered them
+  auto states_back = [&]() -> wl_status {
+    if (deliver) return WL_OK;
+    CU(cudaMemcpyAsync(ctx->hState.p, ctx->state.p, n * sizeof(CubeletState),
+                       cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(ctx->hHead.p, ctx->head.p, kHeadCount * sizeof(long long),
+                       cudaMemcpyDeviceToHost, s));
+    return WL_OK;
+  };
   auto quantize_to_end = [&]() -> wl_status {
     if (anyLog) {
-      CU(cudaMemcpyAsync(ctx->qtable.p, ctx->hTab.p, (size_t)tableTotal * 4,
+      CU(cudaMemcpyAsync(ctx->qtable.p, ctx->hTab.p, hdrBytes + (size_t)tableTotal * 4,
                          cudaMemcpyHostToDevice, s));
-      CU(cudaMemcpyAsync(ctx->logHdr.p, ctx->hLogHdr.p, n * sizeof(int4), cudaMemcpyHostToDevice, s));
       if (nh == 2) {  // the second half starts once the tables are on the device
         CU(cudaEventRecord(ctx->halfT, s));
         CU(cudaStreamWaitEvent(s2, ctx->halfT, 0));
@@ -1286,22 +1319,17 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     TRY(post(0, s));
     if (nh == 2) TRY(post(1, s2));
     TRY(join());
-    CU(cudaMemcpyAsync(ctx->hState.p, ctx->state.p, n * sizeof(CubeletState),
-                       cudaMemcpyDeviceToHost, s));
-    return WL_OK;
+    return states_back();
   };
   auto transform_select = [&]() -> wl_status {
     CU(cudaMemcpyAsync(ctx->passes.p, ctx->hPasses.p, upBytes, cudaMemcpyHostToDevice, s));
-    CU(cudaMemsetAsync(ctx->state.p, 0, n * sizeof(CubeletState), s));
-    CU(cudaMemsetAsync(ctx->selHist.p, 0, (size_t)n * kSelectBins * 4, s));
-    CU(cudaMemsetAsync(ctx->hist.p, 0, (size_t)n * kMaxSymbols * 8, s));
-    if (anyLloyd) CU(cudaMemsetAsync(ctx->lloydHist.p, 0, (size_t)n * kLloydBins * 4, s));
-    launch_select_init(b, s);
-    ctx->launches += 1;
     if (nh == 2) {  // the second half starts with the first
       CU(cudaEventRecord(ctx->halfT, s));
       CU(cudaStreamWaitEvent(s2, ctx->halfT, 0));
+      launch_init(bh[1], anyLloyd, s2);
     }
+    launch_init(bh[0], anyLloyd, s);
+    ctx->launches += nh;
     mark(ctx, 0);
     TRY(launch_phase(ctx, gl, gb[0][0], gb[0][1]));
     mark(ctx, 1);
@@ -1309,7 +1337,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     mark(ctx, 2);
     TRY(launch_phase(ctx, gl, gb[0][2], gb[0][3]));
     mark(ctx, 3);
-    CU(record(ctx, ctx->ev[1]));
     if (nh == 2) {
       for (int ph = 0; ph < 3; ph++)
         TRY(launch_phase_on(ctx, gl, gb[1][ph], gb[1][ph + 1], s2, ctx->side2, ctx->fork2,
@@ -1317,25 +1344,18 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     }
     if (coefOut) return WL_OK;
     launch_select(bh[0], bh[0].coef, pass0[0], s);
-    ctx->launches += pass0[0] ? 8 : 7;
+    ctx->launches += pass0[0] ? 7 : 6;
     if (nh == 2) {
       launch_select(bh[1], bh[1].coef, pass0[1], s2);
-      ctx->launches += pass0[1] ? 8 : 7;
+      ctx->launches += pass0[1] ? 7 : 6;
     }
     CU(cudaGetLastError());
     mark(ctx, 4);
-    if (anyLog) {
-      TRY(join());
-      CU(cudaMemcpyAsync(ctx->hState.p, ctx->state.p, n * sizeof(CubeletState),
-                         cudaMemcpyDeviceToHost, s));
-    } else {
-      if (nh == 2) TRY(post(1, s2));
-      TRY(post(0, s));
-      TRY(join());
-      CU(cudaMemcpyAsync(ctx->hState.p, ctx->state.p, n * sizeof(CubeletState),
-                         cudaMemcpyDeviceToHost, s));
-    }
-    return WL_OK;
+    if (anyLog) return join();  // the select wrote hSel
+    if (nh == 2) TRY(post(1, s2));
+    TRY(post(0, s));
+    TRY(join());
+    return states_back();
   };
 
   GraphEntry *ge = nullptr;
@@ -1344,7 +1364,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     std::vector<long long> key;
     key.reserve(4 + (size_t)n * 18);
     key.push_back(n);
-    key.push_back(onDevice | (ctx->profiling ? 2 : 0) | (nh == 2 ? 4 : 0));
+    key.push_back(onDevice | (ctx->profiling ? 2 : 0) | (nh == 2 ? 4 : 0) | (deliver ? 8 : 0));
     key.push_back((long long)tune_version());
     key.push_back(ctx->encSlices);
     for (int i = 0; i < n; i++) {
@@ -1359,6 +1379,18 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       key.insert(key.end(), v, v + sizeof v / sizeof v[0]);
     }
     ge = graph_for(ctx, std::move(key));
+  }
+
+  // the slab a call holds until its results take it over
+  struct SlabHold {
+    ResultSlab *p = nullptr;
+    ~SlabHold() { if (p) slab_pool().release(p); }
+  } slab;
+  if (deliver) {
+    slab.p = slab_pool().acquire(outCap);
+    if (!slab.p) return fail(ctx, WL_ENOMEM, "cannot allocate %zu bytes of page-locked result storage",
+                             outCap);
+    *H<OutSlab>(ctx->hPasses) = OutSlab{slab.p->base, (long long)slab.p->cap};
   }
 
   // ---- transform ----
@@ -1376,9 +1408,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   // ---- log quantizer tables (host logf) ----
   if (anyLog) {
     CU(cudaStreamSynchronize(s));
-    const CubeletState *hs = H<CubeletState>(ctx->hState);
-    float *tab = H<float>(ctx->hTab);
-    int4 *lh = H<int4>(ctx->hLogHdr);
+    const float2 *sel = H<float2>(ctx->hSel);
+    int4 *lh = H<int4>(ctx->hTab);
+    float *tab = reinterpret_cast<float *>(H<char>(ctx->hTab) + hdrBytes);
     // one table per log cubelet, independent: spread over host threads
     std::vector<int> logIdx;
     for (int i = 0; i < n; i++) {
@@ -1389,7 +1421,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     const std::function<void(int)> one = [&](int k) {
       LogTable t;
       const int i = logIdx[k];
-      log_quant_table(plans[i].p.bin_count, hs[i].threshold, hs[i].maxAbs, t);
+      log_quant_table(plans[i].p.bin_count, sel[i].x, sel[i].y, t);
       if (t.nPos + t.nNeg > 2 * plans[i].p.bin_count) {
         bad.store(i);
         return;
@@ -1405,6 +1437,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   }
 
   // ---- results ----
+  if (deliver) CU(cudaEventRecord(ctx->ev[6], s));
   CU(cudaStreamSynchronize(s));
   const CubeletState *hs = H<CubeletState>(ctx->hState);
   long long hw0[3] = {0, 0, 0};  // words of each half, then their sum
@@ -1422,23 +1455,30 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   const size_t metaInts = hm0[0] + hm0[1];
   // words, then the packed decode tables and codebooks, straight into the slab
   const size_t wordsBytes = ((size_t)totalWords * 4 + 15) & ~(size_t)15;
-  ResultSlab *slab = slab_pool().acquire(wordsBytes + metaInts * 4 + 16);
-  if (!slab) return fail(ctx, WL_ENOMEM, "cannot allocate %zu bytes of page-locked result storage",
-                         wordsBytes + metaInts * 4 + 16);
-  uint32_t *hw = reinterpret_cast<uint32_t *>(slab->base);
-  int *hd = reinterpret_cast<int *>(slab->base + wordsBytes);
+  const long long *head = H<long long>(ctx->hHead);
+  const bool delivered = deliver && head[kHeadDelivered] != 0;
+  if (nh == 1) ctx->outBytes = wordsBytes + metaInts * 4;
+  if (!delivered) {
+    if (slab.p) slab_pool().release(slab.p);
+    slab.p = slab_pool().acquire(wordsBytes + metaInts * 4 + 16);
+    if (!slab.p) return fail(ctx, WL_ENOMEM, "cannot allocate %zu bytes of page-locked result storage",
+                             wordsBytes + metaInts * 4 + 16);
+  }
+  uint32_t *hw = reinterpret_cast<uint32_t *>(slab.p->base);
+  int *hd = reinterpret_cast<int *>(slab.p->base + wordsBytes);
   const long long wAt[2] = {0, hw0[0]};
   const size_t mAt[2] = {0, hm0[0]};
-  for (int h = 0; h < nh; h++) {
-    if (hw0[h]) {
-      const cudaError_t e = cudaMemcpyAsync(hw + wAt[h], bh[h].words, (size_t)hw0[h] * 4,
-                                            cudaMemcpyDeviceToHost, s);
-      if (e != cudaSuccess) { slab_pool().release(slab); CU(e); }
+  if (!delivered) {
+    if (deliver) {  // did not fit: the kernel left the metadata unpacked
+      launch_pack_meta(bh[0], s);
+      ctx->launches++;
+      CU(cudaGetLastError());
     }
-    if (hm0[h]) {
-      const cudaError_t e = cudaMemcpyAsync(hd + mAt[h], bh[h].meta, hm0[h] * 4,
-                                            cudaMemcpyDeviceToHost, s);
-      if (e != cudaSuccess) { slab_pool().release(slab); CU(e); }
+    for (int h = 0; h < nh; h++) {
+      if (hw0[h])
+        CU(cudaMemcpyAsync(hw + wAt[h], bh[h].words, (size_t)hw0[h] * 4, cudaMemcpyDeviceToHost, s));
+      if (hm0[h])
+        CU(cudaMemcpyAsync(hd + mAt[h], bh[h].meta, hm0[h] * 4, cudaMemcpyDeviceToHost, s));
     }
   }
   std::vector<size_t> decOff(n), cbOff(n, 0), wOff(n);
@@ -1448,19 +1488,18 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     cbOff[i] = decOff[i] + hs[i].nDecode;
     wOff[i] = (size_t)(wAt[h] + hs[i].wordsBase);
   }
-  {
-    cudaError_t e = cudaEventRecord(ctx->ev[6], s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { slab_pool().release(slab); CU(e); }
+  if (!delivered) {
+    CU(cudaEventRecord(ctx->ev[6], s));
+    CU(cudaStreamSynchronize(s));
   }
-  slab->refs.store(n);
+  slab.p->refs.store(n);
+  ResultSlab *const owner = slab.p;
+  slab.p = nullptr;
 
-  float t[6];
-  cudaEventElapsedTime(&t[0], ctx->ev[0], ctx->ev[1]);
-  cudaEventElapsedTime(&t[1], ctx->ev[1], ctx->ev[2]);
-  cudaEventElapsedTime(&t[2], ctx->ev[2], ctx->ev[3]);
-  cudaEventElapsedTime(&t[3], ctx->ev[3], ctx->ev[4]);
-  cudaEventElapsedTime(&t[4], ctx->ev[4], ctx->ev[5]);
+  float t[6], staging = 0.f;
+  for (int k = 0; k < 5; k++) t[k] = (float)(head[kMarkStart + k + 1] - head[kMarkStart + k]) * 1e-6f;
+  if (stagedInput) cudaEventElapsedTime(&staging, ctx->ev[0], ctx->ev[1]);
+  t[0] += staging;
   cudaEventElapsedTime(&t[5], ctx->ev[0], ctx->ev[6]);
   memcpy(ctx->timings, t, sizeof t);
   if (ctx->profiling)
@@ -1489,7 +1528,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     r.dup_value = st.dupValue;
     r.dup_key = st.dupValue >= 0 ? pl.p.bin_count : -1;
     r.longest_code = st.longest;
-    r.owner = slab;
+    r.owner = owner;
     r.n_words = st.nWords;
     r.words = hw + wOff[i];
     r.n_decode = st.nDecode;
@@ -2371,12 +2410,12 @@ void wl_destroy(wl_ctx *ctx) {
                    &ctx->encCub, &ctx->sliceOff,
                    &ctx->chunkSpan, &ctx->optIn, &ctx->optOut, &ctx->optErr,
                    &ctx->codes, &ctx->codeLen, &ctx->decode, &ctx->words, &ctx->passes,
-                   &ctx->logHdr, &ctx->outbuf, &ctx->decWords, &ctx->decTable, &ctx->decWs,
+                   &ctx->outbuf, &ctx->head, &ctx->decWords, &ctx->decTable, &ctx->decWs,
                    &ctx->meta, &ctx->errIn, &ctx->errRest, &ctx->errPart};
   for (DevBuf *d : dbs) if (d->p) cudaFree(d->p);
   for (GraphEntry &g : ctx->graphs) drop_graph(g);
   HostBuf *hbs[] = {&ctx->hStage[0], &ctx->hStage[1], &ctx->hState, &ctx->hDecode, &ctx->hPasses,
-                    &ctx->hTab, &ctx->hLogHdr, &ctx->hIn,
+                    &ctx->hTab, &ctx->hHead, &ctx->hSel, &ctx->hIn,
                     &ctx->hFlags};
   for (HostBuf *h : hbs) if (h->p) cudaFreeHost(h->p);
   for (auto &e : ctx->ev) if (e) cudaEventDestroy(e);

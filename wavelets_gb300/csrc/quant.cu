@@ -33,6 +33,7 @@ constexpr int INF = 0x7fffffff;
 
 // ---- quantizer parameters ---------------------------------------------------
 __global__ void quant_params_kernel(DevBatch b) {
+  stage_mark(b.head, kMarkQuant);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
   if (ci >= b.n) return;
   const CubeletDev cd = b.cub[ci];

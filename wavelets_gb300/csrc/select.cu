@@ -64,6 +64,7 @@ __device__ __forceinline__ void load_chunk(const float *src, int len, float (&v)
 __global__ void __launch_bounds__(kThreads, 6)
 select_pass0(DevBatch b, const float *__restrict__ coef) {
   __shared__ unsigned hist[kSelectBins];
+  stage_mark(b.head, kMarkSelect);
   const int ci = b.groupCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
   if (cd.selFused) return;  // the last transform pass gathered these already
@@ -198,9 +199,11 @@ __device__ __forceinline__ void set_lloyd_bins(CubeletState *st, unsigned base, 
 }
 
 // Find the digit bucket holding the remaining rank; one CTA per cubelet.
+// mark: this launch starts the select (no stand-alone first pass).
 template <int PASS>
-__global__ void __launch_bounds__(1024) select_resolve(DevBatch b) {
+__global__ void __launch_bounds__(1024) select_resolve(DevBatch b, bool mark) {
   __shared__ unsigned long long part[1024];
+  if (PASS == 0 && mark) stage_mark(b.head, kMarkSelect);
   const int ci = blockIdx.x;
   CubeletState *st = b.state + ci;
   const CubeletDev cd = b.cub[ci];
@@ -271,6 +274,7 @@ __global__ void __launch_bounds__(1024) select_resolve(DevBatch b) {
           float t = __uint_as_float(bits);
           if (t == 0.0f) t = 1e-16f;  // thresh_cpu.cc:98
           st->threshold = t;
+          if (b.hostSel) b.hostSel[ci] = make_float2(t, st->maxAbs);
           if (cd.quantAlg == WL_LLOYD && st->lloydDeferred) {
             const float hi = st->maxAbs2 > t ? st->maxAbs2 : st->maxAbs;
             set_lloyd_bins(st, __float_as_uint(t), __float_as_uint(hi));
@@ -286,49 +290,58 @@ __global__ void __launch_bounds__(1024) select_resolve(DevBatch b) {
   for (int i = threadIdx.x; i < kSelectBins; i += 1024) g[i] = 0;
 }
 
-// cubelet index of every chunk (and quantize group), so chunk kernels start
-// with one load
-__global__ void chunk_map_kernel(DevBatch b) {
-  const CubeletDev cd = b.cub[blockIdx.x];
-  for (int j = threadIdx.x; j < cd.nChunks; j += blockDim.x)
-    b.chunkCub[cd.chunkBase + j] = (int)blockIdx.x;
+// One launch sets up everything a call's kernels expect: kInitSlices CTAs per
+// cubelet (blockIdx.y) zero its histograms and state and write the cubelet
+// index of its chunks, quantize groups and bit-packer CTAs, so that those
+// kernels start with one load.  (Three memsets, an initialisation and a map
+// kernel before took 20 us at the head of every call, most of it gaps.)
+constexpr int kInitSlices = 8;
+__global__ void __launch_bounds__(kThreads) init_kernel(DevBatch b, bool lloyd) {
+  stage_mark(b.head, kMarkStart);
+  const int ci = blockIdx.y, slice = blockIdx.x;
+  const CubeletDev cd = b.cub[ci];
+  const int t0 = slice * kThreads + threadIdx.x, step = kInitSlices * kThreads;
+  unsigned *sel = b.selHist + (size_t)ci * kSelectBins;
+  for (int i = t0; i < kSelectBins; i += step) sel[i] = 0;
+  unsigned long long *h = b.hist + (size_t)ci * kMaxSymbols;
+  for (int i = t0; i <= cd.binCount; i += step) h[i] = 0;
+  if (lloyd) {
+    unsigned *lh = reinterpret_cast<unsigned *>(b.lloydHist) + (size_t)ci * kLloydBins;
+    for (int i = t0; i < kLloydBins; i += step) lh[i] = 0;
+  }
+  for (int j = t0; j < cd.nChunks; j += step) b.chunkCub[cd.chunkBase + j] = ci;
   const int groups = (cd.nChunks + b.group - 1) / b.group;
-  for (int j = threadIdx.x; j < groups; j += blockDim.x)
-    b.groupCub[cd.groupBase + j] = (int)blockIdx.x;
+  for (int j = t0; j < groups; j += step) b.groupCub[cd.groupBase + j] = ci;
   const int enc = (int)(((long long)cd.nChunks * b.encF + kEncThreads - 1) / kEncThreads);
-  for (int j = threadIdx.x; j < enc; j += blockDim.x) b.encCub[cd.encBase + j] = (int)blockIdx.x;
-}
-
-__global__ void select_init(DevBatch b) {
-  const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ci >= b.n) return;
+  for (int j = t0; j < enc; j += step) b.encCub[cd.encBase + j] = ci;
+  if (slice != 0) return;
   CubeletState *st = b.state + ci;
-  // Traverse starts min at FLT_MAX and max at FLT_MIN (thresh_cpu.cc:67-68)
-  st->minOrd = ord_enc(FLT_MAX);
-  st->maxOrd = ord_enc(FLT_MIN);
-  st->absMax = 0u;
-  st->absMax2 = 0u;
-  st->candCount = 0u;
-  st->lloydDeferred = 0;
+  unsigned *w = reinterpret_cast<unsigned *>(st);
+  for (int i = threadIdx.x; i < (int)(sizeof(CubeletState) / 4); i += kThreads) w[i] = 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // Traverse starts min at FLT_MAX and max at FLT_MIN (thresh_cpu.cc:67-68)
+    st->minOrd = ord_enc(FLT_MAX);
+    st->maxOrd = ord_enc(FLT_MIN);
+  }
 }
 
 }  // namespace
 
-void launch_select_init(DevBatch &b, cudaStream_t s) {
-  select_init<<<(b.n + 127) / 128, 128, 0, s>>>(b);
+void launch_init(DevBatch &b, bool lloyd, cudaStream_t s) {
+  init_kernel<<<dim3(kInitSlices, b.n), kThreads, 0, s>>>(b, lloyd);
 }
 
 void launch_select(DevBatch &b, const float *coef, bool pass0, cudaStream_t s) {
-  chunk_map_kernel<<<b.n, 256, 0, s>>>(b);
   unsigned *cand = reinterpret_cast<unsigned *>(b.coef2);
   const unsigned groups = (unsigned)b.totalGroups;
   if (pass0) select_pass0<<<groups, kThreads, 0, s>>>(b, coef);
-  select_resolve<0><<<b.n, 1024, 0, s>>>(b);
+  select_resolve<0><<<b.n, 1024, 0, s>>>(b, !pass0);
   select_compact<<<groups, kThreads, 0, s>>>(b, coef, cand);
   cand_hist<1><<<dim3(kCandSlices, b.n), kThreads, 0, s>>>(b, cand);
-  select_resolve<1><<<b.n, 1024, 0, s>>>(b);
+  select_resolve<1><<<b.n, 1024, 0, s>>>(b, false);
   cand_hist<2><<<dim3(kCandSlices, b.n), kThreads, 0, s>>>(b, cand);
-  select_resolve<2><<<b.n, 1024, 0, s>>>(b);
+  select_resolve<2><<<b.n, 1024, 0, s>>>(b, false);
 }
 
 }  // namespace wl

@@ -11,6 +11,17 @@
 
 namespace wl {
 
+#ifdef __CUDACC__
+// a stage mark of the call (DevBatch::head)
+__device__ __forceinline__ void stage_mark(long long *head, int i) {
+  if (head && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    head[i] = (long long)t;
+  }
+}
+#endif
+
 __host__ __device__ inline int clz32(unsigned x) {
 #ifdef __CUDA_ARCH__
   return __clz(x);
@@ -177,6 +188,14 @@ struct CubeletDev {
                           // digit and the extremes (no stand-alone first pass)
 };
 
+// Page-locked result storage of a call: words from `base` on, then (at the
+// next multiple of 16 bytes) each cubelet's decode table and codebook; used
+// when they fit in `cap` bytes.
+struct OutSlab {
+  char *base;
+  long long cap;
+};
+
 // Device workspace for one batch.
 struct DevBatch {
   int n;                          // cubelets
@@ -213,7 +232,18 @@ struct DevBatch {
   int *meta;                      // packed decode tables and Lloyd codebooks
   long long totalChunks;
   int maxChunks;                  // most chunks of one cubelet
+  // Stage marks and output sizes of the call (null for a second half): the
+  // marks are nanosecond clock readings taken by the first thread of the
+  // kernel that starts a stage (event nodes between the kernels of a graph
+  // cost 5 to 8 us each)
+  long long *head;
+  float2 *hostSel;                // page-locked: threshold, largest |c| of every cubelet
+  const OutSlab *outSlab;         // in the upload block: where deliver_kernel puts the results
+  CubeletState *hostState;        // page-locked copy of the states, deliver_kernel's
+  long long *hostHead;            // and of head
 };
+enum { kMarkStart, kMarkSelect, kMarkQuant, kMarkBuild, kMarkEncode, kMarkEnd, kHeadWords,
+       kHeadMeta, kHeadDelivered, kHeadCount };
 
 // launchers (dwt.cu)
 // Raise a kernel's dynamic shared-memory limit to at least `bytes`.  The
@@ -280,9 +310,10 @@ void set_tuned_cols_shape(int kind, int typeIdx, int cls, TileShape t,
 unsigned tune_version();  // changes whenever the table does
 
 // launchers (select.cu)
-// per-cubelet select state (extremes from FLT_MAX / FLT_MIN); runs before the
-// transform, whose last pass may gather the first digit
-void launch_select_init(DevBatch &b, cudaStream_t s);
+// everything a call's kernels expect set: histograms and states zeroed, the
+// select state (extremes from FLT_MAX / FLT_MIN), cubelet of every chunk;
+// runs before the transform, whose last pass may gather the first digit
+void launch_init(DevBatch &b, bool lloyd, cudaStream_t s);
 // pass0: run the stand-alone first digit pass for the cubelets whose last
 // transform pass did not gather it (CubeletDev::selFused == 0)
 void launch_select(DevBatch &b, const float *coef, bool pass0, cudaStream_t s);
@@ -307,6 +338,9 @@ void launch_err_sums(const void *orig, int dtype, const float *rest, long long n
 void launch_huffman_build(DevBatch &b, int maxSymbols, cudaStream_t s);
 void launch_encode(DevBatch &b, int maxSymbols, cudaStream_t s);
 void launch_pack_meta(DevBatch &b, cudaStream_t s);
+// states, head and (when they fit in the slab) words, decode tables and
+// codebooks straight to page-locked host memory
+void launch_deliver(DevBatch &b, cudaStream_t s);
 
 // batched Huffman decoding (decode.cu): the streams of n cubelets to their
 // dequantized values
