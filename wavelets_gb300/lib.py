@@ -240,6 +240,10 @@ def make_params(p: Optional[P.Params] = None) -> WlParams:
     return w
 
 
+def _addr(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]
+
+
 @dataclasses.dataclass
 class Compressed:
     """A compressed cubelet (copy of a wl_result)."""
@@ -281,35 +285,24 @@ class Compressed:
                    arr(r.boundaries, r.n_boundaries, np.float32),
                    arr(r.values, r.n_values, np.float32), bool(r.transform_2d))
 
+    def _record(self):
+        """The WlResult field values (in _RESULT_DT order) over this object's
+        arrays, which are kept as self._keep."""
+        self._keep = keep = (np.ascontiguousarray(self.words, np.uint32),
+                             np.ascontiguousarray(self.decode, np.int32),
+                             np.ascontiguousarray(self.boundaries, np.float32),
+                             np.ascontiguousarray(self.values, np.float32))
+        w, d, b, v = keep
+        return (tuple(self.size), tuple(self.original_size), self.original_dtype,
+                tuple(self.steps), self.wavelet, self.quant_alg, self.bin_count,
+                self.threshold_fraction, self.threshold_value, self.max_value, self.min_coef,
+                self.max_coef, self.zero_bin, self.dup_key, self.dup_value, self.longest_code,
+                w.size, _addr(w), d.size, _addr(d), b.size, v.size, _addr(b),
+                _addr(v), 0, 1 if self.transform_2d else 0)
+
     def to_struct(self):
         """A WlResult pointing into this object's arrays (keep self alive)."""
-        r = WlResult()
-        r.size[:] = self.size
-        r.original_size[:] = self.original_size
-        r.original_dtype = self.original_dtype
-        r.steps[:] = self.steps
-        r.wavelet, r.quant_alg, r.bin_count = self.wavelet, self.quant_alg, self.bin_count
-        r.threshold_fraction = self.threshold_fraction
-        r.threshold_value = self.threshold_value
-        r.max_value = self.max_value
-        r.min_coef, r.max_coef = self.min_coef, self.max_coef
-        r.zero_bin, r.dup_key, r.dup_value = self.zero_bin, self.dup_key, self.dup_value
-        r.longest_code = self.longest_code
-        r.transform_2d = 1 if self.transform_2d else 0
-        self._keep = [np.ascontiguousarray(self.words, np.uint32),
-                      np.ascontiguousarray(self.decode, np.int32),
-                      np.ascontiguousarray(self.boundaries, np.float32),
-                      np.ascontiguousarray(self.values, np.float32)]
-        w, d, b, v = self._keep
-        r.n_words = w.size
-        r.words = w.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32))
-        r.n_decode = d.size
-        r.decode = d.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
-        r.n_boundaries = b.size
-        r.boundaries = b.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
-        r.n_values = v.size
-        r.values = v.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
-        return r
+        return WlResult.from_buffer(np.array([self._record()], _result_dtype_cached()))
 
     @property
     def compressed_bytes(self) -> int:
@@ -399,6 +392,14 @@ def _result_dtype():
 
 
 _RESULT_DT = None
+# numpy mirror of WlCubelet (the parameters as their bytes)
+_CUBELET_DT = np.dtype({
+    "names": ["data", "dtype", "size", "params", "row_pitch", "slice_pitch"],
+    "formats": [np.uint64, np.int32, (np.int32, (3,)), np.dtype((np.void, ctypes.sizeof(WlParams))),
+                np.int64, np.int64],
+    "offsets": [getattr(WlCubelet, k).offset for k in ("data", "dtype", "size", "params",
+                                                       "row_pitch", "slice_pitch")],
+    "itemsize": ctypes.sizeof(WlCubelet)})
 
 
 def _result_dtype_cached():
@@ -408,60 +409,93 @@ def _result_dtype_cached():
     return _RESULT_DT
 
 
+_SCALARS = ("original_dtype", "wavelet", "quant_alg", "bin_count", "threshold_fraction",
+            "threshold_value", "max_value", "min_coef", "max_coef", "zero_bin", "dup_key",
+            "dup_value", "longest_code")
+
+
+def _int32_view(lo, hi, owner):
+    """The bytes [lo, hi) at an address as int32; the array holds owner."""
+    buf = (ctypes.c_char * (hi - lo)).from_address(lo)
+    buf._owner = owner
+    return np.frombuffer(buf, np.int32)
+
+
 def adopt_results(lib, outs, n) -> List["Compressed"]:
     """Compressed objects over the results' arrays without copying them.  The
     library keeps a batch's arrays in one block; the numpy views hold a
     reference that releases the results when the last view goes away."""
-    global _RESULT_DT
-    if _RESULT_DT is None:
-        _RESULT_DT = _result_dtype()
-    rec = np.frombuffer(outs, _RESULT_DT, count=n)
-    ptrs = np.stack([rec["words"], rec["decode"], rec["boundaries"], rec["values"]], 1)
+    rec = np.frombuffer(outs, _result_dtype_cached(), count=n)
     cnts = np.stack([rec["n_words"], rec["n_decode"], rec["n_boundaries"], rec["n_values"]],
-                    1).astype(np.int64)
+                    1).astype(np.uint64)
+    ptrs = np.stack([rec["words"], rec["decode"], rec["boundaries"], rec["values"]], 1)
     used = (cnts > 0) & (ptrs != 0)
-    if n == 0 or not used.any() or not (rec["owner"] != 0).all():
+    slab = rec["owner"]
+    if n == 0 or not used.any() or not slab.all():
         res = [Compressed.from_struct(outs[i]) for i in range(n)]
         lib.wl_results_free(outs, n)
         return res
-    # one numpy view per storage block (a pipelined batch has several); all
-    # views share the owner that releases the batch's results
+    # one view per storage block (a pipelined batch has several); all views
+    # share the owner that releases the batch's results
     owner = _ResultsOwner(lib, outs, n)
-    slab = rec["owner"]
-    ends_abs = ptrs + 4 * cnts.astype(np.uint64)
-    bases, lo_of = {}, {}
-    for sid in np.unique(slab).tolist():
-        sel = used & (slab == sid)[:, None]
-        if not sel.any():
-            continue
-        lo = int(ptrs[sel].min())
-        buf = (ctypes.c_char * (int(ends_abs[sel].max()) - lo)).from_address(lo)
-        buf._owner = owner
-        bases[sid], lo_of[sid] = np.frombuffer(buf, np.uint8), lo
-    slab_l = slab.tolist()
-    lo_row = np.array([lo_of.get(x, 0) for x in slab_l], np.uint64)[:, None]
-    rel = np.where(used, ptrs - lo_row, 0).astype(np.int64).tolist()
-    ends = (np.where(used, ptrs - lo_row, 0).astype(np.int64)
-            + 4 * np.where(used, cnts, 0)).tolist()
-    empty_base = np.zeros(0, np.uint8)
-    f = {k: rec[k].tolist() for k in _RESULT_DT.names if k not in ("words", "decode",
-                                                                    "boundaries", "values", "owner")}
-    e32, ef = np.zeros(0, np.float32), np.zeros(0, np.float32)
-    res = []
-    for i in range(n):
-        o, z = rel[i], ends[i]
-        base = bases.get(slab_l[i], empty_base)
-        res.append(Compressed(
-            tuple(f["size"][i]), tuple(f["original_size"][i]), f["original_dtype"][i],
-            tuple(f["steps"][i]), f["wavelet"][i], f["quant_alg"][i], f["bin_count"][i],
-            f["threshold_fraction"][i], f["threshold_value"][i], f["max_value"][i],
-            f["min_coef"][i], f["max_coef"][i], f["zero_bin"][i], f["dup_key"][i],
-            f["dup_value"][i], f["longest_code"][i],
-            base[o[0]:z[0]].view(np.uint32), base[o[1]:z[1]].view(np.int32),
-            base[o[2]:z[2]].view(np.float32) if z[2] > o[2] else e32,
-            base[o[3]:z[3]].view(np.float32) if z[3] > o[3] else ef,
-            bool(f["transform_2d"][i])))
-    return res
+    starts = np.where(used, ptrs, np.uint64(1 << 63))
+    ends = np.where(used, ptrs + 4 * cnts, np.uint64(0))
+    base, rows = [], np.empty(n, np.uint64)
+    for sid in dict.fromkeys(slab.tolist()):
+        sel = slab == sid
+        lo, hi = int(starts[sel].min()), int(ends[sel].max())
+        view = _int32_view(lo, hi, owner) if hi > lo else np.zeros(0, np.int32)
+        base.append((view.view(np.uint32), view, view.view(np.float32)))
+        rows[sel] = lo
+        if sel.all():
+            block = [0] * n
+            break
+        if len(base) == 1:
+            block = np.zeros(n, np.int64)
+        block[sel] = len(base) - 1
+    first = np.where(used, (ptrs - rows[:, None]) // 4, 0).astype(np.int64)
+    last = first + np.where(used, cnts, 0).astype(np.int64)
+
+    def views(kind, column):  # the arrays of one kind, a slice each
+        if not used[:, column].any():
+            return [base[0][kind][:0]] * n
+        lo, hi = first[:, column].tolist(), last[:, column].tolist()
+        if len(base) == 1:
+            v = base[0][kind]
+            return [v[x:y] for x, y in zip(lo, hi)]
+        return [base[k][kind][x:y] for k, x, y in zip(block, lo, hi)]
+
+    cols = [rec[k].tolist() for k in _SCALARS]
+    sizes, originals, steps = (map(tuple, rec[k].tolist())
+                               for k in ("size", "original_size", "steps"))
+    return list(map(Compressed, sizes, originals, cols[0], steps, *cols[1:], views(0, 0),
+                    views(1, 1), views(2, 2), views(2, 3), rec["transform_2d"].astype(bool).tolist()))
+
+
+def _adopt_one(lib, r: WlResult) -> "Compressed":
+    """adopt_results for one result, without the array work of a batch."""
+    n = (r.n_words, r.n_decode, r.n_boundaries, r.n_values)
+    outs = (WlResult * 1).from_buffer(r)
+    rec = np.frombuffer(r, _result_dtype_cached())
+    p = rec[["words", "decode", "boundaries", "values"]].item()
+    if not r.owner or not any(n):
+        res = Compressed.from_struct(r)
+        lib.wl_results_free(outs, 1)
+        return res
+    owner = _ResultsOwner(lib, outs, 1)
+    a = [_int32_view(q, q + 4 * k, owner) if k > 0 and q else _EMPTY for q, k in zip(p, n)]
+    c = Compressed.__new__(Compressed)
+    d = c.__dict__
+    for k in _SCALARS:
+        d[k] = getattr(r, k)
+    d["size"], d["original_size"] = tuple(r.size), tuple(r.original_size)
+    d["steps"], d["transform_2d"] = tuple(r.steps), bool(r.transform_2d)
+    d["words"], d["decode"] = a[0].view(np.uint32), a[1]
+    d["boundaries"], d["values"] = a[2].view(np.float32), a[3].view(np.float32)
+    return c
+
+
+_EMPTY = np.zeros(0, np.int32)
 
 
 class Context:
@@ -512,19 +546,19 @@ class Context:
                                           1 if on_device else 0, ctypes.byref(make_params(params)),
                                           ctypes.byref(res))
         self._check(st)
-        return adopt_results(self.lib, (WlResult * 1)(res), 1)[0]
+        return _adopt_one(self.lib, res)
 
     def prepare_batch(self, items: Sequence, params=None, on_device: bool = False,
                       raw: bool = False) -> PreparedBatch:
         """Describe a batch once (see compress_batch for items)."""
         n = len(items)
-        cubs = (WlCubelet * n)()
-        keep = []
-        for i, it in enumerate(items):
+        keep, rows, made = [], [], {}
+        for it in items:
+            pitch = (0, 0)
             if raw or on_device:
                 ptr, dt, size, prm = it[:4]
                 if len(it) > 4:  # (row pitch, slice pitch) of a sub-volume
-                    cubs[i].row_pitch, cubs[i].slice_pitch = it[4]
+                    pitch = it[4]
             else:
                 if isinstance(it, tuple):
                     a, prm = it
@@ -533,10 +567,12 @@ class Context:
                 a = np.ascontiguousarray(a)
                 keep.append(a)
                 ptr, dt, size = a.ctypes.data, NP_TO_WL[a.dtype], _size_of(a)
-            cubs[i].data = ptr
-            cubs[i].dtype = dt
-            cubs[i].size[:] = size
-            cubs[i].params = make_params(prm if prm is not None else params)
+            prm = prm if prm is not None else params
+            p = made.get(id(prm))  # items of one call often share their Params
+            if p is None:
+                p = made[id(prm)] = bytes(make_params(prm))
+            rows.append((ptr, dt, tuple(size), p, pitch[0], pitch[1]))
+        cubs = (WlCubelet * n).from_buffer(np.array(rows, _CUBELET_DT)) if n else (WlCubelet * 0)()
         return PreparedBatch(cubs, n, on_device, keep)
 
     def compress_prepared(self, pb: PreparedBatch, lazy: bool = False):
@@ -589,15 +625,15 @@ class Context:
         """The wl_decompress_batch arguments for these results (reusable:
         run_decompress(prep) restores them again without rebuilding them)."""
         n = len(cs)
-        rs = (WlResult * n)()
-        keep = []
+        rs = ((WlResult * n).from_buffer(np.array([c._record() for c in cs],
+                                                  _result_dtype_cached()))
+              if n else (WlResult * 0)())
+        # the arrays that the records point into, also if a Compressed is
+        # described again meanwhile
+        keep = [(c, c._keep) for c in cs]
         outs, ptrs = [], (ctypes.c_void_p * n)()
         dts = (ctypes.c_int * n)()
         for i, c in enumerate(cs):
-            r = c.to_struct()
-            keep.append(c)
-            ctypes.memmove(ctypes.byref(rs, i * ctypes.sizeof(WlResult)), ctypes.byref(r),
-                           ctypes.sizeof(WlResult))
             wl_dt = (NP_TO_WL[np.dtype(dtypes[i])] if dtypes is not None and dtypes[i] is not None
                      else c.original_dtype)
             if device_outs is not None:
@@ -992,9 +1028,10 @@ class Server:
 
     def wait(self, ticket: int, timeout_ms: int = -1):
         """(Compressed or None, info dict); None while a poll finds it pending."""
-        res = (WlResult * 1)()
+        res = WlResult()
         info = WlRequestInfo()
-        st = self.lib.wl_serve_wait(self.h, ticket, timeout_ms, res, ctypes.byref(info))
+        st = self.lib.wl_serve_wait(self.h, ticket, timeout_ms, ctypes.byref(res),
+                                    ctypes.byref(info))
         if st == WL_ETIMEOUT:
             return None, None
         req, _ = self._keep.pop(ticket)
@@ -1002,7 +1039,7 @@ class Server:
             raise WlError(st, self.lib.wl_serve_last_error(self.h).decode())
         d = {k: getattr(info, k) for k, _ in WlRequestInfo._fields_}
         if req.kind == REQ_COMPRESS:
-            return adopt_results(self.lib, res, 1)[0], d
+            return _adopt_one(self.lib, res), d
         return None, d
 
     def close(self):

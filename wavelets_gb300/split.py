@@ -19,15 +19,9 @@ def split_grid(volume_xyz: Sequence[int], cube_xyz: Sequence[int],
                overlap: int) -> List[Tuple[Tuple[int, int, int], Tuple[int, int, int]]]:
     """(offset, size) of every cubelet, x y z order, in the reference's output
     order."""
-    counts = [axis_count(n, s, overlap) for n, s in zip(volume_xyz, cube_xyz)]
-    out = []
-    for kz in range(counts[2]):
-        for ky in range(counts[1]):
-            for kx in range(counts[0]):
-                off, size = [], []
-                for k, n, s in zip((kx, ky, kz), volume_xyz, cube_xyz):
-                    o = k * (s - overlap)
-                    off.append(o)
-                    size.append(min(s, n - o))  # trimmed at the end (:475-482)
-                out.append((tuple(off), tuple(size)))
-    return out
+    axes = []
+    for n, s in zip(volume_xyz, cube_xyz):
+        offs = [k * (s - overlap) for k in range(axis_count(n, s, overlap))]
+        axes.append([(o, min(s, n - o)) for o in offs])  # trimmed at the end (:475-482)
+    xs, ys, zs = axes
+    return [((ox, oy, oz), (sx, sy, sz)) for oz, sz in zs for oy, sy in ys for ox, sx in xs]
