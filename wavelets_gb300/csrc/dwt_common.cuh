@@ -36,13 +36,27 @@ template <> __device__ __forceinline__ void store_from_float<uint16_t>(uint16_t 
   *p = (uint16_t)(v < 0 ? 0 : (v > 65535 ? 65535 : v));
 }
 
-// per-level store scale of the lifting form: index t < S detail, t == S low
-__device__ __forceinline__ float lifting_scale(int t, int S) {
-  double k = 1.0;
-  if (t == S) { for (int i = 0; i < S; i++) k *= kK; return (float)k; }
-  for (int i = 0; i < t; i++) k *= kK;
-  return (float)(-k / kK);
+// Per-level store scale of the lifting form: index t < S detail, t == S low;
+// S at most 14 (axes up to 16384).  A table computed by the compiler: every
+// block of every pass began with the double products and a division, on a
+// GPU with few double units (restoring the mixed batch of 512: 5.58 ms a call
+// with them, 5.41 ms without).
+constexpr int kMaxLevels = 14;
+struct ScaleTable {
+  float v[kMaxLevels + 1][kMaxLevels + 1];
+};
+constexpr ScaleTable make_scale_table() {
+  ScaleTable r{};
+  for (int S = 0; S <= kMaxLevels; S++)
+    for (int t = 0; t <= S; t++) {
+      double k = 1.0;
+      for (int i = 0; i < t; i++) k *= kK;
+      r.v[S][t] = t == S ? (float)k : (float)(-k / kK);
+    }
+  return r;
 }
+static __constant__ ScaleTable kScaleTable = make_scale_table();
+__device__ __forceinline__ float lifting_scale(int t, int S) { return kScaleTable.v[S][t]; }
 
 }  // namespace dwtc
 }  // namespace wl
