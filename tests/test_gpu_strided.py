@@ -1,0 +1,44 @@
+"""The register kernel of the y passes (row pairs packed in two floats) against
+the tile kernels: with an even number of z layers the rows pair up, with an
+odd number they go to the tile kernels, and the transforms of the layers both
+volumes share are the same to the bit, forward and inverse.  Forward also
+against the float64 yardstick."""
+import numpy as np
+import pytest
+
+from oracle import lifting64
+from wavelets_gb300 import lib, params as P
+
+pytestmark = pytest.mark.gpu
+
+LEVELS = {16: 4, 32: 5, 48: 4, 64: 5, 96: 4, 128: 5, 192: 4, 256: 5}  # in the register kernel
+CASES = [(L, s) for L, most in LEVELS.items() for s in (1, 2, most, most + 1)
+         if L % (1 << s) == 0 and s <= (L - 1).bit_length()]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from wavelets_gb300 import build
+    build.build()
+    c = lib.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("wavelet", [P.HAAR, P.CDF97])
+@pytest.mark.parametrize("L,s", CASES)
+def test_even_and_odd_layer_counts_agree(ctx, L, s, wavelet):
+    X, Z = 10, 38  # pairs do not fill the last block
+    vol = np.random.default_rng(L + s).normal(0, 100, (Z, L, X)).astype(np.float32)
+    p = P.Params(steps=(1, s, 0), wavelet=wavelet)
+    even, stored = ctx.forward_transform(vol, p)
+    odd, _ = ctx.forward_transform(vol[:Z - 1], p)
+    assert tuple(stored) == (Z, X, L)
+    even, odd = even.reshape(L, X, Z), odd.reshape(L, X, Z - 1)
+    assert np.array_equal(even[:, :, :Z - 1], odd)
+    ref, _ = lifting64.forward(vol, (1, s, 0), wavelet)
+    assert np.abs(even.ravel() - ref).max() <= 2e-6 * np.abs(ref).max()
+    back = ctx.inverse_transform(even, (Z, X, L), (1, s, 0), wavelet, (X, L, Z))
+    back_odd = ctx.inverse_transform(odd, (Z - 1, X, L), (1, s, 0), wavelet, (X, L, Z - 1))
+    assert np.array_equal(back[:Z - 1], back_odd)
+    assert np.abs(back - vol).max() <= 4e-6 * np.abs(vol).max()

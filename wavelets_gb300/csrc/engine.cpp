@@ -94,7 +94,9 @@ int rowreg_key(int L) { return (1 << 20) | L; }
 int rowreg_t_key(int dtype, int L) { return (1 << 21) | (dtype << 16) | L; }
 int rowreg_inv_key(int L) { return (1 << 23) | L; }
 int rowreg_inv_t_key(int outType, int L) { return (1 << 24) | (outType << 16) | L; }
-enum RegKind { kRegNone, kRegInPlace, kRegTile, kRegInvInPlace, kRegInvTile };
+int strided_key(bool inverse, int L) { return (1 << (inverse ? 26 : 25)) | L; }
+enum RegKind { kRegNone, kRegInPlace, kRegTile, kRegInvInPlace, kRegInvTile, kRegStrided,
+               kRegInvStrided };
 
 // ---- result storage ------------------------------------------------------------
 // The arrays of all results of one compression call live in one page-locked
@@ -576,7 +578,7 @@ bool forward_passes_cols(const Plan &pl, const void *in, bool hostIn, float *coe
   e.outSA = Zp; e.outSB = 1; e.outSC = Zp * Xp;
   e.steps = pl.sy;
   e.T = dwt_cols_tile_rows(e.L); e.tiles = (e.rows + e.T - 1) / e.T;
-  ys[group_key(true, WL_F32, e.L)].push_back(e);
+  ys[dwt_strided_fits(e) ? strided_key(false, e.L) : group_key(true, WL_F32, e.L)].push_back(e);
   if (pl.sz == 0) return false;
   // z pass: rows (a = y, b = x) of z-x-y, in place
   PassDesc f = e;
@@ -753,7 +755,9 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
       return fail(ctx, WL_EINVAL, "internal: mixed select-gathering passes in one group");
   if (regL) {
     rows = (regKind == kRegTile || regKind == kRegInvTile) ? dwt_rowreg_t_rows_per_block(regL)
-                                                          : dwt_rowreg_rows_per_block(regL, sel);
+           : (regKind == kRegStrided || regKind == kRegInvStrided)
+               ? dwt_strided_rows_per_block(regL)
+               : dwt_rowreg_rows_per_block(regL, sel);
     for (PassDesc &d : g) {
       d.T = rows;
       d.tiles = (d.rows + rows - 1) / rows;
@@ -793,6 +797,11 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
 wl_status stage_groups(wl_ctx *ctx, const PassGroups &gs, size_t &hoff, int kind, int outType,
                        bool inverse, std::vector<GroupLaunch> &out) {
   for (const auto &kv : gs) {
+    if ((kv.first >> 25) & 1) {
+      TRY(stage_group(ctx, kv.second, hoff, kind, WL_F32, WL_F32, false, false, false, out, nullptr,
+                      kv.second[0].L, kRegStrided));
+      continue;
+    }
     const bool regT = (kv.first >> 21) & 1;
     const int regL = regT || ((kv.first >> 20) & 1) ? kv.second[0].L : 0;
     const int regKind = regT ? kRegTile : regL ? kRegInPlace : kRegNone;
@@ -808,7 +817,9 @@ wl_status launch_one(wl_ctx *ctx, const GroupLaunch &l, cudaStream_t s) {
   const char *base = P<char>(ctx->passes);
   const PassDesc *dp = reinterpret_cast<const PassDesc *>(base + l.off);
   const int *dtp = reinterpret_cast<const int *>(base + l.off + l.n * sizeof(PassDesc));
-  if (l.regKind == kRegTile)
+  if (l.regKind == kRegStrided || l.regKind == kRegInvStrided)
+    launch_dwt_strided(dp, dtp, l.n, l.tiles, l.regL, l.regKind == kRegInvStrided, s);
+  else if (l.regKind == kRegTile)
     launch_dwt_rowreg_t(dp, dtp, l.n, l.tiles, l.regL, l.inType, s);
   else if (l.regKind == kRegInvInPlace)
     launch_dwt_rowreg_inv(dp, dtp, l.n, l.tiles, l.regL, s);
@@ -1632,6 +1643,8 @@ void inverse_passes(const int size[3], const int steps[3], int wavelet, const in
       const int phase = 3 - np + i;
       if (phase == 0 && dwt_rowreg_fits(d[i].L, d[i].steps))  // z rows in registers
         ph[0][rowreg_inv_key(d[i].L)].push_back(d[i]);
+      else if (phase == 1 && dwt_strided_fits(d[i]))  // y rows in registers
+        ph[1][strided_key(true, d[i].L)].push_back(d[i]);
       else if (phase > 0 && dwt_rowreg_fits(d[i].L, d[i].steps))  // y, x: through a tile
         ph[phase][rowreg_inv_t_key(phase == 2 ? outType : WL_F32, d[i].L)].push_back(d[i]);
       else
@@ -1686,6 +1699,11 @@ wl_status stage_inverse_phases(wl_ctx *ctx, PassGroups ph[3], InversePhases &ip)
   const int kinds[3] = {kTuneInvZ, kTuneInvY, kTuneInvX};
   for (int k = 0; k < 3; k++) {
     for (const auto &kv : ph[k]) {
+      if ((kv.first >> 26) & 1) {
+        TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, WL_F32, true, false, false, gl,
+                        nullptr, kv.second[0].L, kRegInvStrided));
+        continue;
+      }
       if ((kv.first >> 24) & 1) {
         TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, (kv.first >> 16) & 15, true, false,
                         false, gl, nullptr, kv.second[0].L, kRegInvTile));

@@ -293,6 +293,13 @@ void launch_dwt_rowreg_inv_t(const PassDesc *d_passes, const int *d_tilePrefix, 
 void launch_dwt_rowreg_t(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
                          int blocks, int L, int inType, cudaStream_t s);
 
+// passes along a strided axis whose rows are neighbours in memory (the y
+// passes), in registers (dwt_strided.cu)
+bool dwt_strided_fits(const PassDesc &d);
+int dwt_strided_rows_per_block(int L);
+void launch_dwt_strided(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
+                        int L, bool inverse, cudaStream_t s);
+
 // ---- column-tile heights per size class (tune.cpp) ----
 enum TuneKind { kTuneFwdX, kTuneFwdY, kTuneFwdZ, kTuneInvZ, kTuneInvY, kTuneInvX, kTuneKinds };
 int tune_type_index(int dtype, bool vec);
