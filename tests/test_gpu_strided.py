@@ -42,3 +42,32 @@ def test_even_and_odd_layer_counts_agree(ctx, L, s, wavelet):
     back_odd = ctx.inverse_transform(odd, (Z - 1, X, L), (1, s, 0), wavelet, (X, L, Z - 1))
     assert np.array_equal(back[:Z - 1], back_odd)
     assert np.abs(back - vol).max() <= 4e-6 * np.abs(vol).max()
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.int32, np.float32])
+@pytest.mark.parametrize("L,s", CASES)
+def test_x_rows_of_every_type(ctx, L, s, dtype):
+    """The x passes: whole rows, rows cut short by the real length (REPEAT
+    padding and crop) and rows that start off the lane vectors."""
+    Y, Z = 6, 38
+    rng = np.random.default_rng(L * s)
+    for X in sorted({L, L - (1 << s) // 2, L - 1}):
+        if P.clamp_steps((s, 1, 0), (X, Y, Z)) != (s, 1, 0) or P.padded_length(X, s) != L:
+            continue
+        if dtype == np.float32:
+            vol = rng.normal(0, 100, (Z, Y, X)).astype(np.float32)
+        else:
+            vol = rng.integers(0, min(np.iinfo(dtype).max, 1 << 20) + 1, (Z, Y, X)).astype(dtype)
+        for wavelet in (P.HAAR, P.CDF97):
+            p = P.Params(steps=(s, 1, 0), wavelet=wavelet)
+            even, stored = ctx.forward_transform(vol, p)
+            odd, _ = ctx.forward_transform(vol[:Z - 1], p)
+            assert tuple(stored) == (Z, L, Y)
+            even, odd = even.reshape(Y, L, Z), odd.reshape(Y, L, Z - 1)
+            assert np.array_equal(even[:, :, :Z - 1], odd)
+            ref, _ = lifting64.forward(vol, (s, 1, 0), wavelet)
+            assert np.abs(even.ravel() - ref).max() <= 2e-6 * np.abs(ref).max()
+            back = ctx.inverse_transform(even, (Z, L, Y), (s, 1, 0), wavelet, (X, Y, Z), dtype)
+            back_odd = ctx.inverse_transform(odd, (Z - 1, L, Y), (s, 1, 0), wavelet,
+                                             (X, Y, Z - 1), dtype)
+            assert np.array_equal(back[:Z - 1], back_odd)

@@ -1,6 +1,8 @@
-// Wavelet passes along an axis that is strided in memory while consecutive
-// rows are neighbours on both sides (the y pass of either direction: z is
-// contiguous), entirely in registers.
+// Wavelet passes entirely in registers, for rows whose neighbours are
+// neighbours in memory: the y pass of either direction (strided rows on both
+// sides, z contiguous), the forward x pass (contiguous source rows of any
+// type, z contiguous in the output) and the inverse x pass (the reverse, into
+// rows of any type).
 //
 // A thread holds K consecutive elements of TWO neighbouring rows, packed as
 // pairs of floats: every lifting operation is one packed instruction
@@ -20,9 +22,20 @@
 // element (2.77 ms in the column-tile kernel), the inverse y passes of the
 // mixed batch 0.55 ms (1.22 ms through the row kernel's tile).
 //
+// The x passes read or write a lane's K elements of a source or output row
+// with vectors of 32 bytes (16 where its address or K asks for it), a run cut
+// by the real row length element by element; they take inputs in device memory
+// and outputs whose rows start at multiples of 16 bytes.
+// The inverse x passes of the mixed batch take 0.73 ms (1.47 ms through the
+// row kernel's tile); forward, the half of a 2 GiB volume's cubelets that the
+// kernel took first (before it accepted 16-byte starts) 0.71 ms against 0.91
+// ms for the other half in the row kernel.
+//
 // Each lifting step does the arithmetic of dwt.cu / dwt_cols.cu / dwt_rows.cu
 // (the same operands, rounded the same), so the values are identical.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "dwt_common.cuh"
 #include "wl_internal.h"
@@ -40,6 +53,14 @@ __device__ __forceinline__ f2 pack(float a) {
   f2 r;
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
   return r;
+}
+__device__ __forceinline__ f2 pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack(f2 v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
 __device__ __forceinline__ f2 add2(f2 a, f2 b) {
   f2 r;
@@ -204,34 +225,170 @@ __device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const float *rscal
   }
 }
 
-template <int K, int G, bool HAAR, bool INV>
+// ---- rows of the source and of the output (x passes) ----
+// bytes per vector access of a lane's K elements
+template <typename T, int K> __host__ __device__ constexpr int vec_bytes() {
+  return (K * (int)sizeof(T)) % 32 == 0 ? 32 : 16;
+}
+template <int VB> __device__ __forceinline__ void load_vec(const void *p, unsigned *w) {
+  if constexpr (VB == 32) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]),
+                   "=r"(w[6]), "=r"(w[7])
+                 : "l"(p));
+  } else {
+    const uint4 q = *static_cast<const uint4 *>(p);
+    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+  }
+}
+template <int VB> __device__ __forceinline__ void store_vec(void *p, const unsigned *w) {
+  if constexpr (VB == 32) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
+                    "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    *static_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+// element k of a vector of 32-bit words as a float, and back
+template <typename T> __device__ __forceinline__ float from_words(const unsigned *w, int k) {
+  if constexpr (std::is_same<T, float>::value) return __uint_as_float(w[k]);
+  else if constexpr (sizeof(T) == 4) return (float)(int)w[k];
+  else if constexpr (sizeof(T) == 2) return (float)((w[k / 2] >> (16 * (k & 1))) & 0xffffu);
+  else return (float)((w[k / 4] >> (8 * (k & 3))) & 0xffu);
+}
+template <typename T> __device__ __forceinline__ unsigned to_bits(float f) {
+  T t;
+  store_from_float(&t, f);
+  if constexpr (std::is_same<T, float>::value) return __float_as_uint(f);
+  else return (unsigned)t;
+}
+
+template <typename T, int K, int VB>
+__device__ __forceinline__ void load_vecs(const T *p, float (&v)[K]) {
+  constexpr int E = VB / (int)sizeof(T);
+#pragma unroll
+  for (int j = 0; j < K / E; j++) {
+    unsigned w[VB / 4];
+    load_vec<VB>(p + j * E, w);
+#pragma unroll
+    for (int k = 0; k < E; k++) v[j * E + k] = from_words<T>(w, k);
+  }
+}
+template <typename T, int K, int VB>
+__device__ __forceinline__ void store_vecs(T *p, const float (&v)[K]) {
+  constexpr int E = VB / (int)sizeof(T), P = 4 / (int)sizeof(T);
+#pragma unroll
+  for (int j = 0; j < K / E; j++) {
+    unsigned w[VB / 4];
+#pragma unroll
+    for (int i = 0; i < VB / 4; i++) {
+      w[i] = 0;
+#pragma unroll
+      for (int k = 0; k < P; k++)
+        w[i] |= to_bits<T>(v[j * E + i * P + k]) << (8 * (int)sizeof(T) * k);
+    }
+    store_vec<VB>(p + j * E, w);
+  }
+}
+
+// K elements [first, first + K) of a row of n real elements (REPEAT clamp)
+template <typename T, int K>
+__device__ __forceinline__ void load_run(const T *row, int first, int n, float (&v)[K]) {
+  if (first + K <= n) {
+    constexpr int VB = vec_bytes<T, K>();
+    if (VB == 32 && (reinterpret_cast<size_t>(row + first) & 31) == 0)
+      load_vecs<T, K, VB>(row + first, v);
+    else
+      load_vecs<T, K, 16>(row + first, v);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < K; k++) v[k] = load_as_float(row + min(first + k, n - 1));
+}
+template <typename T, int K>
+__device__ __forceinline__ void store_run(T *row, int first, int n, const float (&v)[K]) {
+  if (first + K <= n) {
+    constexpr int VB = vec_bytes<T, K>();
+    if (VB == 32 && (reinterpret_cast<size_t>(row + first) & 31) == 0)
+      store_vecs<T, K, VB>(row + first, v);
+    else
+      store_vecs<T, K, 16>(row + first, v);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (first + k < n) store_from_float(row + first + k, v[k]);
+}
+
+enum Pass { kStrided, kStridedInv, kSource, kOutput };  // y forward / inverse, x forward / inverse
+
+template <typename T, int K, int G, bool HAAR, int PASS>
 __device__ __forceinline__ void run_rows(const PassDesc &d, int tile, const float *scale) {
   constexpr int C = 32 / G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Along<G> at{lane / C};
   const int row = 2 * ((tile * (kThreads / 32) + warp) * C + lane % C);
-  Row in{nullptr, d.inSC, row < d.rows}, out{nullptr, d.outSC, row < d.rows};
-  if (in.ok) {
-    const int a = row / d.B, b = row - a * d.B;  // B even: b and b + 1 are one pair
-    in.base = const_cast<float *>(static_cast<const float *>(d.in)) + (long long)a * d.inSA + b;
-    out.base = static_cast<float *>(d.out) + (long long)a * d.outSA + b;
+  const bool ok = row < d.rows;
+  int a = 0, b = 0;
+  if (ok) {
+    a = row / d.B;
+    b = row - a * d.B;  // B even: b and b + 1 are one pair
   }
+  Row in{nullptr, d.inSC, ok}, out{nullptr, d.outSC, ok};
+  if (ok && PASS != kSource)
+    in.base = const_cast<float *>(static_cast<const float *>(d.in)) + (long long)a * d.inSA + b;
+  if (ok && PASS != kOutput)
+    out.base = static_cast<float *>(d.out) + (long long)a * d.outSA + b;
   f2 v[K];
-  if (INV) {
-    inv_to<0, K / 2, G, HAAR>(v, d.steps, scale, at, in);
-#pragma unroll
-    for (int k = 0; k < K; k++) out.put(K * at.seg + k, v[k]);
-  } else {
+  if constexpr (PASS == kStrided) {
 #pragma unroll
     for (int k = 0; k < K; k++) v[k] = in.get(K * at.seg + k);
+  }
+  if constexpr (PASS == kSource) {
+    float x[2][K];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const T *src = static_cast<const T *>(d.in) + (long long)min(a, d.clampA - 1) * d.inSA +
+                     (long long)min(b + r, d.clampB - 1) * d.inSB;
+      if (ok) {
+        load_run<T, K>(src, K * at.seg, min(K * G, d.clampL), x[r]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < K; k++) x[r][k] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = pack(x[0][k], x[1][k]);
+  }
+  if constexpr (PASS == kStrided || PASS == kSource) {
     fwd_from<0, K / 2, G, HAAR>(v, d.steps, scale, at, out);
+  } else {
+    inv_to<0, K / 2, G, HAAR>(v, d.steps, scale, at, in);
+    if constexpr (PASS == kStridedInv) {
+#pragma unroll
+      for (int k = 0; k < K; k++) out.put(K * at.seg + k, v[k]);
+    } else {
+      if (!ok || a >= d.cropA) return;
+      float x[2][K];
+#pragma unroll
+      for (int k = 0; k < K; k++) unpack(v[k], x[0][k], x[1][k]);
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+        if (b + r < d.cropB)
+          store_run<T, K>(static_cast<T *>(d.out) + (long long)a * d.outSA +
+                              (long long)(b + r) * d.outSB,
+                          K * at.seg, min(K * G, d.cropL), x[r]);
+    }
   }
 }
 
-template <int K, int G, bool INV>
+template <typename T, int K, int G, int PASS>
 __global__ void __launch_bounds__(kThreads)
 dwt_strided_kernel(const PassDesc *__restrict__ passes, const int *__restrict__ tilePrefix,
                    int nPasses) {
+  constexpr bool INV = PASS == kStridedInv || PASS == kOutput;
   __shared__ float scale[16];
   const int bid = blockIdx.x;
   int lo = 0, hi = nPasses - 1;
@@ -247,8 +404,8 @@ dwt_strided_kernel(const PassDesc *__restrict__ passes, const int *__restrict__ 
     scale[threadIdx.x] = INV && !haar ? 1.0f / s : s;
   }
   __syncthreads();
-  if (haar) run_rows<K, G, true, INV>(d, bid - tilePrefix[lo], scale);
-  else run_rows<K, G, false, INV>(d, bid - tilePrefix[lo], scale);
+  if (haar) run_rows<T, K, G, true, PASS>(d, bid - tilePrefix[lo], scale);
+  else run_rows<T, K, G, false, PASS>(d, bid - tilePrefix[lo], scale);
 }
 
 // lanes per row pair and elements per lane; 0: another kernel
@@ -262,10 +419,41 @@ int strided_lanes(int L) {
   }
 }
 
-template <int K, int G>
-void launch_kg(const PassDesc *p, const int *tp, int n, int blocks, bool inv, cudaStream_t s) {
-  if (inv) dwt_strided_kernel<K, G, true><<<blocks, kThreads, 0, s>>>(p, tp, n);
-  else dwt_strided_kernel<K, G, false><<<blocks, kThreads, 0, s>>>(p, tp, n);
+template <typename T, int PASS>
+void launch_len(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s) {
+  switch (L) {
+    case 16: dwt_strided_kernel<T, 16, 1, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    case 32: dwt_strided_kernel<T, 32, 1, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    case 48: dwt_strided_kernel<T, 48, 1, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    case 64: dwt_strided_kernel<T, 32, 2, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    case 96: dwt_strided_kernel<T, 48, 2, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    case 128: dwt_strided_kernel<T, 32, 4, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    case 192: dwt_strided_kernel<T, 48, 4, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+    default: dwt_strided_kernel<T, 32, 8, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
+  }
+}
+
+// the x passes by element type
+template <int PASS>
+void launch_type(const PassDesc *p, const int *tp, int n, int blocks, int L, int dtype,
+                 cudaStream_t s) {
+  switch (dtype) {
+    case WL_U8: launch_len<uint8_t, PASS>(p, tp, n, blocks, L, s); break;
+    case WL_U16: launch_len<uint16_t, PASS>(p, tp, n, blocks, L, s); break;
+    case WL_I32: launch_len<int32_t, PASS>(p, tp, n, blocks, L, s); break;
+    default: launch_len<float, PASS>(p, tp, n, blocks, L, s); break;
+  }
+}
+
+// length, levels and paired rows as the kernels take them
+bool shape_fits(const PassDesc &d) {
+  const int g = strided_lanes(d.L);
+  return g && d.steps >= 1 && d.B % 2 == 0 && d.steps <= (d.L / g == 32 ? 5 : 4);
+}
+// rows at base with these strides (elements of es bytes) start at multiples
+// of 16 bytes (K elements are a multiple of 16 bytes for every type)
+bool rows_aligned(const void *base, long long sa, long long sb, int es) {
+  return reinterpret_cast<size_t>(base) % 16 == 0 && sa * es % 16 == 0 && sb * es % 16 == 0;
 }
 
 }  // namespace
@@ -274,25 +462,28 @@ void launch_kg(const PassDesc *p, const int *tp, int n, int blocks, bool inv, cu
 int dwt_strided_rows_per_block(int L) { return 2 * (kThreads / 32) * (32 / strided_lanes(L)); }
 
 bool dwt_strided_fits(const PassDesc &d) {
-  const int g = strided_lanes(d.L);
-  if (!g || d.steps < 1 || d.B % 2 || d.inSB != 1 || d.outSB != 1) return false;
   // neighbouring row pairs stay eight-byte aligned
-  if ((d.inSA | d.inSC | d.outSA | d.outSC) & 1) return false;
-  return d.steps <= (d.L / g == 32 ? 5 : 4);
+  return shape_fits(d) && d.inSB == 1 && d.outSB == 1 &&
+         ((d.inSA | d.inSC | d.outSA | d.outSC) & 1) == 0;
+}
+bool dwt_strided_source_fits(const PassDesc &d, int es) {
+  return shape_fits(d) && d.inSC == 1 && d.outSB == 1 && ((d.outSA | d.outSC) & 1) == 0 &&
+         rows_aligned(d.in, d.inSA, d.inSB, es);
+}
+bool dwt_strided_output_fits(const PassDesc &d, int es) {
+  return shape_fits(d) && d.outSC == 1 && d.inSB == 1 && ((d.inSA | d.inSC) & 1) == 0 &&
+         rows_aligned(d.out, d.outSA, d.outSB, es);
 }
 
 void launch_dwt_strided(const PassDesc *p, const int *tp, int n, int blocks, int L, bool inverse,
                         cudaStream_t s) {
-  switch (L) {
-    case 16: launch_kg<16, 1>(p, tp, n, blocks, inverse, s); break;
-    case 32: launch_kg<32, 1>(p, tp, n, blocks, inverse, s); break;
-    case 48: launch_kg<48, 1>(p, tp, n, blocks, inverse, s); break;
-    case 64: launch_kg<32, 2>(p, tp, n, blocks, inverse, s); break;
-    case 96: launch_kg<48, 2>(p, tp, n, blocks, inverse, s); break;
-    case 128: launch_kg<32, 4>(p, tp, n, blocks, inverse, s); break;
-    case 192: launch_kg<48, 4>(p, tp, n, blocks, inverse, s); break;
-    default: launch_kg<32, 8>(p, tp, n, blocks, inverse, s); break;
-  }
+  if (inverse) launch_len<float, kStridedInv>(p, tp, n, blocks, L, s);
+  else launch_len<float, kStrided>(p, tp, n, blocks, L, s);
+}
+void launch_dwt_strided_x(const PassDesc *p, const int *tp, int n, int blocks, int L, int dtype,
+                          bool inverse, cudaStream_t s) {
+  if (inverse) launch_type<kOutput>(p, tp, n, blocks, L, dtype, s);
+  else launch_type<kSource>(p, tp, n, blocks, L, dtype, s);
 }
 
 }  // namespace wl

@@ -95,8 +95,12 @@ int rowreg_t_key(int dtype, int L) { return (1 << 21) | (dtype << 16) | L; }
 int rowreg_inv_key(int L) { return (1 << 23) | L; }
 int rowreg_inv_t_key(int outType, int L) { return (1 << 24) | (outType << 16) | L; }
 int strided_key(bool inverse, int L) { return (1 << (inverse ? 26 : 25)) | L; }
+int strided_x_key(bool inverse, int dtype, int L) {
+  return (1 << (inverse ? 28 : 27)) | (dtype << 16) | L;
+}
 enum RegKind { kRegNone, kRegInPlace, kRegTile, kRegInvInPlace, kRegInvTile, kRegStrided,
-               kRegInvStrided };
+               kRegInvStrided, kRegStridedX, kRegInvStridedX };
+bool strided_kind(int k) { return k >= kRegStrided; }
 
 // ---- result storage ------------------------------------------------------------
 // The arrays of all results of one compression call live in one page-locked
@@ -559,7 +563,9 @@ bool forward_passes_cols(const Plan &pl, const void *in, bool hostIn, float *coe
   d.out = o2;
   d.outSA = Zp; d.outSB = 1; d.outSC = Zp * Yp;
   d.steps = pl.sx;
-  if (dwt_rowreg_fits(d.L, d.steps)) {
+  if (!hostIn && dwt_strided_source_fits(d, dtype_size(pl.dtype))) {
+    xs[strided_x_key(false, pl.dtype, d.L)].push_back(d);
+  } else if (dwt_rowreg_fits(d.L, d.steps)) {
     d.T = dwt_rowreg_t_rows_per_block(d.L); d.tiles = (d.rows + d.T - 1) / d.T;
     xs[rowreg_t_key(pl.dtype, d.L)].push_back(d);
   } else {
@@ -755,9 +761,8 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
       return fail(ctx, WL_EINVAL, "internal: mixed select-gathering passes in one group");
   if (regL) {
     rows = (regKind == kRegTile || regKind == kRegInvTile) ? dwt_rowreg_t_rows_per_block(regL)
-           : (regKind == kRegStrided || regKind == kRegInvStrided)
-               ? dwt_strided_rows_per_block(regL)
-               : dwt_rowreg_rows_per_block(regL, sel);
+           : strided_kind(regKind) ? dwt_strided_rows_per_block(regL)
+                                   : dwt_rowreg_rows_per_block(regL, sel);
     for (PassDesc &d : g) {
       d.T = rows;
       d.tiles = (d.rows + rows - 1) / rows;
@@ -797,6 +802,11 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
 wl_status stage_groups(wl_ctx *ctx, const PassGroups &gs, size_t &hoff, int kind, int outType,
                        bool inverse, std::vector<GroupLaunch> &out) {
   for (const auto &kv : gs) {
+    if ((kv.first >> 27) & 1) {
+      TRY(stage_group(ctx, kv.second, hoff, kind, (kv.first >> 16) & 15, WL_F32, false, false, false,
+                      out, nullptr, kv.second[0].L, kRegStridedX));
+      continue;
+    }
     if ((kv.first >> 25) & 1) {
       TRY(stage_group(ctx, kv.second, hoff, kind, WL_F32, WL_F32, false, false, false, out, nullptr,
                       kv.second[0].L, kRegStrided));
@@ -819,6 +829,10 @@ wl_status launch_one(wl_ctx *ctx, const GroupLaunch &l, cudaStream_t s) {
   const int *dtp = reinterpret_cast<const int *>(base + l.off + l.n * sizeof(PassDesc));
   if (l.regKind == kRegStrided || l.regKind == kRegInvStrided)
     launch_dwt_strided(dp, dtp, l.n, l.tiles, l.regL, l.regKind == kRegInvStrided, s);
+  else if (l.regKind == kRegStridedX)
+    launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.inType, false, s);
+  else if (l.regKind == kRegInvStridedX)
+    launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.outType, true, s);
   else if (l.regKind == kRegTile)
     launch_dwt_rowreg_t(dp, dtp, l.n, l.tiles, l.regL, l.inType, s);
   else if (l.regKind == kRegInvInPlace)
@@ -1383,7 +1397,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       const wl_params &q = pl.p;
       uint32_t fb;
       memcpy(&fb, &q.threshold_fraction, 4);
-      const long long v[] = {pl.dtype | (hostIn[i] << 8), pl.X, pl.Y, pl.Z, pl.pitchY, pl.pitchZ,
+      // which x pass kernel a cubelet takes depends on its address modulo 16
+      const long long align = (long long)(reinterpret_cast<size_t>(dIn[i]) & 15);
+      const long long v[] = {pl.dtype | (hostIn[i] << 8) | (align << 16), pl.X, pl.Y, pl.Z, pl.pitchY, pl.pitchZ,
                              q.steps[0], q.steps[1], q.steps[2], q.wavelet, (long long)fb,
                              q.bin_count, q.quant_alg, q.compress_zeros, q.lloyd_iters,
                              q.exact_transform, q.transform_2d};
@@ -1645,6 +1661,8 @@ void inverse_passes(const int size[3], const int steps[3], int wavelet, const in
         ph[0][rowreg_inv_key(d[i].L)].push_back(d[i]);
       else if (phase == 1 && dwt_strided_fits(d[i]))  // y rows in registers
         ph[1][strided_key(true, d[i].L)].push_back(d[i]);
+      else if (phase == 2 && dwt_strided_output_fits(d[i], dtype_size(outType)))
+        ph[2][strided_x_key(true, outType, d[i].L)].push_back(d[i]);
       else if (phase > 0 && dwt_rowreg_fits(d[i].L, d[i].steps))  // y, x: through a tile
         ph[phase][rowreg_inv_t_key(phase == 2 ? outType : WL_F32, d[i].L)].push_back(d[i]);
       else
@@ -1699,6 +1717,11 @@ wl_status stage_inverse_phases(wl_ctx *ctx, PassGroups ph[3], InversePhases &ip)
   const int kinds[3] = {kTuneInvZ, kTuneInvY, kTuneInvX};
   for (int k = 0; k < 3; k++) {
     for (const auto &kv : ph[k]) {
+      if ((kv.first >> 28) & 1) {
+        TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, (kv.first >> 16) & 15, true, false,
+                        false, gl, nullptr, kv.second[0].L, kRegInvStridedX));
+        continue;
+      }
       if ((kv.first >> 26) & 1) {
         TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, WL_F32, true, false, false, gl,
                         nullptr, kv.second[0].L, kRegInvStrided));

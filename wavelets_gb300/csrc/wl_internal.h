@@ -293,9 +293,14 @@ void launch_dwt_rowreg_inv_t(const PassDesc *d_passes, const int *d_tilePrefix, 
 void launch_dwt_rowreg_t(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
                          int blocks, int L, int inType, cudaStream_t s);
 
-// passes along a strided axis whose rows are neighbours in memory (the y
-// passes), in registers (dwt_strided.cu)
+// passes in registers whose neighbouring rows are neighbours in memory
+// (dwt_strided.cu): the y passes; the forward x pass of source rows of es-byte
+// elements in device memory; the inverse x pass into such rows
 bool dwt_strided_fits(const PassDesc &d);
+bool dwt_strided_source_fits(const PassDesc &d, int es);
+bool dwt_strided_output_fits(const PassDesc &d, int es);
+void launch_dwt_strided_x(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
+                          int blocks, int L, int dtype, bool inverse, cudaStream_t s);
 int dwt_strided_rows_per_block(int L);
 void launch_dwt_strided(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
                         int L, bool inverse, cudaStream_t s);
