@@ -62,8 +62,8 @@ struct Plan {
   long long n;
   long long inOff;     // bytes into the input staging buffer (host inputs)
   long long coefOff;   // elements
-  long long chunkBase;
-  int nChunks;
+  long long chunkBase;  // token chunks
+  int nChunks, selChunks;
   long long wordsCap;
   int tableOff;
   bool identity;       // all steps zero: no transform, no axis rotation
@@ -307,7 +307,7 @@ struct wl_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   DevBuf input, coef, coef2, bins, tokCount, state, selHist, lloydHist, qtable, dqtable, qlut,
-      hist, chunkRun, chunkBits, chunkCub, groupCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
+      hist, chunkRun, chunkBits, chunkCub, groupCub, quantCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
       words, passes, outbuf, head, decWords, decTable, decWs, meta, optIn, optOut, optErr,
       errIn, errRest, errPart;
   HostBuf hState, hDecode, hPasses, hTab, hIn, hFlags, hHead, hSel;
@@ -923,7 +923,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   if (n <= 0) return fail(ctx, WL_EINVAL, "empty batch");
   CU(cudaSetDevice(ctx->device));
   std::vector<Plan> plans(n);
-  long long coefTotal = 0, chunkTotal = 0, inBytes = 0, wordsTotal = 0;
+  long long coefTotal = 0, chunkTotal = 0, selTotal = 0, inBytes = 0, wordsTotal = 0;
   int tableTotal = 0, maxS = 2, maxTable = 0, maxLloyd = 3;
   bool anyLog = false, anyLloyd = false;
   for (int i = 0; i < n; i++) {
@@ -970,9 +970,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     inBytes += ((long long)pl.X * pl.Y * pl.Z * dtype_size(pl.dtype) + 255) & ~255LL;
     pl.coefOff = coefTotal;
     coefTotal += (pl.n + 63) & ~63LL;
-    pl.chunkBase = chunkTotal;
-    pl.nChunks = (int)((pl.n + kChunk - 1) / kChunk);
-    chunkTotal += pl.nChunks;
+    pl.selChunks = (int)((pl.n + kChunk - 1) / kChunk);
+    selTotal += pl.selChunks;
     // Huffman output bound: < log2(symbols)+1 bits per token plus 3 per dup token
     pl.wordsCap = pl.n / 2 + 64;
     wordsTotal += pl.wordsCap;
@@ -986,6 +985,13 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     if (pl.p.quant_alg == WL_LLOYD) anyLloyd = true;
   }
 
+  const int lgChunk = token_chunk_lg(coefTotal);
+  for (Plan &pl : plans) {
+    pl.chunkBase = chunkTotal;
+    pl.nChunks = (int)((pl.n + (1LL << lgChunk) - 1) >> lgChunk);
+    chunkTotal += pl.nChunks;
+  }
+
   // ---- workspace ----
   TRY(ensure(ctx, ctx->coef, coefTotal * 4));
   TRY(ensure(ctx, ctx->coef2, coefTotal * 4));
@@ -993,7 +999,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   TRY(ensure(ctx, ctx->tokCount, chunkTotal * sizeof(int)));
   TRY(ensure(ctx, ctx->state, n * sizeof(CubeletState)));
   TRY(ensure(ctx, ctx->chunkCub, chunkTotal * sizeof(int)));
-  TRY(ensure(ctx, ctx->groupCub, chunkTotal * sizeof(int)));
+  TRY(ensure(ctx, ctx->groupCub, selTotal * sizeof(int)));
+  TRY(ensure(ctx, ctx->quantCub, chunkTotal * sizeof(int)));
   TRY(ensure(ctx, ctx->encCub, chunkTotal * sizeof(int)));
   TRY(ensure(ctx, ctx->sliceOff, chunkTotal * 32 * sizeof(unsigned)));
   TRY(ensure(ctx, ctx->selHist, (size_t)n * kSelectBins * 4));
@@ -1122,17 +1129,20 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   CubeletDev *hc = reinterpret_cast<CubeletDev *>(H<char>(ctx->hPasses) + slabBytes);
   long long *hp = reinterpret_cast<long long *>(H<char>(ctx->hPasses) + slabBytes + cubBytes);
   long long groupTotal = 0, encTotal = 0;
-  long long chunk0[2] = {0, 0}, group0[2] = {0, 0}, words0[2] = {0, 0}, enc0[2] = {0, 0};
+  long long quantTotal = 0;
+  long long chunk0[2] = {0, 0}, group0[2] = {0, 0}, quant0[2] = {0, 0}, words0[2] = {0, 0},
+            enc0[2] = {0, 0};
   long long wordsAcc = 0;
-  // bit-packer slices per chunk and chunks per quantize group, from each
-  // half's chunk count
+  // bit-packer slices per token chunk and chunks per select group, from each
+  // half's size
   int encF[2] = {1, 1}, group[2] = {1, 1};
   {
     long long halfChunks[2] = {0, 0};
-    for (int i = 0; i < n; i++) halfChunks[half_of(i)] += plans[i].nChunks;
+    for (int i = 0; i < n; i++) halfChunks[half_of(i)] += plans[i].selChunks;
     for (int h = 0; h < nh; h++) {
-      encF[h] = ctx->encSlices ? ctx->encSlices : enc_slices(halfChunks[h]);
-      group[h] = quant_group(halfChunks[h]);
+      const int per = ctx->encSlices ? ctx->encSlices : enc_slices(halfChunks[h]);
+      encF[h] = std::max(1, per >> (kMaxLgChunk - lgChunk));
+      group[h] = sel_group(halfChunks[h]);
     }
   }
   for (int i = 0; i < n; i++) {
@@ -1141,6 +1151,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     if (i == hc0[h]) {
       chunk0[h] = pl.chunkBase;
       group0[h] = groupTotal;
+      quant0[h] = quantTotal;
       words0[h] = wordsAcc;
       enc0[h] = encTotal;
     }
@@ -1152,6 +1163,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     c.wordsOff = 0;
     c.wordsCap = pl.wordsCap;
     c.nChunks = pl.nChunks;
+    c.selChunks = pl.selChunks;
+    c.quantBase = (int)(quantTotal - quant0[h]);
+    quantTotal += (pl.nChunks + kQuantWarps - 1) / kQuantWarps;
     c.binCount = pl.p.bin_count;
     c.quantAlg = pl.p.quant_alg;
     c.compressZeros = pl.p.compress_zeros ? 1 : 0;
@@ -1159,7 +1173,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     c.lloydIters = pl.p.lloyd_iters > 0 ? pl.p.lloyd_iters : 20;
     c.tableOff = pl.tableOff;
     c.groupBase = (int)(groupTotal - group0[h]);
-    groupTotal += (pl.nChunks + group[h] - 1) / group[h];
+    groupTotal += (pl.selChunks + group[h] - 1) / group[h];
     c.encBase = (int)(encTotal - enc0[h]);
     encTotal += ((long long)pl.nChunks * encF[h] + kEncThreads - 1) / kEncThreads;
     wordsAcc += pl.wordsCap;
@@ -1191,6 +1205,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.chunkPrefix = reinterpret_cast<long long *>(P<char>(ctx->passes) + slabBytes + cubBytes);
   b.chunkCub = P<int>(ctx->chunkCub);
   b.groupCub = P<int>(ctx->groupCub);
+  b.quantCub = P<int>(ctx->quantCub);
+  b.totalQuant = quantTotal;
+  b.lgChunk = lgChunk;
   b.totalGroups = groupTotal;
   b.group = group[0];
   b.encCub = P<int>(ctx->encCub);
@@ -1248,6 +1265,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       v.chunkBits += ch;
       v.chunkCub += ch;
       v.groupCub += g;
+      v.quantCub += quant0[h];
+      v.totalQuant = (h ? quantTotal : quant0[1]) - quant0[h];
       v.encCub += enc0[h];
       v.totalEnc = (h ? encTotal : enc0[1]) - enc0[h];
       v.encF = encF[h];
@@ -1297,7 +1316,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     ctx->launches += 1;
     if (anyLloyd) { launch_lloyd(v, v.coef, maxLloyd, st); ctx->launches += 3; }
     if (first) mark(ctx, 5);
-    launch_quantize(v, v.coef, maxTable, maxS, st);
+    launch_quantize(v, v.coef, maxTable, maxS, anyLloyd, st);
     if (first) mark(ctx, 6);
     launch_runs(v, st);
     ctx->launches += 2;
@@ -2447,7 +2466,7 @@ void wl_destroy(wl_ctx *ctx) {
   DevBuf *dbs[] = {&ctx->input, &ctx->coef, &ctx->coef2, &ctx->bins, &ctx->tokCount,
                    &ctx->state,
                    &ctx->selHist, &ctx->lloydHist, &ctx->qtable, &ctx->dqtable, &ctx->qlut, &ctx->hist,
-                   &ctx->chunkRun, &ctx->chunkBits, &ctx->chunkCub, &ctx->groupCub,
+                   &ctx->chunkRun, &ctx->chunkBits, &ctx->chunkCub, &ctx->groupCub, &ctx->quantCub,
                    &ctx->encCub, &ctx->sliceOff,
                    &ctx->chunkSpan, &ctx->optIn, &ctx->optOut, &ctx->optErr,
                    &ctx->codes, &ctx->codeLen, &ctx->decode, &ctx->words, &ctx->passes,

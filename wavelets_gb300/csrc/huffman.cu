@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
 // before any lane of the chunk ORs (the chunk's lanes are one warp); the
 // chunk's first and last words, shared with neighbouring chunks, were zeroed
 // by encode_zero_kernel.  Tokens are read with 16-byte loads: a slot starts
-// at a multiple of 128 bytes and holds kChunk tokens, so the aligned blocks
+// at a multiple of 128 bytes and holds a token per element, so the aligned blocks
 // around a slice stay inside its chunk's slot.
 
 // code bits (below kMaxCodeBits) and length (above) of one symbol
@@ -392,9 +392,9 @@ __global__ void __launch_bounds__(kEncThreads) encode_count_kernel(DevBatch b) {
   for (int i = threadIdx.x; i < S; i += kEncThreads) sLen[i] = b.codeLen[(size_t)ci * kMaxSymbols + i];
   __syncthreads();
   const SliceAt sl = slice_at(b, cd, lgF);
-  unsigned mine = 0;  // at most kChunk tokens of at most 61 bits
+  unsigned mine = 0;  // at most 4096 tokens of at most 61 bits
   if (sl.ok) {
-    const uint16_t *slot = b.tok + cd.coefOff + (long long)sl.cl * kChunk;
+    const uint16_t *slot = b.tok + cd.coefOff + ((long long)sl.cl << b.lgChunk);
     for_tokens(slot, sl.span.x + sl.t0, sl.span.x + sl.t1, sLen, [&](unsigned t, uint8_t l) {
       mine += l + ((int)(t & 0x1fff) == dupKey ? 3u : 0u);
     });
@@ -410,31 +410,51 @@ __global__ void __launch_bounds__(kEncThreads) encode_count_kernel(DevBatch b) {
   }
 }
 
-// per cubelet: exclusive scan of the chunk bit counts
+// Per cubelet: exclusive scan of the chunk bit counts, kScanRun consecutive
+// chunks per thread, so that one round covers 8192 chunks (the most a call
+// that fills no more than the GPU has: a round is all latency).
+constexpr int kScanRun = 8;
 __global__ void __launch_bounds__(1024) encode_scan_kernel(DevBatch b) {
-  __shared__ unsigned long long sh[64];
+  __shared__ unsigned long long sh[32];
   const int ci = blockIdx.x;
   const CubeletDev cd = b.cub[ci];
   CubeletState *st = b.state + ci;
   unsigned long long carry = 0;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int seg = 0; seg < cd.nChunks; seg += 1024) {
-    const int c = seg + threadIdx.x;
-    const unsigned long long v = c < cd.nChunks ? b.chunkBits[cd.chunkBase + c] : 0;
-    unsigned long long inc = v;
+  unsigned long long *bits = b.chunkBits + cd.chunkBase;
+  for (int seg = 0; seg < cd.nChunks; seg += 1024 * kScanRun) {
+    const int c0 = seg + threadIdx.x * kScanRun;
+    unsigned v[kScanRun];  // at most 4096 tokens of 61 bits each
+    unsigned mine = 0;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) {
+      v[k] = c0 + k < cd.nChunks ? (unsigned)bits[c0 + k] : 0u;
+      mine += v[k];
+    }
+    unsigned long long inc = mine;
+#pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      unsigned long long t = __shfl_up_sync(0xffffffffu, inc, off);
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, off);
       if (lane >= off) inc += t;
     }
     if (lane == 31) sh[w] = inc;
     __syncthreads();
-    unsigned long long before = 0, total = 0;
-    for (int i = 0; i < 32; i++) {
-      if (i < w) before += sh[i];
-      total += sh[i];
+    // the warps before this one, and all of them
+    unsigned long long all = sh[lane], before = all;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, before, off);
+      if (lane >= off) before += t;
     }
-    if (c < cd.nChunks) b.chunkBits[cd.chunkBase + c] = carry + before + inc - v;
-    carry += total;
+    all = __shfl_sync(0xffffffffu, before, 31);
+    const unsigned long long upTo = __shfl_sync(0xffffffffu, before, w > 0 ? w - 1 : 0);
+    unsigned long long at = carry + (w > 0 ? upTo : 0) + inc - mine;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) {
+      if (c0 + k < cd.nChunks) bits[c0 + k] = at;
+      at += v[k];
+    }
+    carry += all;
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -589,7 +609,7 @@ __global__ void __launch_bounds__(kEncThreads, 8) encode_write_kernel(DevBatch b
   unsigned nxt = __shfl_down_sync(0xffffffffu, rel, 1, F);
   if (sl.sub == F - 1) nxt = (unsigned)(end - off);
   const unsigned long long sb = nxt - rel, pos = off + rel;
-  const uint16_t *slot = b.tok + cd.coefOff + (long long)sl.cl * kChunk;
+  const uint16_t *slot = b.tok + cd.coefOff + ((long long)sl.cl << b.lgChunk);
   uint32_t *gw = b.words + st->wordsBase;
   const bool any = sl.ok && sb > 0;
   if (any && F > 1) {

@@ -8,7 +8,8 @@
 // (v = 0..7, greedy, longest first, HuffmanDup huffman.h:13-58) plus single
 // zero-bin tokens.
 //
-// A chunk of 4096 consecutive coefficients (reference Z-X-Y order) is one CTA.
+// A token chunk of 512 to 4096 consecutive coefficients (reference Z-X-Y order)
+// is one warp's.
 // Runs wholly inside a chunk are decomposed there; runs that touch a chunk
 // edge are joined across chunks by runs_kernel, which also records for every
 // chunk where the run entering it started and where the run leaving it ends,
@@ -20,8 +21,6 @@
 // because the device has no bit-identical logf; the codebook quantizer is the
 // reference's lower_bound with its last-boundary special case.
 #include <cfloat>
-
-#include <type_traits>
 
 #include "wl_internal.h"
 
@@ -396,27 +395,29 @@ __device__ __forceinline__ QParams load_qparams(const CubeletDev &cd, const Cube
 // in order: a token for every value that is not the zero bin, preceded by the
 // tokens of the zero-bin run before it when that run starts inside the chunk.
 // Runs touching a chunk edge are left to runs_kernel (counts) and the encoder
-// (tokens).  A CTA codes b.group consecutive chunks of one cubelet; warp
-// w owns elements [512 w, 512 w + 512) of each chunk, and everything but one
-// CTA barrier per chunk is warp-local.
+// (tokens).
 //
-// Phase 1 (every element): -thr < x < thr is the zero bin for all three
-// quantizers (uniform and log test |x| <= thr first; the codebook has the
-// boundaries -thr and thr around its zero bin and none in between), so an
-// element costs two compares.  The others are candidates, compacted into the
-// warp's region of shared memory (in word j lane l holds element
-// 512 w + 32 j + l, so loads are coalesced).
-// Phase 2 (per candidate, 32 at a time): the exact bin; a candidate that is
-// not the zero bin is a value.  The zero run before a value ends at the
-// previous value -- the nearest lower lane with one, or the warp's last value
-// of earlier rounds -- so its token count is known here, a warp scan gives
-// each lane its place among the warp's tokens, and the lane stages its run
-// tokens and value token in the warp's buffer (prefilled with the single
-// zero-bin token, so only dup tokens and the value token are stored).
-// After the CTA barrier the warp summaries (first and last value, staged
-// count) give every warp the run before its first value and its place in the
-// chunk, and each warp writes that run's tokens and its staged ones to the
-// chunk's slot with coalesced stores.
+// One warp codes one chunk from its first element to its last, so nothing but
+// the tables and the histogram is shared and there is no barrier inside.  It
+// reads kBlock = 512 elements at a time, 16 consecutive ones per lane (the
+// next block's loads are in flight meanwhile):
+//  - -thr < x < thr is the zero bin for all three quantizers (uniform and log
+//    test |x| <= thr first; the codebook has the boundaries -thr and thr
+//    around its zero bin and none in between), so an element costs a compare;
+//    the positions of the others, the candidates, are appended in order to
+//    the warp's queue (a scan over the lanes' counts places them);
+//  - whenever the queue holds 32 candidates, one per lane, a round gives each
+//    its exact bin (its value is read again, from L1); those that are not the
+//    zero bin are values.  A value's gap to the one before it (the nearest
+//    lower lane with one, else the last value of earlier rounds) gives its
+//    run tokens, a scan its place, and the round's tokens are staged in shared
+//    memory -- prefilled with the single zero-bin token, so only dup tokens
+//    and value tokens are stored -- and written to the chunk's slot two at a
+//    time.
+// Full rounds whatever the density, and no work for the zero bin beyond the
+// compare: 729 cubelets of 128^3 (3% kept) quantize in 1.76 ms, 2.85 ms with
+// eight warps to a chunk that met at a barrier; the kernel is bound by its
+// instructions (issue slots 60% busy).
 // Greedy split of a zero-bin run into dup tokens and single zero-bin tokens
 // (HuffmanDup::dupCount, huffman.h:46-57) in closed form: runs of 1024, then
 // one dup token per set bit of the remainder at or above 8 -- except that a
@@ -433,148 +434,70 @@ __device__ __forceinline__ void run_split_closed(int L, int &singles, int &dups)
   }
 }
 
-// Tokens of a zero-bin run of L < 2^31 elements lying inside one chunk, in
-// the order of run_tokens (whole run, no window): runs of 1024, then one dup
-// token per set bit of the remainder above 8, then single zero-bin tokens.
-template <class F>
-__device__ __forceinline__ void run_tokens_short(int L, int dupKey, int dupV, F f) {
-  for (int j = L >> 10; j > 0; j--) f(make_token(dupKey, 7));
-  int r = L & 1023;
-  while (r > 8) {
-    const int lg = 31 - __clz(r);
-    f(make_token(dupKey, lg - 3));
-    r -= 1 << lg;
-  }
-  for (; r > 0; r--) f(make_token(dupV, 0));
-}
 
-// Token j of run_tokens_short(L, dupKey, dupV) (j below the run's count).
-__device__ __forceinline__ uint16_t run_token_at(int L, int j, int dupKey, int dupV) {
-  const int q = L >> 10;
-  if (j < q) return make_token(dupKey, 7);
-  j -= q;
-  int r = L & 1023;
-  while (r > 8) {
-    const int lg = 31 - __clz(r);
-    if (j == 0) return make_token(dupKey, lg - 3);
-    j--;
-    r -= 1 << lg;
-  }
-  return make_token(dupV, 0);
-}
+constexpr int kBlock = 512, kLaneRun = kBlock / 32;
+constexpr int kQueue = 576;  // less than 32 left over and a block's candidates
+// a round's tokens: a value and at most 17 run tokens per lane (three runs of
+// 1024, one per bit from 512 to 16, the eight and seven singles or eight
+// singles), and one slot for the parity of the place they go to
+constexpr int kStage = 592;
+static_assert(kStage >= 32 * 18 + 2 && kStage % 8 == 0 && kQueue % 8 == 0, "16-byte rows");
+constexpr int kWarpBytes = (kQueue + kStage) * 2;
 
-__global__ void __launch_bounds__(kThreads, 4)
-quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff) {
-  constexpr int kWords = kChunk / kThreads;  // 16 words of 32 elements per warp
-  constexpr int kSpan = 32 * kWords;         // elements per warp
-  constexpr int kWarps = kThreads / 32;
+__global__ void __launch_bounds__(32 * kQuantWarps, 4)
+quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lutOff, int warpOff) {
   constexpr unsigned kAll = 0xffffffffu;
-  // sized by the launch: the quantizer table (Lloyd / log), then the counts
-  // of the batch's largest alphabet
-  extern __shared__ float tab[];
+  // sized by the launch: the quantizer table (Lloyd / log), the counts of the
+  // batch's largest alphabet, the Lloyd cell table, then the warps' buffers
+  extern __shared__ __align__(16) float tab[];
   unsigned *hist = reinterpret_cast<unsigned *>(tab + histOff);
-  __shared__ __align__(16) uint16_t sLut[kLutStride];
-  // by warp region: candidate values and positions (32 extra slots: a dump
-  // for the stores of lanes without a candidate, which keeps the compaction
-  // free of branches)
-  __shared__ __align__(16) float sX[kChunk + 32];
-  __shared__ uint16_t sPos[kChunk + 32];
-  // per warp: its tokens after its first value's zero run, in order (at
-  // most kSpan: each token starts at its own element of the warp's span)
-  __shared__ __align__(16) uint16_t sStage[kWarps][kSpan];
-  // per-warp summaries (first and last value position, staged tokens), two
-  // sets used by alternate chunks
-  __shared__ int wLast[2][kWarps], wFirst[2][kWarps], wTok[2][kWarps];
-  const int ci = b.groupCub[blockIdx.x];
+  uint16_t *lut = reinterpret_cast<uint16_t *>(tab + lutOff);
+  const int ci = b.quantCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
   const CubeletState *st = b.state + ci;
   const QParams q = load_qparams(cd, st);
   const int dupV = st->dupValue;
   const int B = cd.binCount;
   const int nTab = q.alg == WL_LLOYD ? q.nb : (q.alg == WL_LOG ? q.nPos + q.nNeg : 0);
-  const int c0 = ((int)blockIdx.x - cd.groupBase) * b.group;  // first chunk of the cubelet
-  const int nc = min(b.group, cd.nChunks - c0);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int base = w * kSpan;
+  const int c = ((int)blockIdx.x - cd.quantBase) * kQuantWarps + w;  // the warp's chunk
   const unsigned ltMask = (1u << lane) - 1u;
   // zero-bin elements (-thr < x < thr) can be skipped only when they are
   // coded as runs; without runs every element is a candidate (|x| < 0 never)
   const float zthr = dupV >= 0 ? q.thr : 0.f;
-  uint16_t *stage = sStage[w];
+  uint16_t *queue = reinterpret_cast<uint16_t *>(tab + warpOff) + w * (kQueue + kStage);
+  uint16_t *stage = queue + kQueue;
   const unsigned fill2 = dupV >= 0 ? (unsigned)make_token(dupV, 0) * 0x10001u : 0u;
-  int singles = 0, dups = 0;  // the lane's zero-run tokens, over all chunks
+  const uint4 fill8 = make_uint4(fill2, fill2, fill2, fill2);
 
-  for (int i = threadIdx.x; i < B + 1; i += kThreads) hist[i] = 0;
-  for (int i = threadIdx.x; i < nTab; i += kThreads) tab[i] = b.qtable[cd.tableOff + i];
+  for (int i = threadIdx.x; i < B + 1; i += blockDim.x) hist[i] = 0;
+  for (int i = threadIdx.x; i < nTab; i += blockDim.x) tab[i] = b.qtable[cd.tableOff + i];
   if (q.alg == WL_LLOYD) {
     const uint4 *gl = reinterpret_cast<const uint4 *>(b.qlut + (size_t)ci * kLutStride);
-    uint4 *sl = reinterpret_cast<uint4 *>(sLut);
-    for (int i = threadIdx.x; i < kLutStride / 8; i += kThreads) sl[i] = gl[i];
+    uint4 *sl = reinterpret_cast<uint4 *>(lut);
+    for (int i = threadIdx.x; i < kLutStride / 8; i += blockDim.x) sl[i] = gl[i];
   }
+  for (int i = lane; i < kStage / 8; i += 32) reinterpret_cast<uint4 *>(stage)[i] = fill8;
   __syncthreads();
 
-  for (int k = 0; k < nc; k++) {
-    const int par = k & 1;
-    const long long chunk = cd.chunkBase + c0 + k;
-    const long long start = (long long)(c0 + k) * kChunk;
-    const int len = (int)min((long long)kChunk, cd.n - start);
+  if (c < cd.nChunks) {
+    const long long start = (long long)c << b.lgChunk;
+    const int len = (int)min(1LL << b.lgChunk, cd.n - start);
     const float *src = coef + cd.coefOff + start;
+    uint16_t *slot = b.tok + cd.coefOff + start;
+    int singles = 0, dups = 0;           // the lane's zero-run tokens
+    int lead = -1, last = -1, nTok = 0;  // warp-uniform: first and last value, tokens so far
 
-    // ---- phase 1: candidates into the warp's region; the warp's staging
-    // buffer is prefilled with single zero-bin tokens
-    if (dupV >= 0) {
-      uint4 *s4 = reinterpret_cast<uint4 *>(stage);
-      const uint4 f4 = make_uint4(fill2, fill2, fill2, fill2);
-      s4[lane] = f4;
-      s4[lane + 32] = f4;
-    }
-    int nCand = 0;  // warp-uniform
-    auto phase1 = [&](auto full) {
-      constexpr bool kFull = decltype(full)::value;
-      float x[kWords];
-#pragma unroll
-      for (int j = 0; j < kWords; j++) {
-        const int pos = base + 32 * j + lane;
-        x[j] = (kFull || pos < len) ? src[pos] : 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < kWords; j++) {
-        const int pos = base + 32 * j + lane;
-        // zero bin iff |x| < zthr (NaN is a candidate)
-        const bool cand = (kFull || pos < len) && !(fabsf(x[j]) < zthr);
-        const unsigned m = __ballot_sync(kAll, cand);
-        const int l = cand ? base + nCand + __popc(m & ltMask) : kChunk + lane;
-        sX[l] = x[j];
-        sPos[l] = (uint16_t)pos;
-        nCand += __popc(m);
-      }
-    };
-    if (len == kChunk) phase1(std::true_type());
-    else phase1(std::false_type());
-    __syncwarp();
-
-    // ---- phase 2 (per candidate, 32 at a time): the exact bin; a value
-    // (not the zero bin) gets its token and the tokens of the zero run
-    // since the warp's previous value, staged in the warp's buffer.  Single
-    // zero-bin tokens are already there (prefilled), so a lane stores only
-    // its dup tokens (gaps above 8) and its value token.  The warp's first
-    // value stages its own token only: the run before it reaches into
-    // earlier warps and is coded at the copy-out.
-    // (without branches around the loads: lanes past the candidates
-    // quantize whatever their slot of the warp's region holds -- every
-    // quantizer reads only its bounded tables -- and are not values)
-    int nStaged = 0;                  // warp-uniform
-    int firstPos = -1, lastPos = -1;  // warp-uniform: the warp's values so far
-    for (int r = 0; 32 * r < nCand; r++) {
-      const int l = 32 * r + lane;  // < 512: inside the warp's region
-      const int bin = quant_value(sX[base + l], q, tab, sLut);
-      const int pos = sPos[base + l];
-      const bool v = l < nCand && bin != dupV;
+    // one round: candidates queue[at .. at + n), n <= 32
+    auto round = [&](int at, int n) {
+      const int pos = lane < n ? queue[at + lane] : 0;
+      const int bin = quant_value(src[pos], q, tab, lut);
+      const bool v = lane < n && bin != dupV;
       const unsigned m = __ballot_sync(kAll, v);
-      if (m == 0) continue;
+      if (m == 0) return;
       const unsigned lower = m & ltMask;
       const int pp = __shfl_sync(kAll, pos, lower ? 31 - __clz(lower) : 0);
-      const int prev = lower ? pp : lastPos;
+      const int prev = lower ? pp : last;
       const int gap = v && prev >= 0 ? pos - prev - 1 : 0;
       int sg, dp;
       run_split_closed(gap, sg, dp);  // 0, 0 for gap 0
@@ -587,115 +510,122 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff) {
         const int t = __shfl_up_sync(kAll, inc, d);
         if (lane >= d) inc += t;
       }
+      if (lead < 0) lead = __shfl_sync(kAll, pos, __ffs(m) - 1);
+      last = __shfl_sync(kAll, pos, 31 - __clz(m));
+      const int total = __shfl_sync(kAll, inc, 31);
+      const int par = (lead + nTok) & 1;  // tokens pair up as their places do
       if (v) {
-        int t = nStaged + inc - cnt;
-        // dup tokens in the order of run_tokens_short: runs of 1024, then
-        // one per set bit of the remainder from 512 down to 16, then 8 when
-        // more than 8 remain; the rest are single (prefilled) tokens
+        int t = par + inc - cnt;
+        // dup tokens in the order of run_tokens: runs of 1024, then one per
+        // set bit of the remainder from 512 down to 16, then 8 when more than
+        // 8 remain; the rest are single (prefilled) tokens
         for (int j = gap >> 10; j > 0; j--) stage[t++] = make_token(B, 7);
         const int rr = gap & 1023;
+        if (rr >= 16) {
 #pragma unroll
-        for (int lg = 9; lg >= 4; lg--)
-          if ((rr >> lg) & 1) stage[t++] = make_token(B, lg - 3);
+          for (int lg = 9; lg >= 4; lg--)
+            if ((rr >> lg) & 1) stage[t++] = make_token(B, lg - 3);
+        }
         const bool eight = (rr & 8) && (rr & 7);
         if (eight) stage[t++] = make_token(B, 0);
         t += (rr & 8) && !eight ? 8 : (rr & 7);
         stage[t] = make_token(bin, 0);
         atomicAdd(&hist[bin], 1u);
       }
-      if (firstPos < 0) firstPos = __shfl_sync(kAll, pos, __ffs(m) - 1);
-      lastPos = __shfl_sync(kAll, pos, 31 - __clz(m));
-      nStaged += __shfl_sync(kAll, inc, 31);
-    }
-    if (lane == 0) {
-      wFirst[par][w] = firstPos;
-      wLast[par][w] = lastPos;
-      wTok[par][w] = nStaged;
-    }
-    __syncthreads();
+      __syncwarp();
+      {
+        uint16_t *g = slot + lead + nTok - par;  // an even place
+        const int end = par + total;
+        const unsigned *s2 = reinterpret_cast<const unsigned *>(stage);
+        for (int i = lane; 2 * i < end; i += 32) {
+          const unsigned two = s2[i];
+          const bool lo = 2 * i >= par, hi = 2 * i + 1 < end;
+          if (lo && hi) reinterpret_cast<unsigned *>(g)[i] = two;
+          else if (lo) g[2 * i] = (uint16_t)two;
+          else g[2 * i + 1] = (uint16_t)(two >> 16);
+        }
+        __syncwarp();
+        for (int i = lane; 8 * i < end; i += 32) reinterpret_cast<uint4 *>(stage)[i] = fill8;
+        __syncwarp();
+      }
+      nTok += total;
+    };
 
-    // ---- the chunk's layout from the warp summaries (lane u of every warp
-    // reads warp u's; lanes >= kWarps hold an empty warp)
-    int F = -1, Lu = -1, I = 0;
-    if (lane < kWarps) {
-      F = wFirst[par][lane];
-      Lu = wLast[par][lane];
-      I = wTok[par][lane];
-    }
-    // the value before warp u's first: positions grow with the warp index
-    int pv = Lu;
+    float x[kLaneRun];
+    auto load = [&](int base) {
+      const int p0 = base + kLaneRun * lane;
+      if (p0 + kLaneRun <= len) {
+        const float4 *s4 = reinterpret_cast<const float4 *>(src + p0);
 #pragma unroll
-    for (int d = 1; d < kWarps; d <<= 1) {
-      const int t = __shfl_up_sync(kAll, pv, d);
-      if (lane >= d) pv = max(pv, t);
-    }
-    int prevU = __shfl_up_sync(kAll, pv, 1);
-    if (lane == 0) prevU = -1;
-    // warp u's first run lies inside the chunk when a value precedes it
-    const int g0 = F >= 0 && prevU >= 0 ? F - prevU - 1 : 0;
-    int sg0, dp0;
-    run_split_closed(g0, sg0, dp0);
-    if (w == 0) {  // counted once per chunk
-      singles += sg0;
-      dups += dp0;
-    }
-    const int tok = sg0 + dp0 + I;
-    int incT = tok;
+        for (int k = 0; k < kLaneRun / 4; k++) {
+          const float4 f = s4[k];
+          x[4 * k] = f.x; x[4 * k + 1] = f.y; x[4 * k + 2] = f.z; x[4 * k + 3] = f.w;
+        }
+      } else {
 #pragma unroll
-    for (int d = 1; d < kWarps; d <<= 1) {
-      const int t = __shfl_up_sync(kAll, incT, d);
-      if (lane >= d) incT += t;
-    }
-    const int nTok = __shfl_sync(kAll, incT, kWarps - 1);
-    int lead = F >= 0 ? F : len, last = Lu;
+        for (int k = 0; k < kLaneRun; k++) x[k] = p0 + k < len ? src[p0 + k] : 0.f;
+      }
+    };
+    load(0);
+    int nq = 0;  // candidates in the queue
+    for (int base = 0; base < len; base += kBlock) {
+      unsigned mask = 0;
 #pragma unroll
-    for (int d = kWarps / 2; d > 0; d >>= 1) {
-      lead = min(lead, __shfl_xor_sync(kAll, lead, d));
-      last = max(last, __shfl_xor_sync(kAll, last, d));
-    }
-    lead = __shfl_sync(kAll, lead, 0);
-    last = __shfl_sync(kAll, last, 0);
-
-    // ---- copy-out: warp w's tokens (its first run, then the staged ones)
-    // to their place in the chunk's slot, which holds the chunk's tokens from
-    // the first value's position on (the lead zero run's tokens, written
-    // later by runs_kernel, fit before it, since each token starts at its
-    // own element)
-    {
-      const int o = __shfl_sync(kAll, incT - tok, w);
-      const int fr = __shfl_sync(kAll, sg0 + dp0, w);
-      const int gw = __shfl_sync(kAll, g0, w);
-      const int nw = fr + __shfl_sync(kAll, I, w);
-      uint16_t *g = b.tok + cd.coefOff + start + lead + o;
-      // the first run's few tokens, then the staged ones (a plain copy)
-      for (int j = lane; j < fr; j += 32) g[j] = run_token_at(gw, j, B, dupV);
-      for (int j = fr + lane; j < nw; j += 32) g[j] = stage[j - fr];
-    }
-    __syncwarp();  // the staged tokens are read before the next prefill
-    if (threadIdx.x == 0) {
-      b.chunkTok[chunk] = nTok;
-      b.chunkSpan[chunk] = make_int2(lead, nTok);  // runs_kernel adds the edge runs
-      if (dupV >= 0) {
-        const bool any = last >= 0;
-        b.chunkRun[chunk] = make_int4(lead, any ? len - 1 - last : len, any ? 0 : 1, len);
+      for (int k = 0; k < kLaneRun; k++)
+        if (!(fabsf(x[k]) < zthr)) mask |= 1u << k;  // NaN is a candidate
+      const int p0 = base + kLaneRun * lane;
+      if (p0 + kLaneRun > len) mask &= p0 < len ? (1u << (len - p0)) - 1u : 0u;
+      if (base + kBlock < len) load(base + kBlock);
+      const int cnt = __popc(mask);
+      int inc = cnt;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(kAll, inc, d);
+        if (lane >= d) inc += t;
+      }
+      int o = nq + inc - cnt;
+#pragma unroll
+      for (int k = 0; k < kLaneRun; k++)
+        if ((mask >> k) & 1u) queue[o++] = (uint16_t)(p0 + k);
+      nq += __shfl_sync(kAll, inc, 31);
+      __syncwarp();
+      int at = 0;
+      for (; nq - at >= 32; at += 32) round(at, 32);
+      if (at) {  // what is left moves to the front
+        nq -= at;
+        const int left = lane < nq ? queue[at + lane] : 0;
+        __syncwarp();
+        if (lane < nq) queue[lane] = (uint16_t)left;
+        __syncwarp();
       }
     }
-    // one barrier per chunk: the next chunk writes the other summary set,
-    // and a warp reaches this chunk's set again only after every warp has
-    // passed the next chunk's barrier, i.e. has finished this chunk
-  }
+    if (nq) round(0, nq);
+
+    if (lane == 0) {
+      // the tokens sit in the chunk's slot from the first value's position
+      // on (the lead zero run's tokens, written later by runs_kernel, fit
+      // before it, since each token starts at its own element)
+      const long long chunk = cd.chunkBase + c;
+      const bool any = last >= 0;
+      const int first = any ? lead : len;
+      b.chunkTok[chunk] = nTok;
+      b.chunkSpan[chunk] = make_int2(first, nTok);  // runs_kernel adds the edge runs
+      if (dupV >= 0)
+        b.chunkRun[chunk] = make_int4(first, any ? len - 1 - last : len, any ? 0 : 1, len);
+    }
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    singles += __shfl_xor_sync(kAll, singles, d);
-    dups += __shfl_xor_sync(kAll, dups, d);
-  }
-  if (lane == 0 && dupV >= 0) {
-    if (singles) atomicAdd(&hist[dupV], (unsigned)singles);
-    if (dups) atomicAdd(&hist[B], (unsigned)dups);
+    for (int d = 16; d > 0; d >>= 1) {
+      singles += __shfl_xor_sync(kAll, singles, d);
+      dups += __shfl_xor_sync(kAll, dups, d);
+    }
+    if (lane == 0 && dupV >= 0) {
+      if (singles) atomicAdd(&hist[dupV], (unsigned)singles);
+      if (dups) atomicAdd(&hist[B], (unsigned)dups);
+    }
   }
   __syncthreads();
   unsigned long long *gh = b.hist + (size_t)ci * kMaxSymbols;
-  for (int i = threadIdx.x; i <= B; i += kThreads)
+  for (int i = threadIdx.x; i <= B; i += blockDim.x)
     if (hist[i]) atomicAdd(&gh[i], (unsigned long long)hist[i]);
 }
 
@@ -778,10 +708,10 @@ __global__ void __launch_bounds__(kRunChunks) runs_kernel(DevBatch b) {
     int runIn = 0, e = n;
     if (prev >= 0) {
       const int4 o = cr[prev];
-      runIn = prev * kChunk + o.w - o.y;
+      runIn = (prev << b.lgChunk) + o.w - o.y;
     }
-    if (next != INF) e = next * kChunk + cr[next].x;
-    const int cstart = c * kChunk;
+    if (next != INF) e = (next << b.lgChunk) + cr[next].x;
+    const int cstart = c << b.lgChunk;
     if (val) run_split_closed(e - (cstart + me.w - me.y), singles, dups);
     if (c == 0) {  // the run starting at element 0 belongs to no chunk's tail
       int sg, dp;
@@ -837,12 +767,15 @@ void launch_lloyd(DevBatch &b, const float *coef, int maxBins, cudaStream_t s) {
   lloyd_solve_kernel<<<b.n, kSolveThreads, smem, s>>>(b, cbCap);
 }
 
-void launch_quantize(DevBatch &b, const float *coef, int maxTable, int maxSymbols,
+void launch_quantize(DevBatch &b, const float *coef, int maxTable, int maxSymbols, bool lloyd,
                      cudaStream_t s) {
   const int histOff = (maxTable + 3) & ~3;
-  const int smem = (histOff + maxSymbols + 1) * (int)sizeof(float);
+  const int lutOff = (histOff + maxSymbols + 1 + 3) & ~3;
+  const int warpOff = lutOff + (lloyd ? kLutStride / 2 : 0);
+  const int smem = warpOff * (int)sizeof(float) + kQuantWarps * kWarpBytes;
   raise_smem_limit(quantize_kernel, smem);
-  quantize_kernel<<<(unsigned)b.totalGroups, kThreads, smem, s>>>(b, coef, histOff);
+  quantize_kernel<<<(unsigned)b.totalQuant, 32 * kQuantWarps, smem, s>>>(b, coef, histOff, lutOff,
+                                                                          warpOff);
 }
 
 void launch_runs(DevBatch &b, cudaStream_t s) {

@@ -69,7 +69,7 @@ select_pass0(DevBatch b, const float *__restrict__ coef) {
   const CubeletDev cd = b.cub[ci];
   if (cd.selFused) return;  // the last transform pass gathered these already
   const int c0 = ((int)blockIdx.x - cd.groupBase) * b.group;
-  const int nc = min(b.group, cd.nChunks - c0);
+  const int nc = min(b.group, cd.selChunks - c0);
   auto chunk_len = [&](int k) {
     return (int)min((long long)kChunk, cd.n - (long long)(c0 + k) * kChunk);
   };
@@ -104,7 +104,7 @@ select_compact(DevBatch b, const float *__restrict__ coef, unsigned *__restrict_
   const int ci = b.groupCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
   const int c0 = ((int)blockIdx.x - cd.groupBase) * b.group;
-  const int nc = min(b.group, cd.nChunks - c0);
+  const int nc = min(b.group, cd.selChunks - c0);
   CubeletState *st = b.state + ci;
   const unsigned prefix = st->prefix;
   const bool lloyd = cd.quantAlg == WL_LLOYD && !st->lloydDeferred;
@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(1024) select_resolve(DevBatch b, bool mark) {
 
 // One launch sets up everything a call's kernels expect: kInitSlices CTAs per
 // cubelet (blockIdx.y) zero its histograms and state and write the cubelet
-// index of its chunks, quantize groups and bit-packer CTAs, so that those
-// kernels start with one load.  (Three memsets, an initialisation and a map
+// index of its chunks, select groups, quantize and bit-packer CTAs, so that
+// those kernels start with one load.  (Three memsets, an initialisation and a map
 // kernel before took 20 us at the head of every call, most of it gaps.)
 constexpr int kInitSlices = 8;
 __global__ void __launch_bounds__(kThreads) init_kernel(DevBatch b, bool lloyd) {
@@ -310,8 +310,10 @@ __global__ void __launch_bounds__(kThreads) init_kernel(DevBatch b, bool lloyd) 
     for (int i = t0; i < kLloydBins; i += step) lh[i] = 0;
   }
   for (int j = t0; j < cd.nChunks; j += step) b.chunkCub[cd.chunkBase + j] = ci;
-  const int groups = (cd.nChunks + b.group - 1) / b.group;
+  const int groups = (cd.selChunks + b.group - 1) / b.group;
   for (int j = t0; j < groups; j += step) b.groupCub[cd.groupBase + j] = ci;
+  const int quant = (cd.nChunks + kQuantWarps - 1) / kQuantWarps;
+  for (int j = t0; j < quant; j += step) b.quantCub[cd.quantBase + j] = ci;
   const int enc = (int)(((long long)cd.nChunks * b.encF + kEncThreads - 1) / kEncThreads);
   for (int j = t0; j < enc; j += step) b.encCub[cd.encBase + j] = ci;
   if (slice != 0) return;

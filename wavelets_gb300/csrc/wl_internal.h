@@ -32,24 +32,33 @@ __host__ __device__ inline int clz32(unsigned x) {
 
 constexpr int kMaxBins = 4096;          // bins per cubelet (kernel tables)
 constexpr int kMaxSymbols = kMaxBins + 1;
-constexpr int kChunk = 4096;            // elements per quantize/encode chunk
+constexpr int kChunk = 4096;            // elements per select chunk
+// Token chunks: the elements one warp quantizes and a group of bit-packer
+// lanes packs, 1 << lg (DevBatch::lgChunk).  4096 for large batches (little
+// per-chunk work), down to 512 -- a block of the quantizer -- where a call of
+// n elements would otherwise run on fewer than 32 warps per SM of a 152-SM
+// GB300: a warp codes its chunk from end to end (with 4096 always, a 64^2
+// tile took 260 us a call, 180 us with 512; a 2048^2 image 342 and 323 us).
+constexpr int kMinLgChunk = 9, kMaxLgChunk = 12;
+inline int token_chunk_lg(long long n) {
+  int lg = kMinLgChunk;
+  while (lg < kMaxLgChunk && (n >> (lg + 1)) >= 152 * 32) lg++;
+  return lg;
+}
+constexpr int kQuantWarps = 8;  // token chunks per quantize CTA, a warp each
 constexpr int kChunkThreads = 256;
 constexpr int kSelectBins = 4096;       // radix-select digit histogram
 constexpr int kLloydBins = 4096;        // |coefficient| histogram for Lloyd
 constexpr int kCandSlices = 64;        // CTAs per cubelet over its threshold candidates
 constexpr int kLutCells = 4096;         // Lloyd bin lookup: cells of the float order key
 constexpr int kLutStride = kLutCells + 8;  // per-cubelet table stride (16-byte rows)
-// Chunks per select / quantize CTA: up to eight for large batches (few table
-// loads and histogram flushes), fewer where eight would leave CTA slots empty
-// (four CTAs of 256 threads on each of a GB300's 152 SMs: the quantizer's
-// occupancy).  With eight always, the quantizer of a 2048^2 image (1024
-// chunks) ran 128 CTAs of eight chunks in a row: the call took 468 us against
-// 435 us with two, a 147 x 181 x 93 stack 483 against 448 us; 256^3 (4096
-// chunks, seven) 529 and 531 us.
-constexpr int kMaxQuantGroup = 8;
-inline int quant_group(long long chunks) {
+// Chunks per select CTA: up to eight for large batches (few histogram
+// flushes), fewer where eight would leave CTA slots empty (four CTAs of 256
+// threads on each of a GB300's 152 SMs).
+constexpr int kMaxSelGroup = 8;
+inline int sel_group(long long chunks) {
   const long long slots = 152 * 4, g = (chunks + slots - 1) / slots;
-  return (int)(g < 1 ? 1 : g > kMaxQuantGroup ? kMaxQuantGroup : g);
+  return (int)(g < 1 ? 1 : g > kMaxSelGroup ? kMaxSelGroup : g);
 }
 // Bit packer: a chunk's tokens are split into F slices (F a power of two,
 // 1..32), one lane each; a CTA of kEncThreads lanes packs kEncThreads / F
@@ -58,8 +67,9 @@ inline int quant_group(long long chunks) {
 // serial chain): measured on a 512-cubelet batch (92 K chunks), the encode
 // stage (per-slice bit counts, scans, packer) took 0.79, 0.76, 0.60, 0.52,
 // 0.50 and 0.52 ms for F = 1, 2, 4, 8, 16, 32.
-// F = 16 unless the launch would then have fewer lanes than one full wave of
-// a 152-SM GB300 (2048 per SM); small batches take 32.
+// F = 16 per 4096 elements unless the launch would then have fewer lanes than
+// one full wave of a 152-SM GB300 (2048 per SM); small batches take 32.  A
+// smaller token chunk has as many lanes per element.
 constexpr int kEncThreads = 128;
 constexpr long long kEncFullWave = 152LL * 2048;
 inline int enc_slices(long long chunks) { return chunks * 16 >= kEncFullWave ? 16 : 32; }
@@ -171,10 +181,12 @@ struct CubeletState {
 struct CubeletDev {
   long long n;            // padded element count
   long long coefOff;      // float offset of the coefficients
-  long long chunkBase;    // first global chunk index
+  long long chunkBase;    // first token chunk
   long long wordsOff;     // word offset of the Huffman output
   long long wordsCap;     // capacity in words
-  int nChunks;
+  int nChunks;            // token chunks
+  int selChunks;          // chunks of kChunk elements (select)
+  int quantBase;          // first quantize CTA (kQuantWarps token chunks per CTA)
   int binCount;
   int quantAlg;
   int compressZeros;
@@ -182,7 +194,7 @@ struct CubeletDev {
   int lloydIters;
   int tableOff;           // offset into per-cubelet quantizer tables (floats)
   int nTable;             // entries in the table (log: boundaries; lloyd: boundaries)
-  int groupBase;          // first quantize group (DevBatch::group chunks per group)
+  int groupBase;          // first select group (DevBatch::group chunks of kChunk)
   int encBase;            // first bit-packer CTA (kEncThreads / F chunks per CTA)
   int selFused;           // 1: the last transform pass gathered the first select
                           // digit and the extremes (no stand-alone first pass)
@@ -203,7 +215,8 @@ struct DevBatch {
   CubeletState *state;            // [n]
   float *coef;                    // coefficients (ping)
   float *coef2;                   // second buffer (pong)
-  uint16_t *tok;                  // Huffman tokens, one slot of kChunk per chunk
+  uint16_t *tok;                  // Huffman tokens: a token chunk's from its first element's place on
+  int lgChunk;                    // log2 of the elements per token chunk
   int *chunkTok;                  // tokens stored per chunk by quantize
   int2 *chunkSpan;                // per chunk: first token slot, token count
                                   // (with the zero-run tokens at its edges)
@@ -221,9 +234,11 @@ struct DevBatch {
   uint32_t *words;                // Huffman output
   long long *chunkPrefix;         // [n+1] chunk prefix (== cub[i].chunkBase)
   int *chunkCub;                  // [totalChunks] cubelet of every chunk
-  int *groupCub;                  // [totalGroups] cubelet of every quantize group
+  int *groupCub;                  // [totalGroups] cubelet of every select group
+  int *quantCub;                  // [totalQuant] cubelet of every quantize CTA
+  long long totalQuant;
   long long totalGroups;
-  int group;                      // chunks per quantize group
+  int group;                      // chunks per select group
   int *encCub;                    // [totalEnc] cubelet of every bit-packer CTA
   long long totalEnc;
   int encF;                       // bit-packer slices per chunk
@@ -336,7 +351,7 @@ void launch_lloyd(DevBatch &b, const float *coef, int maxBins, cudaStream_t s);
 // sum of squared differences of two u8 arrays into *out (opt.cu)
 void launch_sq_err_u8(const uint8_t *a, const uint8_t *b, long long n, unsigned long long *out,
                       cudaStream_t s);
-void launch_quantize(DevBatch &b, const float *coef, int maxTable, int maxSymbols,
+void launch_quantize(DevBatch &b, const float *coef, int maxTable, int maxSymbols, bool lloyd,
                      cudaStream_t s);
 void launch_runs(DevBatch &b, cudaStream_t s);
 
