@@ -306,8 +306,8 @@ struct wl_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   std::string err;
-  DevBuf input, coef, coef2, bins, tokCount, state, selHist, lloydHist, qtable, dqtable, qlut,
-      hist, chunkRun, chunkBits, chunkCub, groupCub, quantCub, encCub, sliceOff, codes, codeLen, decode, chunkSpan,
+  DevBuf input, coef, coef2, chunkVal, chunkLen, state, selHist, lloydHist, qtable, dqtable, qlut,
+      hist, chunkRun, chunkBits, chunkCub, groupCub, quantCub, encCub, sliceOff, codes, codeLen, decode, chunkEdge,
       words, passes, outbuf, head, decWords, decTable, decWs, meta, optIn, optOut, optErr,
       errIn, errRest, errPart;
   HostBuf hState, hDecode, hPasses, hTab, hIn, hFlags, hHead, hSel;
@@ -995,8 +995,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   // ---- workspace ----
   TRY(ensure(ctx, ctx->coef, coefTotal * 4));
   TRY(ensure(ctx, ctx->coef2, coefTotal * 4));
-  TRY(ensure(ctx, ctx->bins, (coefTotal + (long long)n * kChunk) * 2));
-  TRY(ensure(ctx, ctx->tokCount, chunkTotal * sizeof(int)));
+  TRY(ensure(ctx, ctx->chunkVal, chunkTotal * sizeof(int)));
+  TRY(ensure(ctx, ctx->chunkLen, chunkTotal * sizeof(unsigned)));
   TRY(ensure(ctx, ctx->state, n * sizeof(CubeletState)));
   TRY(ensure(ctx, ctx->chunkCub, chunkTotal * sizeof(int)));
   TRY(ensure(ctx, ctx->groupCub, selTotal * sizeof(int)));
@@ -1012,7 +1012,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   TRY(ensure(ctx, ctx->dqtable, (size_t)n * kMaxBins * 4));
   TRY(ensure(ctx, ctx->hist, (size_t)n * kMaxSymbols * 8));
   TRY(ensure(ctx, ctx->chunkRun, chunkTotal * sizeof(int4)));
-  TRY(ensure(ctx, ctx->chunkSpan, chunkTotal * sizeof(int2)));
+  TRY(ensure(ctx, ctx->chunkEdge, chunkTotal * sizeof(uint2)));
   TRY(ensure(ctx, ctx->chunkBits, chunkTotal * 8));
   TRY(ensure(ctx, ctx->codes, (size_t)n * kMaxSymbols * 8));
   TRY(ensure(ctx, ctx->codeLen, (size_t)n * kMaxSymbols));
@@ -1137,12 +1137,15 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   // half's size
   int encF[2] = {1, 1}, group[2] = {1, 1};
   {
-    long long halfChunks[2] = {0, 0};
-    for (int i = 0; i < n; i++) halfChunks[half_of(i)] += plans[i].selChunks;
+    long long selChunks[2] = {0, 0}, tokChunks[2] = {0, 0};
+    for (int i = 0; i < n; i++) {
+      selChunks[half_of(i)] += plans[i].selChunks;
+      tokChunks[half_of(i)] += plans[i].nChunks;
+    }
     for (int h = 0; h < nh; h++) {
-      const int per = ctx->encSlices ? ctx->encSlices : enc_slices(halfChunks[h]);
-      encF[h] = std::max(1, per >> (kMaxLgChunk - lgChunk));
-      group[h] = sel_group(halfChunks[h]);
+      encF[h] = ctx->encSlices ? std::max(1, ctx->encSlices >> (kMaxLgChunk - lgChunk))
+                               : enc_slices(tokChunks[h], lgChunk);
+      group[h] = sel_group(selChunks[h]);
     }
   }
   for (int i = 0; i < n; i++) {
@@ -1187,8 +1190,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.state = P<CubeletState>(ctx->state);
   b.coef = P<float>(ctx->coef);
   b.coef2 = P<float>(ctx->coef2);
-  b.tok = P<uint16_t>(ctx->bins);
-  b.chunkTok = P<int>(ctx->tokCount);
+  b.items = P<unsigned>(ctx->coef2);
+  b.chunkVal = P<int>(ctx->chunkVal);
+  b.chunkLen = P<unsigned>(ctx->chunkLen);
   b.selHist = P<unsigned>(ctx->selHist);
   b.lloydHist = P<float>(ctx->lloydHist);
   b.qtable = reinterpret_cast<float *>(P<char>(ctx->qtable) + hdrBytes);
@@ -1196,7 +1200,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.dqtable = P<float>(ctx->dqtable);
   b.hist = P<unsigned long long>(ctx->hist);
   b.chunkRun = P<int4>(ctx->chunkRun);
-  b.chunkSpan = P<int2>(ctx->chunkSpan);
+  b.chunkEdge = P<uint2>(ctx->chunkEdge);
   b.chunkBits = P<unsigned long long>(ctx->chunkBits);
   b.codes = P<unsigned long long>(ctx->codes);
   b.codeLen = P<uint8_t>(ctx->codeLen);
@@ -1259,8 +1263,9 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       if (v.hostSel) v.hostSel += c0;
       if (h) v.head = nullptr;
       v.chunkPrefix += c0;
-      v.chunkTok += ch;
-      v.chunkSpan += ch;
+      v.chunkVal += ch;
+      v.chunkLen += ch;
+      v.chunkEdge += ch;
       v.chunkRun += ch;
       v.chunkBits += ch;
       v.chunkCub += ch;
@@ -2463,12 +2468,12 @@ void wl_destroy(wl_ctx *ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  DevBuf *dbs[] = {&ctx->input, &ctx->coef, &ctx->coef2, &ctx->bins, &ctx->tokCount,
+  DevBuf *dbs[] = {&ctx->input, &ctx->coef, &ctx->coef2, &ctx->chunkVal, &ctx->chunkLen,
                    &ctx->state,
                    &ctx->selHist, &ctx->lloydHist, &ctx->qtable, &ctx->dqtable, &ctx->qlut, &ctx->hist,
                    &ctx->chunkRun, &ctx->chunkBits, &ctx->chunkCub, &ctx->groupCub, &ctx->quantCub,
                    &ctx->encCub, &ctx->sliceOff,
-                   &ctx->chunkSpan, &ctx->optIn, &ctx->optOut, &ctx->optErr,
+                   &ctx->chunkEdge, &ctx->optIn, &ctx->optOut, &ctx->optErr,
                    &ctx->codes, &ctx->codeLen, &ctx->decode, &ctx->words, &ctx->passes,
                    &ctx->outbuf, &ctx->head, &ctx->decWords, &ctx->decTable, &ctx->decWs,
                    &ctx->meta, &ctx->errIn, &ctx->errRest, &ctx->errPart};

@@ -17,8 +17,8 @@
 // bit_stream.h:60-162): every coefficient yields zero or one token -- its own
 // code, a single zero-bin code, or at the first element of a dup chunk the
 // zero-run key code followed by 3 length bits.  Token lengths are summed per
-// 4096-element chunk, chunk offsets are scanned per cubelet, and lanes pack
-// slices of a chunk's tokens in registers (the bit packer below).
+// token chunk, chunk offsets are scanned per cubelet, and lanes pack slices of
+// a chunk's values in registers (the bit packer below).
 #include "wl_internal.h"
 
 namespace wl {
@@ -295,75 +295,50 @@ __global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
   }
 }
 
-// ---- tokens -----------------------------------------------------------------
-// A chunk's tokens, in stream order, are slots [span.x, span.x + span.y) of
-// its token slot: the zero-run tokens entering it, its stored tokens and the
-// zero-run tokens leaving it (quantize_kernel and runs_kernel put them there).
-
 // ---- bit packer -------------------------------------------------------------
-// A chunk's tokens are cut into F slices of ceil(n / F) tokens (F from
-// enc_slices, per launch); lane s of the chunk's F lanes packs slice s, and a
-// CTA of kEncThreads lanes takes kEncThreads / F consecutive chunks of one
-// cubelet.  The bit
+// A chunk's stream is the tokens of the zero run entering it that start in it,
+// then for each of its values the tokens of the zero run before it and the
+// value's own, then the tokens of the run leaving it that start in it
+// (quantize_kernel stores the values, runs_kernel the edge runs).
+//
+// A chunk's values are cut into F slices of ceil(n / F) (F from enc_slices,
+// per launch); lane s of the chunk's F lanes packs slice s, the first lane the
+// entering run and the last the leaving run besides, and a CTA of kEncThreads
+// lanes takes kEncThreads / F consecutive chunks of one cubelet.  The bit
 // counter sums each slice's code lengths and places the slices inside their
 // chunk with an F-lane exclusive scan; the packer starts each slice at its
 // chunk's offset (from the per-cubelet scan) plus that place.  A lane keeps
 // its bits in a 64-bit register and stores whole words: words wholly inside
 // its slice are stored directly, its first and last word (which it may share
-// with neighbouring slices) are OR-ed in.  A word shared
-// by slices of one chunk is zeroed by the lane whose slice starts in it,
-// before any lane of the chunk ORs (the chunk's lanes are one warp); the
-// chunk's first and last words, shared with neighbouring chunks, were zeroed
-// by encode_zero_kernel.  Tokens are read with 16-byte loads: a slot starts
-// at a multiple of 128 bytes and holds a token per element, so the aligned blocks
-// around a slice stay inside its chunk's slot.
+// with neighbouring slices) are OR-ed in.  A word shared by slices of one
+// chunk is zeroed by the lane whose slice starts in it, before any lane of the
+// chunk ORs (the chunk's lanes are one warp); the chunk's first and last
+// words, shared with neighbouring chunks, were zeroed by encode_zero_kernel.
+//
+// The run before a value costs no loop over its tokens, which would run as
+// long as the longest in the warp: the tokens of its multiple of 16 below 1024
+// (powers of two) and of what is below 16 (an eight and singles) are two
+// ready-made bit strings, joined with the value's code and appended at once.
+// Only runs of 1024 and more, and alphabets whose codes make such strings
+// longer than 64 bits, take the loops.  Values are read four at a time; a
+// chunk's values start at a multiple of 2 KB, so the aligned blocks around a
+// slice stay inside its chunk's place.
+//
+// The encode stage (bit counts, scans, packer) of the mixed batch takes 0.42
+// ms, of 729 cubelets of 128^3 0.51 ms; 0.49 and 0.79 ms when it read every
+// token as a 16-bit word.
 
 // code bits (below kMaxCodeBits) and length (above) of one symbol
 constexpr unsigned long long kCodeMask = (1ull << kMaxCodeBits) - 1;
 
-// f(token, table entry) for tokens [a, e) of a slot, in order.  In a block
-// of eight tokens that all lie in [a, e) the table entries are read before
-// any is used; in the blocks at the ends only the tokens inside [a, e) are
-// looked up (the other slots hold other slices' tokens or stale values).
-template <class T, class Fn>
-__device__ __forceinline__ void for_tokens(const uint16_t *slot, int a, int e, const T *tab,
-                                           Fn &&f) {
-  if (a >= e) return;
-  const uint4 *p = reinterpret_cast<const uint4 *>(slot) + (a >> 3);
-  const uint4 *pe = reinterpret_cast<const uint4 *>(slot) + ((e + 7) >> 3);
-  for (int i = a & ~7; p < pe; p++, i += 8) {
-    const uint4 q = *p;
-    const unsigned w[4] = {q.x, q.y, q.z, q.w};
-    if (i >= a && i + 8 <= e) {
-      unsigned t[8];
-      T en[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        t[k] = (w[k >> 1] >> (16 * (k & 1))) & 0xffffu;
-        en[k] = tab[t[k] & 0x1fff];
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) f(t[k], en[k]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        if (i + k >= a && i + k < e) {
-          const unsigned t = (w[k >> 1] >> (16 * (k & 1))) & 0xffffu;
-          f(t, tab[t & 0x1fff]);
-        }
-      }
-    }
-  }
-}
-
 // Slice geometry shared by the bit counter and the packer: chunk `cl` of the
-// cubelet (within its CTA's run), slice `sub` of it, tokens [t0, t1) of the
-// chunk's token list.
+// cubelet (within its CTA's run), slice `sub` of it, values [t0, t1) of the
+// chunk's.
 struct SliceAt {
-  int cl, sub, t0, t1;
-  bool ok;        // the chunk exists
+  int cl, sub, n, t0, t1;  // n: values of the chunk
+  bool ok;                 // the chunk exists
   long long chunk;
-  int2 span;      // first token slot, token count
+  uint2 edge;              // run codes at the chunk's edges
 };
 __device__ __forceinline__ SliceAt slice_at(const DevBatch &b, const CubeletDev &cd, int lgF) {
   SliceAt r;
@@ -372,31 +347,62 @@ __device__ __forceinline__ SliceAt slice_at(const DevBatch &b, const CubeletDev 
   r.sub = lane & ((1 << lgF) - 1);
   r.ok = r.cl < cd.nChunks;
   r.chunk = cd.chunkBase + r.cl;
-  r.span = r.ok ? b.chunkSpan[r.chunk] : make_int2(0, 0);
-  const int m = (r.span.y + (1 << lgF) - 1) >> lgF;
-  r.t0 = min(r.span.y, r.sub * m);
-  r.t1 = min(r.span.y, r.t0 + m);
+  const int n = r.ok ? b.chunkVal[r.chunk] : 0;
+  const int m = (n + (1 << lgF) - 1) >> lgF;
+  r.n = n;
+  r.t0 = min(n, r.sub * m);
+  r.t1 = min(n, r.t0 + m);
+  // the chunk's entering run comes before its first value, the leaving run
+  // after its last
+  r.edge = make_uint2(0u, 0u);
+  if (r.ok && b.state[(int)b.encCub[blockIdx.x]].dupValue >= 0) {
+    r.edge = b.chunkEdge[r.chunk];
+    if (r.sub == 0) r.t0 = -1;
+    if (r.sub == (1 << lgF) - 1) r.t1 = n + 1;
+  }
   return r;
 }
-
-// Bits of every slice: lane s of a chunk's F lanes sums its tokens' code
-// lengths, an F-lane exclusive scan places the slice inside the chunk
-// (sliceOff), and the chunk's last lane writes the chunk's bit count.
+// f(bin or -1, run code) for the entries [t0, t1) of the slice, in order: the
+// entering run (-1), the values with the run before each, the leaving run (n).
+// One entry per step and the next value's load in flight: one copy of f keeps
+// the packer's code inside the instruction cache (with four values unrolled
+// and an append for every kind of token, its warps waited for instructions
+// most of the time: 1.46 ms for 729 cubelets against 0.43).
+template <class Fn>
+__device__ __forceinline__ void for_entries(const unsigned *items, const SliceAt &sl, Fn &&f) {
+  auto load = [&](int j) { return (unsigned)j < (unsigned)sl.n ? items[j] : 0u; };
+  unsigned nx = load(sl.t0);
+#pragma unroll 1
+  for (int j = sl.t0; j < sl.t1; j++) {
+    const unsigned it = nx;
+    nx = load(j + 1);
+    if ((unsigned)j < (unsigned)sl.n) f((int)(it >> 16), run_code((int)(it & 0xffff)));
+    else f(-1, j < 0 ? sl.edge.x : sl.edge.y);
+  }
+}
+// Bits of every slice: lane s of a chunk's F lanes sums its values' code
+// lengths and their runs' (a run's length from its token counts), an F-lane
+// exclusive scan places the slice inside the chunk (sliceOff), and the chunk's
+// last lane writes the chunk's bit count.
 __global__ void __launch_bounds__(kEncThreads) encode_count_kernel(DevBatch b) {
   extern __shared__ uint8_t sLen[];
   stage_mark(b.head, kMarkEncode);
   const int ci = b.encCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
   const int lgF = __ffs(b.encF) - 1, F = 1 << lgF;
-  const int dupKey = cd.binCount, S = cd.binCount + 1;
+  const int dupV = b.state[ci].dupValue, dupKey = cd.binCount, S = cd.binCount + 1;
   for (int i = threadIdx.x; i < S; i += kEncThreads) sLen[i] = b.codeLen[(size_t)ci * kMaxSymbols + i];
   __syncthreads();
   const SliceAt sl = slice_at(b, cd, lgF);
   unsigned mine = 0;  // at most 4096 tokens of at most 61 bits
   if (sl.ok) {
-    const uint16_t *slot = b.tok + cd.coefOff + ((long long)sl.cl << b.lgChunk);
-    for_tokens(slot, sl.span.x + sl.t0, sl.span.x + sl.t1, sLen, [&](unsigned t, uint8_t l) {
-      mine += l + ((int)(t & 0x1fff) == dupKey ? 3u : 0u);
+    const unsigned one = dupV >= 0 ? sLen[dupV] : 0u, dup = sLen[dupKey] + 3u;
+    for_entries(b.items + cd.coefOff + ((long long)sl.cl << b.lgChunk), sl,
+                [&](int bin, unsigned run) {
+      if (bin >= 0) mine += sLen[bin];
+      const int lo = run & 255;
+      const int keys = (int)(run >> 16) + __popc(run & 0x3f00) + (lo > 8);
+      mine += dup * keys + one * (lo > 8 ? (lo & 15) - (lo < kEightAlone ? 8 : 0) : lo);
     });
   }
   unsigned inc = mine;
@@ -406,53 +412,64 @@ __global__ void __launch_bounds__(kEncThreads) encode_count_kernel(DevBatch b) {
   }
   if (sl.ok) {
     b.sliceOff[sl.chunk * 32 + sl.sub] = inc - mine;
-    if (sl.sub == F - 1) b.chunkBits[sl.chunk] = inc;
+    if (sl.sub == F - 1) b.chunkLen[sl.chunk] = inc;
   }
 }
 
 // Per cubelet: exclusive scan of the chunk bit counts, kScanRun consecutive
 // chunks per thread, so that one round covers 8192 chunks (the most a call
-// that fills no more than the GPU has: a round is all latency).
+// that fills no more than the GPU has: a round is all latency).  A round's
+// bits fit 32 bits (4096 elements of at most 61 each per chunk).
 constexpr int kScanRun = 8;
 __global__ void __launch_bounds__(1024) encode_scan_kernel(DevBatch b) {
-  __shared__ unsigned long long sh[32];
-  const int ci = blockIdx.x;
+  __shared__ unsigned sh[32];
+  __shared__ unsigned v[1024 * (kScanRun + 1)];  // a thread's run at stride 9
+  const int ci = blockIdx.x, tid = threadIdx.x;
   const CubeletDev cd = b.cub[ci];
   CubeletState *st = b.state + ci;
   unsigned long long carry = 0;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = tid & 31, w = tid >> 5;
+  const unsigned *len = b.chunkLen + cd.chunkBase;
   unsigned long long *bits = b.chunkBits + cd.chunkBase;
   for (int seg = 0; seg < cd.nChunks; seg += 1024 * kScanRun) {
-    const int c0 = seg + threadIdx.x * kScanRun;
-    unsigned v[kScanRun];  // at most 4096 tokens of 61 bits each
-    unsigned mine = 0;
+    const int n = min(1024 * kScanRun, cd.nChunks - seg);
 #pragma unroll
     for (int k = 0; k < kScanRun; k++) {
-      v[k] = c0 + k < cd.nChunks ? (unsigned)bits[c0 + k] : 0u;
-      mine += v[k];
+      const int i = k * 1024 + tid;
+      v[i + i / kScanRun] = i < n ? len[seg + i] : 0u;
     }
-    unsigned long long inc = mine;
+    __syncthreads();
+    unsigned mine = 0;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) {  // exclusive inside the run
+      const unsigned t = v[tid * (kScanRun + 1) + k];
+      v[tid * (kScanRun + 1) + k] = mine;
+      mine += t;
+    }
+    unsigned inc = mine;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, off);
+      const unsigned t = __shfl_up_sync(0xffffffffu, inc, off);
       if (lane >= off) inc += t;
     }
     if (lane == 31) sh[w] = inc;
     __syncthreads();
-    // the warps before this one, and all of them
-    unsigned long long all = sh[lane], before = all;
+    unsigned before = sh[lane];  // inclusive over the warps
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xffffffffu, before, off);
+      const unsigned t = __shfl_up_sync(0xffffffffu, before, off);
       if (lane >= off) before += t;
     }
-    all = __shfl_sync(0xffffffffu, before, 31);
-    const unsigned long long upTo = __shfl_sync(0xffffffffu, before, w > 0 ? w - 1 : 0);
-    unsigned long long at = carry + (w > 0 ? upTo : 0) + inc - mine;
+    const unsigned all = __shfl_sync(0xffffffffu, before, 31);
+    const unsigned upTo = __shfl_sync(0xffffffffu, before, w > 0 ? w - 1 : 0);
+    const unsigned at = (w > 0 ? upTo : 0u) + inc - mine;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) v[tid * (kScanRun + 1) + k] += at;
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < kScanRun; k++) {
-      if (c0 + k < cd.nChunks) bits[c0 + k] = at;
-      at += v[k];
+      const int i = k * 1024 + tid;
+      if (i < n) bits[seg + i] = carry + v[i + i / kScanRun];
     }
     carry += all;
     __syncthreads();
@@ -582,21 +599,52 @@ __global__ void encode_zero_kernel(DevBatch b) {
   w[(end - 1) >> 5] = 0;
 }
 
+// ready-made strings: runs below 16 elements, multiples of 16 below 1024 (in
+// 16s), zero-run keys with their length bits
+constexpr int kLowRuns = 17, kHighRuns = 64, kDupRuns = 8;
+
 __global__ void __launch_bounds__(kEncThreads, 8) encode_write_kernel(DevBatch b) {
   extern __shared__ unsigned long long sTab[];  // code | length << kMaxCodeBits
+  __shared__ unsigned long long sLow[kLowRuns], sHigh[kHighRuns], sDup[kDupRuns];
+  __shared__ unsigned char sLowLen[kLowRuns], sHighLen[kHighRuns];
   const int ci = b.encCub[blockIdx.x];
   const CubeletDev cd = b.cub[ci];
   const CubeletState *st = b.state + ci;
   if (st->error) return;
   const int lane = threadIdx.x;
   const int lgF = __ffs(b.encF) - 1, F = 1 << lgF;
-  const int dupKey = cd.binCount, S = cd.binCount + 1;
-  {
-    const unsigned long long *gc = b.codes + (size_t)ci * kMaxSymbols;
-    const uint8_t *gl = b.codeLen + (size_t)ci * kMaxSymbols;
-    for (int i = lane; i < S; i += kEncThreads)
-      sTab[i] = (gc[i] & kCodeMask) | ((unsigned long long)gl[i] << kMaxCodeBits);
+  const int dupV = st->dupValue, dupKey = cd.binCount, S = cd.binCount + 1;
+  const unsigned long long *gc = b.codes + (size_t)ci * kMaxSymbols;
+  const uint8_t *gl = b.codeLen + (size_t)ci * kMaxSymbols;
+  for (int i = lane; i < S; i += kEncThreads)
+    sTab[i] = (gc[i] & kCodeMask) | ((unsigned long long)gl[i] << kMaxCodeBits);
+  const bool runs = dupV >= 0;
+  const int oneLen = runs ? gl[dupV] : 0, dupLen = runs ? gl[dupKey] + 3 : 0;
+  const unsigned long long one = runs ? gc[dupV] : 0, dup = runs ? gc[dupKey] : 0;
+  // an eight and eight singles, and six powers of two, in 64 bits each: any
+  // but extreme code lengths
+  const bool ready = dupLen + 8 * oneLen <= 64 && 6 * dupLen <= 64;
+  if (ready && lane < kLowRuns) {
+    unsigned long long v = lane > 8 ? dup : 0;
+    int l = lane > 8 ? dupLen : 0;
+    for (int k = lane == kEightAlone ? 0 : lane > 8 ? lane - 8 : lane; k > 0; k--) {
+      if (l < 64) v |= one << l;
+      l += oneLen;
+    }
+    sLow[lane] = v;
+    sLowLen[lane] = (unsigned char)l;
+  } else if (ready && lane >= 32 && lane < 32 + kHighRuns) {
+    unsigned long long v = 0;
+    int l = 0;
+    for (int lg = 5; lg >= 0; lg--)  // 2^(lg + 4) elements, length bits lg + 1
+      if (((lane - 32) >> lg) & 1) {
+        v |= (dup | ((unsigned long long)(lg + 1) << (dupLen - 3))) << l;
+        l += dupLen;
+      }
+    sHigh[lane - 32] = v;
+    sHighLen[lane - 32] = (unsigned char)l;
   }
+  if (lane < kDupRuns && runs) sDup[lane] = dup | ((unsigned long long)lane << (dupLen - 3));
   __syncthreads();
   const SliceAt sl = slice_at(b, cd, lgF);
   unsigned long long off = 0, end = 0;
@@ -609,7 +657,6 @@ __global__ void __launch_bounds__(kEncThreads, 8) encode_write_kernel(DevBatch b
   unsigned nxt = __shfl_down_sync(0xffffffffu, rel, 1, F);
   if (sl.sub == F - 1) nxt = (unsigned)(end - off);
   const unsigned long long sb = nxt - rel, pos = off + rel;
-  const uint16_t *slot = b.tok + cd.coefOff + ((long long)sl.cl << b.lgChunk);
   uint32_t *gw = b.words + st->wordsBase;
   const bool any = sl.ok && sb > 0;
   if (any && F > 1) {
@@ -622,41 +669,67 @@ __global__ void __launch_bounds__(kEncThreads, 8) encode_write_kernel(DevBatch b
   const unsigned long long wFirst = w;
   unsigned long long acc = 0;  // bit 0 = bit 0 of word w
   int bits = (int)(pos & 31);
-  for_tokens(slot, sl.span.x + sl.t0, sl.span.x + sl.t1, sTab,
-             [&](unsigned t, unsigned long long e) {
-    const int sym = t & 0x1fff;
-    int l = (int)(e >> kMaxCodeBits);
-    unsigned long long v = e & kCodeMask;
-    if (sym == dupKey) {
-      v |= (unsigned long long)(t >> 13) << l;
-      l += 3;
-    }
-    // the common case: at most 32 bits, one OR into the accumulator (bits <
-    // 32 here, and a code has no bits above its length)
-    if (l <= 32) {
+  for_entries(b.items + cd.coefOff + ((long long)sl.cl << b.lgChunk), sl,
+              [&](int bin, unsigned run) {
+    const unsigned long long e = bin >= 0 ? sTab[bin] : 0ull;
+    const unsigned long long code = e & kCodeMask;
+    const int codeLen = (int)(e >> kMaxCodeBits);
+    // usually one step: the run's two strings and the code together; else as
+    // many as it takes, the code in the last
+    bool more = true;
+#pragma unroll 1
+    while (more) {
+      const int hi = (run >> 8) & 63, lo = run & 255;
+      unsigned long long v;
+      int l;
+      if (run >> 16) {
+        v = sDup[7];
+        l = dupLen;
+        run -= 1u << 16;
+      } else if (ready) {
+        v = sHigh[hi];
+        l = sHighLen[hi];
+        const int ll = sLowLen[lo];
+        run = (unsigned)lo;
+        if (l + ll <= 64) {
+          v |= l < 64 ? sLow[lo] << l : 0ull;
+          l += ll;
+          run = 0;
+          if (l + codeLen <= 64) {
+            v |= l < 64 ? code << l : 0ull;
+            l += codeLen;
+            more = false;
+          }
+        }
+      } else if (hi) {
+        const int lg = 31 - __clz(hi);
+        v = sDup[lg + 1];
+        l = dupLen;
+        run ^= 256u << lg;
+      } else if (lo > 8) {
+        v = sDup[0];
+        l = dupLen;
+        run = lo == kEightAlone ? 0u : (unsigned)(lo - 8);
+      } else if (lo) {
+        v = one;
+        l = oneLen;
+        run--;
+      } else {
+        v = code;
+        l = codeLen;
+        more = false;
+      }
+      // l <= 64 bits of v, none above them; bits < 32 before and after
+      unsigned long long over = bits ? v >> (64 - bits) : 0;  // above the accumulator
       acc |= v << bits;
       bits += l;
-      if (bits >= 32) {
+#pragma unroll 1
+      while (bits >= 32) {
         if (w == wFirst) atomicOr(&gw[w], (unsigned)acc);
         else gw[w] = (unsigned)acc;
         w++;
-        acc >>= 32;
-        bits -= 32;
-      }
-      return;
-    }
-    // up to 61 bits, appended at most 32 at a time
-    while (l > 0) {
-      const int take = l < 32 ? l : 32;
-      acc |= (v & ((1ull << take) - 1)) << bits;
-      bits += take;
-      v >>= take;
-      l -= take;
-      if (bits >= 32) {
-        if (w == wFirst) atomicOr(&gw[w], (unsigned)acc);
-        else gw[w] = (unsigned)acc;
-        w++;
-        acc >>= 32;
+        acc = (acc >> 32) | (over << 32);
+        over >>= 32;
         bits -= 32;
       }
     }

@@ -390,12 +390,12 @@ __device__ __forceinline__ QParams load_qparams(const CubeletDev &cd, const Cube
   return q;
 }
 
-// ---- quantize + count + tokens of the chunk ----------------------------------
-// Instead of storing a bin per coefficient, a chunk stores its Huffman tokens
-// in order: a token for every value that is not the zero bin, preceded by the
-// tokens of the zero-bin run before it when that run starts inside the chunk.
-// Runs touching a chunk edge are left to runs_kernel (counts) and the encoder
-// (tokens).
+// ---- quantize + count + values of the chunk ----------------------------------
+// Instead of storing a bin per coefficient, a chunk stores its values -- the
+// elements that are not the zero bin -- in order, each with the gap to the
+// value before it in the chunk (make_item).  The bit packer turns a gap into
+// the zero-bin run's Huffman tokens.  Runs touching a chunk edge are left to
+// runs_kernel.
 //
 // One warp codes one chunk from its first element to its last, so nothing but
 // the tables and the histogram is shared and there is no barrier inside.  It
@@ -409,15 +409,14 @@ __device__ __forceinline__ QParams load_qparams(const CubeletDev &cd, const Cube
 //  - whenever the queue holds 32 candidates, one per lane, a round gives each
 //    its exact bin (its value is read again, from L1); those that are not the
 //    zero bin are values.  A value's gap to the one before it (the nearest
-//    lower lane with one, else the last value of earlier rounds) gives its
-//    run tokens, a scan its place, and the round's tokens are staged in shared
-//    memory -- prefilled with the single zero-bin token, so only dup tokens
-//    and value tokens are stored -- and written to the chunk's slot two at a
-//    time.
+//    lower lane with one, else the last value of earlier rounds) gives the
+//    count of its run's tokens, and its item goes out.
 // Full rounds whatever the density, and no work for the zero bin beyond the
-// compare: 729 cubelets of 128^3 (3% kept) quantize in 1.76 ms, 2.85 ms with
-// eight warps to a chunk that met at a barrier; the kernel is bound by its
-// instructions (issue slots 60% busy).
+// compare.  The mixed batch (376 M coefficients, 10% kept) quantizes in 0.49
+// ms, 729 cubelets of 128^3 (1.5 G, 3%) in 1.37 ms; 0.76 and 2.85 ms with
+// eight warps to a chunk that met at a barrier and every token written out
+// here.  Bound by its instructions: 1.5 per coefficient with the tokens,
+// about half of them the tokens'.
 // Greedy split of a zero-bin run into dup tokens and single zero-bin tokens
 // (HuffmanDup::dupCount, huffman.h:46-57) in closed form: runs of 1024, then
 // one dup token per set bit of the remainder at or above 8 -- except that a
@@ -434,21 +433,14 @@ __device__ __forceinline__ void run_split_closed(int L, int &singles, int &dups)
   }
 }
 
-
 constexpr int kBlock = 512, kLaneRun = kBlock / 32;
 constexpr int kQueue = 576;  // less than 32 left over and a block's candidates
-// a round's tokens: a value and at most 17 run tokens per lane (three runs of
-// 1024, one per bit from 512 to 16, the eight and seven singles or eight
-// singles), and one slot for the parity of the place they go to
-constexpr int kStage = 592;
-static_assert(kStage >= 32 * 18 + 2 && kStage % 8 == 0 && kQueue % 8 == 0, "16-byte rows");
-constexpr int kWarpBytes = (kQueue + kStage) * 2;
 
 __global__ void __launch_bounds__(32 * kQuantWarps, 4)
 quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lutOff, int warpOff) {
   constexpr unsigned kAll = 0xffffffffu;
   // sized by the launch: the quantizer table (Lloyd / log), the counts of the
-  // batch's largest alphabet, the Lloyd cell table, then the warps' buffers
+  // batch's largest alphabet, the Lloyd cell table, then the warps' queues
   extern __shared__ __align__(16) float tab[];
   unsigned *hist = reinterpret_cast<unsigned *>(tab + histOff);
   uint16_t *lut = reinterpret_cast<uint16_t *>(tab + lutOff);
@@ -465,10 +457,7 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lut
   // zero-bin elements (-thr < x < thr) can be skipped only when they are
   // coded as runs; without runs every element is a candidate (|x| < 0 never)
   const float zthr = dupV >= 0 ? q.thr : 0.f;
-  uint16_t *queue = reinterpret_cast<uint16_t *>(tab + warpOff) + w * (kQueue + kStage);
-  uint16_t *stage = queue + kQueue;
-  const unsigned fill2 = dupV >= 0 ? (unsigned)make_token(dupV, 0) * 0x10001u : 0u;
-  const uint4 fill8 = make_uint4(fill2, fill2, fill2, fill2);
+  uint16_t *queue = reinterpret_cast<uint16_t *>(tab + warpOff) + w * kQueue;
 
   for (int i = threadIdx.x; i < B + 1; i += blockDim.x) hist[i] = 0;
   for (int i = threadIdx.x; i < nTab; i += blockDim.x) tab[i] = b.qtable[cd.tableOff + i];
@@ -477,16 +466,15 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lut
     uint4 *sl = reinterpret_cast<uint4 *>(lut);
     for (int i = threadIdx.x; i < kLutStride / 8; i += blockDim.x) sl[i] = gl[i];
   }
-  for (int i = lane; i < kStage / 8; i += 32) reinterpret_cast<uint4 *>(stage)[i] = fill8;
   __syncthreads();
 
   if (c < cd.nChunks) {
     const long long start = (long long)c << b.lgChunk;
     const int len = (int)min(1LL << b.lgChunk, cd.n - start);
     const float *src = coef + cd.coefOff + start;
-    uint16_t *slot = b.tok + cd.coefOff + start;
+    unsigned *items = b.items + cd.coefOff + start;
     int singles = 0, dups = 0;           // the lane's zero-run tokens
-    int lead = -1, last = -1, nTok = 0;  // warp-uniform: first and last value, tokens so far
+    int lead = -1, last = -1, nVal = 0;  // warp-uniform: first and last value, values so far
 
     // one round: candidates queue[at .. at + n), n <= 32
     auto round = [&](int at, int n) {
@@ -498,57 +486,18 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lut
       const unsigned lower = m & ltMask;
       const int pp = __shfl_sync(kAll, pos, lower ? 31 - __clz(lower) : 0);
       const int prev = lower ? pp : last;
-      const int gap = v && prev >= 0 ? pos - prev - 1 : 0;
-      int sg, dp;
-      run_split_closed(gap, sg, dp);  // 0, 0 for gap 0
-      singles += sg;
-      dups += dp;
-      const int cnt = v ? 1 + sg + dp : 0;
-      int inc = cnt;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(kAll, inc, d);
-        if (lane >= d) inc += t;
+      if (v) {
+        const int gap = prev >= 0 ? pos - prev - 1 : 0;
+        int sg, dp;
+        run_split_closed(gap, sg, dp);  // 0, 0 for gap 0
+        singles += sg;
+        dups += dp;
+        items[nVal + __popc(lower)] = make_item(bin, gap);
+        atomicAdd(&hist[bin], 1u);
       }
       if (lead < 0) lead = __shfl_sync(kAll, pos, __ffs(m) - 1);
       last = __shfl_sync(kAll, pos, 31 - __clz(m));
-      const int total = __shfl_sync(kAll, inc, 31);
-      const int par = (lead + nTok) & 1;  // tokens pair up as their places do
-      if (v) {
-        int t = par + inc - cnt;
-        // dup tokens in the order of run_tokens: runs of 1024, then one per
-        // set bit of the remainder from 512 down to 16, then 8 when more than
-        // 8 remain; the rest are single (prefilled) tokens
-        for (int j = gap >> 10; j > 0; j--) stage[t++] = make_token(B, 7);
-        const int rr = gap & 1023;
-        if (rr >= 16) {
-#pragma unroll
-          for (int lg = 9; lg >= 4; lg--)
-            if ((rr >> lg) & 1) stage[t++] = make_token(B, lg - 3);
-        }
-        const bool eight = (rr & 8) && (rr & 7);
-        if (eight) stage[t++] = make_token(B, 0);
-        t += (rr & 8) && !eight ? 8 : (rr & 7);
-        stage[t] = make_token(bin, 0);
-        atomicAdd(&hist[bin], 1u);
-      }
-      __syncwarp();
-      {
-        uint16_t *g = slot + lead + nTok - par;  // an even place
-        const int end = par + total;
-        const unsigned *s2 = reinterpret_cast<const unsigned *>(stage);
-        for (int i = lane; 2 * i < end; i += 32) {
-          const unsigned two = s2[i];
-          const bool lo = 2 * i >= par, hi = 2 * i + 1 < end;
-          if (lo && hi) reinterpret_cast<unsigned *>(g)[i] = two;
-          else if (lo) g[2 * i] = (uint16_t)two;
-          else g[2 * i + 1] = (uint16_t)(two >> 16);
-        }
-        __syncwarp();
-        for (int i = lane; 8 * i < end; i += 32) reinterpret_cast<uint4 *>(stage)[i] = fill8;
-        __syncwarp();
-      }
-      nTok += total;
+      nVal += __popc(m);
     };
 
     float x[kLaneRun];
@@ -602,16 +551,10 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lut
     if (nq) round(0, nq);
 
     if (lane == 0) {
-      // the tokens sit in the chunk's slot from the first value's position
-      // on (the lead zero run's tokens, written later by runs_kernel, fit
-      // before it, since each token starts at its own element)
       const long long chunk = cd.chunkBase + c;
       const bool any = last >= 0;
-      const int first = any ? lead : len;
-      b.chunkTok[chunk] = nTok;
-      b.chunkSpan[chunk] = make_int2(first, nTok);  // runs_kernel adds the edge runs
-      if (dupV >= 0)
-        b.chunkRun[chunk] = make_int4(first, any ? len - 1 - last : len, any ? 0 : 1, len);
+      b.chunkVal[chunk] = nVal;
+      b.chunkRun[chunk] = make_int4(any ? lead : len, any ? len - 1 - last : len, any ? 0 : 1, len);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -630,12 +573,11 @@ quantize_kernel(DevBatch b, const float *__restrict__ coef, int histOff, int lut
 }
 
 // Join zero runs across chunk edges: the tokens of the runs entering and
-// leaving every chunk, and their counts.  A CTA takes kRunChunks consecutive
+// leaving every chunk that start in it (run codes), and their counts.  A CTA takes kRunChunks consecutive
 // chunks of one cubelet (blockIdx.y), one thread each; the nearest chunks
 // with a value before and after the CTA's range are searched kRunChunks at a
 // time, usually found in the first step, whose loads are issued with the
-// CTA's own.  Bound by the latency of a few dependent loads and the tokens a
-// thread writes: one CTA of 1024 threads per cubelet left most SMs idle (59
+// CTA's own.  Bound by the latency of a few dependent loads: one CTA of 1024 threads per cubelet left most SMs idle (59
 // us for a 2048^2 image of 1024 chunks, 93 us for a 256^3 volume); spread
 // over the SMs a whole call went from 523 to 468 us and from 623 to 529 us.
 constexpr int kRunChunks = 256;
@@ -703,41 +645,28 @@ __global__ void __launch_bounds__(kRunChunks) runs_kernel(DevBatch b) {
 
   int singles = 0, dups = 0;
   if (c < nc) {
-    const int n = (int)cd.n, dupKey = cd.binCount;  // positions stay below 2^31
-    // the run entering the chunk starts at runIn, the one leaving it ends at e
+    const int n = (int)cd.n;  // positions stay below 2^31
     int runIn = 0, e = n;
     if (prev >= 0) {
       const int4 o = cr[prev];
       runIn = (prev << b.lgChunk) + o.w - o.y;
     }
     if (next != INF) e = (next << b.lgChunk) + cr[next].x;
-    const int cstart = c << b.lgChunk;
-    if (val) run_split_closed(e - (cstart + me.w - me.y), singles, dups);
+    if (val) run_split_closed(e - ((c << b.lgChunk) + me.w - me.y), singles, dups);
     if (c == 0) {  // the run starting at element 0 belongs to no chunk's tail
       int sg, dp;
       run_split_closed(val ? me.x : e, sg, dp);
       singles += sg;
       dups += dp;
     }
-    // Tokens of the zero runs at the chunk's edges that start inside it, in
-    // stream order around the stored tokens [lead, lead + nInt): the entering
-    // run's right before them, the leaving run's right after.
-    uint16_t *slot = b.tok + cd.coefOff + cstart;
-    const int nInt = b.chunkTok[cd.chunkBase + c];
-    int nPre = 0, nPost = 0;
-    if (me.x > 0) {
-      const int re = me.z ? e : cstart + me.x, w1 = cstart + (me.z ? me.w : me.x);
-      run_tokens(runIn, re, cstart, w1, dupKey, dupV, [&](uint16_t) { nPre++; });
-      int i = me.x - nPre;
-      run_tokens(runIn, re, cstart, w1, dupKey, dupV, [&](uint16_t t) { slot[i++] = t; });
-    }
-    if (val && me.y > 0) {
-      const int s0 = cstart + me.w - me.y;
-      int i = me.x + nInt;
-      run_tokens(s0, e, s0, cstart + me.w, dupKey, dupV, [&](uint16_t t) { slot[i++] = t; });
-      nPost = i - (me.x + nInt);
-    }
-    b.chunkSpan[cd.chunkBase + c] = make_int2(me.x - nPre, nPre + nInt + nPost);
+    // the tokens that start in this chunk of the run entering it and of the
+    // one leaving it
+    const int cstart = c << b.lgChunk, cend = cstart + me.w;
+    uint2 edge = make_uint2(0u, 0u);
+    if (me.x > 0)
+      edge.x = run_code_in(runIn, val ? cstart + me.x : e, cstart, val ? cstart + me.x : cend);
+    if (val && me.y > 0) edge.y = run_code_in(cend - me.y, e, cend - me.y, cend);
+    b.chunkEdge[cd.chunkBase + c] = edge;
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
@@ -772,7 +701,7 @@ void launch_quantize(DevBatch &b, const float *coef, int maxTable, int maxSymbol
   const int histOff = (maxTable + 3) & ~3;
   const int lutOff = (histOff + maxSymbols + 1 + 3) & ~3;
   const int warpOff = lutOff + (lloyd ? kLutStride / 2 : 0);
-  const int smem = warpOff * (int)sizeof(float) + kQuantWarps * kWarpBytes;
+  const int smem = warpOff * (int)sizeof(float) + kQuantWarps * kQueue * 2;
   raise_smem_limit(quantize_kernel, smem);
   quantize_kernel<<<(unsigned)b.totalQuant, 32 * kQuantWarps, smem, s>>>(b, coef, histOff, lutOff,
                                                                           warpOff);

@@ -60,19 +60,24 @@ inline int sel_group(long long chunks) {
   const long long slots = 152 * 4, g = (chunks + slots - 1) / slots;
   return (int)(g < 1 ? 1 : g > kMaxSelGroup ? kMaxSelGroup : g);
 }
-// Bit packer: a chunk's tokens are split into F slices (F a power of two,
-// 1..32), one lane each; a CTA of kEncThreads lanes packs kEncThreads / F
+// Bit packer: a token chunk's values are split into F slices (F a power of
+// two, 1..32), one lane each; a CTA of kEncThreads lanes packs kEncThreads / F
 // consecutive chunks of one cubelet (four warps: few CTAs, so kernels of
-// another stream still find CTA slots on the SMs).  Short slices keep many warps in flight (a lane's tokens are a
-// serial chain): measured on a 512-cubelet batch (92 K chunks), the encode
-// stage (per-slice bit counts, scans, packer) took 0.79, 0.76, 0.60, 0.52,
-// 0.50 and 0.52 ms for F = 1, 2, 4, 8, 16, 32.
-// F = 16 per 4096 elements unless the launch would then have fewer lanes than
-// one full wave of a 152-SM GB300 (2048 per SM); small batches take 32.  A
-// smaller token chunk has as many lanes per element.
+// another stream still find CTA slots on the SMs).  Short slices keep many
+// warps in flight (a lane's values are a serial chain), long ones share fewer
+// words with their neighbours: 16 lanes per 4096 elements for large batches
+// (encode stage of the mixed batch 0.53, 0.42 and 0.39 ms with 8, 16 and 32,
+// of 729 sparser cubelets of 128^3 0.52, 0.51 and 0.64 ms); a call with fewer
+// than kEncLanes lanes that way takes as many more as bring it there, at most
+// 32 a chunk (packer of a 256^3 volume: 39, 21 and 14 us with 2^16, 2^17 and
+// 2^18 lanes).
 constexpr int kEncThreads = 128;
-constexpr long long kEncFullWave = 152LL * 2048;
-inline int enc_slices(long long chunks) { return chunks * 16 >= kEncFullWave ? 16 : 32; }
+constexpr long long kEncLanes = 1 << 18;
+inline int enc_slices(long long chunks, int lgChunk) {
+  int f = 16 >> (kMaxLgChunk - lgChunk);
+  while (f < 32 && chunks * f < kEncLanes) f *= 2;
+  return f;
+}
 constexpr int kTileBudget = 16384;      // floats of shared memory per DWT tile
 constexpr int kMaxAxis = 16384;         // longest padded axis (one row per tile)
 
@@ -80,38 +85,46 @@ constexpr int kMaxAxis = 16384;         // longest padded axis (one row per tile
 // row kernel.  Rows are flattened r = b + B*a; row (a,b) of the input starts
 // at in + a*inSA + b*inSB (contiguous along c); element (a,b,c) of the
 // output goes to out + a*outSA + b*outSB + c*outSC.
-// A Huffman token: symbol (bin, or binCount = the zero-run key) in bits 0-12,
-// the zero-run length code v (run of 2^(v+3)) in bits 13-15.
-__host__ __device__ inline uint16_t make_token(int sym, int v) {
-  return (uint16_t)(sym | (v << 13));
+// A value of a token chunk: its bin in bits 16 and up, the zero-bin elements
+// between it and the chunk's value before it (0 for the first) below.
+__host__ __device__ inline unsigned make_item(int bin, int gap) {
+  return ((unsigned)bin << 16) | (unsigned)gap;
 }
 
-// Tokens of a zero-bin run [s, e) that start inside [w0, w1), in order
-// (HuffmanDup::dupCount / Huffman::dupEncodeString, huffman.h:31-57,
-// 278-296: greedy runs of 1024, then the largest power of two >= 8 while
-// more than 8 remain, then single zero-bin tokens).  Calls f(token).  At
-// most 19 tokens start in a window of kChunk elements.
-template <class F>
-__host__ __device__ inline void run_tokens(int s, int e, int w0, int w1, int dupKey, int dupV,
-                                           F f) {
-  const int L = e - s;
-  const int q = L >> 10;
-  int j0 = 0;
-  if (w0 > s) j0 = (int)(((unsigned)(w0 - s) + 1023u) >> 10);
-  for (int j = j0; j < q; j++) {
-    if (s + (j << 10) >= w1) break;
-    f(make_token(dupKey, 7));
-  }
-  int pos = s + (q << 10);
-  int r = L - (q << 10);
+// Tokens of a zero-bin run, or of the part of one that starts in a chunk:
+// 1024s from bit 16 on, powers of two 512 .. 16 as bits 5 .. 0 of bits 8 .. 13,
+// below that 0 .. 8 singles, 8 + k for an eight and k = 1 .. 7 singles, or
+// kEightAlone.  A whole run of L: see run_code.
+constexpr int kEightAlone = 16;
+__host__ __device__ inline unsigned run_code(int L) {
+  return ((unsigned)(L >> 10) << 16) | ((unsigned)((L >> 4) & 63) << 8) | (unsigned)(L & 15);
+}
+
+// Tokens of a zero-bin run [s, e) that start inside [w0, w1) as a run code
+// (HuffmanDup::dupCount / Huffman::dupEncodeString, huffman.h:31-57, 278-296:
+// greedy runs of 1024, then the largest power of two >= 8 while more than 8
+// remain, then single zero-bin tokens).
+__host__ __device__ inline unsigned run_code_in(int s, int e, int w0, int w1) {
+  const int q = (e - s) >> 10;
+  int j0 = w0 > s ? (int)(((unsigned)(w0 - s) + 1023u) >> 10) : 0;
+  int j1 = w1 > s ? (int)(((unsigned)(w1 - s) + 1023u) >> 10) : 0;
+  if (j0 > q) j0 = q;
+  if (j1 > q) j1 = q;
+  unsigned code = (unsigned)(j1 - j0) << 16;
+  int pos = s + (q << 10), r = e - pos;
+  bool eight = false;
   while (r > 8) {
-    int lg = 31 - clz32(r);
-    if (pos >= w0 && pos < w1) f(make_token(dupKey, lg - 3));
+    const int lg = 31 - clz32(r);
+    if (pos >= w0 && pos < w1) {
+      if (lg == 3) eight = true;
+      else code |= 1u << (8 + lg - 4);
+    }
     pos += 1 << lg;
     r -= 1 << lg;
   }
   const int a = pos > w0 ? pos : w0, z = pos + r < w1 ? pos + r : w1;
-  for (int x = a; x < z; x++) f(make_token(dupV, 0));
+  const int singles = z > a ? z - a : 0;
+  return code | (unsigned)(eight ? (singles ? 8 + singles : kEightAlone) : singles);
 }
 
 struct CubeletState;
@@ -215,11 +228,12 @@ struct DevBatch {
   CubeletState *state;            // [n]
   float *coef;                    // coefficients (ping)
   float *coef2;                   // second buffer (pong)
-  uint16_t *tok;                  // Huffman tokens: a token chunk's from its first element's place on
+  unsigned *items;                // values (make_item): a token chunk's from its first element's
+                                  // place on (the second coefficient buffer, free by then)
   int lgChunk;                    // log2 of the elements per token chunk
-  int *chunkTok;                  // tokens stored per chunk by quantize
-  int2 *chunkSpan;                // per chunk: first token slot, token count
-                                  // (with the zero-run tokens at its edges)
+  int *chunkVal;                  // values per token chunk
+  uint2 *chunkEdge;               // per chunk: tokens (run_code) that start in it of the zero run
+                                  // entering it and of the one leaving it
   unsigned *selHist;              // [n][kSelectBins]
   float *lloydHist;               // [n][kLloydBins][2] (count, sum)
   float *qtable;                  // quantizer tables
@@ -227,7 +241,8 @@ struct DevBatch {
   float *dqtable;                 // dequant values [n][binCount]
   unsigned long long *hist;       // [n][kMaxSymbols] Huffman counts
   int4 *chunkRun;                 // per chunk: lead, trail, allZero, len
-  unsigned long long *chunkBits;  // per chunk bit count / offset
+  unsigned *chunkLen;             // per chunk bit count
+  unsigned long long *chunkBits;  // per chunk bit offset in its cubelet's stream
   unsigned long long *codes;      // [n][kMaxSymbols] code bits
   uint8_t *codeLen;               // [n][kMaxSymbols]
   int *decode;                    // [n][4*kMaxSymbols]
