@@ -11,8 +11,9 @@ from wavelets_gb300 import lib, params as P
 
 pytestmark = pytest.mark.gpu
 
-LEVELS = {16: 4, 32: 5, 48: 4, 64: 5, 96: 4, 128: 5, 192: 4, 256: 5}  # in the register kernel
-CASES = [(L, s) for L, most in LEVELS.items() for s in (1, 2, most, most + 1)
+# most levels in the register kernel
+LEVELS = {16: 4, 32: 5, 48: 4, 64: 6, 96: 4, 128: 7, 192: 4, 256: 8, 512: 9, 1024: 10, 2048: 11}
+CASES = [(L, s) for L, most in LEVELS.items() for s in sorted({1, 2, 4, 5, most - 1, most, most + 1})
          if L % (1 << s) == 0 and s <= (L - 1).bit_length()]
 
 
@@ -71,3 +72,29 @@ def test_x_rows_of_every_type(ctx, L, s, dtype):
             back_odd = ctx.inverse_transform(odd, (Z - 1, L, Y), (s, 1, 0), wavelet,
                                              (X, Y, Z - 1), dtype)
             assert np.array_equal(back[:Z - 1], back_odd)
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32])
+@pytest.mark.parametrize("Y,X,steps", [(64, 64, (-1, -1)), (128, 256, (-1, -1)), (256, 48, (3, 5)),
+                                       (512, 96, (4, 9)), (96, 512, (7, 4)), (1024, 64, (6, 10)),
+                                       (2048, 128, (-1, -1)), (32, 2048, (11, 5)),
+                                       (1024, 2048, (3, 2)), (600, 1000, (-1, -1)),
+                                       (2048, 1023, (10, 1))])
+def test_images(ctx, Y, X, steps, dtype):
+    """One layer (rows paired along the other axis) against the middle one of
+    three layers, which the other kernels take; deep levels, long axes, cut
+    rows; integers restored the same."""
+    rng = np.random.default_rng(Y + X)
+    img = rng.normal(128, 60, (1, Y, X))
+    img = img.astype(np.float32) if dtype == np.float32 else np.clip(img, 0, 255).astype(dtype)
+    three = np.repeat(img, 3, 0)
+    for wavelet in (P.HAAR, P.CDF97):
+        p = P.Params(steps=(steps[0], steps[1], 0), wavelet=wavelet)
+        one, (_, Xp, Yp) = ctx.forward_transform(img, p)
+        all3, _ = ctx.forward_transform(three, p)
+        one, all3 = one.reshape(Yp, Xp), all3.reshape(Yp, Xp, 3)
+        assert np.array_equal(one, all3[:, :, 1])
+        st = P.clamp_steps(p.steps, (X, Y, 1))
+        back = ctx.inverse_transform(one, (1, Xp, Yp), st, wavelet, (X, Y, 1), dtype)
+        back3 = ctx.inverse_transform(all3, (3, Xp, Yp), st, wavelet, (X, Y, 3), dtype)
+        assert np.array_equal(back[0], back3[1])

@@ -1,454 +1,49 @@
-// Wavelet passes entirely in registers, for rows whose neighbours are
-// neighbours in memory: the y pass of either direction (strided rows on both
-// sides, z contiguous), the forward x pass (contiguous source rows of any
-// type, z contiguous in the output) and the inverse x pass (the reverse, into
-// rows of any type).
-//
-// A thread holds K consecutive elements of TWO neighbouring rows, packed as
-// pairs of floats: every lifting operation is one packed instruction
-// (add / fma .f32x2) for both, and every load and store moves eight bytes.
-// G = L / K lanes hold a row pair; they lie C = 32 / G lanes apart, so the C
-// lanes next to each other touch neighbouring memory.  All levels run on the
-// K elements in place (M = K/2, K/4, .. pairs a lane), with two 64-bit
-// shuffles down and two up per level for the pairs at the lane edges, and a
-// finished value goes straight from its register to its place in global
-// memory: no shared memory, no barriers.
-//
-// K = 32 for L = 32 .. 256 (five levels), 48 for L = 48, 96, 192 (four), 16
-// for L = 16 (four); deeper transforms, other lengths and an odd number of
-// neighbouring rows stay with the tile kernels.  With 64 to 96 values per
-// thread in flight the pass is bound by HBM: the y passes of 729 cubelets of
-// 128^3 (1.5 G elements) take 1.56 ms, 7.8 TB/s of their eight bytes an
-// element (2.77 ms in the column-tile kernel), the inverse y passes of the
-// mixed batch 0.55 ms (1.22 ms through the row kernel's tile).
-//
-// The x passes read or write a lane's K elements of a source or output row
-// with vectors of 32 bytes (16 where its address or K asks for it), a run cut
-// by the real row length element by element; they take inputs in device memory
-// and outputs whose rows start at multiples of 16 bytes.
-// The inverse x passes of the mixed batch take 0.73 ms (1.47 ms through the
-// row kernel's tile); forward, the half of a 2 GiB volume's cubelets that the
-// kernel took first (before it accepted 16-byte starts) 0.71 ms against 0.91
-// ms for the other half in the row kernel.
-//
-// Each lifting step does the arithmetic of dwt.cu / dwt_cols.cu / dwt_rows.cu
-// (the same operands, rounded the same), so the values are identical.
-#include <cuda_runtime.h>
-
-#include <type_traits>
-
-#include "dwt_common.cuh"
+// Register passes (dwt_strided.cuh): which passes they take, and their launch.
 #include "wl_internal.h"
 
 namespace wl {
+
+// one per pass and element type (dwt_strided_*.cu)
+#define WL_STRIDED_DECLARE(NAME) \
+  void NAME(const PassDesc *p, const int *tp, int n, int blocks, int L, bool full,  \
+            cudaStream_t s);
+WL_STRIDED_DECLARE(strided_y)
+WL_STRIDED_DECLARE(strided_y_inv)
+WL_STRIDED_DECLARE(strided_x_u8)
+WL_STRIDED_DECLARE(strided_x_u16)
+WL_STRIDED_DECLARE(strided_x_i32)
+WL_STRIDED_DECLARE(strided_x_f32)
+WL_STRIDED_DECLARE(strided_x_inv_u8)
+WL_STRIDED_DECLARE(strided_x_inv_u16)
+WL_STRIDED_DECLARE(strided_x_inv_i32)
+WL_STRIDED_DECLARE(strided_x_inv_f32)
+
 namespace {
-using namespace dwtc;
 
-constexpr int kThreads = 128;
-constexpr unsigned kAll = 0xffffffffu;
+constexpr int kWarps = 4;  // per block (dwt_strided.cuh kThreads)
 
-typedef unsigned long long f2;  // two floats: the same element of two rows
-
-__device__ __forceinline__ f2 pack(float a) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
-  return r;
-}
-__device__ __forceinline__ f2 pack(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack(f2 v, float &a, float &b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
-// lane position along the row: lane `seg` of G, C lanes between neighbours
-template <int G> struct Along {
-  static constexpr int C = 32 / G;
-  int seg;
-  // the value of the next / previous lane of the row, `own` at its end
-  __device__ __forceinline__ f2 next(f2 v, f2 own) const {
-    if (G == 1) return own;
-    const f2 o = __shfl_down_sync(kAll, v, C);
-    return seg == G - 1 ? own : o;
-  }
-  __device__ __forceinline__ f2 prev(f2 v, f2 own) const {
-    if (G == 1) return own;
-    const f2 o = __shfl_up_sync(kAll, v, C);
-    return seg == 0 ? own : o;
-  }
-};
-
-// One forward level on M pairs a lane: low-pass values in e[], details in o[]
-// (dwt_rows.cu fwd_level; mirrored ends s[h] = s[h-1], d[-1] = d[0]).
-template <int M, int G, bool HAAR>
-__device__ __forceinline__ void fwd_level(f2 (&e)[M], f2 (&o)[M], const Along<G> &at) {
-  if (HAAR) {  // dwt_cpu.cc:159-162
-    const f2 c = pack(kInvSqrt2), neg = pack(-1.0f);
-#pragma unroll
-    for (int k = 0; k < M; k++) {
-      const f2 a = e[k], b = o[k];
-      o[k] = mul2(fma2(b, neg, a), c);  // a - b, rounded once
-      e[k] = mul2(add2(a, b), c);
-    }
-    return;
-  }
-  const f2 ka = pack(kAlpha), kb = pack(kBeta), kg = pack(kGamma), kd = pack(kDelta);
-  const f2 eN = at.next(e[0], e[M - 1]);
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = fma2(ka, add2(e[k], k + 1 < M ? e[(k + 1) % M] : eN), o[k]);
-  const f2 d1P = at.prev(o[M - 1], o[0]);
-#pragma unroll
-  for (int k = 0; k < M; k++) e[k] = fma2(kb, add2(k ? o[(k + M - 1) % M] : d1P, o[k]), e[k]);
-  const f2 s1N = at.next(e[0], e[M - 1]);
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = fma2(kg, add2(e[k], k + 1 < M ? e[(k + 1) % M] : s1N), o[k]);
-  const f2 d2P = at.prev(o[M - 1], o[0]);
-#pragma unroll
-  for (int k = 0; k < M; k++) e[k] = fma2(kd, add2(k ? o[(k + M - 1) % M] : d2P, o[k]), e[k]);
-}
-
-// The inverse: low-pass e[], details o[] in, even and odd elements out
-// (dwt_rows.cu inv_level).
-template <int M, int G, bool HAAR>
-__device__ __forceinline__ void inv_level(f2 (&e)[M], f2 (&o)[M], const Along<G> &at) {
-  if (HAAR) {  // dwt_cpu.cc:193-196
-    const f2 c = pack(kInvSqrt2), neg = pack(-1.0f);
-#pragma unroll
-    for (int k = 0; k < M; k++) {
-      const f2 a = e[k], b = o[k];
-      e[k] = mul2(c, add2(a, b));
-      o[k] = mul2(c, fma2(b, neg, a));
-    }
-    return;
-  }
-  const f2 ka = pack(-kAlpha), kb = pack(-kBeta), kg = pack(-kGamma), kd = pack(-kDelta);
-  const f2 d2P = at.prev(o[M - 1], o[0]);
-#pragma unroll
-  for (int k = 0; k < M; k++) e[k] = fma2(kd, add2(k ? o[(k + M - 1) % M] : d2P, o[k]), e[k]);
-  const f2 s1N = at.next(e[0], e[M - 1]);
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = fma2(kg, add2(e[k], k + 1 < M ? e[(k + 1) % M] : s1N), o[k]);
-  const f2 d1P = at.prev(o[M - 1], o[0]);
-#pragma unroll
-  for (int k = 0; k < M; k++) e[k] = fma2(kb, add2(k ? o[(k + M - 1) % M] : d1P, o[k]), e[k]);
-  const f2 eN = at.next(e[0], e[M - 1]);
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = fma2(ka, add2(e[k], k + 1 < M ? e[(k + 1) % M] : eN), o[k]);
-}
-
-// A row pair in global memory: position q at base + q * stride floats.
-struct Row {
-  float *base;
-  long long stride;
-  bool ok;
-  __device__ __forceinline__ f2 get(int q) const {
-    return ok ? *reinterpret_cast<const f2 *>(base + q * stride) : 0ull;
-  }
-  __device__ __forceinline__ void put(int q, f2 v) const {
-    if (ok) *reinterpret_cast<f2 *>(base + q * stride) = v;
-  }
-};
-
-// Levels LEV .. S-1 on the 2 M values v[] of a lane, each band to its place
-// with the deferred lifting scale.
-template <int LEV, int M, int G, bool HAAR>
-__device__ __forceinline__ void fwd_from(const f2 (&v)[2 * M], int S, const float *scale,
-                                         const Along<G> &at, const Row &out) {
-  constexpr int H = M * G;  // pairs of this level
-  f2 e[M], o[M];
-#pragma unroll
-  for (int k = 0; k < M; k++) {
-    e[k] = v[2 * k];
-    o[k] = v[2 * k + 1];
-  }
-  fwd_level<M, G, HAAR>(e, o, at);
-  const f2 sc = pack(scale[LEV]);
-#pragma unroll
-  for (int k = 0; k < M; k++) out.put(H + M * at.seg + k, mul2(o[k], sc));
-  if constexpr (M % 2 == 0) {
-    if (LEV + 1 < S) {
-      fwd_from<LEV + 1, M / 2, G, HAAR>(e, S, scale, at, out);
-      return;
-    }
-  }
-  const f2 low = pack(scale[LEV + 1]);
-#pragma unroll
-  for (int k = 0; k < M; k++) out.put(M * at.seg + k, mul2(e[k], low));
-}
-
-// The 2 M values v[] of level LEV's input from the bands of levels LEV ..
-// S-1 (rscale: the reciprocal of the deferred scale).
-template <int LEV, int M, int G, bool HAAR>
-__device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const float *rscale,
-                                       const Along<G> &at, const Row &in) {
-  constexpr int H = M * G;
-  f2 e[M], o[M];
-  const f2 sc = pack(rscale[LEV]);
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = in.get(H + M * at.seg + k);
-  bool deeper = false;
-  if constexpr (M % 2 == 0) {
-    if (LEV + 1 < S) {
-      inv_to<LEV + 1, M / 2, G, HAAR>(e, S, rscale, at, in);
-      deeper = true;
-    }
-  }
-  if (!deeper) {
-    const f2 low = pack(rscale[LEV + 1]);
-#pragma unroll
-    for (int k = 0; k < M; k++) e[k] = mul2(in.get(M * at.seg + k), low);
-  }
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = mul2(o[k], sc);
-  inv_level<M, G, HAAR>(e, o, at);
-#pragma unroll
-  for (int k = 0; k < M; k++) {
-    v[2 * k] = e[k];
-    v[2 * k + 1] = o[k];
-  }
-}
-
-// ---- rows of the source and of the output (x passes) ----
-// bytes per vector access of a lane's K elements
-template <typename T, int K> __host__ __device__ constexpr int vec_bytes() {
-  return (K * (int)sizeof(T)) % 32 == 0 ? 32 : 16;
-}
-template <int VB> __device__ __forceinline__ void load_vec(const void *p, unsigned *w) {
-  if constexpr (VB == 32) {
-    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]),
-                   "=r"(w[6]), "=r"(w[7])
-                 : "l"(p));
-  } else {
-    const uint4 q = *static_cast<const uint4 *>(p);
-    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
-  }
-}
-template <int VB> __device__ __forceinline__ void store_vec(void *p, const unsigned *w) {
-  if constexpr (VB == 32) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 :: "l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
-                    "r"(w[6]), "r"(w[7])
-                 : "memory");
-  } else {
-    *static_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
-// element k of a vector of 32-bit words as a float, and back
-template <typename T> __device__ __forceinline__ float from_words(const unsigned *w, int k) {
-  if constexpr (std::is_same<T, float>::value) return __uint_as_float(w[k]);
-  else if constexpr (sizeof(T) == 4) return (float)(int)w[k];
-  else if constexpr (sizeof(T) == 2) return (float)((w[k / 2] >> (16 * (k & 1))) & 0xffffu);
-  else return (float)((w[k / 4] >> (8 * (k & 3))) & 0xffu);
-}
-template <typename T> __device__ __forceinline__ unsigned to_bits(float f) {
-  T t;
-  store_from_float(&t, f);
-  if constexpr (std::is_same<T, float>::value) return __float_as_uint(f);
-  else return (unsigned)t;
-}
-
-template <typename T, int K, int VB>
-__device__ __forceinline__ void load_vecs(const T *p, float (&v)[K]) {
-  constexpr int E = VB / (int)sizeof(T);
-#pragma unroll
-  for (int j = 0; j < K / E; j++) {
-    unsigned w[VB / 4];
-    load_vec<VB>(p + j * E, w);
-#pragma unroll
-    for (int k = 0; k < E; k++) v[j * E + k] = from_words<T>(w, k);
-  }
-}
-template <typename T, int K, int VB>
-__device__ __forceinline__ void store_vecs(T *p, const float (&v)[K]) {
-  constexpr int E = VB / (int)sizeof(T), P = 4 / (int)sizeof(T);
-#pragma unroll
-  for (int j = 0; j < K / E; j++) {
-    unsigned w[VB / 4];
-#pragma unroll
-    for (int i = 0; i < VB / 4; i++) {
-      w[i] = 0;
-#pragma unroll
-      for (int k = 0; k < P; k++)
-        w[i] |= to_bits<T>(v[j * E + i * P + k]) << (8 * (int)sizeof(T) * k);
-    }
-    store_vec<VB>(p + j * E, w);
-  }
-}
-
-// K elements [first, first + K) of a row of n real elements (REPEAT clamp)
-template <typename T, int K>
-__device__ __forceinline__ void load_run(const T *row, int first, int n, float (&v)[K]) {
-  if (first + K <= n) {
-    constexpr int VB = vec_bytes<T, K>();
-    if (VB == 32 && (reinterpret_cast<size_t>(row + first) & 31) == 0)
-      load_vecs<T, K, VB>(row + first, v);
-    else
-      load_vecs<T, K, 16>(row + first, v);
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < K; k++) v[k] = load_as_float(row + min(first + k, n - 1));
-}
-template <typename T, int K>
-__device__ __forceinline__ void store_run(T *row, int first, int n, const float (&v)[K]) {
-  if (first + K <= n) {
-    constexpr int VB = vec_bytes<T, K>();
-    if (VB == 32 && (reinterpret_cast<size_t>(row + first) & 31) == 0)
-      store_vecs<T, K, VB>(row + first, v);
-    else
-      store_vecs<T, K, 16>(row + first, v);
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < K; k++)
-    if (first + k < n) store_from_float(row + first + k, v[k]);
-}
-
-enum Pass { kStrided, kStridedInv, kSource, kOutput };  // y forward / inverse, x forward / inverse
-
-template <typename T, int K, int G, bool HAAR, int PASS>
-__device__ __forceinline__ void run_rows(const PassDesc &d, int tile, const float *scale) {
-  constexpr int C = 32 / G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const Along<G> at{lane / C};
-  const int row = 2 * ((tile * (kThreads / 32) + warp) * C + lane % C);
-  const bool ok = row < d.rows;
-  int a = 0, b = 0;
-  if (ok) {
-    a = row / d.B;
-    b = row - a * d.B;  // B even: b and b + 1 are one pair
-  }
-  Row in{nullptr, d.inSC, ok}, out{nullptr, d.outSC, ok};
-  if (ok && PASS != kSource)
-    in.base = const_cast<float *>(static_cast<const float *>(d.in)) + (long long)a * d.inSA + b;
-  if (ok && PASS != kOutput)
-    out.base = static_cast<float *>(d.out) + (long long)a * d.outSA + b;
-  f2 v[K];
-  if constexpr (PASS == kStrided) {
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = in.get(K * at.seg + k);
-  }
-  if constexpr (PASS == kSource) {
-    float x[2][K];
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const T *src = static_cast<const T *>(d.in) + (long long)min(a, d.clampA - 1) * d.inSA +
-                     (long long)min(b + r, d.clampB - 1) * d.inSB;
-      if (ok) {
-        load_run<T, K>(src, K * at.seg, min(K * G, d.clampL), x[r]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < K; k++) x[r][k] = 0.f;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = pack(x[0][k], x[1][k]);
-  }
-  if constexpr (PASS == kStrided || PASS == kSource) {
-    fwd_from<0, K / 2, G, HAAR>(v, d.steps, scale, at, out);
-  } else {
-    inv_to<0, K / 2, G, HAAR>(v, d.steps, scale, at, in);
-    if constexpr (PASS == kStridedInv) {
-#pragma unroll
-      for (int k = 0; k < K; k++) out.put(K * at.seg + k, v[k]);
-    } else {
-      if (!ok || a >= d.cropA) return;
-      float x[2][K];
-#pragma unroll
-      for (int k = 0; k < K; k++) unpack(v[k], x[0][k], x[1][k]);
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-        if (b + r < d.cropB)
-          store_run<T, K>(static_cast<T *>(d.out) + (long long)a * d.outSA +
-                              (long long)(b + r) * d.outSB,
-                          K * at.seg, min(K * G, d.cropL), x[r]);
-    }
-  }
-}
-
-template <typename T, int K, int G, int PASS>
-__global__ void __launch_bounds__(kThreads)
-dwt_strided_kernel(const PassDesc *__restrict__ passes, const int *__restrict__ tilePrefix,
-                   int nPasses) {
-  constexpr bool INV = PASS == kStridedInv || PASS == kOutput;
-  __shared__ float scale[16];
-  const int bid = blockIdx.x;
-  int lo = 0, hi = nPasses - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tilePrefix[mid] <= bid) lo = mid; else hi = mid - 1;
-  }
-  const PassDesc &d = passes[lo];
-  const int S = d.steps;
-  const bool haar = d.wavelet == WL_HAAR;
-  if ((int)threadIdx.x <= S) {
-    const float s = haar ? 1.0f : lifting_scale(threadIdx.x, S);
-    scale[threadIdx.x] = INV && !haar ? 1.0f / s : s;
-  }
-  __syncthreads();
-  if (haar) run_rows<T, K, G, true, PASS>(d, bid - tilePrefix[lo], scale);
-  else run_rows<T, K, G, false, PASS>(d, bid - tilePrefix[lo], scale);
-}
-
-// lanes per row pair and elements per lane; 0: another kernel
+// lanes per row pair (0: another kernel), elements per lane and the most levels
 int strided_lanes(int L) {
   switch (L) {
     case 16: case 32: case 48: return 1;
     case 64: case 96: return 2;
     case 128: case 192: return 4;
     case 256: return 8;
+    case 512: return 16;
+    case 1024: case 2048: return 32;
     default: return 0;
   }
 }
-
-template <typename T, int PASS>
-void launch_len(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s) {
-  switch (L) {
-    case 16: dwt_strided_kernel<T, 16, 1, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    case 32: dwt_strided_kernel<T, 32, 1, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    case 48: dwt_strided_kernel<T, 48, 1, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    case 64: dwt_strided_kernel<T, 32, 2, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    case 96: dwt_strided_kernel<T, 48, 2, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    case 128: dwt_strided_kernel<T, 32, 4, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    case 192: dwt_strided_kernel<T, 48, 4, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-    default: dwt_strided_kernel<T, 32, 8, PASS><<<blocks, kThreads, 0, s>>>(p, tp, n); break;
-  }
-}
-
-// the x passes by element type
-template <int PASS>
-void launch_type(const PassDesc *p, const int *tp, int n, int blocks, int L, int dtype,
-                 cudaStream_t s) {
-  switch (dtype) {
-    case WL_U8: launch_len<uint8_t, PASS>(p, tp, n, blocks, L, s); break;
-    case WL_U16: launch_len<uint16_t, PASS>(p, tp, n, blocks, L, s); break;
-    case WL_I32: launch_len<int32_t, PASS>(p, tp, n, blocks, L, s); break;
-    default: launch_len<float, PASS>(p, tp, n, blocks, L, s); break;
-  }
+int strided_levels(int L) {
+  if (L % 48 == 0) return 4;  // 48 elements a lane halve four times
+  int n = 0;
+  while ((2 << n) <= L) n++;
+  return n;
 }
 
 // length, levels and paired rows as the kernels take them
 bool shape_fits(const PassDesc &d) {
-  const int g = strided_lanes(d.L);
-  return g && d.steps >= 1 && d.B % 2 == 0 && d.steps <= (d.L / g == 32 ? 5 : 4);
+  return strided_lanes(d.L) && d.steps >= 1 && d.B % 2 == 0 && d.steps <= strided_levels(d.L);
 }
 // rows at base with these strides (elements of es bytes) start at multiples
 // of 16 bytes (K elements are a multiple of 16 bytes for every type)
@@ -458,8 +53,8 @@ bool rows_aligned(const void *base, long long sa, long long sb, int es) {
 
 }  // namespace
 
-// rows per block (both rows of kThreads / 32 warps of 32 / G pairs)
-int dwt_strided_rows_per_block(int L) { return 2 * (kThreads / 32) * (32 / strided_lanes(L)); }
+// rows per block (both rows of kWarps warps of 32 / G pairs)
+int dwt_strided_rows_per_block(int L) { return 2 * kWarps * (32 / strided_lanes(L)); }
 
 bool dwt_strided_fits(const PassDesc &d) {
   // neighbouring row pairs stay eight-byte aligned
@@ -475,15 +70,24 @@ bool dwt_strided_output_fits(const PassDesc &d, int es) {
          rows_aligned(d.out, d.outSA, d.outSB, es);
 }
 
+bool dwt_strided_full(const PassDesc &d, bool inverse) {
+  int own = 0;  // levels on a lane's own elements
+  for (int k = d.L / strided_lanes(d.L); k % 2 == 0; k /= 2) own++;
+  return d.steps > own || (inverse && d.exact);
+}
+
 void launch_dwt_strided(const PassDesc *p, const int *tp, int n, int blocks, int L, bool inverse,
-                        cudaStream_t s) {
-  if (inverse) launch_len<float, kStridedInv>(p, tp, n, blocks, L, s);
-  else launch_len<float, kStrided>(p, tp, n, blocks, L, s);
+                        bool full, cudaStream_t s) {
+  (inverse ? strided_y_inv : strided_y)(p, tp, n, blocks, L, full, s);
 }
 void launch_dwt_strided_x(const PassDesc *p, const int *tp, int n, int blocks, int L, int dtype,
-                          bool inverse, cudaStream_t s) {
-  if (inverse) launch_type<kOutput>(p, tp, n, blocks, L, dtype, s);
-  else launch_type<kSource>(p, tp, n, blocks, L, dtype, s);
+                          bool inverse, bool full, cudaStream_t s) {
+  switch (dtype) {
+    case WL_U8: (inverse ? strided_x_inv_u8 : strided_x_u8)(p, tp, n, blocks, L, full, s); break;
+    case WL_U16: (inverse ? strided_x_inv_u16 : strided_x_u16)(p, tp, n, blocks, L, full, s); break;
+    case WL_I32: (inverse ? strided_x_inv_i32 : strided_x_i32)(p, tp, n, blocks, L, full, s); break;
+    default: (inverse ? strided_x_inv_f32 : strided_x_f32)(p, tp, n, blocks, L, full, s); break;
+  }
 }
 
 }  // namespace wl

@@ -94,9 +94,12 @@ int rowreg_key(int L) { return (1 << 20) | L; }
 int rowreg_t_key(int dtype, int L) { return (1 << 21) | (dtype << 16) | L; }
 int rowreg_inv_key(int L) { return (1 << 23) | L; }
 int rowreg_inv_t_key(int outType, int L) { return (1 << 24) | (outType << 16) | L; }
-int strided_key(bool inverse, int L) { return (1 << (inverse ? 26 : 25)) | L; }
-int strided_x_key(bool inverse, int dtype, int L) {
-  return (1 << (inverse ? 28 : 27)) | (dtype << 16) | L;
+int strided_key(bool inverse, const PassDesc &d) {
+  return (1 << (inverse ? 26 : 25)) | (dwt_strided_full(d, inverse) ? 1 << 14 : 0) | d.L;
+}
+int strided_x_key(bool inverse, int dtype, const PassDesc &d) {
+  return (1 << (inverse ? 28 : 27)) | (dtype << 16) |
+         (dwt_strided_full(d, inverse) ? 1 << 14 : 0) | d.L;
 }
 enum RegKind { kRegNone, kRegInPlace, kRegTile, kRegInvInPlace, kRegInvTile, kRegStrided,
                kRegInvStrided, kRegStridedX, kRegInvStridedX };
@@ -534,6 +537,28 @@ wl_status check_params(wl_ctx *ctx, const wl_params &p) {
   return WL_OK;
 }
 
+// A pass with one row per `a` with its rows along `b` (images have one layer),
+// where the register kernels look for a row's neighbour.
+PassDesc rows_along_b(PassDesc d) {
+  if (d.B == 1) {
+    std::swap(d.inSA, d.inSB);
+    std::swap(d.outSA, d.outSB);
+    std::swap(d.clampA, d.clampB);
+    std::swap(d.cropA, d.cropB);
+    d.inSA = d.outSA = 0;  // a is 0 throughout
+    d.B = d.rows;
+  }
+  return d;
+}
+// Put a forward pass whose source rows are contiguous on the register kernel
+// when it takes it (elements of dtype; not over the host link).
+bool put_source_pass(const PassDesc &pass, int dtype, bool hostIn, PassGroups &gs) {
+  const PassDesc d = rows_along_b(pass);
+  if (hostIn || !dwt_strided_source_fits(d, dtype_size(dtype))) return false;
+  gs[strided_x_key(false, dtype, d)].push_back(d);
+  return true;
+}
+
 // Build PassDescs for one cubelet's forward transform.
 // Column-tile layouts: x pass [raw x-y-z] -> z-y-x, y pass z-y-x -> z-x-y,
 // z pass z-x-y in place (a-b-c lists axes from fastest to slowest).  Rows
@@ -563,8 +588,7 @@ bool forward_passes_cols(const Plan &pl, const void *in, bool hostIn, float *coe
   d.out = o2;
   d.outSA = Zp; d.outSB = 1; d.outSC = Zp * Yp;
   d.steps = pl.sx;
-  if (!hostIn && dwt_strided_source_fits(d, dtype_size(pl.dtype))) {
-    xs[strided_x_key(false, pl.dtype, d.L)].push_back(d);
+  if (put_source_pass(d, pl.dtype, hostIn, xs)) {
   } else if (dwt_rowreg_fits(d.L, d.steps)) {
     d.T = dwt_rowreg_t_rows_per_block(d.L); d.tiles = (d.rows + d.T - 1) / d.T;
     xs[rowreg_t_key(pl.dtype, d.L)].push_back(d);
@@ -584,7 +608,9 @@ bool forward_passes_cols(const Plan &pl, const void *in, bool hostIn, float *coe
   e.outSA = Zp; e.outSB = 1; e.outSC = Zp * Xp;
   e.steps = pl.sy;
   e.T = dwt_cols_tile_rows(e.L); e.tiles = (e.rows + e.T - 1) / e.T;
-  ys[dwt_strided_fits(e) ? strided_key(false, e.L) : group_key(true, WL_F32, e.L)].push_back(e);
+  // (the rows are contiguous where there is one layer)
+  if (!put_source_pass(e, WL_F32, false, ys))
+    ys[dwt_strided_fits(e) ? strided_key(false, e) : group_key(true, WL_F32, e.L)].push_back(e);
   if (pl.sz == 0) return false;
   // z pass: rows (a = y, b = x) of z-x-y, in place
   PassDesc f = e;
@@ -697,7 +723,9 @@ bool forward_passes(const Plan &pl, const void *in, bool hostIn, float *coef, fl
   }
   d.T = dwt_tile_rows(d.L, d.exact && d.wavelet == WL_CDF97);
   d.tiles = (d.rows + d.T - 1) / d.T;
-  xs[group_key(false, pl.dtype, d.L)].push_back(d);
+  const bool filterBank = d.exact && d.wavelet == WL_CDF97;
+  if (filterBank || pl.identity || !put_source_pass(d, pl.dtype, hostIn, xs))
+    xs[group_key(false, pl.dtype, d.L)].push_back(d);
   if (pl.identity) return false;
   // y pass: rows (x, z) of the y-z-x cube -> z-x-y
   PassDesc e;
@@ -712,7 +740,8 @@ bool forward_passes(const Plan &pl, const void *in, bool hostIn, float *coef, fl
   e.steps = pl.sy; e.wavelet = pl.p.wavelet; e.exact = pl.p.exact_transform;
   e.T = dwt_tile_rows(e.L, e.exact && e.wavelet == WL_CDF97);
   e.tiles = (e.rows + e.T - 1) / e.T;
-  ys[group_key(false, WL_F32, e.L)].push_back(e);
+  if (filterBank || !put_source_pass(e, WL_F32, false, ys))
+    ys[group_key(false, WL_F32, e.L)].push_back(e);
   if (pl.sz == 0) return false;
   // z pass: rows (y, x) of the z-x-y cube, in place
   PassDesc f = e;
@@ -737,6 +766,7 @@ struct GroupLaunch {
   int regL;  // row-register pass of rows of regL elements (0: another kernel)
   int regKind;  // which row-register kernel (RegKind)
   bool sel;     // in-place row-register pass gathering the select statistics
+  bool full;    // register pass needing the full kernel (dwt_strided_full)
   // bytes a launch moves, for ordering concurrent groups
   double weight() const { return (double)tiles * (regL ? 4.0 * regL * rows : (double)smem); }
 };
@@ -793,7 +823,7 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
   }
   tp[n] = tiles;
   out.push_back({hoff, (int)n, tiles, smem, rows, warps, inType, outType, inverse, cols, vec,
-                 regL, regKind, sel});
+                 regL, regKind, sel, strided_kind(regKind) && dwt_strided_full(g[0], inverse)});
   hoff += (bytes + 255) & ~(size_t)255;
   return WL_OK;
 }
@@ -828,11 +858,11 @@ wl_status launch_one(wl_ctx *ctx, const GroupLaunch &l, cudaStream_t s) {
   const PassDesc *dp = reinterpret_cast<const PassDesc *>(base + l.off);
   const int *dtp = reinterpret_cast<const int *>(base + l.off + l.n * sizeof(PassDesc));
   if (l.regKind == kRegStrided || l.regKind == kRegInvStrided)
-    launch_dwt_strided(dp, dtp, l.n, l.tiles, l.regL, l.regKind == kRegInvStrided, s);
+    launch_dwt_strided(dp, dtp, l.n, l.tiles, l.regL, l.regKind == kRegInvStrided, l.full, s);
   else if (l.regKind == kRegStridedX)
-    launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.inType, false, s);
+    launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.inType, false, l.full, s);
   else if (l.regKind == kRegInvStridedX)
-    launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.outType, true, s);
+    launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.outType, true, l.full, s);
   else if (l.regKind == kRegTile)
     launch_dwt_rowreg_t(dp, dtp, l.n, l.tiles, l.regL, l.inType, s);
   else if (l.regKind == kRegInvInPlace)
@@ -1676,17 +1706,37 @@ void inverse_passes(const int size[3], const int steps[3], int wavelet, const in
     b.L = Yp; b.B = Xp; b.rows = Xp * Zp; b.steps = sy2;
     b.T = dwt_tile_rows(b.L, false); b.tiles = (b.rows + b.T - 1) / b.T;
     put(2, cols, b);
-  } else if (use_cols(Xp, Yp, Zp, identity, wp)) {
-    PassDesc d[3];
-    const int np = inverse_passes_cols(Xp, Yp, Zp, original_size, steps, wavelet, c1, c2, dst, d);
+    return;
+  }
+  // the register kernels take y and x passes of these lengths: true when put.
+  // They undo the deferred scale as the passes' former kernels did (the row
+  // kernel by its reciprocal, the tile kernels by division), so that restored
+  // integers do not change.
+  auto put_registers = [&](int phase, const PassDesc &pass, bool division, bool apply) {
+    PassDesc d = rows_along_b(pass);
+    d.exact = division || !dwt_rowreg_fits(d.L, d.steps) ? 1 : 0;
+    const int type = phase == 2 ? outType : WL_F32;
+    int key = 0;
+    if (phase == 1 && dwt_strided_fits(d)) key = strided_key(true, d);
+    else if (dwt_strided_output_fits(d, dtype_size(type))) key = strided_x_key(true, type, d);
+    if (key && apply) ph[phase][key].push_back(d);
+    return key != 0;
+  };
+  PassDesc d[3];
+  const int np = identity ? 0 : inverse_passes_cols(Xp, Yp, Zp, original_size, steps, wavelet, c1,
+                                                    c2, dst, d);
+  // an image with an axis above the column tiles' limit, both passes in
+  // registers
+  const bool columns = use_cols(Xp, Yp, Zp, identity, wp);
+  const bool longImage = !columns && np == 2 && put_registers(1, d[0], true, false) &&
+                         put_registers(2, d[1], true, false);
+  if (columns || longImage) {
     for (int i = 0; i < np; i++) {
       const int phase = 3 - np + i;
       if (phase == 0 && dwt_rowreg_fits(d[i].L, d[i].steps))  // z rows in registers
         ph[0][rowreg_inv_key(d[i].L)].push_back(d[i]);
-      else if (phase == 1 && dwt_strided_fits(d[i]))  // y rows in registers
-        ph[1][strided_key(true, d[i].L)].push_back(d[i]);
-      else if (phase == 2 && dwt_strided_output_fits(d[i], dtype_size(outType)))
-        ph[2][strided_x_key(true, outType, d[i].L)].push_back(d[i]);
+      else if (phase > 0 && put_registers(phase, d[i], longImage, true))
+        continue;
       else if (phase > 0 && dwt_rowreg_fits(d[i].L, d[i].steps))  // y, x: through a tile
         ph[phase][rowreg_inv_t_key(phase == 2 ? outType : WL_F32, d[i].L)].push_back(d[i]);
       else

@@ -142,7 +142,8 @@ struct PassDesc {
   int tiles;
   int steps;
   int wavelet;    // WL_HAAR / WL_CDF97
-  int exact;      // reference float order (filter bank) instead of lifting
+  int exact;      // reference float order (filter bank) instead of lifting; inverse passes of
+                  // the register kernels: the deferred scale undone by division
   int clampL, clampB, clampA;  // forward load: source sizes (REPEAT padding)
   int cropL, cropB, cropA;     // inverse store: destination sizes (crop)
   int vecLoad;                 // source is page-locked host memory: 16-byte row loads
@@ -329,11 +330,14 @@ void launch_dwt_rowreg_t(const PassDesc *d_passes, const int *d_tilePrefix, int 
 bool dwt_strided_fits(const PassDesc &d);
 bool dwt_strided_source_fits(const PassDesc &d, int es);
 bool dwt_strided_output_fits(const PassDesc &d, int es);
+// full: the kernel with levels across lanes and division (all passes of a
+// launch, or none, need it)
+bool dwt_strided_full(const PassDesc &d, bool inverse);
 void launch_dwt_strided_x(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
-                          int blocks, int L, int dtype, bool inverse, cudaStream_t s);
+                          int blocks, int L, int dtype, bool inverse, bool full, cudaStream_t s);
 int dwt_strided_rows_per_block(int L);
 void launch_dwt_strided(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
-                        int L, bool inverse, cudaStream_t s);
+                        int L, bool inverse, bool full, cudaStream_t s);
 
 // ---- column-tile heights per size class (tune.cpp) ----
 enum TuneKind { kTuneFwdX, kTuneFwdY, kTuneFwdZ, kTuneInvZ, kTuneInvY, kTuneInvX, kTuneKinds };
