@@ -9,13 +9,13 @@
 // The stream is cut into subsequences of 256 bits, one thread each, and a CTA
 // decodes a tile of kTileSubs consecutive ones:
 //  - tile_kernel: every thread decodes speculatively from its first bit to
-//    the end of its subsequence and keeps its first kRec token boundaries.
-//    Huffman codes resynchronise after a few tokens, so a thread's exit (the
-//    first boundary past its end) rarely depends on where it started.  Then,
-//    in rounds inside the CTA, a thread whose start differs from its
-//    predecessor's exit decodes again from there until it meets one of its
-//    recorded boundaries.  Thread 0 decodes the subsequence before the tile
-//    only to find the tile's entry.
+//    the end of its subsequence and keeps the last token boundary in each of
+//    its words.  Huffman codes resynchronise after some tokens, so a thread's
+//    exit (the first boundary past its end) rarely depends on where it
+//    started.  Then, in rounds inside the CTA, a thread whose start differs
+//    from its predecessor's exit decodes again from there until it is on the
+//    speculative path at one of those words.  Thread 0 decodes the
+//    subsequence before the tile only to find the tile's entry.
 //  - check_kernel: a tile whose entry is not the exit of the tile before it
 //    (rare: no resynchronisation within a subsequence) is decoded again from
 //    that exit.  It is launched twice; the second launch changes nothing
@@ -23,8 +23,8 @@
 //    repairs with more launches (codes that never resynchronise, e.g. all of
 //    one length).
 //  - scan_kernel: output offset of every tile.
-//  - write_kernel: decodes each subsequence from its true start and writes
-//    the values.
+//  - write_kernel: decodes each subsequence from its true start, lists the
+//    tile's values in shared memory and writes the output a window at a time.
 // A token costs two shared-memory reads of the stream and one of a 12-bit
 // table that also expands zero-run lengths where they fit; longer codes go on
 // four bits at a time.
@@ -33,8 +33,10 @@
 // thread has only 256 bits and nothing waits on the host between the passes:
 // with 1024 bits a thread, tables in global memory and a host wait after
 // every round, decoding a 2048^2 image (4.7 Mbit) took 830 us of a 1213 us
-// call; the call now takes 394 us.  256^3 volume 900 -> 339 us, mixed batch
-// of 512 (464 Mbit) 7.02 -> 5.86 ms.
+// call.  A wrong start is found out a word at a time: with only the first
+// eight boundaries recorded a warp went through its bits five times over
+// (tile_kernel 62 us, and 520 us for the mixed batch of 512, 464 Mbit);
+// recorded per word it takes 34 and 345 us.
 #include <cstring>
 
 #include "wl_internal.h"
@@ -47,7 +49,6 @@ constexpr int kSubBits = 256, kSubWords = kSubBits / 32;
 constexpr int kTileSubs = kThreads - 1;      // thread 0 warms up on the one before
 constexpr int kTileBits = kTileSubs * kSubBits;
 constexpr int kTileWords = kTileSubs * kSubWords;
-constexpr int kRec = 8;                      // token boundaries kept per speculative decode
 constexpr int kLutBits = 12, kLutSize = 1 << kLutBits;
 constexpr int kStepBits = 4, kStep = 1 << kStepBits;  // longer codes, per step
 constexpr int kMaxCode = 60;                 // longest code accepted
@@ -90,23 +91,27 @@ __device__ __forceinline__ TileAt stage_words(const DecodeCub &c, int tile, uint
   t.tot = (int)min(bits, (long long)2 * kTileBits);
   return t;
 }
-// A stream's tables for one CTA: the 12-bit table and the first step tables
-// in shared memory, the other step tables in global memory.
+// A stream's tables for one CTA: the 12-bit table and the first `nNear` step
+// tables in shared memory, the other step tables in global memory.
 struct Tables {
-  __align__(16) unsigned lut[kLutSize];
-  __align__(16) unsigned steps[kStageSteps * kStep];
+  const unsigned *lut, *near, *steps;
+  int nNear;
 };
-__device__ __forceinline__ void stage_tables(const DecodeCub &c, const DecodeArrays &d, int ci,
-                                             Tables &t) {
+__device__ __forceinline__ void stage_lut(const DecodeCub &c, const DecodeArrays &d,
+                                          unsigned *lut) {
   const uint4 *g = reinterpret_cast<const uint4 *>(d.lut + c.lutOff);
-  uint4 *s = reinterpret_cast<uint4 *>(t.lut);
-  const int n = min(d.stepCount[ci], kStageSteps) * (kStep / 4);
+  uint4 *s = reinterpret_cast<uint4 *>(lut);
 #pragma unroll
   for (int i = 0; i < kLutSize / 4 / kThreads; i++)
     s[threadIdx.x + i * kThreads] = g[threadIdx.x + i * kThreads];
-  g = reinterpret_cast<const uint4 *>(d.steps + (size_t)c.stepOff * kStep);
-  s = reinterpret_cast<uint4 *>(t.steps);
-  for (int i = threadIdx.x; i < n; i += kThreads) s[i] = g[i];
+}
+__device__ __forceinline__ Tables stage_steps(const DecodeCub &c, const DecodeArrays &d, int ci,
+                                              const unsigned *lut, unsigned *near, int room) {
+  const Tables t{lut, near, d.steps + (size_t)c.stepOff * kStep, min(d.stepCount[ci], room)};
+  const uint4 *g = reinterpret_cast<const uint4 *>(t.steps);
+  uint4 *s = reinterpret_cast<uint4 *>(near);
+  for (int i = threadIdx.x; i < t.nNear * (kStep / 4); i += kThreads) s[i] = g[i];
+  return t;
 }
 __device__ __forceinline__ unsigned bits_at(const uint32_t *sw, int p) {
   const int k = p >> 5, a = k + (k >> 3);
@@ -114,90 +119,81 @@ __device__ __forceinline__ unsigned bits_at(const uint32_t *sw, int p) {
 }
 
 // a code longer than the table, or a zero-run key whose length bits are
-// outside it; returns the bits consumed, 0 when malformed
-__device__ __noinline__ int slow_token(const uint32_t *sw, const unsigned *near,
-                                       const unsigned *steps, int p, unsigned e, int dupValue,
-                                       int &lg, int &sym) {
-  int used = 0, width = kLutBits;
+// outside it: the token in the table's format, 0 when malformed
+__device__ __noinline__ unsigned slow_token(const uint32_t *sw, const unsigned *near,
+                                            const unsigned *steps, int nNear, int p, unsigned e,
+                                            int dupValue) {
+  unsigned used = 0, width = kLutBits;
   while (e & kSlow) {
     if (e & kRun) {
       if (e & kBad) return 0;
-      used += (int)(e & 63u);
-      lg = (int)(bits_at(sw, p + used) & 7u) + 3;
-      sym = dupValue;
-      return used + 3;
+      used += e & 63u;
+      const unsigned lg = (bits_at(sw, p + used) & 7u) + 3;
+      return (used + 3) | (lg << 6) | ((unsigned)dupValue << 10);
     }
     used += width;
     width = kStepBits;
-    const unsigned slot = e & 0xffffu;
+    const int slot = (int)(e & 0xffffu);
     const unsigned at = slot * kStep + (bits_at(sw, p + used) & (kStep - 1));
-    e = slot < kStageSteps ? near[at] : steps[at];
+    e = slot < nNear ? near[at] : steps[at];
   }
-  lg = (int)((e >> 6) & 15u);
-  sym = (int)((e >> 10) & 0x1fffu);
-  return used + (int)(e & 63u);
+  return e + used;  // at most 60 bits
 }
 
-// one token at bit p of the staged words: bits consumed (0: malformed)
-__device__ __forceinline__ int token_at(const uint32_t *sw, const Tables &t,
-                                        const unsigned *steps, int p, int dupValue, int &lg,
-                                        int &sym) {
+// the token at bit p of the staged words: bits consumed in bits 0-5 (0:
+// malformed), log2 of its elements in 6-9, its symbol above
+__device__ __forceinline__ unsigned token_at(const uint32_t *sw, const Tables &t, int p,
+                                             int dupValue) {
   const unsigned e = t.lut[bits_at(sw, p) & (kLutSize - 1)];
-  if (e & kSlow) return slow_token(sw, t.steps, steps, p, e, dupValue, lg, sym);
-  lg = (int)((e >> 6) & 15u);
-  sym = (int)((e >> 10) & 0x1fffu);
-  return (int)(e & 63u);
+  return e & kSlow ? slow_token(sw, t.near, t.steps, t.nNear, p, e, dupValue) : e;
+}
+
+// Elements of tokens, and above them how many are values to write (not the
+// zero bin): a subsequence of 256 bits and a token has less than 2^17 and 2^9.
+constexpr int kCountBits = 17, kRecShift = 26;
+__device__ __forceinline__ unsigned token_count(unsigned e, int dupValue) {
+  return (1u << ((e >> 6) & 15u)) + ((int)(e >> 10) != dupValue ? 1u << kCountBits : 0u);
 }
 
 struct TileSmem {
-  Tables tab;
+  __align__(16) unsigned lut[kLutSize];
+  __align__(16) unsigned near[kStageSteps * kStep];
   uint32_t sw[kStageSize];
-  unsigned rec[kRec][kThreads];
+  // last token boundary of the speculative decode in each word: the bit in
+  // bits 26-30, the counts before it below; all ones: none
+  unsigned rec[kSubWords][kThreads];
   int exits[kThreads];
   unsigned sums[kThreads / 32];
 };
 
 // Decode a tile; entry: the tile's true first token boundary (bits past the
 // tile's first bit), or -1 to find it speculatively.  Writes the start and
-// element count of every subsequence and the tile's entry, exit and total.
+// counts of every subsequence and the tile's entry, exit and total.
 __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, TileSmem &sm,
                             int entry) {
   constexpr unsigned kAll = 0xffffffffu;
   const int tile = t - c.tileBase, tid = threadIdx.x;
+  const int dupValue = c.dupValue;
   const TileAt at = stage_words(c, tile, sm.sw);
-  stage_tables(c, d, d.tileCub[t], sm.tab);
+  stage_lut(c, d, sm.lut);
+  const Tables tab = stage_steps(c, d, d.tileCub[t], sm.lut, sm.near, kStageSteps);
   __syncthreads();
-  const unsigned *steps = d.steps + (size_t)c.stepOff * kStep;
   const long long sub = (long long)tile * kTileSubs + tid - 1;  // subsequence of the stream
   const bool active = sub >= 0 && sub < c.nSub;
-  const int s0 = tid * kSubBits, lim = min(s0 + kSubBits, at.tot);
+  const int s0 = tid * kSubBits, lim = active ? min(s0 + kSubBits, at.tot) : s0;
+  bool bad = false;
   int p = s0;
   unsigned n = 0;
-  bool bad = false;
-  // speculative decode, the first boundaries recorded (unused: all ones)
 #pragma unroll
-  for (int k = 0; k < kRec; k++) {
-    unsigned r = ~0u;
-    if (active && !bad && p < lim) {
-      int lg, sym;
-      const int used = token_at(sm.sw, sm.tab, steps, p, c.dupValue, lg, sym);
-      bad = used == 0;
-      if (!bad) {
-        p += used;
-        n += 1u << lg;
-        r = (unsigned)(p - s0) | (n << 16);
-      }
-    }
-    sm.rec[k][tid] = r;
+  for (int j = 0; j < kSubWords; j++) sm.rec[j][tid] = ~0u;
+  while (p < lim) {
+    sm.rec[(p - s0) >> 5][tid] = ((unsigned)(p & 31) << kRecShift) | n;
+    const unsigned e = token_at(sm.sw, tab, p, dupValue);
+    if ((e & 63u) == 0) { bad = true; break; }
+    p += (int)(e & 63u);
+    n += token_count(e, dupValue);
   }
-  while (active && !bad && p < lim) {
-    int lg, sym;
-    const int used = token_at(sm.sw, sm.tab, steps, p, c.dupValue, lg, sym);
-    if (used == 0) { bad = true; break; }
-    p += used;
-    n += 1u << lg;
-  }
-  const int x0 = p;           // the speculative exit and element count
+  const int x0 = p;           // the speculative exit and counts
   const unsigned n0 = n;
   int start = s0;
   // the first tile starts with the stream
@@ -210,29 +206,21 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
     __syncthreads();
     const int ns = tid > 0 ? sm.exits[tid - 1] : start;
     bool changed = false;
-    if (active && tid > 0 && ns != start) {
+    if (active && tid > 0 && ns != start && !bad) {
       start = ns;
-      int q = ns, k = -1, bk = s0;  // boundary k of the speculative decode (-1: s0)
-      unsigned m = 0, ck = 0;
-      for (;;) {
-        while (bk < q && k + 1 < kRec) {
-          const unsigned r = sm.rec[k + 1][tid];
-          if (r == ~0u) break;
-          k++;
-          bk = s0 + (int)(r & 0xffffu);
-          ck = r >> 16;
-        }
-        if (bk == q) {  // on the speculative path from here
-          m += n0 - ck;
+      int q = ns;
+      unsigned m = 0;
+      while (q < lim) {
+        const unsigned r = sm.rec[(q - s0) >> 5][tid];
+        if (r >> kRecShift == (unsigned)(q & 31)) {  // on the speculative path from here
+          m += n0 - (r & ((1u << kRecShift) - 1));
           q = x0;
           break;
         }
-        if (bad || q >= lim) break;
-        int lg, sym;
-        const int used = token_at(sm.sw, sm.tab, steps, q, c.dupValue, lg, sym);
-        if (used == 0) { bad = true; break; }
-        q += used;
-        m += 1u << lg;
+        const unsigned e = token_at(sm.sw, tab, q, dupValue);
+        if ((e & 63u) == 0) { bad = true; break; }
+        q += (int)(e & 63u);
+        m += token_count(e, dupValue);
       }
       changed = q != p;
       p = q;
@@ -245,7 +233,7 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
     d.subStart[c.subBase + sub] = (uint8_t)(start - s0);
     d.subCount[c.subBase + sub] = n;
   }
-  unsigned sum = out ? n : 0u;
+  unsigned sum = out ? n & ((1u << kCountBits) - 1) : 0u;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
   if ((tid & 31) == 0) sm.sums[tid >> 5] = sum;
@@ -321,20 +309,40 @@ __global__ void __launch_bounds__(kThreads) scan_kernel(const DecodeCub *__restr
   if (threadIdx.x == 0 && carry < c.n) atomicAdd(&d.flags[kDecodeShort], 1);
 }
 
+// Shared memory of write_kernel: with kPool words four CTAs fit on an SM.  The
+// pool holds the list of the tile's values and, before them, the step tables
+// that fit (kMinNear at least, else the values are written one by one).
+constexpr int kPool = 7600, kMinNear = 16, kWindow = 6400;
+constexpr int kPosBits = 19;  // elements of a listed tile, a bin above them
 struct WriteSmem {
-  Tables tab;
-  uint32_t sw[kStageSize];
-  unsigned sums[kThreads / 32];
-  float dq[1];  // binCount entries
+  union {
+    struct {
+      __align__(16) unsigned lut[kLutSize];
+      uint32_t sw[kStageSize];
+    };
+    float4 window[kWindow / 4];  // once the tile is decoded
+  };
+  __align__(16) unsigned pool[kPool];
+  uint2 sums[kThreads / 32];
 };
 
-// The values, from each subsequence's true start.  With zero runs
-// (dupValue >= 0) only the other values are written one by one; the zero
-// bin's value is set before: by this CTA over its tile's output range
-// (DecodeCub::fill), so that the scattered values land in lines still in L2,
-// or, where a tile covers so much output that one CTA would be long at it, by
-// launch_fill_batch.  Filling everything first cost the mixed batch (1.5 GB
-// of output) 252 us and 48 us more in this kernel.
+// The values, from each subsequence's true start.
+//
+// With zero runs (dupValue >= 0) a tile's output is mostly the zero bin's
+// value.  All threads decode their subsequences at once into a list of the
+// tile's values, then the output goes by in windows: a window of the zero
+// bin's value in shared memory, the list's next values into it, and out with
+// 16-byte stores, every output line written once.  Writing the values one by
+// one over a filled output cost the mixed batch 0.90 ms (the lines of all
+// resident tiles, some 200 MB, do not stay in L2 between fill and value; every
+// value is a partial sector); this way 0.55 ms
+// (volume 256^3: 52 -> 51 us, one tile per SM).  Step tables beyond the pool
+// are read from memory: with 64 of them the volume's 1024 bins took 57 us.
+//
+// Tiles with more values than the pool holds are filled and written one by
+// one; so are sparse cubelets, whose tiles cover so much output that one CTA
+// would be long at it (filled beforehand by launch_fill_batch,
+// DecodeCub::fill 0), and streams without zero runs, which have no fill.
 __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__restrict__ cubs,
                                                          DecodeArrays d) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -344,51 +352,119 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__rest
   const DecodeCub c = cubs[d.tileCub[t]];
   const long long tileOff = d.tileOff[t];
   if (tileOff >= c.n) return;  // padding bits after the last value
-  const int tile = t - c.tileBase;
+  const int tile = t - c.tileBase, dupValue = c.dupValue, bins = c.binCount;
   const TileAt at = stage_words(c, tile, sm.sw);
-  stage_tables(c, d, d.tileCub[t], sm.tab);
-  for (int i = tid; i < c.binCount; i += kThreads) sm.dq[i] = c.dq[i];
+  stage_lut(c, d, sm.lut);
   const long long sub = (long long)tile * kTileSubs + tid - 1;
   const bool active = tid > 0 && sub < c.nSub;
-  const unsigned n = active ? d.subCount[c.subBase + sub] : 0u;
+  const unsigned cnt = active ? d.subCount[c.subBase + sub] : 0u;
   int p = tid * kSubBits + (active ? (int)d.subStart[c.subBase + sub] : 0);
-  unsigned inc = n;
+  // elements and values before the subsequence
+  const unsigned n = cnt & ((1u << kCountBits) - 1), nv = cnt >> kCountBits;
+  uint2 inc = make_uint2(n, nv);
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const unsigned x = __shfl_up_sync(kAll, inc, o);
-    if (lane >= o) inc += x;
+    const unsigned x = __shfl_up_sync(kAll, inc.x, o), y = __shfl_up_sync(kAll, inc.y, o);
+    if (lane >= o) {
+      inc.x += x;
+      inc.y += y;
+    }
   }
   if (lane == 31) sm.sums[w] = inc;
   __syncthreads();
-  unsigned before = inc - n;
+  unsigned o = inc.x - n, v = inc.y - nv, values = 0;
 #pragma unroll
-  for (int k = 0; k < kThreads / 32; k++) before += k < w ? sm.sums[k] : 0u;
+  for (int k = 0; k < kThreads / 32; k++) {
+    const uint2 x = sm.sums[k];
+    if (k < w) {
+      o += x.x;
+      v += x.y;
+    }
+    values += x.y;
+  }
+  const unsigned vEnd = v + nv;
   const long long room = c.n - tileOff;  // elements from the tile's first on
   const unsigned end = (unsigned)min(room, (long long)0xffffffffu);
-  if (c.fill) {
-    const float v = sm.dq[min(c.dupValue, c.binCount - 1)];
-    float *g = c.out + tileOff;
-    const int total = (int)min(end, d.tileCount[t]);
-    const int head = min((int)((16 - (reinterpret_cast<size_t>(g) & 15)) & 15) / 4, total);
-    const int quads = (total - head) / 4, tail = head + 4 * quads;
-    if (tid < head) g[tid] = v;
-    float4 *g4 = reinterpret_cast<float4 *>(g + head);
-    for (int i = tid; i < quads; i += kThreads) g4[i] = make_float4(v, v, v, v);
-    if (tid < total - tail) g[tail + tid] = v;
-    __syncthreads();  // the values below come after
-  }
-  if (!active) return;
-  const int lim = min(tid * kSubBits + kSubBits, at.tot);
-  const unsigned *steps = d.steps + (size_t)c.stepOff * kStep;
+  const int lim = active ? min(tid * kSubBits + kSubBits, at.tot) : p;
   float *F = c.out + tileOff;
-  unsigned o = before;
+  const unsigned tileEnd = (unsigned)min((long long)end, (long long)d.tileCount[t]);
+  const bool listed = c.fill && tileEnd < (1u << kPosBits) &&
+                      values <= kPool - kMinNear * kStep;
+  // the pool: step tables, then the list (element from the tile's first on,
+  // ascending, and bin)
+  const int listAt = listed ? (int)(kPool - values) : kPool;
+  unsigned *list = sm.pool + listAt;
+  const Tables tab = stage_steps(c, d, d.tileCub[t], sm.lut, sm.pool, listAt / kStep);
+  const float zero = dupValue >= 0 ? c.dq[min(dupValue, bins - 1)] : 0.f;
+  if (c.fill && !listed) {
+    const int total = (int)tileEnd;
+    const int head = min((int)((16 - (reinterpret_cast<size_t>(F) & 15)) & 15) / 4, total);
+    const int quads = (total - head) / 4, tail = head + 4 * quads;
+    if (tid < head) F[tid] = zero;
+    float4 *g4 = reinterpret_cast<float4 *>(F + head);
+    for (int i = tid; i < quads; i += kThreads) g4[i] = make_float4(zero, zero, zero, zero);
+    if (tid < total - tail) F[tail + tid] = zero;
+  }
+  __syncthreads();  // the tables are there, and the fill comes before the values
   while (p < lim && o < end) {
-    int lg, sym;
-    const int used = token_at(sm.sw, sm.tab, steps, p, c.dupValue, lg, sym);
-    if (used == 0) break;
-    p += used;
-    if (sym != c.dupValue) F[o] = sm.dq[min(sym, c.binCount - 1)];
-    o += 1u << lg;
+    const unsigned e = token_at(sm.sw, tab, p, dupValue);
+    if ((e & 63u) == 0) break;
+    p += (int)(e & 63u);
+    const int sym = (int)(e >> 10);
+    if (sym != dupValue) {
+      if (listed) {
+        list[v++] = o | ((unsigned)min(sym, bins - 1) << kPosBits);
+      } else {
+        F[o] = __ldg(c.dq + min(sym, bins - 1));
+      }
+    }
+    o += 1u << ((e >> 6) & 15u);
+  }
+  if (!listed) return;
+  // values counted in the padding bits past the cubelet's end
+  for (; v < vEnd; v++) list[v] = ~0u;
+
+  // ---- the tile's output, window by window: windows start at multiples of
+  // 16 bytes, the first up to three floats before the tile
+  if (tileEnd == 0) return;
+  const unsigned shift = (unsigned)((reinterpret_cast<size_t>(F) & 15) / 4);
+  const unsigned span = tileEnd + shift;
+  float4 *G = reinterpret_cast<float4 *>(F - shift);
+  float *win = reinterpret_cast<float *>(sm.window);
+  const float4 zero4 = make_float4(zero, zero, zero, zero);
+  __syncthreads();  // the list is complete, the tables are done with
+  const float *dq = c.dq;
+  if (bins <= listAt) {  // in the place of the step tables
+    float *near = reinterpret_cast<float *>(sm.pool);
+    for (int i = tid; i < bins; i += kThreads) near[i] = c.dq[i];
+    dq = near;
+  }
+  for (int i = tid; i < kWindow / 4; i += kThreads) sm.window[i] = zero4;
+  __syncthreads();
+  unsigned i = tid;  // the thread's next value of the list
+  for (unsigned w0 = 0; w0 < span; w0 += kWindow) {
+    const unsigned w1 = min(w0 + kWindow, span);
+    for (; i < values; i += kThreads) {
+      const unsigned x = list[i], at = (x & ((1u << kPosBits) - 1)) + shift;
+      if (at >= w1) break;
+      win[at - w0] = dq[x >> kPosBits];
+    }
+    __syncthreads();
+    for (unsigned k = tid; k < kWindow / 4; k += kThreads) {
+      const unsigned q = w0 + 4 * k;
+      if (q >= span) break;
+      const float4 x = sm.window[k];
+      if (q >= shift && q + 4 <= span) {
+        G[q / 4] = x;
+      } else {
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (q + j >= shift && q + j < span) F[q + j - shift] = xs[j];
+      }
+      sm.window[k] = zero4;
+    }
+    __syncthreads();
   }
 }
 
@@ -519,7 +595,7 @@ void launch_decode_check(const DecodeCub *cubs, const DecodeBatch &b, const Deco
 int launch_decode_write(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,
                         cudaStream_t s) {
   scan_kernel<<<b.n, kThreads, 0, s>>>(cubs, d);
-  const int smem = (int)sizeof(WriteSmem) + b.maxBins * 4;
+  const int smem = (int)sizeof(WriteSmem);
   if (smem > 48 * 1024) raise_smem_limit(write_kernel, smem);
   write_kernel<<<b.tiles, kThreads, smem, s>>>(cubs, d);
   return 2;

@@ -2241,7 +2241,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
   int *hmap = reinterpret_cast<int *>(hu + mapAt);
   int *ht = reinterpret_cast<int *>(hu + tabAt);
   float *hq = reinterpret_cast<float *>(hu + dqAt);
-  DecodeBatch db{nStreams, (int)tileTotal, 2, 2};
+  DecodeBatch db{nStreams, (int)tileTotal, 2};
   int nFill = 0, k = 0;
   long long fillBlocks = 0, tableOff = 0, binOff = 0, subOff = 0, tileOff = 0, stepOff = 0;
   for (int i = 0; i < n; i++) {
@@ -2283,7 +2283,6 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
       tileOff += c.nTiles;
       stepOff += c.nSteps;
       db.maxTable = std::max(db.maxTable, r->n_decode);
-      db.maxBins = std::max(db.maxBins, r->bin_count);
       k++;
     }
     tableOff += ((long long)r->n_decode + 3) & ~3LL;

@@ -413,7 +413,7 @@ struct DecodeArrays {
   unsigned *lut, *steps;
   int *stepCount;         // step tables of every stream
   uint8_t *subStart;      // first token boundary of every subsequence
-  unsigned *subCount;     // elements of every subsequence
+  unsigned *subCount;     // elements and values of every subsequence
   const int *tileCub;     // cubelet of every tile
   int *tileEntry, *tileExit;
   unsigned *tileCount;
@@ -428,7 +428,7 @@ enum {
 };
 struct DecodeBatch {
   int n, tiles;           // streams, tiles in all
-  int maxTable, maxBins;
+  int maxTable;
 };
 long long decode_subs(long long nWords);
 int decode_tiles(long long nWords);
