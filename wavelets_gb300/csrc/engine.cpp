@@ -1344,11 +1344,15 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   // computes the log quantizer tables); each may run as a CUDA graph ----
   ctx->launches = 0;
   // everything after the select for half h on stream st
-  auto post = [&](int h, cudaStream_t st) -> wl_status {
+  auto post = [&](int h, cudaStream_t st, const Upload &up) -> wl_status {
     DevBatch &v = bh[h];
     const bool first = h == 0;
-    launch_quant_params(v, st);
+    launch_quant_params(v, up, st);
     ctx->launches += 1;
+    if (up.src && nh == 2) {  // the second half starts once the tables are on the device
+      CU(cudaEventRecord(ctx->halfT, s));
+      CU(cudaStreamWaitEvent(s2, ctx->halfT, 0));
+    }
     if (anyLloyd) { launch_lloyd(v, v.coef, maxLloyd, st); ctx->launches += 3; }
     if (first) mark(ctx, 5);
     launch_quantize(v, v.coef, maxTable, maxS, anyLloyd, st);
@@ -1387,27 +1391,21 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     return WL_OK;
   };
   auto quantize_to_end = [&]() -> wl_status {
-    if (anyLog) {
-      CU(cudaMemcpyAsync(ctx->qtable.p, ctx->hTab.p, hdrBytes + (size_t)tableTotal * 4,
-                         cudaMemcpyHostToDevice, s));
-      if (nh == 2) {  // the second half starts once the tables are on the device
-        CU(cudaEventRecord(ctx->halfT, s));
-        CU(cudaStreamWaitEvent(s2, ctx->halfT, 0));
-      }
-    }
-    TRY(post(0, s));
-    if (nh == 2) TRY(post(1, s2));
+    TRY(post(0, s, anyLog ? Upload{H<uint4>(ctx->hTab), P<uint4>(ctx->qtable),
+                                   (int)((hdrBytes + (size_t)tableTotal * 4) / 16)}
+                          : Upload{}));
+    if (nh == 2) TRY(post(1, s2, Upload{}));
     TRY(join());
     return states_back();
   };
   auto transform_select = [&]() -> wl_status {
-    CU(cudaMemcpyAsync(ctx->passes.p, ctx->hPasses.p, upBytes, cudaMemcpyHostToDevice, s));
-    if (nh == 2) {  // the second half starts with the first
+    launch_init(bh[0], anyLloyd,
+                Upload{H<uint4>(ctx->hPasses), P<uint4>(ctx->passes), (int)((upBytes + 15) / 16)}, s);
+    if (nh == 2) {  // the second half starts once the block is on the device
       CU(cudaEventRecord(ctx->halfT, s));
       CU(cudaStreamWaitEvent(s2, ctx->halfT, 0));
-      launch_init(bh[1], anyLloyd, s2);
+      launch_init(bh[1], anyLloyd, Upload{}, s2);
     }
-    launch_init(bh[0], anyLloyd, s);
     ctx->launches += nh;
     mark(ctx, 0);
     TRY(launch_phase(ctx, gl, gb[0][0], gb[0][1]));
@@ -1431,8 +1429,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     CU(cudaGetLastError());
     mark(ctx, 4);
     if (anyLog) return join();  // the select wrote hSel
-    if (nh == 2) TRY(post(1, s2));
-    TRY(post(0, s));
+    if (nh == 2) TRY(post(1, s2, Upload{}));
+    TRY(post(0, s, Upload{}));
     TRY(join());
     return states_back();
   };

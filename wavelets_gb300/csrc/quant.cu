@@ -22,6 +22,8 @@
 // reference's lower_bound with its last-boundary special case.
 #include <cfloat>
 
+#include <algorithm>
+
 #include "wl_internal.h"
 
 namespace wl {
@@ -31,9 +33,12 @@ constexpr int kThreads = kChunkThreads;
 constexpr int INF = 0x7fffffff;
 
 // ---- quantizer parameters ---------------------------------------------------
-__global__ void quant_params_kernel(DevBatch b) {
+// Copies the log quantizers' tables over on its way.
+__global__ void quant_params_kernel(DevBatch b, Upload up) {
   stage_mark(b.head, kMarkQuant);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
+  if (up.src)
+    for (int i = ci; i < up.vecs; i += gridDim.x * blockDim.x) up.dst[i] = up.src[i];
   if (ci >= b.n) return;
   const CubeletDev cd = b.cub[ci];
   CubeletState *st = b.state + ci;
@@ -50,7 +55,7 @@ __global__ void quant_params_kernel(DevBatch b) {
     st->zeroBin = (B - 1) >> 1;
   } else if (cd.quantAlg == WL_LOG) {
     st->zeroBin = (B - 1) >> 1;
-    const int4 h = b.logHdr[ci];  // computed on the host (quant_host.cpp)
+    const int4 h = *up.host(b.logHdr + ci);  // computed on the host (quant_host.cpp)
     st->lowBin = h.x;
     st->highNeg = h.y;
     st->nPos = h.z;
@@ -682,8 +687,9 @@ __global__ void __launch_bounds__(kRunChunks) runs_kernel(DevBatch b) {
 
 }  // namespace
 
-void launch_quant_params(DevBatch &b, cudaStream_t s) {
-  quant_params_kernel<<<(b.n + 127) / 128, 128, 0, s>>>(b);
+void launch_quant_params(DevBatch &b, const Upload &up, cudaStream_t s) {
+  const int copy = up.src ? std::min((up.vecs + 127) / 128, 1024) : 0;
+  quant_params_kernel<<<std::max((b.n + 127) / 128, copy), 128, 0, s>>>(b, up);
 }
 
 void launch_lloyd(DevBatch &b, const float *coef, int maxBins, cudaStream_t s) {

@@ -290,17 +290,20 @@ __global__ void __launch_bounds__(1024) select_resolve(DevBatch b, bool mark) {
   for (int i = threadIdx.x; i < kSelectBins; i += 1024) g[i] = 0;
 }
 
-// One launch sets up everything a call's kernels expect: kInitSlices CTAs per
+// One launch sets up everything a call's kernels expect: the CTAs copy the
+// upload block over from the host, and kInitSlices of them per
 // cubelet (blockIdx.y) zero its histograms and state and write the cubelet
 // index of its chunks, select groups, quantize and bit-packer CTAs, so that
 // those kernels start with one load.  (Three memsets, an initialisation and a map
 // kernel before took 20 us at the head of every call, most of it gaps.)
 constexpr int kInitSlices = 8;
-__global__ void __launch_bounds__(kThreads) init_kernel(DevBatch b, bool lloyd) {
+__global__ void __launch_bounds__(kThreads) init_kernel(DevBatch b, bool lloyd, Upload up) {
   stage_mark(b.head, kMarkStart);
   const int ci = blockIdx.y, slice = blockIdx.x;
-  const CubeletDev cd = b.cub[ci];
   const int t0 = slice * kThreads + threadIdx.x, step = kInitSlices * kThreads;
+  if (up.src)
+    for (int i = ci * step + t0; i < up.vecs; i += b.n * step) up.dst[i] = up.src[i];
+  const CubeletDev cd = *up.host(b.cub + ci);
   unsigned *sel = b.selHist + (size_t)ci * kSelectBins;
   for (int i = t0; i < kSelectBins; i += step) sel[i] = 0;
   unsigned long long *h = b.hist + (size_t)ci * kMaxSymbols;
@@ -330,8 +333,8 @@ __global__ void __launch_bounds__(kThreads) init_kernel(DevBatch b, bool lloyd) 
 
 }  // namespace
 
-void launch_init(DevBatch &b, bool lloyd, cudaStream_t s) {
-  init_kernel<<<dim3(kInitSlices, b.n), kThreads, 0, s>>>(b, lloyd);
+void launch_init(DevBatch &b, bool lloyd, const Upload &up, cudaStream_t s) {
+  init_kernel<<<dim3(kInitSlices, b.n), kThreads, 0, s>>>(b, lloyd, up);
 }
 
 void launch_select(DevBatch &b, const float *coef, bool pass0, cudaStream_t s) {

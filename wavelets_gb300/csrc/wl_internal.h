@@ -359,13 +359,30 @@ unsigned tune_version();  // changes whenever the table does
 // everything a call's kernels expect set: histograms and states zeroed, the
 // select state (extremes from FLT_MAX / FLT_MIN), cubelet of every chunk;
 // runs before the transform, whose last pass may gather the first digit
-void launch_init(DevBatch &b, bool lloyd, cudaStream_t s);
+// A block of page-locked host memory that a kernel copies to the device on its
+// way.  A copy node in front of a graph's kernels is handed to the copy engine
+// apart from them; with a
+// copy node each graph of a 64^3 call and of a 2048^2 image took some 3 us more
+// (calls: 160 -> 155 us, 250 -> 244 us, mixed batch of 40: 797 -> 761 us).
+struct Upload {
+  const uint4 *src;  // null: already there
+  uint4 *dst;
+  int vecs;          // of 16 bytes
+  // the host's copy of something at a device address inside the block
+  template <typename T> __device__ const T *host(const T *p) const {
+    return src ? reinterpret_cast<const T *>(
+                     reinterpret_cast<const char *>(src) +
+                     (reinterpret_cast<const char *>(p) - reinterpret_cast<const char *>(dst)))
+               : p;
+  }
+};
+void launch_init(DevBatch &b, bool lloyd, const Upload &up, cudaStream_t s);
 // pass0: run the stand-alone first digit pass for the cubelets whose last
 // transform pass did not gather it (CubeletDev::selFused == 0)
 void launch_select(DevBatch &b, const float *coef, bool pass0, cudaStream_t s);
 
 // launchers (quant.cu)
-void launch_quant_params(DevBatch &b, cudaStream_t s);
+void launch_quant_params(DevBatch &b, const Upload &up, cudaStream_t s);
 void launch_lloyd(DevBatch &b, const float *coef, int maxBins, cudaStream_t s);
 // sum of squared differences of two u8 arrays into *out (opt.cu)
 void launch_sq_err_u8(const uint8_t *a, const uint8_t *b, long long n, unsigned long long *out,
