@@ -16,6 +16,14 @@ LEVELS = {16: 4, 32: 5, 48: 4, 64: 6, 96: 4, 128: 7, 192: 4, 256: 8, 512: 9, 102
 CASES = [(L, s) for L, most in LEVELS.items() for s in sorted({1, 2, 4, 5, most - 1, most, most + 1})
          if L % (1 << s) == 0 and s <= (L - 1).bit_length()]
 
+# lengths whose lanes a row are not a power of two: 8, 16 and 32 elements a
+# lane at most 16 times, and just beyond
+LEVELS_ANY = {8: 3, 24: 3, 40: 3, 80: 4, 112: 4, 120: 3, 136: 3, 144: 4, 160: 5, 208: 4, 224: 5,
+              240: 4, 272: 4, 480: 5, 544: 5}
+ANY = [(L, s) for L, most in LEVELS_ANY.items() for s in sorted({1, 2, most, most + 1})
+       if L % (1 << s) == 0 and s <= (L - 1).bit_length()]
+CASES += ANY
+
 
 @pytest.fixture(scope="module")
 def ctx():
@@ -98,3 +106,27 @@ def test_images(ctx, Y, X, steps, dtype):
         back = ctx.inverse_transform(one, (1, Xp, Yp), st, wavelet, (X, Y, 1), dtype)
         back3 = ctx.inverse_transform(all3, (3, Xp, Yp), st, wavelet, (X, Y, 3), dtype)
         assert np.array_equal(back[0], back3[1])
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.int32, np.float32])
+def test_rows_at_any_address(ctx, dtype):
+    """Cubelets in device memory that start off the lane vectors and have rows
+    of odd length, several lengths in one launch: as alone from the host, where
+    they start at an aligned address."""
+    import torch
+    rng = np.random.default_rng(5)
+    p = P.Params(steps=(3, 2, 1), threshold_fraction=0.7, bin_count=64)
+    es = np.dtype(dtype).itemsize
+    vols, items, keep = [], [], []
+    for k, x in enumerate((77, 80, 113, 120, 161, 131, 131, 255)):
+        v = rng.integers(0, 200, (16, 20, x)).astype(dtype)
+        buf = torch.zeros(v.nbytes + 16 * es, dtype=torch.uint8, device="cuda")
+        buf[k * es:k * es + v.nbytes] = torch.from_numpy(v.reshape(-1).view(np.uint8)).cuda()
+        vols.append(v)
+        keep.append(buf)
+        items.append((buf.data_ptr() + k * es, lib.NP_TO_WL[np.dtype(dtype)], (x, 20, 16), p))
+    torch.cuda.synchronize()
+    for v, c in zip(vols, ctx.compress_batch(items, on_device=True, raw=True)):
+        want = ctx.compress(v, p)
+        assert np.array_equal(c.words, want.words)
+        assert (c.threshold_value, c.max_value) == (want.threshold_value, want.max_value)

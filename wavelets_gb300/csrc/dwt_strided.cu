@@ -18,6 +18,10 @@ WL_STRIDED_DECLARE(strided_x_inv_u16)
 WL_STRIDED_DECLARE(strided_x_inv_i32)
 WL_STRIDED_DECLARE(strided_x_inv_f32)
 
+bool dwt_strided_own(int L) {
+  return (L >= 16 && (L & (L - 1)) == 0) || L == 48 || L == 96 || L == 192;
+}
+
 namespace {
 
 constexpr int kWarps = 4;  // per block (dwt_strided.cuh kThreads)
@@ -31,11 +35,15 @@ int strided_lanes(int L) {
     case 256: return 8;
     case 512: return 16;
     case 1024: case 2048: return 32;
-    default: return 0;
+    default: return strided_elems(L) ? L / strided_elems(L) : 0;
   }
 }
 int strided_levels(int L) {
-  if (L % 48 == 0) return 4;  // 48 elements a lane halve four times
+  if (!dwt_strided_own(L) || L % 48 == 0) {  // as often as a lane's elements halve
+    int n = 0;
+    for (int k = dwt_strided_own(L) ? 48 : strided_elems(L); k % 2 == 0; k /= 2) n++;
+    return n;
+  }
   int n = 0;
   while ((2 << n) <= L) n++;
   return n;
@@ -46,7 +54,7 @@ bool shape_fits(const PassDesc &d) {
   return strided_lanes(d.L) && d.steps >= 1 && d.B % 2 == 0 && d.steps <= strided_levels(d.L);
 }
 // rows at base with these strides (elements of es bytes) start at multiples
-// of 16 bytes (K elements are a multiple of 16 bytes for every type)
+// of 16 bytes, so that every lane's K elements start at their vectors' size
 bool rows_aligned(const void *base, long long sa, long long sb, int es) {
   return reinterpret_cast<size_t>(base) % 16 == 0 && sa * es % 16 == 0 && sb * es % 16 == 0;
 }
@@ -63,7 +71,7 @@ bool dwt_strided_fits(const PassDesc &d) {
 }
 bool dwt_strided_source_fits(const PassDesc &d, int es) {
   return shape_fits(d) && d.inSC == 1 && d.outSB == 1 && ((d.outSA | d.outSC) & 1) == 0 &&
-         rows_aligned(d.in, d.inSA, d.inSB, es);
+         (!dwt_strided_own(d.L) || rows_aligned(d.in, d.inSA, d.inSB, es));
 }
 bool dwt_strided_output_fits(const PassDesc &d, int es) {
   return shape_fits(d) && d.outSC == 1 && d.inSB == 1 && ((d.inSA | d.inSC) & 1) == 0 &&

@@ -16,18 +16,27 @@
 //
 // K = 32 for L = 32 .. 1024, 64 for 2048, 16 for 16 (every level: after one
 // value is left per lane a level gathers pair j into lane j), 48 for L = 48,
-// 96, 192 (four levels); other lengths, deeper ones of the latter and an odd
-// number of neighbouring rows stay with the tile kernels.  Levels below one
-// value per lane and scales undone by division (FULL) are instantiations of
-// their own: in one kernel they cost the shallow passes registers and
-// branches (restoring the mixed batch 4.36 ms a call instead of 4.19).
-// A 2048^2 image's passes take 17 us each forward, 21 us inverse (42 and 60
-// to 70 us in the row-cooperative kernel).
+// 96, 192 (four levels).  Other lengths of K = 32, 16 or 8 times at most 16
+// (five, four or three levels; strided_elems) take their number of lanes from
+// the pass (G = 0; the lanes of a warp that do not make a row are idle), so
+// one launch holds rows of all such lengths; their source rows start at any
+// address.  The x passes of 400 cubelets of odd sizes take 0.40 ms, their y
+// passes 0.33 (0.55 and 0.37 in the column-tile kernel), restoring as many
+// 3.4 ms a call (3.74); the x pass of a 93 x 181 x 147 16-bit volume 13 us
+// (25).  Longer lengths, deeper levels and an odd number of neighbouring rows
+// stay with the tile kernels.
 //
-// With 64 to 96 values per thread in flight a large pass is bound by HBM: the y passes of 729 cubelets of
-// 128^3 (1.5 G elements) take 1.56 ms, 7.8 TB/s of their eight bytes an
-// element (2.77 ms in the column-tile kernel), the inverse y passes of the
-// mixed batch 0.55 ms (1.22 ms through the row kernel's tile).
+// Levels below one value per lane and scales undone by division (FULL) are
+// instantiations of their own: in one kernel they cost the shallow passes
+// registers and branches (restoring the mixed batch 4.36 ms a call instead of
+// 4.19).  A 2048^2 image's passes take 17 us each forward, 21 us inverse (42
+// and 60 to 70 us in the row-cooperative kernel).
+//
+// With 64 to 96 values per thread in flight a large pass is bound by HBM: the
+// y passes of 729 cubelets of 128^3 (1.5 G elements) take 1.56 ms, 7.8 TB/s
+// of their eight bytes an element (2.77 ms in the column-tile kernel), the
+// inverse y passes of the mixed batch 0.55 ms (1.22 ms through the row
+// kernel's tile).
 //
 // The x passes read or write a lane's K elements of a source or output row
 // with vectors of 32 bytes (16 where its address or K asks for it), a run cut
@@ -86,20 +95,21 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
   return r;
 }
 
-// lane position along the row: lane `seg` of G, C lanes between neighbours;
-// lanes [0, na) hold the level's pairs
+// lane position along the row: lane `seg` of `lanes` (G, or the pass's own
+// number where G is 0), `c` lanes between neighbours; lanes [0, na) hold the
+// level's pairs
 template <int G> struct Along {
-  static constexpr int C = 32 / G;
-  int seg, na = G;
+  static constexpr int C = G ? 32 / G : 0;
+  int seg, lanes, c, na;
   // the value of the next / previous lane of the row, `own` at its end
   __device__ __forceinline__ f2 next(f2 v, f2 own) const {
     if (G == 1) return own;
-    const f2 o = __shfl_down_sync(kAll, v, C);
+    const f2 o = __shfl_down_sync(kAll, v, c);
     return seg == na - 1 ? own : o;
   }
   __device__ __forceinline__ f2 prev(f2 v, f2 own) const {
     if (G == 1) return own;
-    const f2 o = __shfl_up_sync(kAll, v, C);
+    const f2 o = __shfl_up_sync(kAll, v, c);
     return seg == 0 ? own : o;
   }
   // the value of lane s of the row
@@ -184,7 +194,7 @@ struct Row {
 template <int LEV, int M, int G, bool HAAR, bool FULL>
 __device__ __forceinline__ void fwd_from(const f2 (&v)[2 * M], int S, const float *scale,
                                          const Along<G> &at, const Row &out) {
-  constexpr int H = M * G;  // pairs of this level
+  const int H = M * at.lanes;  // pairs of this level
   f2 e[M], o[M];
 #pragma unroll
   for (int k = 0; k < M; k++) {
@@ -248,7 +258,7 @@ template <bool FULL> struct Unscale {
 template <int LEV, int M, int G, bool HAAR, bool FULL>
 __device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL> &un,
                                        const Along<G> &at, const Row &in) {
-  constexpr int H = M * G;
+  const int H = M * at.lanes;
   f2 e[M], o[M];
 #pragma unroll
   for (int k = 0; k < M; k++) o[k] = in.get(H + M * at.seg + k);
@@ -303,7 +313,7 @@ __device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL
 // ---- rows of the source and of the output (x passes) ----
 // bytes per vector access of a lane's K elements
 template <typename T, int K> __host__ __device__ constexpr int vec_bytes() {
-  return (K * (int)sizeof(T)) % 32 == 0 ? 32 : 16;
+  return (K * (int)sizeof(T)) % 32 == 0 ? 32 : (K * (int)sizeof(T)) % 16 == 0 ? 16 : 8;
 }
 template <int VB> __device__ __forceinline__ void load_vec(const void *p, unsigned *w) {
   if constexpr (VB == 32) {
@@ -311,6 +321,9 @@ template <int VB> __device__ __forceinline__ void load_vec(const void *p, unsign
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]),
                    "=r"(w[6]), "=r"(w[7])
                  : "l"(p));
+  } else if constexpr (VB == 8) {
+    const uint2 q = *static_cast<const uint2 *>(p);
+    w[0] = q.x; w[1] = q.y;
   } else {
     const uint4 q = *static_cast<const uint4 *>(p);
     w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
@@ -322,6 +335,8 @@ template <int VB> __device__ __forceinline__ void store_vec(void *p, const unsig
                  :: "l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
                     "r"(w[6]), "r"(w[7])
                  : "memory");
+  } else if constexpr (VB == 8) {
+    *static_cast<uint2 *>(p) = make_uint2(w[0], w[1]);
   } else {
     *static_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
   }
@@ -368,15 +383,40 @@ __device__ __forceinline__ void store_vecs(T *p, const float (&v)[K]) {
   }
 }
 
-// K elements [first, first + K) of a row of n real elements (REPEAT clamp)
+// K elements at any address: 16- and 8-bit ones from the aligned words that
+// hold them
 template <typename T, int K>
+__device__ __forceinline__ void load_unaligned(const T *p, float (&v)[K]) {
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = load_as_float(p + k);
+  } else {
+    constexpr int E = 4 / (int)sizeof(T), W = K / E;
+    const size_t at = reinterpret_cast<size_t>(p);
+    const unsigned *w = reinterpret_cast<const unsigned *>(at & ~(size_t)3);
+    const int shift = 8 * (int)(at & 3);
+    unsigned lo = w[0];
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+      const unsigned hi = j + 1 < W || shift ? w[j + 1] : 0u;
+      const unsigned x = __funnelshift_r(lo, hi, shift);
+#pragma unroll
+      for (int k = 0; k < E; k++) v[j * E + k] = from_words<T>(&x, k);
+      lo = hi;
+    }
+  }
+}
+
+// K elements [first, first + K) of a row of n real elements (REPEAT clamp);
+// ANY: whatever the row's address
+template <typename T, int K, bool ANY>
 __device__ __forceinline__ void load_run(const T *row, int first, int n, float (&v)[K]) {
   if (first + K <= n) {
-    constexpr int VB = vec_bytes<T, K>();
-    if (VB == 32 && (reinterpret_cast<size_t>(row + first) & 31) == 0)
-      load_vecs<T, K, VB>(row + first, v);
-    else
-      load_vecs<T, K, 16>(row + first, v);
+    constexpr int VB = vec_bytes<T, K>(), VS = VB < 16 ? VB : 16;
+    const size_t at = reinterpret_cast<size_t>(row + first);
+    if (VB == 32 && (at & 31) == 0) load_vecs<T, K, VB>(row + first, v);
+    else if (ANY && (at & (VS - 1))) load_unaligned<T, K>(row + first, v);
+    else load_vecs<T, K, VS>(row + first, v);
     return;
   }
 #pragma unroll
@@ -389,7 +429,7 @@ __device__ __forceinline__ void store_run(T *row, int first, int n, const float 
     if (VB == 32 && (reinterpret_cast<size_t>(row + first) & 31) == 0)
       store_vecs<T, K, VB>(row + first, v);
     else
-      store_vecs<T, K, 16>(row + first, v);
+      store_vecs<T, K, VB < 16 ? VB : 16>(row + first, v);
     return;
   }
 #pragma unroll
@@ -402,11 +442,11 @@ enum Pass { kStrided, kStridedInv, kSource, kOutput };  // y forward / inverse, 
 template <typename T, int K, int G, bool HAAR, int PASS, bool FULL>
 __device__ __forceinline__ void run_rows(const PassDesc &d, int tile, const float *scale,
                                          const float *rscale) {
-  constexpr int C = 32 / G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const Along<G> at{lane / C};
-  const int row = 2 * ((tile * (kThreads / 32) + warp) * C + lane % C);
-  const bool ok = row < d.rows;
+  const int g = G ? G : d.L / K, c = G ? Along<G>::C : 32 / g;
+  const Along<G> at{lane / c, g, c, g};
+  const int row = 2 * ((tile * (kThreads / 32) + warp) * c + lane % c);
+  const bool ok = row < d.rows && (G || at.seg < g);
   int a = 0, b = 0;
   if (ok) {
     a = row / d.B;
@@ -429,7 +469,7 @@ __device__ __forceinline__ void run_rows(const PassDesc &d, int tile, const floa
       const T *src = static_cast<const T *>(d.in) + (long long)min(a, d.clampA - 1) * d.inSA +
                      (long long)min(b + r, d.clampB - 1) * d.inSB;
       if (ok) {
-        load_run<T, K>(src, K * at.seg, min(K * G, d.clampL), x[r]);
+        load_run<T, K, G == 0>(src, K * at.seg, min(K * g, d.clampL), x[r]);
       } else {
 #pragma unroll
         for (int k = 0; k < K; k++) x[r][k] = 0.f;
@@ -456,7 +496,7 @@ __device__ __forceinline__ void run_rows(const PassDesc &d, int tile, const floa
         if (b + r < d.cropB)
           store_run<T, K>(static_cast<T *>(d.out) + (long long)a * d.outSA +
                               (long long)(b + r) * d.outSB,
-                          K * at.seg, min(K * G, d.cropL), x[r]);
+                          K * at.seg, min(K * g, d.cropL), x[r]);
     }
   }
 }
@@ -496,8 +536,24 @@ void launch_kg(const PassDesc *p, const int *tp, int n, int blocks, bool full, c
   }
   dwt_strided_kernel<T, K, G, PASS, true><<<blocks, kThreads, 0, s>>>(p, tp, n);
 }
+template <typename T, int PASS, int K>
+void launch_any(const PassDesc *p, const int *tp, int n, int blocks, cudaStream_t s) {
+  dwt_strided_kernel<T, K, 0, PASS, PASS == kStridedInv || PASS == kOutput>
+      <<<blocks, kThreads, 0, s>>>(p, tp, n);
+}
+// rows of any other length: strided_elems(L) elements a lane
 template <typename T, int PASS>
-void launch_len(const PassDesc *p, const int *tp, int n, int blocks, int L, bool full,
+void launch_ragged(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s) {
+  switch (strided_elems(L)) {
+    case 8: launch_any<T, PASS, 8>(p, tp, n, blocks, s); break;
+    case 16: launch_any<T, PASS, 16>(p, tp, n, blocks, s); break;
+    default: launch_any<T, PASS, 32>(p, tp, n, blocks, s); break;
+  }
+}
+typedef void LaunchRagged(const PassDesc *p, const int *tp, int n, int blocks, int L,
+                          cudaStream_t s);
+template <typename T, int PASS>
+void launch_len(LaunchRagged *ragged, const PassDesc *p, const int *tp, int n, int blocks, int L, bool full,
                 cudaStream_t s) {
   switch (L) {
     case 16: launch_kg<T, PASS, 16, 1>(p, tp, n, blocks, full, s); break;
@@ -510,7 +566,8 @@ void launch_len(const PassDesc *p, const int *tp, int n, int blocks, int L, bool
     case 256: launch_kg<T, PASS, 32, 8>(p, tp, n, blocks, full, s); break;
     case 512: launch_kg<T, PASS, 32, 16>(p, tp, n, blocks, full, s); break;
     case 1024: launch_kg<T, PASS, 32, 32>(p, tp, n, blocks, full, s); break;
-    default: launch_kg<T, PASS, 64, 32>(p, tp, n, blocks, full, s); break;
+    case 2048: launch_kg<T, PASS, 64, 32>(p, tp, n, blocks, full, s); break;
+    default: ragged(p, tp, n, blocks, L, s); break;
   }
 }
 
@@ -519,9 +576,15 @@ void launch_len(const PassDesc *p, const int *tp, int n, int blocks, int L, bool
 // the instantiations of one pass and element type, each in a file of its own
 // (they are many, and compile in parallel)
 #define WL_STRIDED_LAUNCH(NAME, T, PASS)                                                     \
+  LaunchRagged NAME##_ragged;                                                                \
   void NAME(const PassDesc *p, const int *tp, int n, int blocks, int L, bool full,           \
             cudaStream_t s) {                                                                \
-    launch_len<T, PASS>(p, tp, n, blocks, L, full, s);                                       \
+    launch_len<T, PASS>(NAME##_ragged, p, tp, n, blocks, L, full, s);                        \
+  }
+#define WL_RAGGED_LAUNCH(NAME, T, PASS)                                                      \
+  void NAME##_ragged(const PassDesc *p, const int *tp, int n, int blocks, int L,             \
+                     cudaStream_t s) {                                                       \
+    launch_ragged<T, PASS>(p, tp, n, blocks, L, s);                                          \
   }
 
 }  // namespace wl

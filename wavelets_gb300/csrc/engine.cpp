@@ -94,12 +94,15 @@ int rowreg_key(int L) { return (1 << 20) | L; }
 int rowreg_t_key(int dtype, int L) { return (1 << 21) | (dtype << 16) | L; }
 int rowreg_inv_key(int L) { return (1 << 23) | L; }
 int rowreg_inv_t_key(int outType, int L) { return (1 << 24) | (outType << 16) | L; }
+int strided_len_key(bool inverse, const PassDesc &d) {
+  return (dwt_strided_full(d, inverse) ? 1 << 14 : 0) |
+         (dwt_strided_own(d.L) ? d.L : (1 << 15) | strided_elems(d.L));
+}
 int strided_key(bool inverse, const PassDesc &d) {
-  return (1 << (inverse ? 26 : 25)) | (dwt_strided_full(d, inverse) ? 1 << 14 : 0) | d.L;
+  return (1 << (inverse ? 26 : 25)) | strided_len_key(inverse, d);
 }
 int strided_x_key(bool inverse, int dtype, const PassDesc &d) {
-  return (1 << (inverse ? 28 : 27)) | (dtype << 16) |
-         (dwt_strided_full(d, inverse) ? 1 << 14 : 0) | d.L;
+  return (1 << (inverse ? 28 : 27)) | (dtype << 16) | strided_len_key(inverse, d);
 }
 enum RegKind { kRegNone, kRegInPlace, kRegTile, kRegInvInPlace, kRegInvTile, kRegStrided,
                kRegInvStrided, kRegStridedX, kRegInvStridedX };
@@ -794,6 +797,8 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
            : strided_kind(regKind) ? dwt_strided_rows_per_block(regL)
                                    : dwt_rowreg_rows_per_block(regL, sel);
     for (PassDesc &d : g) {
+      // the rows of a launch may differ in length there
+      if (strided_kind(regKind)) rows = dwt_strided_rows_per_block(d.L);
       d.T = rows;
       d.tiles = (d.rows + rows - 1) / rows;
     }

@@ -336,6 +336,18 @@ bool dwt_strided_full(const PassDesc &d, bool inverse);
 void launch_dwt_strided_x(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
                           int blocks, int L, int dtype, bool inverse, bool full, cudaStream_t s);
 int dwt_strided_rows_per_block(int L);
+// a length with a kernel of its own (else: all of strided_elems(L) in one launch)
+bool dwt_strided_own(int L);
+// elements a lane holds of rows whose length has no kernel of its own, 0: not
+// taken.  They halve five, four or three times; at most 16 lanes a row, so
+// that neighbouring lanes still share sectors.  (With 48, 40 and 24 besides, a
+// batch of 40 odd sizes had a third more launches and took as long, and the y
+// passes of 400 of them took 0.38 ms instead of 0.34.)
+constexpr int strided_elems(int L) {
+  for (int k : {32, 16, 8})
+    if (L % k == 0 && L / k <= 16) return k;
+  return 0;
+}
 void launch_dwt_strided(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
                         int L, bool inverse, bool full, cudaStream_t s);
 
