@@ -1,6 +1,7 @@
 """The Huffman tree build against the oracle's priority queue
 (huffman.cc:42-97): alphabets around the sizes where the build changes shape
-(powers of two of the sort, the wide-CTA limit, one to a few symbols) with
+(powers of two of the sort, the list one warp merges, the wide-CTA limit, one to
+a few symbols) with
 counts that tie, that grow geometrically (long codes, many merge rounds) and
 that are random.  Decode table, longest code and stream are exact."""
 import numpy as np
@@ -11,7 +12,7 @@ from wavelets_gb300 import lib, params as P
 
 pytestmark = pytest.mark.gpu
 
-BINS = (2, 3, 31, 32, 33, 255, 256, 257, 511, 599, 600, 1023, 1024, 2047, 4096)
+BINS = (2, 3, 31, 32, 33, 63, 64, 65, 255, 256, 257, 511, 599, 600, 1023, 1024, 2047, 4096)
 
 
 @pytest.fixture(scope="module")

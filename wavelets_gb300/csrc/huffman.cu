@@ -52,15 +52,8 @@ __host__ __device__ inline size_t build_smem_bytes(int S) {
   return (size_t)build_pow2(S) * 8 + s * 4 + (s / 2 + 4) * 4 + s * 2 * 3 + s * 2 * 2;
 }
 
-// number of entries of the ascending list v[0..n) below x (below or equal
-// with LE)
-template <bool LE> __device__ __forceinline__ int list_rank(const unsigned *v, int n, unsigned x) {
-  int pos = 0;
-  for (int step = n ? 1 << (31 - __clz(n)) : 0; step > 0; step >>= 1)
-    if (step <= n - pos && (LE ? v[pos + step - 1] <= x : v[pos + step - 1] < x)) pos += step;
-  return pos;
-}
-// the same for one x by a whole warp: 32 probes at a time
+// number of entries of the ascending list v[0..n) below x, by a whole warp:
+// 32 probes at a time
 __device__ __forceinline__ int list_rank_warp(const unsigned *v, int n, unsigned x, int lane) {
   int lo = 0, len = n;
   while (len > 0) {
@@ -74,10 +67,16 @@ __device__ __forceinline__ int list_rank_warp(const unsigned *v, int n, unsigned
 }
 
 // One CTA builds one cubelet's tree, codes and decode table; nothing in it is
-// a serial chain over the symbols.  It is bound by shared-memory latency: a
-// one-thread merge, depth pass and breadth-first walk took 120 and 578 us for
-// 257 and 1025 symbols; with this form a whole call on a 2048^2 image (257
-// symbols) went from 624 to 523 us, on a 256^3 volume (1025) from 1079 to 623.
+// a serial chain over the symbols.  A one-thread merge, depth pass and
+// breadth-first walk took 120 and 578 us for 257 and 1025 symbols.  It is bound
+// by the latency of its dependent steps in shared memory and, with many warps,
+// by the instructions they all issue between two barriers; so the searches of
+// a round run side by side, the last rounds and the breadth-first numbering,
+// whose lists are short, belong to one warp without barriers, and the other
+// warps walk the codes meanwhile: 42 K cycles instead of 55 K for 257 symbols
+// and 82 K instead of 118 K for 1025 (a 256^3 volume's call 380 -> 363 us), of
+// which the rounds take 27 and 46 K, the numbering 9 and 20 K.  (Ranks by
+// ballots over a warp's registers in the last rounds were no faster.)
 //
 // Merging in rounds.  The active list holds the parentless nodes in the order
 // the reference pops them (count ascending, on equal counts the larger index
@@ -95,11 +94,11 @@ __device__ __forceinline__ int list_rank_warp(const unsigned *v, int n, unsigned
 // by level.
 template <int T>
 __global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
-  constexpr int kWarps = T / 32;
   constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kTail = 64;  // lists that one warp merges
   extern __shared__ __align__(16) unsigned char hsm[];
   __shared__ int nLeaves;
-  __shared__ int wSum[2][kWarps];
+  __shared__ bool overflow;
   stage_mark(b.head, kMarkBuild);
   const int ci = blockIdx.x;
   const CubeletDev cd = b.cub[ci];
@@ -181,14 +180,14 @@ __global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
   unsigned *cc = m.cntA, *cn = m.cntB;
   uint16_t *ic = m.idA, *in = m.idB;
   int len = nL, next = S;
-  bool bad = false;
-  while (len > 1) {
+  // one round by threads t0, t0 + step, .. (sync: a barrier among them); false
+  // when the counts overflow 32 bits: not from a token count
+  auto merge_round = [&](int t0, int step, auto sync) {
     const unsigned s = cc[0] + cc[1];
     const int kp = list_rank_warp(cc, len, s, lane) & ~1;  // entries paired off
-    bad = kp < 2;  // the counts overflow 32 bits: not from a token count
-    if (bad) break;
+    if (kp < 2) return false;
     const int q = kp >> 1, r = len - kp;
-    for (int j = tid; j < q; j += T) {
+    for (int j = t0; j < q; j += step) {
       const int a = ic[2 * j], c = ic[2 * j + 1], node = next - S + j;
       m.sum[j] = cc[2 * j] + cc[2 * j + 1];
       m.lch[node] = (uint16_t)a;
@@ -196,97 +195,119 @@ __global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
       m.par[a] = (uint16_t)(2 * node);
       m.par[c] = (uint16_t)(2 * node + 1);
     }
-    __syncthreads();
+    sync();
     const unsigned *rest = cc + kp;
-    for (int j = tid; j < q; j += T) {
-      const unsigned c = m.sum[j];
-      int at = j;  // among the new nodes: a run of equal counts is reversed
-      const bool le = j > 0 && m.sum[j - 1] == c, re = j + 1 < q && m.sum[j + 1] == c;
-      if (le || re) {
-        const int gs = le ? list_rank<false>(m.sum, j, c) : j;
-        const int ge = re ? list_rank<true>(m.sum, q, c) - 1 : j;
-        at = gs + ge - j;
+    const int top = 1 << (31 - __clz(max(q, r)));
+    // new nodes go before, old ones after entries of equal count in the other
+    // list; a run of equal counts among the new nodes is reversed
+    for (int t = t0; t < len - q; t += step) {
+      const bool isNew = t < q;
+      const unsigned c = isNew ? m.sum[t] : rest[t - q];
+      const unsigned *v = isNew ? rest : m.sum;
+      const int n = isNew ? r : q;
+      const bool run = isNew && ((t > 0 && m.sum[max(t - 1, 0)] == c) |
+                                 (t + 1 < q && m.sum[min(t + 1, q - 1)] == c));
+      // three searches side by side, without branches: in the other list, and
+      // for a run's ends (an index at or past the end reads some entry of ours)
+      int at = 0, lo = 0, hi = 0;
+      for (int d = top; d > 0; d >>= 1) {
+        const unsigned x = v[min(at + d, n) - (n > 0)], y = m.sum[min(lo + d, q) - 1],
+                       z = m.sum[min(hi + d, q) - 1];
+        at += (d <= n - at) & ((x < c) | (!isNew & (x == c))) ? d : 0;
+        lo += (d <= q - lo) & (y < c) ? d : 0;
+        hi += (d <= q - hi) & (z <= c) ? d : 0;
       }
-      at += list_rank<false>(rest, r, c);
+      at += !isNew ? t - q : run ? lo + hi - 1 - t : t;
       cn[at] = c;
-      in[at] = (uint16_t)(next + j);
-    }
-    for (int i = tid; i < r; i += T) {
-      const unsigned c = rest[i];
-      const int at = i + list_rank<true>(m.sum, q, c);
-      cn[at] = c;
-      in[at] = ic[kp + i];
+      in[at] = isNew ? (uint16_t)(next + t) : ic[kp + t - q];
     }
     next += q;
-    len = q + r;
+    len -= q;
     unsigned *tc = cc;
     cc = cn;
     cn = tc;
     uint16_t *ti = ic;
     ic = in;
     in = ti;
-    __syncthreads();
+    sync();
+    return true;
+  };
+  bool bad = false;
+  while (len > kTail && !bad) bad = !merge_round(tid, T, [] { __syncthreads(); });
+  if (warp == 0) {
+    while (len > 1 && !bad) bad = !merge_round(lane, 32, [] { __syncwarp(); });
+    if (lane == 0) overflow = bad;
   }
+  __syncthreads();
+  bad = overflow;
+  const int root = S + nL - 2;  // with two or more leaves
 
   // ---- codes: up from each leaf (root-first bits, bit d = branch at depth d)
-  const int root = next - 1;  // with two or more leaves
-  unsigned long long *gcode = b.codes + (size_t)ci * kMaxSymbols;
-  uint8_t *glen = b.codeLen + (size_t)ci * kMaxSymbols;
-  for (int i = tid; i < S; i += T) {
-    unsigned long long code = 0;
-    int d = 0;
-    if (nL > 1 && cnt[i] > 0 && !bad) {
-      int nd = i;
-      while (nd != root && d < 64) {
-        const int pb = m.par[nd];
-        code = (code << 1) | (unsigned)(pb & 1);
-        d++;
-        nd = S + (pb >> 1);
+  if (warp > 0) {
+    unsigned long long *gcode = b.codes + (size_t)ci * kMaxSymbols;
+    uint8_t *glen = b.codeLen + (size_t)ci * kMaxSymbols;
+    for (int i = tid - 32; i < S; i += T - 32) {
+      unsigned long long code = 0;
+      int d = 0;
+      if (nL > 1 && cnt[i] > 0 && !bad) {
+        int nd = i;
+        while (nd != root && d < 64) {
+          const int pb = m.par[nd];
+          code = (code << 1) | (unsigned)(pb & 1);
+          d++;
+          nd = S + (pb >> 1);
+        }
       }
+      gcode[i] = code;
+      glen[i] = (uint8_t)d;
     }
-    gcode[i] = code;
-    glen[i] = (uint8_t)d;
+    return;
   }
 
-  // ---- decode table, breadth first: (left id, right id) or (0, symbol)
+  // ---- decode table, breadth first: (left id, right id) or (0, symbol);
+  // kWide nodes a lane and step
+  constexpr int kWide = 2;
   int2 *dec = reinterpret_cast<int2 *>(b.decode + (size_t)ci * 4 * kMaxSymbols);
-  int base = 0, width = nL > 0 && !bad ? 1 : 0, levels = 0, par = 0;
-  if (nL > 0 && tid == 0) m.bfs[0] = (uint16_t)(nL > 1 ? root : 8191 - (int)(m.keys[0] & 8191ull));
-  __syncthreads();
+  int base = 0, width = nL > 0 && !bad ? 1 : 0, levels = 0;
+  if (nL > 0 && lane == 0)
+    m.bfs[0] = (uint16_t)(nL > 1 ? root : 8191 - (int)(m.keys[0] & 8191ull));
+  __syncwarp();
   while (width > 0) {
-    const int nb = base + width;  // the next level's first node
-    int inner = 0;                // inner nodes of this level so far
-    for (int t0 = 0; t0 < width; t0 += T) {
-      const int t = t0 + tid;
-      const int nd = t < width ? m.bfs[base + t] : 0;
-      const bool isIn = t < width && nd >= S;
-      const unsigned bal = __ballot_sync(kAll, isIn);
-      if (lane == 0) wSum[par][warp] = __popc(bal);
-      __syncthreads();
-      int before = 0, all = 0;
+    int child = base + width;  // the next level's first node
+    for (int t0 = 0; t0 < width; t0 += 32 * kWide) {
+      int nd[kWide], left[kWide], right[kWide];
 #pragma unroll
-      for (int v = 0; v < kWarps; v++) {
-        const int x = wSum[par][v];
-        before += v < warp ? x : 0;
-        all += x;
+      for (int k = 0; k < kWide; k++) {
+        const int t = t0 + 32 * k + lane;
+        const int x = m.bfs[base + min(t, width - 1)];
+        nd[k] = t < width ? x : -1;
       }
-      par ^= 1;  // two sets: a warp overwrites one only after the next barrier
-      if (isIn) {
-        const int c = nb + 2 * (inner + before + __popc(bal & ((1u << lane) - 1u)));
-        m.bfs[c] = m.lch[nd - S];
-        m.bfs[c + 1] = m.rch[nd - S];
-        dec[base + t] = make_int2(c, c + 1);
-      } else if (t < width) {
-        dec[base + t] = make_int2(0, nd);
+#pragma unroll
+      for (int k = 0; k < kWide; k++) {
+        left[k] = m.lch[max(nd[k] - S, 0)];
+        right[k] = m.rch[max(nd[k] - S, 0)];
       }
-      inner += all;
+#pragma unroll
+      for (int k = 0; k < kWide; k++) {
+        const unsigned bal = __ballot_sync(kAll, nd[k] >= S);
+        const int at = base + t0 + 32 * k + lane;
+        const int c = child + 2 * __popc(bal & ((1u << lane) - 1u));
+        if (nd[k] >= S) {
+          m.bfs[c] = (uint16_t)left[k];
+          m.bfs[c + 1] = (uint16_t)right[k];
+          dec[at] = make_int2(c, c + 1);
+        } else if (nd[k] >= 0) {
+          dec[at] = make_int2(0, nd[k]);
+        }
+        child += 2 * __popc(bal);
+      }
     }
-    __syncthreads();
-    base = nb;
-    width = 2 * inner;
+    __syncwarp();
+    base += width;
+    width = child - base;
     levels++;
   }
-  if (tid == 0) {
+  if (lane == 0) {
     const int longest = levels > 0 ? levels - 1 : 0;
     st->nDecode = 2 * base;
     st->longest = longest;
