@@ -130,3 +130,22 @@ def test_rows_at_any_address(ctx, dtype):
         want = ctx.compress(v, p)
         assert np.array_equal(c.words, want.words)
         assert (c.threshold_value, c.max_value) == (want.threshold_value, want.max_value)
+
+
+@pytest.mark.parametrize("wavelet", [P.HAAR, P.CDF97])
+@pytest.mark.parametrize("L,s", ANY + [(512, 5), (512, 6)])
+def test_z_rows(ctx, L, s, wavelet):
+    """z passes of the same lengths, an odd number of rows: against the float64
+    yardstick, back again, and the extremes gathered on the way."""
+    X, Y = 13, 11
+    vol = np.random.default_rng(L * s).normal(0, 100, (L, Y, X)).astype(np.float32)
+    p = P.Params(steps=(0, 0, s), wavelet=wavelet, threshold_fraction=0.5, bin_count=64)
+    got, stored = ctx.forward_transform(vol, p)
+    ref, _ = lifting64.forward(vol, (0, 0, s), wavelet)
+    assert np.abs(got.ravel() - ref).max() <= 2e-6 * np.abs(ref).max()
+    back = ctx.inverse_transform(got, stored, (0, 0, s), wavelet, (X, Y, L))
+    assert np.abs(back - vol).max() <= 4e-6 * np.abs(vol).max()
+    c = ctx.compress(vol, p)
+    a = np.sort(np.abs(got.ravel()))
+    assert (c.min_coef, c.max_coef, c.max_value) == (got.min(), got.max(), a[-1])
+    assert c.threshold_value in a and abs(np.searchsorted(a, c.threshold_value) - a.size / 2) <= 2

@@ -17,6 +17,9 @@ WL_STRIDED_DECLARE(strided_x_inv_u8)
 WL_STRIDED_DECLARE(strided_x_inv_u16)
 WL_STRIDED_DECLARE(strided_x_inv_i32)
 WL_STRIDED_DECLARE(strided_x_inv_f32)
+void strided_z(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s);
+void strided_z_sel(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s);
+void strided_z_inv(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s);
 
 bool dwt_strided_own(int L) {
   return (L >= 16 && (L & (L - 1)) == 0) || L == 48 || L == 96 || L == 192;
@@ -76,6 +79,29 @@ bool dwt_strided_source_fits(const PassDesc &d, int es) {
 bool dwt_strided_output_fits(const PassDesc &d, int es) {
   return shape_fits(d) && d.outSC == 1 && d.inSB == 1 && ((d.inSA | d.inSC) & 1) == 0 &&
          rows_aligned(d.out, d.outSA, d.outSB, es);
+}
+
+bool dwt_z_fits(const PassDesc &d) {
+  // lengths of the row kernel stay with it, which is faster there: the z pass
+  // of the mixed batch takes 0.67 ms there and 0.89 here, with whole sectors
+  // a lane but a quarter of the warps
+  const int k = strided_elems(d.L);
+  if (!k || (dwt_strided_own(d.L) && d.L <= 256) || d.steps < 1 || d.inSC != 1 || d.outSC != 1)
+    return false;
+  int own = 0;
+  for (int e = k; e % 2 == 0; e /= 2) own++;
+  const auto at32 = [](const void *p, long long a, long long b) {
+    return reinterpret_cast<size_t>(p) % 32 == 0 && a % 8 == 0 && b % 8 == 0;
+  };
+  return d.steps <= own && at32(d.in, d.inSA, d.inSB) && at32(d.out, d.outSA, d.outSB);
+}
+int dwt_z_rows_per_block(int L) {
+  const int k = strided_elems(L);
+  return 2 * 8 * (32 / (L / k)) * strided_z_rounds(k);
+}
+void launch_dwt_z(const PassDesc *p, const int *tp, int n, int blocks, int L, bool inverse,
+                  bool sel, cudaStream_t s) {
+  (inverse ? strided_z_inv : sel ? strided_z_sel : strided_z)(p, tp, n, blocks, L, s);
 }
 
 bool dwt_strided_full(const PassDesc &d, bool inverse) {

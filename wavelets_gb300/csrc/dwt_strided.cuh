@@ -55,6 +55,7 @@
 #include <type_traits>
 
 #include "dwt_common.cuh"
+#include "select_common.cuh"
 #include "wl_internal.h"
 
 namespace wl {
@@ -176,141 +177,7 @@ __device__ __forceinline__ void inv_level(f2 (&e)[M], f2 (&o)[M], const Along<G>
   for (int k = 0; k < M; k++) o[k] = fma2(ka, add2(e[k], k + 1 < M ? e[(k + 1) % M] : eN), o[k]);
 }
 
-// A row pair in global memory: position q at base + q * stride floats.
-struct Row {
-  float *base;
-  long long stride;
-  bool ok;
-  __device__ __forceinline__ f2 get(int q) const {
-    return ok ? *reinterpret_cast<const f2 *>(base + q * stride) : 0ull;
-  }
-  __device__ __forceinline__ void put(int q, f2 v) const {
-    if (ok) *reinterpret_cast<f2 *>(base + q * stride) = v;
-  }
-};
-
-// Levels LEV .. S-1 on the 2 M values v[] of a lane, each band to its place
-// with the deferred lifting scale.
-template <int LEV, int M, int G, bool HAAR, bool FULL>
-__device__ __forceinline__ void fwd_from(const f2 (&v)[2 * M], int S, const float *scale,
-                                         const Along<G> &at, const Row &out) {
-  const int H = M * at.lanes;  // pairs of this level
-  f2 e[M], o[M];
-#pragma unroll
-  for (int k = 0; k < M; k++) {
-    e[k] = v[2 * k];
-    o[k] = v[2 * k + 1];
-  }
-  fwd_level<M, G, HAAR>(e, o, at);
-  const f2 sc = pack(scale[LEV]);
-#pragma unroll
-  for (int k = 0; k < M; k++) out.put(H + M * at.seg + k, mul2(o[k], sc));
-  if constexpr (M % 2 == 0) {
-    if (LEV + 1 < S) {
-      fwd_from<LEV + 1, M / 2, G, HAAR, FULL>(e, S, scale, at, out);
-      return;
-    }
-  }
-  if constexpr (FULL && M == 1 && G > 1) {
-    if (LEV + 1 < S) {
-      // one low-pass value per lane: each further level gathers pair j into
-      // lane j
-      f2 s = e[0];
-      Along<G> in = at;
-#pragma unroll 1
-      for (int lev = LEV + 1; lev < S; lev++) {
-        f2 ge[1] = {at.from(s, 2 * at.seg)}, go[1] = {at.from(s, 2 * at.seg + 1)};
-        in.na >>= 1;
-        fwd_level<1, G, HAAR>(ge, go, in);
-        if (at.seg < in.na) out.put(in.na + at.seg, mul2(go[0], pack(scale[lev])));
-        s = ge[0];
-      }
-      if (at.seg < in.na) out.put(at.seg, mul2(s, pack(scale[S])));
-      return;
-    }
-  }
-  const f2 low = pack(scale[LEV + 1]);
-#pragma unroll
-  for (int k = 0; k < M; k++) out.put(M * at.seg + k, mul2(e[k], low));
-}
-
-// The deferred lifting scale of level t undone, as the kernel that had the
-// pass before did: by its reciprocal, or (divide) by a correctly rounded
-// division -- the quotient by the reciprocal with one correction step, which
-// gives it for every scale of up to kMaxLevels levels and every significand
-// (checked exhaustively); an infinite quotient stays.
-template <bool FULL> struct Unscale {
-  const float *scale, *rscale;
-  bool divide;
-  __device__ __forceinline__ f2 operator()(f2 v, int t) const {
-    const f2 r = pack(rscale[t]);
-    const f2 q = mul2(v, r);
-    if (!FULL || !divide) return q;
-    float qa, qb, ca, cb;
-    unpack(q, qa, qb);
-    unpack(fma2(fma2(q, pack(-scale[t]), v), r, q), ca, cb);
-    return pack(isinf(qa) ? qa : ca, isinf(qb) ? qb : cb);
-  }
-};
-
-// The 2 M values v[] of level LEV's input from the bands of levels LEV ..
-// S-1.
-template <int LEV, int M, int G, bool HAAR, bool FULL>
-__device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL> &un,
-                                       const Along<G> &at, const Row &in) {
-  const int H = M * at.lanes;
-  f2 e[M], o[M];
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = in.get(H + M * at.seg + k);
-  bool deeper = false;
-  if constexpr (M % 2 == 0) {
-    if (LEV + 1 < S) {
-      inv_to<LEV + 1, M / 2, G, HAAR, FULL>(e, S, un, at, in);
-      deeper = true;
-    }
-  }
-  if constexpr (FULL && M == 1 && G > 1) {
-    if (LEV + 1 < S) {
-      // the levels below one pair per lane: lane j holds pair j
-      constexpr int kDeep = G == 32 ? 5 : G == 16 ? 4 : G == 8 ? 3 : G == 4 ? 2 : 1;
-      f2 dg[kDeep];
-#pragma unroll
-      for (int k = 0; k < kDeep; k++) {
-        const int n = G >> (k + 1);
-        dg[k] = LEV + 1 + k < S && at.seg < n ? un(in.get(n + at.seg), LEV + 1 + k) : 0ull;
-      }
-      const int n0 = G >> (S - LEV - 1);
-      f2 s = at.seg < n0 ? un(in.get(at.seg), S) : 0ull;
-      Along<G> now = at;
-#pragma unroll
-      for (int k = kDeep - 1; k >= 0; k--) {
-        if (LEV + 1 + k < S) {  // the same for the whole warp
-          now.na = G >> (k + 1);
-          f2 se[1] = {s}, so[1] = {dg[k]};
-          inv_level<1, G, HAAR>(se, so, now);
-          const f2 a = at.from(se[0], at.seg >> 1), b = at.from(so[0], at.seg >> 1);
-          s = at.seg & 1 ? b : a;
-        }
-      }
-      e[0] = s;
-      deeper = true;
-    }
-  }
-  if (!deeper) {
-#pragma unroll
-    for (int k = 0; k < M; k++) e[k] = un(in.get(M * at.seg + k), LEV + 1);
-  }
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = un(o[k], LEV);
-  inv_level<M, G, HAAR>(e, o, at);
-#pragma unroll
-  for (int k = 0; k < M; k++) {
-    v[2 * k] = e[k];
-    v[2 * k + 1] = o[k];
-  }
-}
-
-// ---- rows of the source and of the output (x passes) ----
+// ---- contiguous rows (x passes: source and output; z passes) ----
 // bytes per vector access of a lane's K elements
 template <typename T, int K> __host__ __device__ constexpr int vec_bytes() {
   return (K * (int)sizeof(T)) % 32 == 0 ? 32 : (K * (int)sizeof(T)) % 16 == 0 ? 16 : 8;
@@ -324,6 +191,8 @@ template <int VB> __device__ __forceinline__ void load_vec(const void *p, unsign
   } else if constexpr (VB == 8) {
     const uint2 q = *static_cast<const uint2 *>(p);
     w[0] = q.x; w[1] = q.y;
+  } else if constexpr (VB == 4) {
+    w[0] = *static_cast<const unsigned *>(p);
   } else {
     const uint4 q = *static_cast<const uint4 *>(p);
     w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
@@ -337,6 +206,8 @@ template <int VB> __device__ __forceinline__ void store_vec(void *p, const unsig
                  : "memory");
   } else if constexpr (VB == 8) {
     *static_cast<uint2 *>(p) = make_uint2(w[0], w[1]);
+  } else if constexpr (VB == 4) {
+    *static_cast<unsigned *>(p) = w[0];
   } else {
     *static_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
   }
@@ -380,6 +251,195 @@ __device__ __forceinline__ void store_vecs(T *p, const float (&v)[K]) {
         w[i] |= to_bits<T>(v[j * E + i * P + k]) << (8 * (int)sizeof(T) * k);
     }
     store_vec<VB>(p + j * E, w);
+  }
+}
+
+// A row pair in global memory: position q at base + q * stride floats.
+struct Row {
+  float *base;
+  long long stride;
+  bool ok;
+  __device__ __forceinline__ f2 get(int q) const {
+    return ok ? *reinterpret_cast<const f2 *>(base + q * stride) : 0ull;
+  }
+  __device__ __forceinline__ void put(int q, f2 v) const {
+    if (ok) *reinterpret_cast<f2 *>(base + q * stride) = v;
+  }
+  template <int M> __device__ __forceinline__ void get_run(int q, f2 (&v)[M]) const {
+#pragma unroll
+    for (int k = 0; k < M; k++) v[k] = get(q + k);
+  }
+  template <int M> __device__ __forceinline__ void put_run(int q, const f2 (&v)[M]) {
+#pragma unroll
+    for (int k = 0; k < M; k++) put(q + k, v[k]);
+  }
+};
+
+// A pair of contiguous rows (z passes); SEL: every value put also goes into
+// the select statistics.
+template <bool SEL> struct ZRow {
+  float *base[2];  // null: no such row
+  selc::SelAcc *acc;
+  template <int M> __host__ __device__ static constexpr int vb() {
+    return M % 8 == 0 ? 32 : M % 4 == 0 ? 16 : M % 2 == 0 ? 8 : 4;
+  }
+  __device__ __forceinline__ f2 get(int q) const {
+    return pack(base[0] ? base[0][q] : 0.f, base[1] ? base[1][q] : 0.f);
+  }
+  __device__ __forceinline__ void put(int q, f2 v) {
+    const f2 x[1] = {v};
+    put_run<1>(q, x);
+  }
+  template <int M> __device__ __forceinline__ void get_run(int q, f2 (&v)[M]) const {
+    float x[2][M];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      if (base[r]) {
+        load_vecs<float, M, vb<M>()>(base[r] + q, x[r]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < M; k++) x[r][k] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < M; k++) v[k] = pack(x[0][k], x[1][k]);
+  }
+  template <int M> __device__ __forceinline__ void put_run(int q, const f2 (&v)[M]) {
+    float x[2][M];
+#pragma unroll
+    for (int k = 0; k < M; k++) unpack(v[k], x[0][k], x[1][k]);
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      if (!base[r]) continue;
+      store_vecs<float, M, vb<M>()>(base[r] + q, x[r]);
+      if (SEL) {
+#pragma unroll
+        for (int k = 0; k < M; k++) acc->visit(x[r][k]);
+      }
+    }
+  }
+};
+
+// Levels LEV .. S-1 on the 2 M values v[] of a lane, each band to its place
+// with the deferred lifting scale.
+template <int LEV, int M, int G, bool HAAR, bool FULL, typename Out>
+__device__ __forceinline__ void fwd_from(const f2 (&v)[2 * M], int S, const float *scale,
+                                         const Along<G> &at, Out &out) {
+  const int H = M * at.lanes;  // pairs of this level
+  f2 e[M], o[M];
+#pragma unroll
+  for (int k = 0; k < M; k++) {
+    e[k] = v[2 * k];
+    o[k] = v[2 * k + 1];
+  }
+  fwd_level<M, G, HAAR>(e, o, at);
+  const f2 sc = pack(scale[LEV]);
+#pragma unroll
+  for (int k = 0; k < M; k++) o[k] = mul2(o[k], sc);
+  out.template put_run<M>(H + M * at.seg, o);
+  if constexpr (M % 2 == 0) {
+    if (LEV + 1 < S) {
+      fwd_from<LEV + 1, M / 2, G, HAAR, FULL>(e, S, scale, at, out);
+      return;
+    }
+  }
+  if constexpr (FULL && M == 1 && G > 1) {
+    if (LEV + 1 < S) {
+      // one low-pass value per lane: each further level gathers pair j into
+      // lane j
+      f2 s = e[0];
+      Along<G> in = at;
+#pragma unroll 1
+      for (int lev = LEV + 1; lev < S; lev++) {
+        f2 ge[1] = {at.from(s, 2 * at.seg)}, go[1] = {at.from(s, 2 * at.seg + 1)};
+        in.na >>= 1;
+        fwd_level<1, G, HAAR>(ge, go, in);
+        if (at.seg < in.na) out.put(in.na + at.seg, mul2(go[0], pack(scale[lev])));
+        s = ge[0];
+      }
+      if (at.seg < in.na) out.put(at.seg, mul2(s, pack(scale[S])));
+      return;
+    }
+  }
+  const f2 low = pack(scale[LEV + 1]);
+#pragma unroll
+  for (int k = 0; k < M; k++) e[k] = mul2(e[k], low);
+  out.template put_run<M>(M * at.seg, e);
+}
+
+// The deferred lifting scale of level t undone, as the kernel that had the
+// pass before did: by its reciprocal, or (divide) by a correctly rounded
+// division -- the quotient by the reciprocal with one correction step, which
+// gives it for every scale of up to kMaxLevels levels and every significand
+// (checked exhaustively); an infinite quotient stays.
+template <bool FULL> struct Unscale {
+  const float *scale, *rscale;
+  bool divide;
+  __device__ __forceinline__ f2 operator()(f2 v, int t) const {
+    const f2 r = pack(rscale[t]);
+    const f2 q = mul2(v, r);
+    if (!FULL || !divide) return q;
+    float qa, qb, ca, cb;
+    unpack(q, qa, qb);
+    unpack(fma2(fma2(q, pack(-scale[t]), v), r, q), ca, cb);
+    return pack(isinf(qa) ? qa : ca, isinf(qb) ? qb : cb);
+  }
+};
+
+// The 2 M values v[] of level LEV's input from the bands of levels LEV ..
+// S-1.
+template <int LEV, int M, int G, bool HAAR, bool FULL, typename In>
+__device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL> &un,
+                                       const Along<G> &at, const In &in) {
+  const int H = M * at.lanes;
+  f2 e[M], o[M];
+  in.template get_run<M>(H + M * at.seg, o);
+  bool deeper = false;
+  if constexpr (M % 2 == 0) {
+    if (LEV + 1 < S) {
+      inv_to<LEV + 1, M / 2, G, HAAR, FULL>(e, S, un, at, in);
+      deeper = true;
+    }
+  }
+  if constexpr (FULL && M == 1 && G > 1) {
+    if (LEV + 1 < S) {
+      // the levels below one pair per lane: lane j holds pair j
+      constexpr int kDeep = G == 32 ? 5 : G == 16 ? 4 : G == 8 ? 3 : G == 4 ? 2 : 1;
+      f2 dg[kDeep];
+#pragma unroll
+      for (int k = 0; k < kDeep; k++) {
+        const int n = G >> (k + 1);
+        dg[k] = LEV + 1 + k < S && at.seg < n ? un(in.get(n + at.seg), LEV + 1 + k) : 0ull;
+      }
+      const int n0 = G >> (S - LEV - 1);
+      f2 s = at.seg < n0 ? un(in.get(at.seg), S) : 0ull;
+      Along<G> now = at;
+#pragma unroll
+      for (int k = kDeep - 1; k >= 0; k--) {
+        if (LEV + 1 + k < S) {  // the same for the whole warp
+          now.na = G >> (k + 1);
+          f2 se[1] = {s}, so[1] = {dg[k]};
+          inv_level<1, G, HAAR>(se, so, now);
+          const f2 a = at.from(se[0], at.seg >> 1), b = at.from(so[0], at.seg >> 1);
+          s = at.seg & 1 ? b : a;
+        }
+      }
+      e[0] = s;
+      deeper = true;
+    }
+  }
+  if (!deeper) {
+    in.template get_run<M>(M * at.seg, e);
+#pragma unroll
+    for (int k = 0; k < M; k++) e[k] = un(e[k], LEV + 1);
+  }
+#pragma unroll
+  for (int k = 0; k < M; k++) o[k] = un(o[k], LEV);
+  inv_level<M, G, HAAR>(e, o, at);
+#pragma unroll
+  for (int k = 0; k < M; k++) {
+    v[2 * k] = e[k];
+    v[2 * k + 1] = o[k];
   }
 }
 
@@ -523,6 +583,86 @@ dwt_strided_kernel(const PassDesc *__restrict__ passes, const int *__restrict__ 
   __syncthreads();
   if (haar) run_rows<T, K, G, true, PASS, FULL>(d, bid - tilePrefix[lo], scale, rscale);
   else run_rows<T, K, G, false, PASS, FULL>(d, bid - tilePrefix[lo], scale, rscale);
+}
+
+// ---- z passes: contiguous rows, in place ----
+// Lengths without a row kernel (dwt_rows.cu), which went to the column tiles
+// and then needed the first select pass: the z pass of a 93 x 181 x 147 16-bit
+// volume takes 18 us (23), of a 200 x 176 x 208 float volume 22 (32, and its
+// select 39 instead of 45); restoring 400 cubelets of odd sizes 3.0 ms a call
+// (3.4).
+constexpr int kZThreads = 256;
+
+template <int K, bool HAAR, bool INV, bool SEL>
+__device__ __forceinline__ void run_z(const PassDesc &d, int pair0, const float *scale,
+                                      const float *rscale, selc::SelAcc &acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = d.L / K, c = 32 / g;
+  const Along<0> at{lane / c, g, c, g};
+  const int row = 2 * (pair0 + warp * c + lane % c);
+  ZRow<false> in{{nullptr, nullptr}, nullptr};
+  ZRow<SEL> out{{nullptr, nullptr}, &acc};
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    if (row + r >= d.rows || at.seg >= g) continue;
+    const int a = (row + r) / d.B, b = row + r - a * d.B;
+    in.base[r] = const_cast<float *>(static_cast<const float *>(d.in)) + (long long)a * d.inSA +
+                 (long long)b * d.inSB;
+    out.base[r] = static_cast<float *>(d.out) + (long long)a * d.outSA + (long long)b * d.outSB;
+  }
+  f2 v[K];
+  if constexpr (!INV) {
+    in.template get_run<K>(K * at.seg, v);
+    __syncwarp();  // the row's lanes have read it
+    fwd_from<0, K / 2, 0, HAAR, false>(v, d.steps, scale, at, out);
+  } else {
+    inv_to<0, K / 2, 0, HAAR, true>(v, d.steps, Unscale<true>{scale, rscale, d.exact != 0}, at,
+                                    in);
+    __syncwarp();
+    out.template put_run<K>(K * at.seg, v);
+  }
+}
+
+template <int K, bool INV, bool SEL>
+__global__ void __launch_bounds__(kZThreads)
+dwt_z_kernel(const PassDesc *__restrict__ passes, const int *__restrict__ tilePrefix, int nPasses) {
+  __shared__ float scale[16], rscale[16];
+  __shared__ unsigned hist[SEL ? kSelectBins : 1];
+  const int bid = blockIdx.x;
+  int lo = 0, hi = nPasses - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (tilePrefix[mid] <= bid) lo = mid; else hi = mid - 1;
+  }
+  const PassDesc &d = passes[lo];
+  const int S = d.steps;
+  const bool haar = d.wavelet == WL_HAAR;
+  if ((int)threadIdx.x <= S) {
+    const float s = haar ? 1.0f : lifting_scale(threadIdx.x, S);
+    scale[threadIdx.x] = s;
+    rscale[threadIdx.x] = 1.0f / s;
+  }
+  if (SEL) selc::clear_hist<kZThreads>(hist);
+  selc::SelAcc acc{hist};
+  __syncthreads();
+  constexpr int kRounds = K < 32 ? 32 / K : 1;  // strided_z_rounds
+  const int round = (kZThreads / 32) * (32 / (d.L / K));  // pairs
+  for (int r = 0; r < kRounds; r++) {
+    const int pair0 = ((bid - tilePrefix[lo]) * kRounds + r) * round;
+    if (2 * pair0 >= d.rows) break;  // the same for every thread of the block
+    if (haar) run_z<K, true, INV, SEL>(d, pair0, scale, rscale, acc);
+    else run_z<K, false, INV, SEL>(d, pair0, scale, rscale, acc);
+  }
+  if (SEL) selc::flush<kZThreads>(acc, d.selHist, d.selState);
+}
+
+template <bool INV, bool SEL>
+void launch_z(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s) {
+  switch (strided_elems(L)) {
+    case 8: dwt_z_kernel<8, INV, SEL><<<blocks, kZThreads, 0, s>>>(p, tp, n); break;
+    case 16: dwt_z_kernel<16, INV, SEL><<<blocks, kZThreads, 0, s>>>(p, tp, n); break;
+    default: dwt_z_kernel<32, INV, SEL><<<blocks, kZThreads, 0, s>>>(p, tp, n); break;
+  }
 }
 
 // launch for rows of L elements

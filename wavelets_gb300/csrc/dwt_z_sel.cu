@@ -1,0 +1,8 @@
+// Register passes (dwt_strided.cuh): the z passes that gather the select statistics.
+#include "dwt_strided.cuh"
+
+namespace wl {
+void strided_z_sel(const PassDesc *p, const int *tp, int n, int blocks, int L, cudaStream_t s) {
+  launch_z<false, true>(p, tp, n, blocks, L, s);
+}
+}  // namespace wl

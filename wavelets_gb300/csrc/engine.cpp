@@ -105,8 +105,10 @@ int strided_x_key(bool inverse, int dtype, const PassDesc &d) {
   return (1 << (inverse ? 28 : 27)) | (dtype << 16) | strided_len_key(inverse, d);
 }
 enum RegKind { kRegNone, kRegInPlace, kRegTile, kRegInvInPlace, kRegInvTile, kRegStrided,
-               kRegInvStrided, kRegStridedX, kRegInvStridedX };
-bool strided_kind(int k) { return k >= kRegStrided; }
+               kRegInvStrided, kRegStridedX, kRegInvStridedX, kRegZ, kRegInvZ };
+bool strided_kind(int k) { return k >= kRegStrided && k < kRegZ; }
+bool z_kind(int k) { return k >= kRegZ; }
+int z_key(bool inverse, int L) { return (1 << (inverse ? 30 : 29)) | strided_elems(L); }
 
 // ---- result storage ------------------------------------------------------------
 // The arrays of all results of one compression call live in one page-locked
@@ -623,6 +625,12 @@ bool forward_passes_cols(const Plan &pl, const void *in, bool hostIn, float *coe
   f.out = o;
   f.outSA = Zp * Xp; f.outSB = Zp; f.outSC = 1;
   f.steps = pl.sz;
+  if (dwt_z_fits(f)) {
+    f.selHist = selHist;
+    f.selState = selState;
+    zs[z_key(false, f.L)].push_back(f);
+    return selHist != nullptr;
+  }
   if (dwt_rowreg_fits(f.L, f.steps)) {
     f.selHist = selHist;
     f.selState = selState;
@@ -788,17 +796,18 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
   if (hoff + bytes > ctx->hPasses.cap || hoff + bytes > ctx->passes.cap)
     return fail(ctx, WL_ENOMEM, "pass staging too small");
   int rows = 0, warps = 4;
-  const bool sel = regKind == kRegInPlace && g[0].selHist != nullptr;
+  const bool sel = (regKind == kRegInPlace || regKind == kRegZ) && g[0].selHist != nullptr;
   for (const PassDesc &d : g)
     if ((d.selHist != nullptr) != sel)
       return fail(ctx, WL_EINVAL, "internal: mixed select-gathering passes in one group");
   if (regL) {
-    rows = (regKind == kRegTile || regKind == kRegInvTile) ? dwt_rowreg_t_rows_per_block(regL)
-           : strided_kind(regKind) ? dwt_strided_rows_per_block(regL)
-                                   : dwt_rowreg_rows_per_block(regL, sel);
+    rows = regKind == kRegTile || regKind == kRegInvTile     ? dwt_rowreg_t_rows_per_block(regL)
+           : regKind == kRegInPlace || regKind == kRegInvInPlace ? dwt_rowreg_rows_per_block(regL, sel)
+                                                                 : 0;
     for (PassDesc &d : g) {
       // the rows of a launch may differ in length there
       if (strided_kind(regKind)) rows = dwt_strided_rows_per_block(d.L);
+      else if (z_kind(regKind)) rows = dwt_z_rows_per_block(d.L);
       d.T = rows;
       d.tiles = (d.rows + rows - 1) / rows;
     }
@@ -837,6 +846,11 @@ wl_status stage_group(wl_ctx *ctx, std::vector<PassDesc> g, size_t &hoff, int ki
 wl_status stage_groups(wl_ctx *ctx, const PassGroups &gs, size_t &hoff, int kind, int outType,
                        bool inverse, std::vector<GroupLaunch> &out) {
   for (const auto &kv : gs) {
+    if ((kv.first >> 29) & 1) {
+      TRY(stage_group(ctx, kv.second, hoff, kind, WL_F32, WL_F32, false, false, false, out, nullptr,
+                      kv.second[0].L, kRegZ));
+      continue;
+    }
     if ((kv.first >> 27) & 1) {
       TRY(stage_group(ctx, kv.second, hoff, kind, (kv.first >> 16) & 15, WL_F32, false, false, false,
                       out, nullptr, kv.second[0].L, kRegStridedX));
@@ -862,7 +876,9 @@ wl_status launch_one(wl_ctx *ctx, const GroupLaunch &l, cudaStream_t s) {
   const char *base = P<char>(ctx->passes);
   const PassDesc *dp = reinterpret_cast<const PassDesc *>(base + l.off);
   const int *dtp = reinterpret_cast<const int *>(base + l.off + l.n * sizeof(PassDesc));
-  if (l.regKind == kRegStrided || l.regKind == kRegInvStrided)
+  if (z_kind(l.regKind))
+    launch_dwt_z(dp, dtp, l.n, l.tiles, l.regL, l.regKind == kRegInvZ, l.sel, s);
+  else if (l.regKind == kRegStrided || l.regKind == kRegInvStrided)
     launch_dwt_strided(dp, dtp, l.n, l.tiles, l.regL, l.regKind == kRegInvStrided, l.full, s);
   else if (l.regKind == kRegStridedX)
     launch_dwt_strided_x(dp, dtp, l.n, l.tiles, l.regL, l.inType, false, l.full, s);
@@ -1736,7 +1752,10 @@ void inverse_passes(const int size[3], const int steps[3], int wavelet, const in
   if (columns || longImage) {
     for (int i = 0; i < np; i++) {
       const int phase = 3 - np + i;
-      if (phase == 0 && dwt_rowreg_fits(d[i].L, d[i].steps))  // z rows in registers
+      if (phase == 0 && dwt_z_fits(d[i])) {  // z rows in registers; the scale as above
+        d[i].exact = !dwt_rowreg_fits(d[i].L, d[i].steps);
+        ph[0][z_key(true, d[i].L)].push_back(d[i]);
+      } else if (phase == 0 && dwt_rowreg_fits(d[i].L, d[i].steps))
         ph[0][rowreg_inv_key(d[i].L)].push_back(d[i]);
       else if (phase > 0 && put_registers(phase, d[i], longImage, true))
         continue;
@@ -1794,6 +1813,11 @@ wl_status stage_inverse_phases(wl_ctx *ctx, PassGroups ph[3], InversePhases &ip)
   const int kinds[3] = {kTuneInvZ, kTuneInvY, kTuneInvX};
   for (int k = 0; k < 3; k++) {
     for (const auto &kv : ph[k]) {
+      if ((kv.first >> 30) & 1) {
+        TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, WL_F32, true, false, false, gl,
+                        nullptr, kv.second[0].L, kRegInvZ));
+        continue;
+      }
       if ((kv.first >> 28) & 1) {
         TRY(stage_group(ctx, kv.second, hoff, kinds[k], WL_F32, (kv.first >> 16) & 15, true, false,
                         false, gl, nullptr, kv.second[0].L, kRegInvStridedX));

@@ -348,6 +348,15 @@ constexpr int strided_elems(int L) {
     if (L % k == 0 && L / k <= 16) return k;
   return 0;
 }
+// z passes of the same kernels: contiguous rows, in place, as many levels as a
+// lane's elements halve; the forward pass may gather the select statistics.
+// One launch for all lengths of the same strided_elems.
+bool dwt_z_fits(const PassDesc &d);
+int dwt_z_rows_per_block(int L);
+void launch_dwt_z(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
+                  int L, bool inverse, bool sel, cudaStream_t s);
+// rounds of a block over rows of k elements a lane: some 16 K values
+constexpr int strided_z_rounds(int k) { return k < 32 ? 32 / k : 1; }
 void launch_dwt_strided(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
                         int L, bool inverse, bool full, cudaStream_t s);
 
