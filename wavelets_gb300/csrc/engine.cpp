@@ -1071,13 +1071,11 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   TRY(ensure(ctx, ctx->words, wordsTotal * 4));
   TRY(ensure(ctx, ctx->head, kHeadCount * sizeof(long long)));
   TRY(ensure(ctx, ctx->meta, (size_t)n * (4 * kMaxSymbols + 2 * kMaxBins) * 4));
-  // upload block: result slab | cubelet records | chunk prefix | transform
-  // pass groups
+  // upload block: result slab | cubelet records | transform pass groups
   const size_t slabBytes = 256;
   const size_t cubBytes = ((size_t)n * sizeof(CubeletDev) + 255) & ~(size_t)255;
-  const size_t prefBytes = ((size_t)n * sizeof(long long) + 255) & ~(size_t)255;
   const size_t passBytes =
-      slabBytes + cubBytes + prefBytes + (size_t)3 * n * (sizeof(PassDesc) + sizeof(int) + 260) + 4096;
+      slabBytes + cubBytes + (size_t)3 * n * (sizeof(PassDesc) + sizeof(int) + 260) + 4096;
   TRY(ensure(ctx, ctx->passes, passBytes));
   TRY(ensure_host(ctx, ctx->hPasses, passBytes));
   TRY(ensure_host(ctx, ctx->hState, n * sizeof(CubeletState)));
@@ -1178,7 +1176,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
 
   // ---- descriptors (host side of the upload block) ----
   CubeletDev *hc = reinterpret_cast<CubeletDev *>(H<char>(ctx->hPasses) + slabBytes);
-  long long *hp = reinterpret_cast<long long *>(H<char>(ctx->hPasses) + slabBytes + cubBytes);
   long long groupTotal = 0, encTotal = 0;
   long long quantTotal = 0;
   long long chunk0[2] = {0, 0}, group0[2] = {0, 0}, quant0[2] = {0, 0}, words0[2] = {0, 0},
@@ -1231,7 +1228,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     c.encBase = (int)(encTotal - enc0[h]);
     encTotal += ((long long)pl.nChunks * encF[h] + kEncThreads - 1) / kEncThreads;
     wordsAcc += pl.wordsCap;
-    hp[i] = c.chunkBase;
   }
 
   DevBatch b;
@@ -1257,7 +1253,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.codeLen = P<uint8_t>(ctx->codeLen);
   b.decode = P<int>(ctx->decode);
   b.words = P<uint32_t>(ctx->words);
-  b.chunkPrefix = reinterpret_cast<long long *>(P<char>(ctx->passes) + slabBytes + cubBytes);
   b.chunkCub = P<int>(ctx->chunkCub);
   b.groupCub = P<int>(ctx->groupCub);
   b.quantCub = P<int>(ctx->quantCub);
@@ -1313,7 +1308,6 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       v.logHdr += c0;
       if (v.hostSel) v.hostSel += c0;
       if (h) v.head = nullptr;
-      v.chunkPrefix += c0;
       v.chunkVal += ch;
       v.chunkLen += ch;
       v.chunkEdge += ch;
@@ -1347,7 +1341,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     pass0[h] |= !fused;
   }
   std::vector<GroupLaunch> gl;
-  size_t hoff = slabBytes + cubBytes + prefBytes;
+  size_t hoff = slabBytes + cubBytes;
   size_t gb[2][4];  // per half: group index bounds of the x, y, z phases
   for (int h = 0; h < nh; h++) {
     gb[h][0] = gl.size();

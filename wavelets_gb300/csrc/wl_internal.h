@@ -248,7 +248,6 @@ struct DevBatch {
   uint8_t *codeLen;               // [n][kMaxSymbols]
   int *decode;                    // [n][4*kMaxSymbols]
   uint32_t *words;                // Huffman output
-  long long *chunkPrefix;         // [n+1] chunk prefix (== cub[i].chunkBase)
   int *chunkCub;                  // [totalChunks] cubelet of every chunk
   int *groupCub;                  // [totalGroups] cubelet of every select group
   int *quantCub;                  // [totalQuant] cubelet of every quantize CTA
