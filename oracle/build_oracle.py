@@ -39,11 +39,12 @@ def build_port(verbose=False):
 
 def reference_dir():
     """The reference checkout: $WL_REFERENCE_DIR, else a directory named
-    `reference` beside this repository (None when neither exists; the GPU
-    box has no checkout, and nothing there needs one)."""
+    `reference` beside this repository.  None when neither holds the sources
+    that oracle/ref compiles (no directory, or an empty one): nothing else
+    needs them."""
     d = os.environ.get("WL_REFERENCE_DIR") or os.path.join(
         os.path.dirname(os.path.dirname(HERE)), "reference")
-    return d if os.path.isdir(d) else None
+    return d if os.path.isfile(os.path.join(d, "test_compress_cpu.cc")) else None
 
 
 def build_reference(ref_dir):
