@@ -51,7 +51,6 @@ constexpr int kTileBits = kTileSubs * kSubBits;
 constexpr int kTileWords = kTileSubs * kSubWords;
 constexpr int kLutBits = 12, kLutSize = 1 << kLutBits;
 constexpr int kStepBits = 4, kStep = 1 << kStepBits;  // longer codes, per step
-constexpr int kMaxCode = 60;                 // longest code accepted
 // step tables kept in shared memory: the first ones built belong to the
 // shortest of the long codes (a global read of a step costs the whole warp
 // several hundred cycles, and with 1024 bins most warps have one per token)
@@ -193,6 +192,14 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
     p += (int)(e & 63u);
     n += token_count(e, dupValue);
   }
+  // A malformed token ends its subsequence: the exit is the next one's first
+  // bit, never a bit before it, and nothing is counted.  (The host refuses the
+  // tables that hold such tokens; whatever a table holds, a start lies in its
+  // subsequence or past it and the write pass stays inside the counts.)
+  if (bad) {
+    p = s0 + kSubBits;
+    n = 0;
+  }
   const int x0 = p;           // the speculative exit and counts
   const unsigned n0 = n;
   int start = s0;
@@ -207,10 +214,11 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
     const int ns = tid > 0 ? sm.exits[tid - 1] : start;
     bool changed = false;
     if (active && tid > 0 && ns != start && !bad) {
-      start = ns;
-      int q = ns;
+      bad = ns < s0;
+      start = bad ? s0 : ns;
+      int q = start;
       unsigned m = 0;
-      while (q < lim) {
+      while (q < lim && !bad) {
         const unsigned r = sm.rec[(q - s0) >> 5][tid];
         if (r >> kRecShift == (unsigned)(q & 31)) {  // on the speculative path from here
           m += n0 - (r & ((1u << kRecShift) - 1));
@@ -221,6 +229,10 @@ __device__ void decode_tile(const DecodeCub &c, const DecodeArrays &d, int t, Ti
         if ((e & 63u) == 0) { bad = true; break; }
         q += (int)(e & 63u);
         m += token_count(e, dupValue);
+      }
+      if (bad) {
+        q = s0 + kSubBits;
+        m = 0;
       }
       changed = q != p;
       p = q;
@@ -351,7 +363,8 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__rest
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const DecodeCub c = cubs[d.tileCub[t]];
   const long long tileOff = d.tileOff[t];
-  if (tileOff >= c.n) return;  // padding bits after the last value
+  const int refused = d.flags[kDecodeBad];  // settled by the launches before
+  if (refused || tileOff >= c.n) return;  // padding bits after the last value
   const int tile = t - c.tileBase, dupValue = c.dupValue, bins = c.binCount;
   const TileAt at = stage_words(c, tile, sm.sw);
   stage_lut(c, d, sm.lut);
@@ -413,7 +426,7 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__rest
     const int sym = (int)(e >> 10);
     if (sym != dupValue) {
       if (listed) {
-        list[v++] = o | ((unsigned)min(sym, bins - 1) << kPosBits);
+        if (v < vEnd) list[v++] = o | ((unsigned)min(sym, bins - 1) << kPosBits);
       } else {
         F[o] = __ldg(c.dq + min(sym, bins - 1));
       }
@@ -502,7 +515,7 @@ __global__ void __launch_bounds__(1024) build_lut_kernel(const DecodeCub *__rest
       v = node(k);
     }
     if (v.x != 0) {  // goes on: a step table of its own
-      if (above + dep + kStepBits > kMaxCode) return kSlow | kRun | kBad;
+      if (above + dep + kStepBits > kMaxDecodeCode) return kSlow | kRun | kBad;
       const int slot = atomicAdd(&nSlots, 1);
       if (slot >= c.nSteps) return kSlow | kRun | kBad;
       T[slot * kStep] = (unsigned)k;  // until it is filled

@@ -1896,12 +1896,8 @@ wl_status check_result(wl_ctx *ctx, const wl_result *r, int outType, long long &
     return fail(ctx, WL_EFORMAT, "missing Huffman stream");
   if (r->dup_key >= 0 && (r->dup_value < 0 || r->dup_value >= r->bin_count))
     return fail(ctx, WL_EFORMAT, "zero-run value out of range");
-  for (int i = 0; i < r->n_decode; i += 2) {  // every entry must be a node or a symbol
-    const int a = r->decode[i], b = r->decode[i + 1];
-    if (a == 0 ? (b < 0 || (b >= r->bin_count && b != r->dup_key))
-               : (a < 0 || 2 * a >= r->n_decode || b < 0 || 2 * b >= r->n_decode))
-      return fail(ctx, WL_EFORMAT, "corrupt Huffman decode table");
-  }
+  if (!decode_table_ok(r->decode, r->n_decode, r->bin_count, r->dup_key))
+    return fail(ctx, WL_EFORMAT, "corrupt Huffman decode table");
   if (r->quant_alg == WL_LLOYD && (!r->values || r->n_values != r->bin_count))
     return fail(ctx, WL_EFORMAT, "codebook values missing");
   return WL_OK;

@@ -467,6 +467,9 @@ struct DecodeBatch {
   int n, tiles;           // streams, tiles in all
   int maxTable;
 };
+constexpr int kMaxDecodeCode = 60;  // longest code decoded (with its length bits 63)
+// a table that the decoder takes (decode_table.cpp)
+bool decode_table_ok(const int *t, int n, int binCount, int dupKey);
 long long decode_subs(long long nWords);
 int decode_tiles(long long nWords);
 int decode_lut_size();
