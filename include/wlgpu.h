@@ -147,7 +147,9 @@ wl_status wl_decompress_cubelet(wl_ctx *ctx, const wl_result *in, int out_dtype,
  * transform in concurrent launch groups).  out_dtypes: per cubelet (NULL =
  * each one's original type); outs[i]: original_size elements of that type,
  * all host or all device memory (outs_on_device).  Results are those of
- * wl_decompress_cubelet on each. */
+ * wl_decompress_cubelet on each.  A malformed or short stream is refused with
+ * WL_EFORMAT and leaves every output as it was (also in
+ * wl_decompress_cubelet). */
 wl_status wl_decompress_batch(wl_ctx *ctx, const wl_result *in, int n, const int *out_dtypes,
                               void *const *outs, int outs_on_device);
 

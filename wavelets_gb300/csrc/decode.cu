@@ -363,7 +363,10 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const DecodeCub *__rest
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const DecodeCub c = cubs[d.tileCub[t]];
   const long long tileOff = d.tileOff[t];
-  const int refused = d.flags[kDecodeBad];  // settled by the launches before
+  // the launches before settled the flags; the host looks at them before it
+  // lets anything reach the outputs
+  const int refused = d.flags[kDecodeBad];
+  if (t == 0 && tid < kDecodeFlags) d.hostFlags[tid] = d.flags[tid];
   if (refused || tileOff >= c.n) return;  // padding bits after the last value
   const int tile = t - c.tileBase, dupValue = c.dupValue, bins = c.binCount;
   const TileAt at = stage_words(c, tile, sm.sw);

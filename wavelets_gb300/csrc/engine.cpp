@@ -333,6 +333,7 @@ struct wl_ctx {
   long long graphStats[4] = {0, 0, 0, 0};  // direct runs, captures, replays, capture failures
   std::string graphErr;
   cudaEvent_t ev[7] = {};
+  cudaEvent_t decodedEv = nullptr;  // a decompression's streams are decoded
   // side streams for the independent launch groups of one transform phase
   static constexpr int kSide = 3;
   cudaStream_t side[kSide] = {};
@@ -1842,9 +1843,9 @@ wl_status stage_inverse_phases(wl_ctx *ctx, PassGroups ph[3], InversePhases &ip)
   return WL_OK;
 }
 
-// Launch them in order; the groups of a phase run concurrently.
-wl_status launch_inverse_phases(wl_ctx *ctx, const InversePhases &ip) {
-  for (int k = 0; k < 3; k++) TRY(launch_phase(ctx, ip.gl, ip.bound[k], ip.bound[k + 1]));
+// Launch phases [a, b) in order; the groups of a phase run concurrently.
+wl_status launch_inverse_phases(wl_ctx *ctx, const InversePhases &ip, int a, int b) {
+  for (int k = a; k < b; k++) TRY(launch_phase(ctx, ip.gl, ip.bound[k], ip.bound[k + 1]));
   return WL_OK;
 }
 
@@ -1861,7 +1862,7 @@ wl_status inverse_impl(wl_ctx *ctx, const int size[3], const int steps[3], int w
                  P<float>(ctx->coef2), dst, ph);
   InversePhases ip;
   TRY(stage_inverse_phases(ctx, ph, ip));
-  TRY(launch_inverse_phases(ctx, ip));
+  TRY(launch_inverse_phases(ctx, ip, 0, 3));
   if (!outOnDevice) CU(cudaMemcpyAsync(out, dst, outBytes, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
   return WL_OK;
@@ -2172,9 +2173,11 @@ wl_status optimize_impl(wl_ctx *ctx, const void *data, const int size[3], int on
 // records, decode tables and dequantization tables; every stream decoded by
 // one set of launches straight to the dequantized values; the inverse
 // transform as three phases of concurrent launch groups; the outputs copied
-// back per cubelet.  The host waits once, at the end, and looks at the
-// decoder's flags then: a malformed stream is refused, and a batch whose
-// tiles the two checks did not settle is repaired and written again.
+// back per cubelet.  The host looks at the decoder's flags before it launches
+// the last pass, the one that writes the outputs (the passes before it run
+// meanwhile): a malformed stream is refused with every output untouched, and a
+// batch whose tiles the two checks did not settle is repaired and written
+// again.
 wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const int *outTypes,
                                 void *const *outs, int outOnDevice) {
   CU(cudaSetDevice(ctx->device));
@@ -2330,32 +2333,28 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
   da.stepCount = reinterpret_cast<int *>(ws + scntAt);
   da.flags = reinterpret_cast<int *>(ws + flagAt);
   int *hf = H<int>(ctx->hFlags);
+  da.hostFlags = hf;
   ctx->launches = 0;
   auto fill = [&] {
     if (!nFill) return;
     launch_fill_batch(reinterpret_cast<const FillItem *>(du + fillAt), nFill, fillBlocks, s);
     ctx->launches++;
   };
-  // the values on, and the flags and outputs back
-  auto finish = [&]() -> wl_status {
+  // The decoder's flags, which the write pass leaves in hf, with the passes
+  // before the last queued meanwhile.  Only the last pass touches the outputs:
+  // a refused call leaves them as they were.
+  auto decoded = [&]() -> wl_status {
     CU(cudaGetLastError());
-    TRY(launch_inverse_phases(ctx, ip));
-    CU(cudaMemcpyAsync(hf, da.flags, kDecodeFlags * 4, cudaMemcpyDeviceToHost, s));
-    if (!outOnDevice)
-      for (int i = 0; i < n; i++) {
-        const wl_result *r = rs + i;
-        const size_t bytes = (size_t)r->original_size[0] * r->original_size[1] *
-                             r->original_size[2] * dtype_size(ot[i]);
-        CU(cudaMemcpyAsync(outs[i], P<char>(ctx->outbuf) + outOff[i], bytes,
-                           cudaMemcpyDeviceToHost, s));
-      }
-    CU(cudaStreamSynchronize(s));
+    CU(cudaEventRecord(ctx->decodedEv, s));
+    TRY(launch_inverse_phases(ctx, ip, 0, 2));
+    if (nStreams) CU(cudaEventSynchronize(ctx->decodedEv));
     return WL_OK;
   };
+  std::fill(hf, hf + kDecodeFlags, 0);
   CU(cudaMemsetAsync(da.flags, 0, kDecodeFlags * 4, s));
   fill();
   if (nStreams) ctx->launches += launch_decode(dc, db, da, s);
-  TRY(finish());
+  TRY(decoded());
   if (hf[kDecodeAgain] && !hf[kDecodeBad]) {
     // a chain of tiles took another entry: each check settles at least the
     // first wrong one, so they end within the longest stream's tile count
@@ -2372,12 +2371,24 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
       CU(cudaMemsetAsync(da.flags, 0, kDecodeFlags * 4, s));
       fill();
       ctx->launches += launch_decode_write(dc, db, da, s);
-      TRY(finish());
+      TRY(decoded());
     }
   }
-  if (hf[kDecodeBad] || hf[kDecodeShort])
+  if (hf[kDecodeBad] || hf[kDecodeShort]) {
+    CU(cudaStreamSynchronize(s));
     return fail(ctx, WL_EFORMAT, n == 1 ? "corrupt Huffman stream"
                                         : "corrupt Huffman stream in the batch");
+  }
+  TRY(launch_inverse_phases(ctx, ip, 2, 3));
+  if (!outOnDevice)
+    for (int i = 0; i < n; i++) {
+      const wl_result *r = rs + i;
+      const size_t bytes = (size_t)r->original_size[0] * r->original_size[1] *
+                           r->original_size[2] * dtype_size(ot[i]);
+      CU(cudaMemcpyAsync(outs[i], P<char>(ctx->outbuf) + outOff[i], bytes,
+                         cudaMemcpyDeviceToHost, s));
+    }
+  CU(cudaStreamSynchronize(s));
   return WL_OK;
 }
 
@@ -2505,6 +2516,7 @@ wl_status wl_init(int device, wl_ctx **out) {
     return WL_ECUDA;
   }
   for (auto &e : ctx->ev) cudaEventCreate(&e);
+  cudaEventCreateWithFlags(&ctx->decodedEv, cudaEventDisableTiming);
   bool sideOk = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming) == cudaSuccess;
   for (int k = 0; k < wl_ctx::kSide && sideOk; k++)
     sideOk = cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking) == cudaSuccess &&
@@ -2550,6 +2562,7 @@ void wl_destroy(wl_ctx *ctx) {
                     &ctx->hFlags};
   for (HostBuf *h : hbs) if (h->p) cudaFreeHost(h->p);
   for (auto &e : ctx->ev) if (e) cudaEventDestroy(e);
+  if (ctx->decodedEv) cudaEventDestroy(ctx->decodedEv);
   for (auto &e : ctx->pev) if (e) cudaEventDestroy(e);
   for (int k = 0; k < wl_ctx::kSide; k++) {
     if (ctx->side[k]) cudaStreamDestroy(ctx->side[k]);

@@ -456,6 +456,7 @@ struct DecodeArrays {
   unsigned *tileCount;
   long long *tileOff;
   int *flags;             // kDecodeFlags counters, zero before the first launch
+  int *hostFlags;         // page-locked copy of them, the write pass's
 };
 enum {
   kDecodeFirst, kDecodeAgain,  // tiles decoded again by the first / second check
