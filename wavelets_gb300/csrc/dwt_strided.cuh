@@ -367,22 +367,63 @@ __device__ __forceinline__ void fwd_from(const f2 (&v)[2 * M], int S, const floa
   out.template put_run<M>(M * at.seg, e);
 }
 
+// v / s of both, rounded correctly (rarely called: not inline)
+__device__ __noinline__ f2 divide(f2 v, float s) {
+  float a, b;
+  unpack(v, a, b);
+  return pack(__fdiv_rn(a, s), __fdiv_rn(b, s));
+}
+
+// neither zero nor within 2^-97 .. 2^125
+__device__ __forceinline__ bool out_of_range(float v) {
+  constexpr unsigned kLow = (127u - 97u) << 23, kSpan = (97u + 125u) << 23;
+  return (v != 0.f) & ((__float_as_uint(v) & 0x7fffffffu) - kLow > kSpan);
+}
+
 // The deferred lifting scale of level t undone, as the kernel that had the
-// pass before did: by its reciprocal, or (divide) by a correctly rounded
-// division -- the quotient by the reciprocal with one correction step, which
-// gives it for every scale of up to kMaxLevels levels and every significand
-// (checked exhaustively); an infinite quotient stays.
+// pass before did: by its reciprocal, or (divides) by a correctly rounded
+// division.  That is the quotient by the reciprocal with one correction step,
+// which gives it for every scale of up to kMaxLevels levels (1/K .. K^14, so
+// at most 2^3) and every significand while the quotient lies in 2^-100 ..
+// 2^126, where the remainder is a float (tests/test_unscale.py); a zero keeps
+// its first quotient's sign, and a run with any other value is divided.
 template <bool FULL> struct Unscale {
   const float *scale, *rscale;
-  bool divide;
-  __device__ __forceinline__ f2 operator()(f2 v, int t) const {
+  bool divides;
+  template <int M> __device__ __forceinline__ void operator()(f2 (&v)[M], int t) const {
     const f2 r = pack(rscale[t]);
-    const f2 q = mul2(v, r);
-    if (!FULL || !divide) return q;
-    float qa, qb, ca, cb;
-    unpack(q, qa, qb);
-    unpack(fma2(fma2(q, pack(-scale[t]), v), r, q), ca, cb);
-    return pack(isinf(qa) ? qa : ca, isinf(qb) ? qb : cb);
+    if (!FULL || !divides) {
+#pragma unroll
+      for (int k = 0; k < M; k++) v[k] = mul2(v[k], r);
+      return;
+    }
+    bool other = false;
+#pragma unroll
+    for (int k = 0; k < M; k++) {
+      float a, b;
+      unpack(v[k], a, b);
+      other |= out_of_range(a) | out_of_range(b);
+    }
+    if (other) {
+#pragma unroll
+      for (int k = 0; k < M; k++) v[k] = divide(v[k], scale[t]);
+      return;
+    }
+    const f2 neg = pack(-scale[t]);
+#pragma unroll
+    for (int k = 0; k < M; k++) {
+      const f2 q = mul2(v[k], r);
+      float a, b, qa, qb, ca, cb;
+      unpack(v[k], a, b);
+      unpack(q, qa, qb);
+      unpack(fma2(fma2(q, neg, v[k]), r, q), ca, cb);
+      v[k] = pack(a == 0.f ? qa : ca, b == 0.f ? qb : cb);
+    }
+  }
+  __device__ __forceinline__ f2 operator()(f2 v, int t) const {
+    f2 x[1] = {v};
+    (*this)(x, t);
+    return x[0];
   }
 };
 
@@ -430,11 +471,9 @@ __device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL
   }
   if (!deeper) {
     in.template get_run<M>(M * at.seg, e);
-#pragma unroll
-    for (int k = 0; k < M; k++) e[k] = un(e[k], LEV + 1);
+    un(e, LEV + 1);
   }
-#pragma unroll
-  for (int k = 0; k < M; k++) o[k] = un(o[k], LEV);
+  un(o, LEV);
   inv_level<M, G, HAAR>(e, o, at);
 #pragma unroll
   for (int k = 0; k < M; k++) {
