@@ -407,10 +407,11 @@ void wl_tune_reset(void);
 wl_status wl_set_graph_mode(wl_ctx *ctx, int mode);
 
 /* Bit-packer slices per 4096-element chunk (no reference counterpart): the
- * Huffman tokens of a chunk are packed by `slices` lanes (1, 2, 4, 8, 16 or
- * 32) that each take a contiguous share.  0 (default): the smallest count
- * that gives the launch at least 16 warps per SM.  The packed bits do not
- * depend on it. */
+ * values of a chunk are packed by `slices` lanes (1, 2, 4, 8, 16 or 32) that
+ * each take a contiguous share.  0 (default): chunks of 512 to 4096 elements,
+ * by the size of the call, and 16 lanes per 4096 elements, more in calls that
+ * would have fewer than 2^18 lanes that way (at most 32 a chunk).  The packed
+ * bits do not depend on it. */
 wl_status wl_set_encode_slices(wl_ctx *ctx, int slices);
 wl_status wl_graph_stats(const wl_ctx *ctx, long long out[4]);
 const char *wl_graph_error(const wl_ctx *ctx);

@@ -345,7 +345,7 @@ struct wl_ctx {
   cudaStream_t side2[kSide] = {};  // the second half's side streams
   cudaEvent_t fork2 = nullptr, join2[kSide] = {};
   int splitMode = 1;  // 1: split large batches into two staggered halves
-  int encSlices = 0;  // bit-packer slices per chunk; 0: from the batch size
+  int encSlices = 0;  // bit-packer slices per 4096-element chunk; 0: chunks and slices from the batch size
   float timings[6] = {0, 0, 0, 0, 0, 0};
   bool profiling = false;
   cudaEvent_t pev[10] = {};
@@ -1037,7 +1037,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     if (pl.p.quant_alg == WL_LLOYD) anyLloyd = true;
   }
 
-  const int lgChunk = token_chunk_lg(coefTotal);
+  // (a forced slice count is per 4096 elements)
+  const int lgChunk = ctx->encSlices ? kMaxLgChunk : token_chunk_lg(coefTotal);
   for (Plan &pl : plans) {
     pl.chunkBase = chunkTotal;
     pl.nChunks = (int)((pl.n + (1LL << lgChunk) - 1) >> lgChunk);
@@ -1192,8 +1193,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
       tokChunks[half_of(i)] += plans[i].nChunks;
     }
     for (int h = 0; h < nh; h++) {
-      encF[h] = ctx->encSlices ? std::max(1, ctx->encSlices >> (kMaxLgChunk - lgChunk))
-                               : enc_slices(tokChunks[h], lgChunk);
+      encF[h] = ctx->encSlices ? ctx->encSlices : enc_slices(tokChunks[h], lgChunk);
       group[h] = sel_group(selChunks[h]);
     }
   }

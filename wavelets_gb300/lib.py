@@ -794,7 +794,7 @@ class Context:
 
     def set_encode_slices(self, slices: int):
         """Bit-packer lanes per 4096-element chunk (1, 2, 4, 8, 16, 32);
-        0 = chosen from the batch size.  The output does not depend on it."""
+        0 = chunks and lanes chosen from the batch size.  The output does not depend on it."""
         self._check(self.lib.wl_set_encode_slices(self.h, int(slices)))
 
     def set_graph_mode(self, mode: int):
