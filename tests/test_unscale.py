@@ -29,7 +29,9 @@ def quotient(v, s):
     s = np.full_like(v, s)
     r = np.float32(1) / s
     q = v * r
-    return fma(fma(q, -s, v), r, q)
+    # |s| q - v, or |s| q + v with a negative scale, times -|r|
+    rest = fma(q, np.abs(s), np.where(s > 0, -v, v))
+    return fma(rest, -np.abs(r), q)
 
 
 @pytest.mark.parametrize("s", SCALES)
@@ -53,9 +55,8 @@ def test_ends_of_the_range(e):
         assert np.array_equal(quotient(v[keep], np.float32(s)), want[keep])
 
 
-def test_zero_needs_its_own_sign():
-    """Minus zero by a positive scale: the correction step loses the sign, which
-    is why the kernel keeps the first quotient of a zero."""
-    s, v = np.float32(K), np.array([-0.0], np.float32)
-    assert not np.signbit(quotient(v, s))[0] and np.signbit(v / s)[0]
-    assert np.signbit(v * (np.float32(1) / s))[0]
+@pytest.mark.parametrize("v", [0.0, -0.0])
+def test_zeros_keep_their_sign(v):
+    v = np.array([v], np.float32)
+    for s in SCALES:
+        assert np.signbit(quotient(v, np.float32(s)))[0] == np.signbit(v / np.float32(s))[0]

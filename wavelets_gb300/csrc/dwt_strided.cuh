@@ -374,55 +374,66 @@ __device__ __noinline__ f2 divide(f2 v, float s) {
   return pack(__fdiv_rn(a, s), __fdiv_rn(b, s));
 }
 
-// neither zero nor within 2^-97 .. 2^125
-__device__ __forceinline__ bool out_of_range(float v) {
-  constexpr unsigned kLow = (127u - 97u) << 23, kSpan = (97u + 125u) << 23;
-  return (v != 0.f) & ((__float_as_uint(v) & 0x7fffffffu) - kLow > kSpan);
-}
+// Magnitudes of a run: the smallest but zero, the largest (NaN above all).
+struct Range {
+  unsigned low = ~0u;
+  float high = 0.f;
+  __device__ __forceinline__ void add(float v) {
+    low = min(low, (__float_as_uint(v) << 1) - 1u);  // a zero becomes the largest
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(v)));
+  }
+  // within 2^-97 .. 2^125 or zero
+  __device__ __forceinline__ bool ok() const {
+    return low >= ((127u - 97u) << 24) - 1u && high <= 0x1p125f;
+  }
+};
 
 // The deferred lifting scale of level t undone, as the kernel that had the
 // pass before did: by its reciprocal, or (divides) by a correctly rounded
 // division.  That is the quotient by the reciprocal with one correction step,
 // which gives it for every scale of up to kMaxLevels levels (1/K .. K^14, so
 // at most 2^3) and every significand while the quotient lies in 2^-100 ..
-// 2^126, where the remainder is a float (tests/test_unscale.py); a zero keeps
-// its first quotient's sign, and a run with any other value is divided.
-template <bool FULL> struct Unscale {
+// 2^126, where the remainder is a float (tests/test_unscale.py); a run with
+// any other value but zero is divided.  The remainder's sign is chosen so that
+// a zero keeps its first quotient's: the step adds minus zero.  LOW: the
+// low-pass band, whose scale is positive; the details' are negative.  The
+// scales of the Haar wavelet are 1.
+template <bool HAAR, bool FULL> struct Unscale {
   const float *scale, *rscale;
   bool divides;
-  template <int M> __device__ __forceinline__ void operator()(f2 (&v)[M], int t) const {
+  template <bool LOW, int M> __device__ __forceinline__ void run(f2 (&v)[M], int t) const {
+    if (HAAR) return;
     const f2 r = pack(rscale[t]);
     if (!FULL || !divides) {
 #pragma unroll
       for (int k = 0; k < M; k++) v[k] = mul2(v[k], r);
       return;
     }
-    bool other = false;
+    Range range;
 #pragma unroll
     for (int k = 0; k < M; k++) {
       float a, b;
       unpack(v[k], a, b);
-      other |= out_of_range(a) | out_of_range(b);
+      range.add(a);
+      range.add(b);
     }
-    if (other) {
+    if (!range.ok()) {
 #pragma unroll
       for (int k = 0; k < M; k++) v[k] = divide(v[k], scale[t]);
       return;
     }
-    const f2 neg = pack(-scale[t]);
+    // |s| q - v or (s < 0) |s| q + v, times -|1 / s|
+    const f2 s = pack(LOW ? scale[t] : -scale[t]), rn = pack(LOW ? -rscale[t] : rscale[t]);
+    const f2 minus = pack(-1.0f);
 #pragma unroll
     for (int k = 0; k < M; k++) {
       const f2 q = mul2(v[k], r);
-      float a, b, qa, qb, ca, cb;
-      unpack(v[k], a, b);
-      unpack(q, qa, qb);
-      unpack(fma2(fma2(q, neg, v[k]), r, q), ca, cb);
-      v[k] = pack(a == 0.f ? qa : ca, b == 0.f ? qb : cb);
+      v[k] = fma2(fma2(q, s, LOW ? mul2(v[k], minus) : v[k]), rn, q);
     }
   }
-  __device__ __forceinline__ f2 operator()(f2 v, int t) const {
+  template <bool LOW> __device__ __forceinline__ f2 one(f2 v, int t) const {
     f2 x[1] = {v};
-    (*this)(x, t);
+    run<LOW>(x, t);
     return x[0];
   }
 };
@@ -430,7 +441,7 @@ template <bool FULL> struct Unscale {
 // The 2 M values v[] of level LEV's input from the bands of levels LEV ..
 // S-1.
 template <int LEV, int M, int G, bool HAAR, bool FULL, typename In>
-__device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL> &un,
+__device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<HAAR, FULL> &un,
                                        const Along<G> &at, const In &in) {
   const int H = M * at.lanes;
   f2 e[M], o[M];
@@ -450,10 +461,10 @@ __device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL
 #pragma unroll
       for (int k = 0; k < kDeep; k++) {
         const int n = G >> (k + 1);
-        dg[k] = LEV + 1 + k < S && at.seg < n ? un(in.get(n + at.seg), LEV + 1 + k) : 0ull;
+        dg[k] = LEV + 1 + k < S && at.seg < n ? un.template one<false>(in.get(n + at.seg), LEV + 1 + k) : 0ull;
       }
       const int n0 = G >> (S - LEV - 1);
-      f2 s = at.seg < n0 ? un(in.get(at.seg), S) : 0ull;
+      f2 s = at.seg < n0 ? un.template one<true>(in.get(at.seg), S) : 0ull;
       Along<G> now = at;
 #pragma unroll
       for (int k = kDeep - 1; k >= 0; k--) {
@@ -471,9 +482,9 @@ __device__ __forceinline__ void inv_to(f2 (&v)[2 * M], int S, const Unscale<FULL
   }
   if (!deeper) {
     in.template get_run<M>(M * at.seg, e);
-    un(e, LEV + 1);
+    un.template run<true>(e, LEV + 1);  // LEV + 1 is S here
   }
-  un(o, LEV);
+  un.template run<false>(o, LEV);
   inv_level<M, G, HAAR>(e, o, at);
 #pragma unroll
   for (int k = 0; k < M; k++) {
@@ -580,7 +591,7 @@ __device__ __forceinline__ void run_rows(const PassDesc &d, int tile, const floa
   if constexpr (PASS == kStrided || PASS == kSource) {
     fwd_from<0, K / 2, G, HAAR, FULL>(v, d.steps, scale, at, out);
   } else {
-    inv_to<0, K / 2, G, HAAR, FULL>(v, d.steps, Unscale<FULL>{scale, rscale, d.exact != 0}, at,
+    inv_to<0, K / 2, G, HAAR, FULL>(v, d.steps, Unscale<HAAR, FULL>{scale, rscale, d.exact != 0}, at,
                                      in);
     if constexpr (PASS == kStridedInv) {
 #pragma unroll
@@ -655,7 +666,7 @@ __device__ __forceinline__ void run_z(const PassDesc &d, int pair0, const float 
     __syncwarp();  // the row's lanes have read it
     fwd_from<0, K / 2, 0, HAAR, false>(v, d.steps, scale, at, out);
   } else {
-    inv_to<0, K / 2, 0, HAAR, true>(v, d.steps, Unscale<true>{scale, rscale, d.exact != 0}, at,
+    inv_to<0, K / 2, 0, HAAR, true>(v, d.steps, Unscale<HAAR, true>{scale, rscale, d.exact != 0}, at,
                                     in);
     __syncwarp();
     out.template put_run<K>(K * at.seg, v);
