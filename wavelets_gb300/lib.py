@@ -240,6 +240,24 @@ def make_params(p: Optional[P.Params] = None) -> WlParams:
     return w
 
 
+class _ParamsBytes:
+    """make_params as bytes, made once for items in a row with the same object
+    and the same values (items of one call often share their parameters, and
+    an object may change between items)."""
+
+    def __init__(self):
+        self.p, self.values, self.made = self, None, b""
+
+    def __call__(self, p: Optional[P.Params]) -> bytes:
+        if p is self.p and (p is None or vars(p) == self.values):
+            return self.made
+        self.made = bytes(make_params(p))
+        # values that can change in place are not compared
+        fixed = p is None or (type(p) is P.Params and type(p.steps) is tuple)
+        self.p, self.values = (p if fixed else self), (dict(vars(p)) if fixed and p else None)
+        return self.made
+
+
 def _addr(a: np.ndarray) -> int:
     return a.__array_interface__["data"][0]
 
@@ -552,7 +570,7 @@ class Context:
                       raw: bool = False) -> PreparedBatch:
         """Describe a batch once (see compress_batch for items)."""
         n = len(items)
-        keep, rows, made = [], [], {}
+        keep, rows, params_bytes = [], [], _ParamsBytes()
         for it in items:
             pitch = (0, 0)
             if raw or on_device:
@@ -568,10 +586,7 @@ class Context:
                 keep.append(a)
                 ptr, dt, size = a.ctypes.data, NP_TO_WL[a.dtype], _size_of(a)
             prm = prm if prm is not None else params
-            p = made.get(id(prm))  # items of one call often share their Params
-            if p is None:
-                p = made[id(prm)] = bytes(make_params(prm))
-            rows.append((ptr, dt, tuple(size), p, pitch[0], pitch[1]))
+            rows.append((ptr, dt, tuple(size), params_bytes(prm), pitch[0], pitch[1]))
         cubs = (WlCubelet * n).from_buffer(np.array(rows, _CUBELET_DT)) if n else (WlCubelet * 0)()
         return PreparedBatch(cubs, n, on_device, keep)
 
