@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import itertools
 import os
 from typing import List, Optional, Sequence
 
@@ -420,6 +421,39 @@ _CUBELET_DT = np.dtype({
     "itemsize": ctypes.sizeof(WlCubelet)})
 
 
+def _ints(*columns) -> bool:
+    """Whether every value of every column is a plain int."""
+    return all(set(map(type, c)) <= {int} for c in columns)
+
+
+def _cubelet_array(rows):
+    """The WlCubelet array of (data, dtype, size, params bytes, row pitch,
+    slice pitch) rows.  Plain integers go in column by column; anything else
+    one by one, which takes and refuses what the ctypes fields do (pointer
+    objects and None, no fractions, no sizes of another length)."""
+    n = len(rows)
+    if not n:
+        return (WlCubelet * 0)()
+    data, dtypes, sizes, prms, row, sl = zip(*rows)
+    if (_ints(data, dtypes, row, sl, itertools.chain.from_iterable(sizes))
+            and set(map(len, sizes)) == {3}):
+        try:
+            a = np.empty(n, _CUBELET_DT)
+            a["data"], a["dtype"], a["size"] = np.array(data, np.uint64), dtypes, sizes
+            a["params"] = np.frombuffer(b"".join(prms), _CUBELET_DT["params"])
+            a["row_pitch"], a["slice_pitch"] = row, sl
+            return (WlCubelet * n).from_buffer(a)
+        except OverflowError:
+            pass
+    cubs = (WlCubelet * n)()
+    for c, (ptr, dt, size, prm, row_pitch, slice_pitch) in zip(cubs, rows):
+        c.data, c.dtype = ptr, dt
+        c.size[:] = size
+        c.params = WlParams.from_buffer_copy(prm)
+        c.row_pitch, c.slice_pitch = row_pitch, slice_pitch
+    return cubs
+
+
 def _result_dtype_cached():
     global _RESULT_DT
     if _RESULT_DT is None:
@@ -587,8 +621,7 @@ class Context:
                 ptr, dt, size = a.ctypes.data, NP_TO_WL[a.dtype], _size_of(a)
             prm = prm if prm is not None else params
             rows.append((ptr, dt, tuple(size), params_bytes(prm), pitch[0], pitch[1]))
-        cubs = (WlCubelet * n).from_buffer(np.array(rows, _CUBELET_DT)) if n else (WlCubelet * 0)()
-        return PreparedBatch(cubs, n, on_device, keep)
+        return PreparedBatch(_cubelet_array(rows), n, on_device, keep)
 
     def compress_prepared(self, pb: PreparedBatch, lazy: bool = False):
         """Compress a prepared batch; lazy returns a ResultBatch."""
