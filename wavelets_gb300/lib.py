@@ -11,8 +11,8 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
-import itertools
 import os
+import struct
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -411,40 +411,38 @@ def _result_dtype():
 
 
 _RESULT_DT = None
-# numpy mirror of WlCubelet (the parameters as their bytes)
-_CUBELET_DT = np.dtype({
-    "names": ["data", "dtype", "size", "params", "row_pitch", "slice_pitch"],
-    "formats": [np.uint64, np.int32, (np.int32, (3,)), np.dtype((np.void, ctypes.sizeof(WlParams))),
-                np.int64, np.int64],
-    "offsets": [getattr(WlCubelet, k).offset for k in ("data", "dtype", "size", "params",
-                                                       "row_pitch", "slice_pitch")],
-    "itemsize": ctypes.sizeof(WlCubelet)})
+def _packer(t) -> struct.Struct:
+    """The layout of a ctypes structure as a struct format: a pointer is an
+    address, an array its elements, a structure its bytes."""
+    codes = {ctypes.c_int: "i", ctypes.c_float: "f", ctypes.c_longlong: "q"}
+    fmt, end = "=", 0
+    for name, ct in t._fields_:
+        f = getattr(t, name)
+        if issubclass(ct, ctypes.Array):
+            code = codes[ct._type_] * ct._length_
+        elif issubclass(ct, ctypes.Structure):
+            code = f"{ctypes.sizeof(ct)}s"
+        else:
+            code = codes.get(ct, "Q")
+        fmt += f"{f.offset - end}x{code}"
+        end = f.offset + f.size
+    return struct.Struct(fmt + f"{ctypes.sizeof(t) - end}x")
 
 
-def _ints(*columns) -> bool:
-    """Whether every value of every column is a plain int."""
-    return all(set(map(type, c)) <= {int} for c in columns)
+_PACK_CUBELET = _packer(WlCubelet).pack
 
 
 def _cubelet_array(rows):
     """The WlCubelet array of (data, dtype, size, params bytes, row pitch,
-    slice pitch) rows.  Plain integers go in column by column; anything else
-    one by one, which takes and refuses what the ctypes fields do (pointer
-    objects and None, no fractions, no sizes of another length)."""
+    slice pitch) rows.  Integers are packed at once; anything else goes in
+    field by field, which takes and refuses what ctypes does (pointer objects
+    and None, no fractions, no sizes of another length)."""
     n = len(rows)
-    if not n:
-        return (WlCubelet * 0)()
-    data, dtypes, sizes, prms, row, sl = zip(*rows)
-    if (_ints(data, dtypes, row, sl, itertools.chain.from_iterable(sizes))
-            and set(map(len, sizes)) == {3}):
-        try:
-            a = np.empty(n, _CUBELET_DT)
-            a["data"], a["dtype"], a["size"] = np.array(data, np.uint64), dtypes, sizes
-            a["params"] = np.frombuffer(b"".join(prms), _CUBELET_DT["params"])
-            a["row_pitch"], a["slice_pitch"] = row, sl
-            return (WlCubelet * n).from_buffer(a)
-        except OverflowError:
-            pass
+    try:
+        return (WlCubelet * n).from_buffer(bytearray().join(
+            [_PACK_CUBELET(d, t, x, y, z, p, r, s) for d, t, (x, y, z), p, r, s in rows]))
+    except (struct.error, OverflowError, TypeError, ValueError):
+        pass
     cubs = (WlCubelet * n)()
     for c, (ptr, dt, size, prm, row_pitch, slice_pitch) in zip(cubs, rows):
         c.data, c.dtype = ptr, dt
