@@ -88,3 +88,63 @@ def test_other_values_are_refused(ctx, item):
     for items in ([item], [good, item, good]):
         with pytest.raises((TypeError, ValueError)):
             ctx.prepare_batch(items, raw=True)
+
+
+def compressed(**over):
+    f = dict(size=(4, 5, 6), original_size=(6, 4, 5), original_dtype=lib.WL_F32, steps=(1, 2, 3),
+             wavelet=P.CDF97, quant_alg=P.LLOYD, bin_count=9, threshold_fraction=0.5,
+             threshold_value=0.25, max_value=3.5, min_coef=-2.5, max_coef=3.25, zero_bin=4,
+             dup_key=9, dup_value=4, longest_code=7, words=np.arange(11, dtype=np.uint32),
+             decode=np.arange(34, dtype=np.int32), boundaries=np.arange(8, dtype=np.float32),
+             values=np.arange(9, dtype=np.float32), transform_2d=True)
+    return lib.Compressed(**{**f, **over})
+
+
+def fields(r):
+    """A WlResult's values, its arrays as lists."""
+    out = {}
+    for name, ct in lib.WlResult._fields_:
+        v = getattr(r, name)
+        n = {"words": r.n_words, "decode": r.n_decode, "boundaries": r.n_boundaries,
+             "values": r.n_values}.get(name)
+        out[name] = v[:n] if n is not None else list(v) if hasattr(v, "__len__") else v
+    return out
+
+
+def test_result_records(ctx):
+    c = compressed()
+    got = fields(c.to_struct())
+    assert got.pop("owner") is None
+    for name, v in got.items():
+        if name.startswith("n_"):
+            assert v == getattr(c, {"n_words": "words", "n_decode": "decode",
+                                    "n_boundaries": "boundaries", "n_values": "values"}[name]).size
+        elif isinstance(v, list):
+            assert v == [x for x in getattr(c, name)]
+        else:
+            assert v == getattr(c, name)
+    rs = ctx.prepare_decompress([c, compressed(dup_key=-1, size=[7, 8, 9]), c])["rs"]
+    assert fields(rs[0]) == fields(rs[2]) == fields(c.to_struct())
+    assert rs[1].dup_key == -1 and list(rs[1].size) == [7, 8, 9]
+
+
+@pytest.mark.parametrize("over", [dict(size=(4.5, 5, 6)), dict(size=(4, 5)), dict(steps=(1,)),
+                                  dict(bin_count=8.5), dict(dup_key=None), dict(wavelet="2"),
+                                  dict(threshold_value=None), dict(original_size=(1, 2, 3, 4))])
+def test_result_values_refused(ctx, over):
+    with pytest.raises((TypeError, ValueError)):
+        compressed(**over).to_struct()
+
+
+def test_converted_arrays_stay_alive(ctx):
+    """Arrays of other types are converted; the copies live as long as the
+    description, also of a result described twice."""
+    c = compressed(words=list(range(11)), decode=np.arange(34.0), values=np.arange(18)[::2])
+    prep = ctx.prepare_decompress([c, c], device_outs=[0, 0])
+    c.to_struct()
+    live = {a.__array_interface__["data"][0] for arrays in prep["keep"] for a in arrays}
+    for r in prep["rs"]:
+        for name in ("words", "decode", "boundaries", "values"):
+            assert ctypes.cast(getattr(r, name), ctypes.c_void_p).value in live
+        assert r.words[:11] == list(range(11)) and r.decode[:34] == list(range(34))
+        assert r.values[:9] == [2.0 * k for k in range(9)]

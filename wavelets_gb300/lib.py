@@ -305,23 +305,23 @@ class Compressed:
                    arr(r.values, r.n_values, np.float32), bool(r.transform_2d))
 
     def _record(self):
-        """The WlResult field values (in _RESULT_DT order) over this object's
-        arrays, which are kept as self._keep."""
-        self._keep = keep = (np.ascontiguousarray(self.words, np.uint32),
+        """The WlResult field values over this object's arrays, and those
+        arrays."""
+        keep = w, d, b, v = (np.ascontiguousarray(self.words, np.uint32),
                              np.ascontiguousarray(self.decode, np.int32),
                              np.ascontiguousarray(self.boundaries, np.float32),
                              np.ascontiguousarray(self.values, np.float32))
-        w, d, b, v = keep
-        return (tuple(self.size), tuple(self.original_size), self.original_dtype,
-                tuple(self.steps), self.wavelet, self.quant_alg, self.bin_count,
+        return (self.size, self.original_size, self.original_dtype,
+                self.steps, self.wavelet, self.quant_alg, self.bin_count,
                 self.threshold_fraction, self.threshold_value, self.max_value, self.min_coef,
                 self.max_coef, self.zero_bin, self.dup_key, self.dup_value, self.longest_code,
                 w.size, _addr(w), d.size, _addr(d), b.size, v.size, _addr(b),
-                _addr(v), 0, 1 if self.transform_2d else 0)
+                _addr(v), 0, 1 if self.transform_2d else 0), keep
 
     def to_struct(self):
         """A WlResult pointing into this object's arrays (keep self alive)."""
-        return WlResult.from_buffer(np.array([self._record()], _result_dtype_cached()))
+        rec, self._keep = self._record()
+        return _result_array([rec])[0]
 
     @property
     def compressed_bytes(self) -> int:
@@ -429,7 +429,7 @@ def _packer(t) -> struct.Struct:
     return struct.Struct(fmt + f"{ctypes.sizeof(t) - end}x")
 
 
-_PACK_CUBELET = _packer(WlCubelet).pack
+_PACK_CUBELET, _PACK_RESULT = _packer(WlCubelet).pack, _packer(WlResult).pack
 
 
 def _cubelet_array(rows):
@@ -450,6 +450,27 @@ def _cubelet_array(rows):
         c.params = WlParams.from_buffer_copy(prm)
         c.row_pitch, c.slice_pitch = row_pitch, slice_pitch
     return cubs
+
+
+def _result_array(recs):
+    """The WlResult array of Compressed._record values (see _cubelet_array)."""
+    n = len(recs)
+    try:
+        return (WlResult * n).from_buffer(bytearray().join(
+            [_PACK_RESULT(x, y, z, ox, oy, oz, t, sx, sy, sz, *rest)
+             for (x, y, z), (ox, oy, oz), t, (sx, sy, sz), *rest in recs]))
+    except (struct.error, OverflowError, TypeError, ValueError):
+        pass
+    rs = (WlResult * n)()
+    for r, rec in zip(rs, recs):
+        for (name, ct), value in zip(WlResult._fields_, rec):
+            if issubclass(ct, ctypes.Array):
+                getattr(r, name)[:] = value
+            elif issubclass(ct, ctypes._Pointer):
+                setattr(r, name, ctypes.cast(value, ct))
+            else:
+                setattr(r, name, value)
+    return rs
 
 
 def _result_dtype_cached():
@@ -671,12 +692,9 @@ class Context:
         """The wl_decompress_batch arguments for these results (reusable:
         run_decompress(prep) restores them again without rebuilding them)."""
         n = len(cs)
-        rs = ((WlResult * n).from_buffer(np.array([c._record() for c in cs],
-                                                  _result_dtype_cached()))
-              if n else (WlResult * 0)())
-        # the arrays that the records point into, also if a Compressed is
-        # described again meanwhile
-        keep = [(c, c._keep) for c in cs]
+        recs = [c._record() for c in cs]
+        rs = _result_array([rec for rec, _ in recs])
+        keep = [arrays for _, arrays in recs]  # that the records point into
         outs, ptrs = [], (ctypes.c_void_p * n)()
         dts = (ctypes.c_int * n)()
         for i, c in enumerate(cs):
