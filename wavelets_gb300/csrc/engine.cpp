@@ -121,24 +121,30 @@ struct ResultSlab {
   size_t cap = 0;
 };
 
+// size of a new slab for `bytes`: powers of two from 1 MiB, so that freed
+// slabs fit later requests
+constexpr size_t kMinSlab = (size_t)1 << 20;
+size_t slab_bytes(size_t bytes) {
+  size_t cap = kMinSlab;
+  while (cap < bytes) cap <<= 1;
+  return cap;
+}
+
 class SlabPool {
  public:
+  // (a larger free slab is left: a few words would pin it)
   ResultSlab *acquire(size_t bytes) {
+    const size_t cap = slab_bytes(bytes);
     {
       std::lock_guard<std::mutex> g(mu_);
-      int bi = -1;
-      for (int i = 0; i < (int)free_.size(); i++)
-        if (free_[i]->cap >= bytes && (bi < 0 || free_[i]->cap < free_[bi]->cap)) bi = i;
-      if (bi >= 0) {
-        ResultSlab *s = free_[bi];
-        free_.erase(free_.begin() + bi);
+      for (size_t i = 0; i < free_.size(); i++) {
+        if (free_[i]->cap != cap) continue;
+        ResultSlab *s = free_[i];
+        free_.erase(free_.begin() + i);
         return s;
       }
     }
     ResultSlab *s = new ResultSlab;
-    // power-of-two sizes from 1 MiB, so that freed slabs fit later requests
-    size_t cap = (size_t)1 << 20;
-    while (cap < bytes) cap <<= 1;
     if (cudaHostAlloc(reinterpret_cast<void **>(&s->base), cap, cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       delete s;
@@ -1277,11 +1283,14 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   b.head = P<long long>(ctx->head);
   b.hostSel = anyLog ? H<float2>(ctx->hSel) : nullptr;
   // Small results go to the host by a kernel at the end of the call, into a
-  // slab acquired beforehand: room for a quarter more than the last such
-  // call's and at most what the streams can take.  Larger ones are copied by
-  // the copy engine once the host knows their size.
-  size_t outCap = std::max<size_t>((size_t)1 << 20, ctx->outBytes + ctx->outBytes / 4);
-  outCap = std::min(outCap, (size_t)wordsTotal * 4 + (size_t)n * (4 * kMaxSymbols + 2 * kMaxBins) * 4);
+  // slab acquired beforehand: as large as the last such call's results would
+  // get, and no larger than what the streams can take.  Others are copied by
+  // the copy engine once the host knows their size: larger ones, and those
+  // that a smaller slab would hold, which would pin this one for as long as
+  // the caller keeps them.
+  const size_t outCap =
+      std::min(slab_bytes(ctx->outBytes),
+               (size_t)wordsTotal * 4 + (size_t)n * (4 * kMaxSymbols + 2 * kMaxBins) * 4);
   const bool deliver = nh == 1 && !coefOut && outCap <= kDeliverMax;
   b.outSlab = reinterpret_cast<const OutSlab *>(P<char>(ctx->passes));
   if (deliver) {
@@ -1485,7 +1494,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     slab.p = slab_pool().acquire(outCap);
     if (!slab.p) return fail(ctx, WL_ENOMEM, "cannot allocate %zu bytes of page-locked result storage",
                              outCap);
-    *H<OutSlab>(ctx->hPasses) = OutSlab{slab.p->base, (long long)slab.p->cap};
+    const long long cap = (long long)slab.p->cap;
+    *H<OutSlab>(ctx->hPasses) = OutSlab{slab.p->base, cap, cap > (long long)kMinSlab ? cap / 2 : -1};
   }
 
   // ---- transform ----
@@ -1564,7 +1574,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
   const long long wAt[2] = {0, hw0[0]};
   const size_t mAt[2] = {0, hm0[0]};
   if (!delivered) {
-    if (deliver) {  // did not fit: the kernel left the metadata unpacked
+    if (deliver) {  // not this slab: the kernel left the metadata unpacked
       launch_pack_meta(bh[0], s);
       ctx->launches++;
       CU(cudaGetLastError());

@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(kDeliverThreads) deliver_kernel(DevBatch b) {
   const OutSlab o = *b.outSlab;
   const long long words = b.head[kHeadWords], meta = b.head[kHeadMeta];
   const long long wordsBytes = (words * 4 + 15) & ~15LL;
-  const bool fits = wordsBytes + meta * 4 <= o.cap;
+  const bool fits = wordsBytes + meta * 4 <= o.cap && wordsBytes + meta * 4 > o.above;
   const int t0 = blockIdx.x * kDeliverThreads + threadIdx.x, step = kDeliverBlocks * kDeliverThreads;
   if (fits) {
     const uint4 *src = reinterpret_cast<const uint4 *>(b.words);

@@ -216,10 +216,10 @@ struct CubeletDev {
 
 // Page-locked result storage of a call: words from `base` on, then (at the
 // next multiple of 16 bytes) each cubelet's decode table and codebook; used
-// when they fit in `cap` bytes.
+// when they take more than `above` and at most `cap` bytes.
 struct OutSlab {
   char *base;
-  long long cap;
+  long long cap, above;
 };
 
 // Device workspace for one batch.
