@@ -413,6 +413,11 @@ wl_status wl_set_graph_mode(wl_ctx *ctx, int mode);
  * would have fewer than 2^18 lanes that way (at most 32 a chunk).  The packed
  * bits do not depend on it. */
 wl_status wl_set_encode_slices(wl_ctx *ctx, int slices);
+/* Elements per chunk that the quantizer and the bit packer work on (no
+ * reference counterpart): 512, 1024, 2048 or 4096; 0 (default): by the size of
+ * the call.  With both set, a chunk of `elements` is packed by `slices` lanes.
+ * The results do not depend on it. */
+wl_status wl_set_token_chunk(wl_ctx *ctx, int elements);
 wl_status wl_graph_stats(const wl_ctx *ctx, long long out[4]);
 const char *wl_graph_error(const wl_ctx *ctx);
 

@@ -351,7 +351,8 @@ struct wl_ctx {
   cudaStream_t side2[kSide] = {};  // the second half's side streams
   cudaEvent_t fork2 = nullptr, join2[kSide] = {};
   int splitMode = 1;  // 1: split large batches into two staggered halves
-  int encSlices = 0;  // bit-packer slices per 4096-element chunk; 0: chunks and slices from the batch size
+  int encSlices = 0;  // bit-packer slices per token chunk; 0: from the batch size
+  int lgChunk = 0;    // log2 of the elements per token chunk; 0: from the batch size
   float timings[6] = {0, 0, 0, 0, 0, 0};
   bool profiling = false;
   cudaEvent_t pev[10] = {};
@@ -1043,8 +1044,10 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     if (pl.p.quant_alg == WL_LLOYD) anyLloyd = true;
   }
 
-  // (a forced slice count is per 4096 elements)
-  const int lgChunk = ctx->encSlices ? kMaxLgChunk : token_chunk_lg(coefTotal);
+  // (a forced slice count is per 4096 elements where no chunk is forced)
+  const int lgChunk = ctx->lgChunk     ? ctx->lgChunk
+                      : ctx->encSlices ? kMaxLgChunk
+                                       : token_chunk_lg(coefTotal);
   for (Plan &pl : plans) {
     pl.chunkBase = chunkTotal;
     pl.nChunks = (int)((pl.n + (1LL << lgChunk) - 1) >> lgChunk);
@@ -1468,7 +1471,7 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
     key.push_back(n);
     key.push_back(onDevice | (ctx->profiling ? 2 : 0) | (nh == 2 ? 4 : 0) | (deliver ? 8 : 0));
     key.push_back((long long)tune_version());
-    key.push_back(ctx->encSlices);
+    key.push_back(ctx->encSlices | (lgChunk << 8));
     for (int i = 0; i < n; i++) {
       const Plan &pl = plans[i];
       const wl_params &q = pl.p;
@@ -2875,6 +2878,18 @@ wl_status wl_set_host_input_mode(wl_ctx *ctx, int mode) {
 wl_status wl_set_encode_slices(wl_ctx *ctx, int slices) {
   if (!ctx || slices < 0 || slices > 32 || (slices & (slices - 1))) return WL_EINVAL;
   ctx->encSlices = slices;
+  return WL_OK;
+}
+
+wl_status wl_set_token_chunk(wl_ctx *ctx, int elements) {
+  if (!ctx) return WL_EINVAL;
+  int lg = 0;
+  if (elements) {
+    lg = kMinLgChunk;
+    while (lg < kMaxLgChunk && 1 << lg < elements) lg++;
+    if (1 << lg != elements) return WL_EINVAL;
+  }
+  ctx->lgChunk = lg;
   return WL_OK;
 }
 

@@ -189,6 +189,7 @@ EXPORTS = {
     "wl_tune_reset": (None, []),
     "wl_set_graph_mode": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "wl_set_encode_slices": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
+    "wl_set_token_chunk": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "wl_graph_stats": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_longlong)]),
     "wl_graph_error": (ctypes.c_char_p, [ctypes.c_void_p]),
     "wl_error_metrics": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(WlResult),
@@ -860,6 +861,12 @@ class Context:
         """Bit-packer lanes per 4096-element chunk (1, 2, 4, 8, 16, 32);
         0 = chunks and lanes chosen from the batch size.  The output does not depend on it."""
         self._check(self.lib.wl_set_encode_slices(self.h, int(slices)))
+
+    def set_token_chunk(self, elements: int):
+        """Elements per chunk of the quantizer and the bit packer (512, 1024,
+        2048, 4096); 0 = by the size of the call.  The output does not depend
+        on it."""
+        self._check(self.lib.wl_set_token_chunk(self.h, int(elements)))
 
     def set_graph_mode(self, mode: int):
         """1: capture a batch geometry seen twice in a row as a CUDA graph
