@@ -16,15 +16,20 @@ LONGEST = 60
 
 
 @pytest.fixture(scope="module")
-def ok():
+def steps():
     from wavelets_gb300 import build
-    fn = ctypes.CDLL(build.build()).wl_internal_decode_table_ok
+    fn = ctypes.CDLL(build.build()).wl_internal_decode_table_steps
     fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int]
 
     def call(table, bins, key=-1):
         t = np.ascontiguousarray(table, np.int32)
-        return bool(fn(t.ctypes.data, t.size, bins, key))
+        return fn(t.ctypes.data, t.size, bins, key)
     return call
+
+
+@pytest.fixture(scope="module")
+def ok(steps):
+    return lambda *a: steps(*a) >= 0
 
 
 def comb(bits):
@@ -143,3 +148,32 @@ def test_accepted_tables_are_trees(ok):
             assert walk_ok(t, leaves - 1, leaves - 1), t
             passed += 1
     assert passed > 100
+
+
+def test_step_tables(steps):
+    """One per inner node at depth 12, 16, 20 .."""
+    rng = np.random.default_rng(2)
+
+    def shuffled(t):
+        """The same tree with its nodes numbered depth first."""
+        out = []
+
+        def place(i):
+            k = len(out)
+            out.append((0, t[2 * i + 1]))
+            if t[2 * i]:
+                out[k] = (place(t[2 * i]), place(t[2 * i + 1]))
+            return k
+        place(0)
+        return [x for p in out for x in p]
+    trees = [comb(k) for k in (1, 11, 12, 13, 16, 17, 40, LONGEST)]
+    trees += [random_tree(rng, k) for k in (2, 300, 5000)]
+    for t in trees:
+        want, todo = 0, [(0, 0)]
+        while todo:
+            i, d = todo.pop()
+            if t[2 * i]:
+                want += d >= 12 and (d - 12) % 4 == 0
+                todo += [(t[2 * i], d + 1), (t[2 * i + 1], d + 1)]
+        assert steps(t, 5000) == want
+        assert steps(shuffled(t), 5000) == want

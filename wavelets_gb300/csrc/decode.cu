@@ -49,8 +49,8 @@ constexpr int kSubBits = 256, kSubWords = kSubBits / 32;
 constexpr int kTileSubs = kThreads - 1;      // thread 0 warms up on the one before
 constexpr int kTileBits = kTileSubs * kSubBits;
 constexpr int kTileWords = kTileSubs * kSubWords;
-constexpr int kLutBits = 12, kLutSize = 1 << kLutBits;
-constexpr int kStepBits = 4, kStep = 1 << kStepBits;  // longer codes, per step
+constexpr int kLutBits = kDecodeLutBits, kLutSize = 1 << kLutBits;
+constexpr int kStepBits = kDecodeStepBits, kStep = 1 << kStepBits;  // longer codes, per step
 // step tables kept in shared memory: the first ones built belong to the
 // shortest of the long codes (a global read of a step costs the whole warp
 // several hundred cycles, and with 1024 bins most warps have one per token)
@@ -65,9 +65,9 @@ constexpr int kBuildNodes = 2 * kMaxSymbols;  // decode tables staged in shared 
 
 // Table entry.  Token: bits 0-5 bits consumed, 6-9 log2 of its elements,
 // 10-22 symbol.  kSlow: kRun: the zero-run key with a code of bits 0-5 bits
-// whose length bits come after it (kBad: malformed table), else bits 0-15
+// whose length bits come after it (kBad: malformed table), else bits 0-28
 // the step table to go on with.
-constexpr unsigned kSlow = 1u << 31, kRun = 1u << 30, kBad = 1u << 29;
+constexpr unsigned kSlow = 1u << 31, kRun = 1u << 30, kBad = 1u << 29, kSlots = kBad - 1;
 
 struct TileAt {
   int tile;    // tile of the cubelet
@@ -132,7 +132,7 @@ __device__ __noinline__ unsigned slow_token(const uint32_t *sw, const unsigned *
     }
     used += width;
     width = kStepBits;
-    const int slot = (int)(e & 0xffffu);
+    const int slot = (int)(e & kSlots);
     const unsigned at = slot * kStep + (bits_at(sw, p + used) & (kStep - 1));
     e = slot < nNear ? near[at] : steps[at];
   }
@@ -587,11 +587,6 @@ int decode_tiles(long long nWords) {
   return (int)((decode_subs(nWords) + kTileSubs - 1) / kTileSubs);
 }
 int decode_lut_size() { return kLutSize; }
-// step tables a decode table of nTable ints can need: one per inner node
-int decode_steps(int nTable) {
-  const int k = nTable / 4 + 1;
-  return k < 0xffff ? k : 0xffff;
-}
 size_t decode_step_bytes(long long steps) { return (size_t)steps * kStep * sizeof(unsigned); }
 
 int launch_decode(const DecodeCub *cubs, const DecodeBatch &b, const DecodeArrays &d,

@@ -16,17 +16,25 @@ namespace wl {
 // to each other (Huffman::computeDecodeTable, huffman.cc:177-228); that layout
 // is checked in one pass without a branch per node, anything else with a depth
 // per node.
-bool decode_table_ok(const int *t, int n, int binCount, int dupKey) {
-  if (n < 2 || n % 2) return false;
+//
+// Returns the step tables that the decoder builds for it, -1 when it is not
+// accepted.  A step table belongs to an inner node at the depth where the
+// lookup table or another step table ends.
+int decode_table_steps(const int *t, int n, int binCount, int dupKey) {
+  if (n < 2 || n % 2) return -1;
   const int nodes = n / 2;
   const unsigned bins = (unsigned)binCount;
   const int key = dupKey < 0 ? 0 : dupKey;
   const auto symbol = [&](int s) { return ((unsigned)s < bins) | (s == key); };
-  if (t[0] == 0) return nodes == 1 && symbol(t[1]);
-  int next = 1, levelEnd = 1, depth = 0;
+  const auto stepDepth = [](int d) {
+    return d >= kDecodeLutBits && (d - kDecodeLutBits) % kDecodeStepBits == 0;
+  };
+  if (t[0] == 0) return nodes == 1 && symbol(t[1]) ? 0 : -1;
+  int next = 1, levelEnd = 1, depth = 0, steps = 0;
   unsigned off = 0;  // anything but the reference's layout
   for (int i = 0; i < nodes; i++) {
-    if (i == levelEnd) {
+    if (i == levelEnd) {  // the next level: two nodes for every inner one of this
+      if (stepDepth(depth)) steps += (next - i) / 2;
       levelEnd = next;
       depth++;
     }
@@ -37,26 +45,28 @@ bool decode_table_ok(const int *t, int n, int binCount, int dupKey) {
            (inner & ((unsigned)(a ^ next) | (unsigned)(b ^ (next + 1))));
     next += (int)(inner & 2u);
   }
-  if (off == 0 && next == nodes) return depth <= kMaxDecodeCode;
+  if (off == 0 && next == nodes) return depth <= kMaxDecodeCode ? steps : -1;
+  steps = 0;
   std::vector<unsigned char> at(nodes, 0);  // depth, 0: no parent yet
   for (int i = 0; i < nodes; i++) {
     const int a = t[2 * i], b = t[2 * i + 1];
-    if (i > 0 && at[i] == 0) return false;
+    if (i > 0 && at[i] == 0) return -1;
     if (a == 0) {
-      if (!symbol(b)) return false;
+      if (!symbol(b)) return -1;
       continue;
     }
     if (a <= i || a >= nodes || b <= i || b >= nodes || a == b || at[a] || at[b] ||
         at[i] >= kMaxDecodeCode)
-      return false;
+      return -1;
+    steps += stepDepth(at[i]);
     at[a] = at[b] = (unsigned char)(at[i] + 1);
   }
-  return true;
+  return steps;
 }
 
 }  // namespace wl
 
 // for callers without a GPU
-extern "C" int wl_internal_decode_table_ok(const int *t, int n, int binCount, int dupKey) {
-  return wl::decode_table_ok(t, n, binCount, dupKey) ? 1 : 0;
+extern "C" int wl_internal_decode_table_steps(const int *t, int n, int binCount, int dupKey) {
+  return wl::decode_table_steps(t, n, binCount, dupKey);
 }

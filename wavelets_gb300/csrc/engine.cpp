@@ -1897,8 +1897,9 @@ wl_status check_sizes(wl_ctx *ctx, const int size[3], const int steps[3], const 
   return WL_OK;
 }
 
-// Checks of a compressed cubelet before decoding; n = its padded element count.
-wl_status check_result(wl_ctx *ctx, const wl_result *r, int outType, long long &n) {
+// Checks of a compressed cubelet before decoding; n = its padded element count,
+// steps = the decoder's step tables.
+wl_status check_result(wl_ctx *ctx, const wl_result *r, int outType, long long &n, int &steps) {
   if (!r) return fail(ctx, WL_EINVAL, "null argument");
   if (dtype_size(outType) == 0) return fail(ctx, WL_EINVAL, "bad output dtype %d", outType);
   TRY(check_sizes(ctx, r->size, r->steps, r->original_size, n, r->transform_2d != 0));
@@ -1910,7 +1911,8 @@ wl_status check_result(wl_ctx *ctx, const wl_result *r, int outType, long long &
     return fail(ctx, WL_EFORMAT, "missing Huffman stream");
   if (r->dup_key >= 0 && (r->dup_value < 0 || r->dup_value >= r->bin_count))
     return fail(ctx, WL_EFORMAT, "zero-run value out of range");
-  if (!decode_table_ok(r->decode, r->n_decode, r->bin_count, r->dup_key))
+  steps = decode_table_steps(r->decode, r->n_decode, r->bin_count, r->dup_key);
+  if (steps < 0)
     return fail(ctx, WL_EFORMAT, "corrupt Huffman decode table");
   if (r->quant_alg == WL_LLOYD && (!r->values || r->n_values != r->bin_count))
     return fail(ctx, WL_EFORMAT, "codebook values missing");
@@ -2197,7 +2199,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
   if (n <= 0) return fail(ctx, WL_EINVAL, "empty batch");
   if (!rs || !outs) return fail(ctx, WL_EINVAL, "null argument");
   std::vector<long long> N(n), coefOff(n), wordsOff(n), outOff(n);
-  std::vector<int> ot(n);
+  std::vector<int> ot(n), nSteps(n);
   long long coefTotal = 0, wordsTotal = 0, tableTotal = 0, outTotal = 0, binTotal = 0;
   long long subTotal = 0, tileTotal = 0, stepTotal = 0;
   int nStreams = 0;
@@ -2211,7 +2213,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
     const wl_result *r = rs + i;
     ot[i] = outTypes ? outTypes[i] : r->original_dtype;
     if (!outs[i]) return fail(ctx, WL_EINVAL, "cubelet %d: null output", i);
-    TRY(check_result(ctx, r, ot[i], N[i]));
+    TRY(check_result(ctx, r, ot[i], N[i], nSteps[i]));
     coefOff[i] = coefTotal;
     coefTotal += (N[i] + 63) & ~63LL;
     wordsOff[i] = follows(i) ? wordsOff[i - 1] + rs[i - 1].n_words : (wordsTotal + 3) & ~3LL;
@@ -2225,7 +2227,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
       nStreams++;
       subTotal += decode_subs(r->n_words);
       tileTotal += decode_tiles(r->n_words);
-      stepTotal += decode_steps(r->n_decode);
+      stepTotal += nSteps[i];
     }
   }
   if (tileTotal > 0x7fffffffLL) return fail(ctx, WL_EINVAL, "batch too large");
@@ -2310,7 +2312,7 @@ wl_status decompress_batch_impl(wl_ctx *ctx, const wl_result *rs, int n, const i
       c.nTiles = decode_tiles(r->n_words);
       c.lutOff = (long long)k * decode_lut_size();
       c.stepOff = stepOff;
-      c.nSteps = decode_steps(r->n_decode);
+      c.nSteps = nSteps[i];
       std::fill(hmap + tileOff, hmap + tileOff + c.nTiles, k);
       subOff += c.nSub;
       tileOff += c.nTiles;

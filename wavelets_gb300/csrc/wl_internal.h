@@ -441,7 +441,7 @@ struct DecodeCub {
   long long subBase, nSub;   // subsequences (decode_subs)
   int tileBase, nTiles;      // tiles (decode_tiles)
   long long lutOff;          // decode_lut_size() entries
-  long long stepOff;         // step tables (decode_steps)
+  long long stepOff;         // step tables (decode_table_steps)
   int nSteps;
 };
 // elements of a tile's output up to which the decoder fills it itself
@@ -469,12 +469,13 @@ struct DecodeBatch {
   int maxTable;
 };
 constexpr int kMaxDecodeCode = 60;  // longest code decoded (with its length bits 63)
-// a table that the decoder takes (decode_table.cpp)
-bool decode_table_ok(const int *t, int n, int binCount, int dupKey);
+constexpr int kDecodeLutBits = 12, kDecodeStepBits = 4;  // of a code, per table
+// step tables of a decode table, -1: not one that the decoder takes
+// (decode_table.cpp)
+int decode_table_steps(const int *t, int n, int binCount, int dupKey);
 long long decode_subs(long long nWords);
 int decode_tiles(long long nWords);
 int decode_lut_size();
-int decode_steps(int nTable);
 size_t decode_step_bytes(long long steps);
 // the whole decode (returns the kernels launched); if flags[kDecodeAgain] is
 // not zero afterwards: zero it and launch_decode_check until it stays zero,
