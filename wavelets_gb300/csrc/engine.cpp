@@ -303,7 +303,7 @@ namespace {
 // and kernel arguments are functions of the geometry (key) and of the
 // context's buffers (gen); what changes from call to call -- input
 // addresses, thresholds' host tables -- travels through the page-locked
-// upload block and tables that the graph's copy nodes read at launch time.
+// upload block and tables, which the first kernel of each graph reads.
 struct GraphEntry {
   std::vector<long long> key;
   unsigned long long gen = 0;
@@ -345,7 +345,8 @@ struct wl_ctx {
   cudaStream_t side[kSide] = {};
   cudaEvent_t fork = nullptr, join[kSide] = {};
   // second half of a large batch: its own stream, started when the first
-  // half's transform has finished (halfT), joined back at the end (halfJ)
+  // half's first kernel has copied the upload block or, after the host's log
+  // tables, those (halfT), joined back at the end (halfJ)
   cudaStream_t stream2 = nullptr;
   cudaEvent_t halfT = nullptr, halfJ = nullptr;
   cudaStream_t side2[kSide] = {};  // the second half's side streams
@@ -1165,8 +1166,8 @@ wl_status compress_impl(wl_ctx *ctx, const wl_cubelet *items, int n, int onDevic
 
   // ---- halves ----
   // A large batch runs as two halves (cubelets [0, cut) and [cut, n), cut at
-  // half of the padded elements) on two streams: the second half's transform
-  // starts when the first half's has finished, so each half's latency-bound
+  // half of the padded elements) on two streams, the second once the first
+  // half's init_kernel has the upload block on the device: each half's latency-bound
   // steps (radix-select resolves, Lloyd solve, zero-run join, Huffman tree
   // build) run beside the other half's bulk passes.  Each half is a view of
   // the same buffers (per-cubelet and per-chunk arrays offset to its first

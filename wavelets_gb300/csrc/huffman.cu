@@ -341,9 +341,8 @@ __global__ void __launch_bounds__(T) huffman_build_kernel(DevBatch b) {
 // (powers of two) and of what is below 16 (an eight and singles) are two
 // ready-made bit strings, joined with the value's code and appended at once.
 // Only runs of 1024 and more, and alphabets whose codes make such strings
-// longer than 64 bits, take the loops.  Values are read four at a time; a
-// chunk's values start at a multiple of 2 KB, so the aligned blocks around a
-// slice stay inside its chunk's place.
+// longer than 64 bits, take the loops.  Values are read one at a time, the
+// next one ahead (for_entries).
 //
 // The encode stage (bit counts, scans, packer) of the mixed batch takes 0.42
 // ms, of 729 cubelets of 128^3 0.51 ms; 0.49 and 0.79 ms when it read every

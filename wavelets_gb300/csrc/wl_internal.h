@@ -81,10 +81,6 @@ inline int enc_slices(long long chunks, int lgChunk) {
 constexpr int kTileBudget = 16384;      // floats of shared memory per DWT tile
 constexpr int kMaxAxis = 16384;         // longest padded axis (one row per tile)
 
-// One pass of the separable transform over one cubelet, as seen by the
-// row kernel.  Rows are flattened r = b + B*a; row (a,b) of the input starts
-// at in + a*inSA + b*inSB (contiguous along c); element (a,b,c) of the
-// output goes to out + a*outSA + b*outSB + c*outSC.
 // A value of a token chunk: its bin in bits 16 and up, the zero-bin elements
 // between it and the chunk's value before it (0 for the first) below.
 __host__ __device__ inline unsigned make_item(int bin, int gap) {
@@ -129,6 +125,10 @@ __host__ __device__ inline unsigned run_code_in(int s, int e, int w0, int w1) {
 
 struct CubeletState;
 
+// One pass of the separable transform over one cubelet, as seen by the
+// row kernel.  Rows are flattened r = b + B*a; row (a,b) of the input starts
+// at in + a*inSA + b*inSB (contiguous along c); element (a,b,c) of the
+// output goes to out + a*outSA + b*outSB + c*outSC.
 struct PassDesc {
   const void *in;
   void *out;
@@ -307,9 +307,6 @@ bool dwt_rowreg_fits(int L, int steps);
 int dwt_rowreg_rows_per_block(int L, bool sel = false);
 void launch_dwt_rowreg(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses, int blocks,
                        int L, bool sel, cudaStream_t s);
-// the same with the rows read from any element type (REPEAT clamp) and
-// stored through a shared-memory tile to an output where consecutive rows
-// are neighbours (forward x and y passes)
 // the inverse of the in-place pass (the first inverse pass, z)
 void launch_dwt_rowreg_inv(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
                            int blocks, int L, cudaStream_t s);
@@ -320,6 +317,9 @@ int dwt_rowreg_t_rows_per_block(int L);
 // contiguous in the output, cropped) or back through the tile (the y pass)
 void launch_dwt_rowreg_inv_t(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
                              int blocks, int L, int outType, cudaStream_t s);
+// the same with the rows read from any element type (REPEAT clamp) and
+// stored through a shared-memory tile to an output where consecutive rows
+// are neighbours (forward x and y passes)
 void launch_dwt_rowreg_t(const PassDesc *d_passes, const int *d_tilePrefix, int nPasses,
                          int blocks, int L, int inType, cudaStream_t s);
 
@@ -375,10 +375,6 @@ void set_tuned_cols_shape(int kind, int typeIdx, int cls, TileShape t,
                           const float us[kTileShapes]);
 unsigned tune_version();  // changes whenever the table does
 
-// launchers (select.cu)
-// everything a call's kernels expect set: histograms and states zeroed, the
-// select state (extremes from FLT_MAX / FLT_MIN), cubelet of every chunk;
-// runs before the transform, whose last pass may gather the first digit
 // A block of page-locked host memory that a kernel copies to the device on its
 // way.  A copy node in front of a graph's kernels is handed to the copy engine
 // apart from them; with a
@@ -396,6 +392,10 @@ struct Upload {
                : p;
   }
 };
+// launchers (select.cu)
+// everything a call's kernels expect set: histograms and states zeroed, the
+// select state (extremes from FLT_MAX / FLT_MIN), cubelet of every chunk;
+// runs before the transform, whose last pass may gather the first digit
 void launch_init(DevBatch &b, bool lloyd, const Upload &up, cudaStream_t s);
 // pass0: run the stand-alone first digit pass for the cubelets whose last
 // transform pass did not gather it (CubeletDev::selFused == 0)
