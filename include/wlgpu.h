@@ -147,9 +147,10 @@ wl_status wl_decompress_cubelet(wl_ctx *ctx, const wl_result *in, int out_dtype,
  * transform in concurrent launch groups).  out_dtypes: per cubelet (NULL =
  * each one's original type); outs[i]: original_size elements of that type,
  * all host or all device memory (outs_on_device).  Results are those of
- * wl_decompress_cubelet on each.  A malformed or short stream is refused with
- * WL_EFORMAT and leaves every output as it was (also in
- * wl_decompress_cubelet). */
+ * wl_decompress_cubelet on each.  A decode table that is no tree (children
+ * after their parent, every node but the root the child of exactly one, codes
+ * of at most 60 bits) and a short stream are refused with WL_EFORMAT and leave
+ * every output as it was (also in wl_decompress_cubelet). */
 wl_status wl_decompress_batch(wl_ctx *ctx, const wl_result *in, int n, const int *out_dtypes,
                               void *const *outs, int outs_on_device);
 
