@@ -1,5 +1,6 @@
 // What a Huffman decode table has to be before a stream is decoded with it.
-#include <vector>
+#include <cstdlib>
+#include <memory>
 
 #include "wl_internal.h"
 
@@ -47,7 +48,11 @@ int decode_table_steps(const int *t, int n, int binCount, int dupKey) {
   }
   if (off == 0 && next == nodes) return depth <= kMaxDecodeCode ? steps : -1;
   steps = 0;
-  std::vector<unsigned char> at(nodes, 0);  // depth, 0: no parent yet
+  // depth of every node, 0: no parent yet
+  const std::unique_ptr<unsigned char, void (*)(void *)> depths(
+      static_cast<unsigned char *>(calloc(nodes, 1)), free);
+  unsigned char *at = depths.get();
+  if (!at) return -1;
   for (int i = 0; i < nodes; i++) {
     const int a = t[2 * i], b = t[2 * i + 1];
     if (i > 0 && at[i] == 0) return -1;
